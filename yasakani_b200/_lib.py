@@ -5,6 +5,7 @@ There is no fallback: if the library is missing or an entry fails, callers get a
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 from . import build as _build
@@ -152,6 +153,24 @@ def load():
             fn.restype, fn.argtypes = res, args
         _LIB = L
     return _LIB
+
+
+class _Host:
+    """The extension module `_host` (csrc/host_py.cpp), loaded at the first use of one of its functions."""
+
+    def __getattr__(self, name):
+        import torch  # noqa: F401  (the extension links against torch's libraries)
+        load()
+        if not os.path.exists(_build.HOST):
+            _build.build()
+        spec = importlib.util.spec_from_file_location("yasakani_b200._host", _build.HOST)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        self.__dict__.update({k: v for k, v in vars(mod).items() if not k.startswith("__")})
+        return self.__dict__[name]
+
+
+host = _Host()
 
 
 def check(rc: int, what: str) -> None:

@@ -3,7 +3,8 @@
 Function names and argument meaning follow the reference's launchers (src/args.hpp:14-21,
 src/post_kernels.hpp:26,39-41); tensors are torch CUDA tensors used purely as device memory, and
 every call is enqueue-only on torch's current stream.  All arithmetic happens in libyskn_kv4.so;
-there is no torch or CPU fallback.
+there is no torch or CPU fallback.  The launchers of a decode or prefill step marshal their arguments in
+native code (`_lib.host`, csrc/host_py.cpp), the others through ctypes.
 """
 from __future__ import annotations
 
@@ -13,7 +14,7 @@ import math
 import torch
 
 from . import _lib
-from ._lib import F16, BF16, F32, KvLayerC, KvQuantArgsC, AttnGArgsC, AttnGCombineArgsC, KvAppendArgsC, PeerExchangeC, AttnExtC, MsRowsC, check
+from ._lib import F16, BF16, F32, KvLayerC, KvQuantArgsC, AttnGArgsC, AttnGCombineArgsC, PeerExchangeC, AttnExtC, check, host
 
 _NAMES = ("kq", "kscale", "kzero", "kshadow", "vq", "vscale", "vzero")
 
@@ -107,10 +108,7 @@ def launch_rope_table_g(out: torch.Tensor, max_ctx: int, theta: float, rd: int, 
 
 def launch_kv_append(kv: KvLayer, k_in: torch.Tensor, v_in: torch.Tensor, d_pos: torch.Tensor, M: int, stream=None) -> None:
     """K/V branches of launch_qkv_post (src/post_kernels.cu:48-82) + launch_kv_group_quant_g."""
-    assert k_in.shape == v_in.shape and k_in.dtype == v_in.dtype and k_in.numel() == M * kv.hkv * kv.hd
-    a = KvAppendArgsC(k_in.data_ptr(), v_in.data_ptr(), _dtype_code(k_in), kv.struct(), d_pos.data_ptr(), M, kv.max_ctx, kv.hkv, kv.hd)
-    assert k_in.is_cuda and k_in.is_contiguous() and v_in.is_contiguous() and d_pos.dtype == torch.int32
-    check(_lib.load().yskn_kv4_append(C.byref(a), _stream(stream)), "yskn_kv4_append")
+    host.kv_append(kv, k_in, v_in, d_pos, M, stream)
 
 
 def launch_kv_group_quant_g(kv: KvLayer, d_pos: torch.Tensor, M: int, stream=None) -> None:
@@ -142,11 +140,7 @@ def attn_ext(early: bool = False, splits_short: int = 0, long_len: int = 0, wk=N
 def launch_attention_gqa(q16, kv: KvLayer, M: int, d_pos, splits: int, pm, pl, pacc, rope, nh: int, qscale: float,
                          rd: int, stream=None, ext: AttnExtC | None = None) -> None:
     """launch_attention_gqa (src/attention_gqa.cu:168-175): split-K partials for M rows."""
-    a = _attn_args(q16, kv, M, d_pos, splits, pm, pl, pacc, rope, nh, qscale)
-    if ext is not None:
-        check(_lib.load().yskn_kv4_attention_ex(C.byref(a), C.byref(ext), nh // kv.hkv, kv.hd, rd, _dtype_code(q16), _stream(stream)), "yskn_kv4_attention_ex")
-        return
-    check(_lib.load().yskn_kv4_attention(C.byref(a), nh // kv.hkv, kv.hd, rd, _dtype_code(q16), _stream(stream)), "yskn_kv4_attention")
+    host.attention(q16, kv, M, d_pos, splits, pm, pl, pacc, rope, nh, qscale, rd, stream, ext)
 
 
 class MsSlots:
@@ -169,12 +163,7 @@ class MsSlots:
 def launch_attention_ms(q16, slots: MsSlots, M: int, pos, slot, splits: int, pm, pl, pacc, rope, nh: int, qscale: float, rd: int,
                         stream=None) -> None:
     """Partials for M rows of several sequences in one launch (yskn_kv4_attention_ms): pos, slot int32 device tensors [M]."""
-    assert pos.dtype == torch.int32 and slot.dtype == torch.int32 and pos.numel() >= M and slot.numel() >= M
-    a = AttnGArgsC(q16.data_ptr(), KvLayerC(), slots.max_ctx, M, None, splits, pm.data_ptr(), pl.data_ptr(), pacc.data_ptr(),
-                   rope.data_ptr() if rope is not None else None, slots.hkv, nh, qscale)
-    ms = MsRowsC(pos.data_ptr(), slot.data_ptr(), slots.d_layers.data_ptr(), slots.maps_ptr, slots.n)
-    check(_lib.load().yskn_kv4_attention_ms(C.byref(a), C.byref(ms), nh // slots.hkv, slots.hd, rd, _dtype_code(q16), _stream(stream)),
-          "yskn_kv4_attention_ms")
+    host.attention_ms(q16, slots, M, pos, slot, splits, pm, pl, pacc, rope, nh, qscale, rd, stream)
 
 
 def launch_attention_shard(q16, kv: KvLayer, M: int, d_pos, splits: int, pm, pl, pacc, rope, nh: int, qscale: float,
@@ -189,12 +178,7 @@ def launch_decode(q16, kv: KvLayer, M: int, d_pos, splits: int, pm, pl, pacc, ro
                   bv=None, gate=None, stream=None, ext: AttnExtC | None = None) -> None:
     """launch_attention_gqa + the merge of launch_attn_combine_gqa_xform as one launch where the shape allows
     (src/attention_gqa.cu:168-181).  Calls on one device must not overlap."""
-    a = _attn_args(q16, kv, M, d_pos, splits, pm, pl, pacc, rope, nh, qscale)
-    g = nh // kv.hkv
-    c = AttnGCombineArgsC(pm.data_ptr(), pl.data_ptr(), pacc.data_ptr(), splits, M, bv.data_ptr() if bv is not None else None,
-                          o16.data_ptr(), gate.data_ptr() if gate is not None else None, nh, g)
-    check(_lib.load().yskn_kv4_decode_ex(C.byref(a), C.byref(c), C.byref(ext) if ext is not None else None, g, kv.hd, rd, _dtype_code(q16),
-                                        _stream(stream)), "yskn_kv4_decode")
+    host.decode(q16, kv, M, d_pos, splits, pm, pl, pacc, rope, nh, qscale, rd, o16, bv, gate, stream, ext)
 
 
 def launch_decode_shard_triple(q16, kv: KvLayer, M: int, d_pos, splits: int, pm, pl, pacc, rope, nh: int, qscale: float, rd: int,
@@ -207,10 +191,7 @@ def launch_decode_shard_triple(q16, kv: KvLayer, M: int, d_pos, splits: int, pm,
 
 def launch_attn_combine_gqa(pm, pl, pacc, splits: int, M: int, o16, nh: int, g: int, bv=None, gate=None, stream=None) -> None:
     """Merge half of launch_attn_combine_gqa_xform (src/attention_gqa.cu:123-134,176-181), up to the o16 store."""
-    hd = o16.numel() // (M * nh)
-    a = AttnGCombineArgsC(pm.data_ptr(), pl.data_ptr(), pacc.data_ptr(), splits, M, bv.data_ptr() if bv is not None else None,
-                          o16.data_ptr(), gate.data_ptr() if gate is not None else None, nh, g)
-    check(_lib.load().yskn_kv4_combine(C.byref(a), hd, _dtype_code(o16), _stream(stream)), "yskn_kv4_combine")
+    host.combine(pm, pl, pacc, splits, M, o16, nh, g, bv, gate, stream)
 
 
 def launch_xform_a8(o16, signs, qx, alpha, stream=None) -> None:
@@ -249,19 +230,14 @@ def launch_attention_tc(q16, kv: KvLayer, M: int, d_pos, splits: int, pm, pl, pa
                         workspace: torch.Tensor | None, valid_tokens: int = 0, stream=None) -> None:
     """launch_kv_dequant + launch_attention_f32 (src/attention_kv4q.cu:198-285) on tcgen05: partials for M rows.
     workspace None: the kernel converts the packed cache itself (no dequantised copy, one launch)."""
-    a = _attn_args(q16, kv, M, d_pos, splits, pm, pl, pacc, rope, nh, qscale)
-    check(_lib.load().yskn_kv4_attention_tc(C.byref(a), nh // kv.hkv, kv.hd, rd, _dtype_code(q16), _ptr(workspace) if workspace is not None else None,
-                                           workspace.numel() if workspace is not None else 0, valid_tokens, _stream(stream)), "yskn_kv4_attention_tc")
+    host.attention_tc(q16, kv, M, d_pos, splits, pm, pl, pacc, rope, nh, qscale, rd, workspace, valid_tokens, stream)
 
 
 def launch_attention_prefill_tc(q16, kv: KvLayer, M: int, d_pos, splits: int, pm, pl, pacc, rope, nh: int, qscale: float, rd: int,
                                 o16, workspace: torch.Tensor | None, bv=None, valid_tokens: int = 0, stream=None) -> None:
     """launch_attention_prefill_f32 (src/attention_kv4q.cu:287-323) on tcgen05: M appended rows, merged to o16.
     workspace None: the kernel converts the packed cache itself."""
-    a = _attn_args(q16, kv, M, d_pos, splits, pm, pl, pacc, rope, nh, qscale)
-    check(_lib.load().yskn_kv4_prefill_tc(C.byref(a), nh // kv.hkv, kv.hd, rd, _dtype_code(q16), bv.data_ptr() if bv is not None else None,
-                                         _ptr(o16), _ptr(workspace) if workspace is not None else None,
-                                         workspace.numel() if workspace is not None else 0, valid_tokens, _stream(stream)), "yskn_kv4_prefill_tc")
+    host.prefill_tc(q16, kv, M, d_pos, splits, pm, pl, pacc, rope, nh, qscale, rd, o16, workspace, bv, valid_tokens, stream)
 
 
 def launch_local_triple(pm, pl, pacc, splits: int, M: int, nh: int, hd: int, triple, stream=None) -> None:

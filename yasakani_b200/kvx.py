@@ -9,7 +9,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import check, Kv8AttnArgsC
+from ._lib import check, host
 from .kv4 import _ptr, _stream, _dtype_code
 
 
@@ -50,17 +50,7 @@ def launch_attn_post(q_rows, k_rows, v_rows, qn_w, kn_w, eps: float, d_pos, rope
     """launch_q35_attn_post (src/q35_kernels.cu:1013-1069) from the bf16 projection rows on: RMS norm, partial RoPE and
     rotation of the query and key heads, INT8 rows of keys and values appended at *d_pos + token, gate copied.
     q_rows bf16 [M, nh, 512]; k_rows / v_rows bf16 [M, kvh, 256]; k8 / v8 int8 [kvh, max_ctx, 256]; ks / vs fp32 [kvh, max_ctx]."""
-    M, nh = q_rows.shape[0], q_rows.shape[1]
-    kvh, max_ctx = k8.shape[0], k8.shape[1]
-    for t in (q_rows, k_rows, v_rows, qn_w, kn_w, q16, gate16):
-        if t.dtype != torch.bfloat16:
-            raise TypeError("yskn_kvx_attn_post takes bf16 rows and norm weights")
-    if tuple(q_rows.shape) != (M, nh, 512) or tuple(k_rows.shape) != (M, kvh, 256) or tuple(v_rows.shape) != (M, kvh, 256):
-        raise ValueError("q_rows [M, nh, 512], k_rows / v_rows [M, kvh, 256]")
-    a = _lib.KvxAttnPostArgsC(_ptr(q_rows), _ptr(k_rows), _ptr(v_rows), _ptr(qn_w), _ptr(kn_w), eps, M, _ptr(d_pos),
-                              _ptr(rope) if rope is not None else None, rd, _ptr(q16), _ptr(gate16), _ptr(k8), _ptr(v8), _ptr(ks), _ptr(vs),
-                              max_ctx, nh, kvh, 1 if pm else 0)
-    check(_lib.load().yskn_kvx_attn_post(C.byref(a), _stream(stream)), "yskn_kvx_attn_post")
+    host.attn_post(q_rows, k_rows, v_rows, qn_w, kn_w, eps, d_pos, rope, rd, q16, gate16, k8, ks, v8, vs, pm, stream)
 
 
 def probe(x: np.ndarray):
@@ -76,37 +66,24 @@ def probe(x: np.ndarray):
     return q, sc, y
 
 
-def _dp(t):
-    return None if t is None else t.data_ptr()
-
-
 def launch_kv8_attention(q16: torch.Tensor, k8: torch.Tensor, v8: torch.Tensor, ks: torch.Tensor, vs: torch.Tensor, M: int,
                          d_pos: torch.Tensor, splits: int, pm: torch.Tensor, pl: torch.Tensor, pacc: torch.Tensor, nh: int,
                          qscale: float = 0.0625, stream=None) -> None:
     """launch_q35_attention, INT8 branch (src/q35_kernels.cu:1176-1281): k8/v8 [kvh, max_ctx, 256] int8, ks/vs [kvh, max_ctx]."""
-    kvh, max_ctx = k8.shape[0], k8.shape[1]
-    for t in (q16, k8, v8, ks, vs, d_pos, pm, pl, pacc):
-        assert t.is_cuda and t.is_contiguous()
-    a = Kv8AttnArgsC(_dp(q16), _dp(k8), _dp(v8), _dp(ks), _dp(vs), max_ctx, M, _dp(d_pos), splits, _dp(pm), _dp(pl), _dp(pacc), kvh, nh, qscale)
-    check(_lib.load().yskn_kv8_attention(C.byref(a), _dtype_code(q16), _stream(stream)), "yskn_kv8_attention")
+    host.kv8_attention(q16, k8, v8, ks, vs, M, d_pos, splits, pm, pl, pacc, nh, qscale, stream)
 
 
 def launch_kv8_attention_tc(q16: torch.Tensor, k8: torch.Tensor, v8: torch.Tensor, ks: torch.Tensor, vs: torch.Tensor, M: int,
                             d_pos: torch.Tensor, splits: int, pm: torch.Tensor, pl: torch.Tensor, pacc: torch.Tensor, nh: int,
                             qscale: float = 0.0625, stream=None) -> None:
     """Many rows over INT8 rows on the tcgen05 kernel (launch_q35_atx, src/q35_atx.cu:92-793): same arguments and partials."""
-    kvh, max_ctx = k8.shape[0], k8.shape[1]
-    for t in (q16, k8, v8, ks, vs, d_pos, pm, pl, pacc):
-        assert t.is_cuda and t.is_contiguous()
-    a = Kv8AttnArgsC(_dp(q16), _dp(k8), _dp(v8), _dp(ks), _dp(vs), max_ctx, M, _dp(d_pos), splits, _dp(pm), _dp(pl), _dp(pacc), kvh, nh, qscale)
-    check(_lib.load().yskn_kv8_attention_tc(C.byref(a), _dtype_code(q16), _stream(stream)), "yskn_kv8_attention_tc")
+    host.kv8_attention_tc(q16, k8, v8, ks, vs, M, d_pos, splits, pm, pl, pacc, nh, qscale, stream)
 
 
 def launch_kv8_combine(pm, pl, pacc, splits: int, M: int, nh: int, o16: torch.Tensor, gate: torch.Tensor | None = None,
                        inverse_rotate: bool = True, stream=None) -> None:
     """Split merge, inverse rotation, rounding, optional sigmoid gate (src/q35_kernels.cu:1400-1424)."""
-    check(_lib.load().yskn_kv8_combine(_ptr(pm), _ptr(pl), _ptr(pacc), splits, M, nh, _ptr(gate), _ptr(o16), _dtype_code(o16),
-                                       1 if inverse_rotate else 0, _stream(stream)), "yskn_kv8_combine")
+    host.kv8_combine(pm, pl, pacc, splits, M, nh, o16, gate, inverse_rotate, stream)
 
 
 # ---------------------------------------------------------------- step 2: trellis rows (src/kvq_gpu.cuh, src/kvq_fast.cuh)
@@ -151,8 +128,4 @@ def launch_tb_attention(profile: TrellisProfile, q16, k_pay, k_side, v_pay, v_si
     """Decode attention straight over packed trellis rows (the reference's launch_q35_atxpk for a few rows): k_pay / v_pay uint8
     [kvh, max_ctx, stride], k_side / v_side int32-bits [kvh, max_ctx, 2], grp_k / grp_v int32 [kvh]; rows the profile leaves
     unpacked come from k_plain / v_plain fp32 [kvh, max_ctx, 256].  Partials as launch_kv8_attention."""
-    kvh, max_ctx, stride = k_pay.shape
-    a = _lib.TbAttnArgsC(_ptr(q16), _ptr(profile.dev), _ptr(k_pay), _ptr(v_pay), stride, _ptr(k_side), _ptr(v_side), _ptr(grp_k), _ptr(grp_v),
-                         _ptr(k_plain) if k_plain is not None else None, _ptr(v_plain) if v_plain is not None else None,
-                         max_ctx, M, _ptr(d_pos), splits, _ptr(pm), _ptr(pl), _ptr(pacc), kvh, nh, qscale)
-    check(_lib.load().yskn_tb_attention(C.byref(a), _dtype_code(q16), _stream(stream)), "yskn_tb_attention")
+    host.tb_attention(profile, q16, k_pay, k_side, v_pay, v_side, grp_k, grp_v, M, d_pos, splits, pm, pl, pacc, nh, k_plain, v_plain, qscale, stream)
