@@ -25,6 +25,18 @@ inline int launch_status(const char* what) {
   return 0;
 }
 
+// Launch with programmatic stream serialization allowed (for kernels that wait in griddepcontrol.wait before they read what a predecessor wrote).
+template <class K, class... Args>
+inline int launch_pdl(const char* who, K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  KV4_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  return launch_status(who);
+}
+
 // Function attributes are per device: true the first time a launcher runs on the current device (flags = one word per
 // launcher, bit d = done on device d).  The reference sets them once per process (src/q35_fa.cu:305-307) because an engine
 // owns one GPU; a process that drives several GPUs through this library gets them on each.

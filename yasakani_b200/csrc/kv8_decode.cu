@@ -17,7 +17,7 @@
 // permutation of the channels (slot (w, s, 2j+x) <-> channel 16(4w+j)+4s+x), applied to Q once at set-up; for P.V a lane
 // owns channels [32g, 32g+32) of token rows 2j, 2j+1, 2j+8, 2j+9 and PRMT pairs the two tokens of a k-slot.
 // HBM-bound: 2,080 bytes per token (4 kv-heads x 2 x 260).
-#include "kv4_common.cuh"
+#include "kvx_rotate.cuh"
 
 namespace kv4 {
 namespace {
@@ -42,47 +42,20 @@ __device__ __forceinline__ uint4 ldg16(const void* p) { return __ldcs(reinterpre
 template <int DT>
 __global__ void __launch_bounds__(KV8_WARPS * 32, 1) kv8_decode_kernel(const Kv8P P) {
   extern __shared__ __align__(16) uint8_t smem[];
-  // [16 k-steps][32 lanes] uint2 Q fragments | bias[8] | merge area [warps][8 heads][258]
+  // [16 k-steps][32 lanes] uint2 Q fragments | q sums [4][8] | merge area [warps][8 heads][258]
   uint2* s_q = reinterpret_cast<uint2*>(smem);
   float* s_bias = reinterpret_cast<float*>(smem + 16 * 32 * 8);
-  float* s_merge = s_bias + 8;
+  float* s_merge = s_bias + 32;
   const yskn_kv8_attn_args& A = P.a;
   const int split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z, G = P.g;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+  // Programmatic dependent launch: this grid may be scheduled while the row epilogue in front of it drains, and waits here before it
+  // reads the position, the queries and the new rows; the merge behind it may be scheduled early in turn.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int len = *A.d_pos + r + 1;                        // keys 0 .. pos
   const int tiles = (len + 15) / 16, per = (tiles + (int)gridDim.x - 1) / (int)gridDim.x;
   const int ti0 = min(tiles, split * per), ti1 = min(tiles, ti0 + per);
-
-  // ---- set-up: Q as B fragments in the slot order of the K loads, scaled by qscale * log2(e); the per-head bias
-  const float qs = A.qscale * KV8_LOG2E;
-  for (int e = threadIdx.x; e < 16 * 32 * 2; e += KV8_WARPS * 32) {
-    const int x = e & 1, ln = (e >> 1) & 31, kstep = e >> 6, w = kstep >> 2, s = kstep & 3, hh = ln >> 2, jj = ln & 3;
-    const int c = 16 * (4 * w + jj) + 4 * s + 2 * x;
-    float lo = 0.f, hi = 0.f;
-    if (hh < G) {
-      const size_t qb = ((size_t)r * A.nh + kvh * G + hh) * KV8_HD;
-      lo = act_load<DT>(A.q16, qb + c) * qs; hi = act_load<DT>(A.q16, qb + c + 1) * qs;
-    }
-    reinterpret_cast<uint32_t*>(s_q)[e] = pack_h2(lo, hi);
-  }
-  __syncthreads();
-  if (threadIdx.x < 8) {                                   // bias[h] = 1152 * sum over the fp16 values the MMAs multiply by
-    float sum = 0.f;
-    for (int kstep = 0; kstep < 16; ++kstep)
-      for (int jj = 0; jj < 4; ++jj) {
-        const uint2 u = s_q[kstep * 32 + threadIdx.x * 4 + jj];
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-        sum += (a.x + a.y) + (b.x + b.y);
-      }
-    s_bias[threadIdx.x] = KV8_OFF * sum;
-  }
-  __syncthreads();
-  const float bias0 = s_bias[2 * j], bias1 = s_bias[2 * j + 1];
-
-  float acc[16][4];                                        // O^T: [m-tile][(channel 32g+2mt | +1) x (head 2j | 2j+1)]
-  #pragma unroll
-  for (int mt = 0; mt < 16; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
-  float m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f}, zs[2] = {0.f, 0.f};   // heads 2j, 2j+1 (log2 domain); zs = sum of rounded p'
 
   const size_t plane = (size_t)kvh * A.max_ctx;
   const int8_t* kbase = A.k8 + plane * KV8_HD + 16 * j;    // + token*256 + 64*w : this lane's 16 channels of block w
@@ -96,7 +69,38 @@ __global__ void __launch_bounds__(KV8_WARPS * 32, 1) kv8_decode_kernel(const Kv8
     for (int w = 0; w < 4; ++w) { kx[w] = ldg16(kbase + t * KV8_HD + 64 * w); ky[w] = ldg16(kbase + (t + 8) * KV8_HD + 64 * w); }
   };
   int ti = ti0 + warp;
-  if (ti < ti1) load_k(ti);
+  if (ti < ti1) load_k(ti);                                // the first keys are on their way while Q is prepared
+
+  // ---- set-up: Q as B fragments in the slot order of the K loads, scaled by qscale * log2(e); the per-head bias 1152 * sum of the
+  //      fp16 values the MMAs multiply by.  A thread keeps one head over its four entries (head = bits 3-5 of e), so the sum is
+  //      three shuffles and four partials per head (one thread per head walking the fragments took about 1 us).
+  const float qs = A.qscale * KV8_LOG2E;
+  float qsum = 0.f;
+  for (int e = threadIdx.x; e < 16 * 32 * 2; e += KV8_WARPS * 32) {
+    const int x = e & 1, ln = (e >> 1) & 31, kstep = e >> 6, w = kstep >> 2, s = kstep & 3, hh = ln >> 2, jj = ln & 3;
+    const int c = 16 * (4 * w + jj) + 4 * s + 2 * x;
+    float lo = 0.f, hi = 0.f;
+    if (hh < G) {
+      const size_t qb = ((size_t)r * A.nh + kvh * G + hh) * KV8_HD + c;
+      lo = act_load<DT>(A.q16, qb) * qs; hi = act_load<DT>(A.q16, qb + 1) * qs;
+    }
+    const uint32_t p = pack_h2(lo, hi);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&p));
+    qsum += f.x + f.y;
+    reinterpret_cast<uint32_t*>(s_q)[e] = p;
+  }
+  #pragma unroll
+  for (int o = 1; o <= 4; o <<= 1) qsum += __shfl_xor_sync(0xffffffffu, qsum, o);
+  if ((lane & 7) == 0) s_bias[(warp >> 1) * 8 + (threadIdx.x >> 3 & 7)] = qsum;
+  __syncthreads();
+  auto bias_of = [&](int h) { return KV8_OFF * ((s_bias[h] + s_bias[8 + h]) + (s_bias[16 + h] + s_bias[24 + h])); };
+  const float bias0 = bias_of(2 * j), bias1 = bias_of(2 * j + 1);
+
+  float acc[16][4];                                        // O^T: [m-tile][(channel 32g+2mt | +1) x (head 2j | 2j+1)]
+  #pragma unroll
+  for (int mt = 0; mt < 16; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
+  float m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f}, zs[2] = {0.f, 0.f};   // heads 2j, 2j+1 (log2 domain); zs = sum of rounded p'
+
   for (; ti < ti1; ti += KV8_WARPS) {
     const int tg = 16 * ti + g;
     const bool v0 = tg < len, v1 = tg + 8 < len;
@@ -197,46 +201,136 @@ __global__ void __launch_bounds__(KV8_WARPS * 32, 1) kv8_decode_kernel(const Kv8
   }
 }
 
-// ---- merge of the splits + inverse rotation + rounding (+ gate): one block per (head, row), one thread per channel
+// ---- merge of the splits + inverse rotation + rounding (+ gate), in two shapes.
+// What bounds both is latency, not bytes (a decode step merges 0.9 MB).  The former kernel (one block of 256 threads per row, splits
+// walked one after the other, sixteen block barriers for the rotation) took 20 us for 24 rows of 37 splits and 64 us for
+// 24,000 rows of one split.
+__device__ __forceinline__ float kv8_round(int dt, float v) { return dt == YSKN_KV4_BF16 ? bf2f(f2bf(v)) : h2f(f2h(v)); }
+template <int DT> __device__ __forceinline__ float kv8_gated(float y, float gt) {   // y * sigmoid(gate), each factor and the product rounded (src/q35_kernels.cu:1423-1424)
+  return kv8_round(DT, __fmul_rn(y, kv8_round(DT, __fdiv_rn(1.f, __fadd_rn(1.f, expf(-gt))))));
+}
+
+// Many splits: one block per (head, row), four runs of splits x 256 channels, every thread's loads issued at once; one warp
+// forms the weights meanwhile.  The butterflies (inverse kvx_rotate, src/kvx_codec.cuh:35-49, stages h = 1 ... 128 in order): 1 ... 16 by
+// shuffles, 32 ... 128 from one exchange through shared memory, each thread folding the eight values its output depends on.
+constexpr int KV8_CQ = 4, KV8_CB = 10;
 template <int DT>
-__global__ void __launch_bounds__(256) kv8_combine_kernel(const float* pm, const float* pl, const float* pacc, int S, int M, int nh,
-                                                         const void* gate, void* o16, int inverse_rotate) {
-  __shared__ float s_w[64], s_buf[256];
+__global__ void __launch_bounds__(KV8_CQ * 256) kv8_combine_kernel(const float* pm, const float* pl, const float* pacc, int S, int nh,
+                                                                  const void* gate, uint16_t* o16, int inverse_rotate) {
+  __shared__ float s_w[64], s_part[KV8_CQ][256], s_buf[256];
   __shared__ float s_L;
-  const int head = blockIdx.x, r = blockIdx.y, d = threadIdx.x;
+  const int head = blockIdx.x, r = blockIdx.y, tid = threadIdx.x, q = tid >> 8, d = tid & 255;
   auto slot = [&](int s) -> size_t { return ((size_t)r * S + s) * nh + head; };
-  float M2 = -1e30f;
-  for (int s = 0; s < S; ++s) M2 = fmaxf(M2, __ldcg(pm + slot(s)));
-  if (d < S) { const float pmv = __ldcg(pm + slot(d)); s_w[d] = pmv > -1e29f ? expf(pmv - M2) : 0.f; }
-  __syncthreads();
-  if (d == 0) { float L2 = 0.f; for (int s = 0; s < S; ++s) L2 += s_w[s] * __ldcg(pl + slot(s)); s_L = L2; }
-  float o = 0.f;
-  for (int s = 0; s < S; ++s) o += s_w[s] * __ldcg(pacc + slot(s) * KV8_HD + d);
-  __syncthreads();
-  float y = __fdiv_rn(o, s_L);
-  if (inverse_rotate) {                                    // inverse kvx_rotate (src/kvx_codec.cuh:35-49): butterflies, x 1/16, then the sign
-    s_buf[d] = y;
-    __syncthreads();
-    for (int h = 1; h < 256; h *= 2) {
-      const float a = s_buf[d], b = s_buf[d ^ h];
-      __syncthreads();
-      s_buf[d] = (d & h) ? __fsub_rn(b, a) : __fadd_rn(a, b);
-      __syncthreads();
-    }
-    uint32_t x = (uint32_t)d + 1u;
-    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
-    y = __fmul_rn(s_buf[d], 0.0625f);
-    if (x & 1u) y = -y;
-  }
+  const int per = (S + KV8_CQ - 1) / KV8_CQ, s0 = min(S, q * per), s1 = min(S, s0 + per);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");       // the attention grid's partials are visible from here on
   const size_t e = ((size_t)r * nh + head) * KV8_HD + d;
-  auto rnd = [](float v) -> float { return DT == YSKN_KV4_BF16 ? bf2f(f2bf(v)) : h2f(f2h(v)); };
-  y = rnd(y);
-  if (gate) {                                              // y * sigmoid(gate), each factor and the product rounded (src/q35_kernels.cu:1423-1424)
-    const float gt = act_load<DT>(gate, e);
-    const float sg = rnd(__fdiv_rn(1.f, __fadd_rn(1.f, expf(-gt))));
-    y = rnd(__fmul_rn(y, sg));
+  const float gt = gate && q == 0 ? act_load<DT>(gate, e) : 0.f;
+  float v[KV8_CB];
+  #pragma unroll
+  for (int k = 0; k < KV8_CB; ++k) v[k] = s0 + k < s1 ? __ldcg(pacc + slot(s0 + k) * KV8_HD + d) : 0.f;
+  if (tid < 32) {                                          // at most 64 splits: two per lane
+    const float m0 = tid < S ? __ldcg(pm + slot(tid)) : -1e30f, m1 = tid + 32 < S ? __ldcg(pm + slot(tid + 32)) : -1e30f;
+    const float l0 = tid < S ? __ldcg(pl + slot(tid)) : 0.f, l1 = tid + 32 < S ? __ldcg(pl + slot(tid + 32)) : 0.f;
+    float mx = fmaxf(m0, m1);
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float w0 = m0 > -1e29f ? expf(m0 - mx) : 0.f, w1 = m1 > -1e29f ? expf(m1 - mx) : 0.f;
+    s_w[tid] = w0; s_w[tid + 32] = w1;
+    float ls = w0 * l0 + w1 * l1;
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);
+    if (tid == 0) s_L = ls;
   }
-  static_cast<uint16_t*>(o16)[e] = act_store16<DT>(y);
+  __syncthreads();
+  float o = 0.f;
+  #pragma unroll
+  for (int k = 0; k < KV8_CB; ++k) if (s0 + k < s1) o += s_w[s0 + k] * v[k];
+  for (int s = s0 + KV8_CB; s < s1; ++s) o += s_w[s] * __ldcg(pacc + slot(s) * KV8_HD + d);     // more than 40 splits
+  s_part[q][d] = o;
+  __syncthreads();
+  if (q != 0) return;
+  float y = __fdiv_rn((s_part[0][d] + s_part[1][d]) + (s_part[2][d] + s_part[3][d]), s_L);
+  if (inverse_rotate) {
+    #pragma unroll
+    for (int h = 1; h < 32; h *= 2) {                      // lower index: a + b; upper: lower - upper
+      const float other = __shfl_xor_sync(0xffffffffu, y, h);
+      y = (d & h) ? __fsub_rn(other, y) : __fadd_rn(y, other);
+    }
+    s_buf[d] = y;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    float t[8];
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) t[k] = s_buf[32 * k + (d & 31)];
+    const uint32_t f0 = (d & 32) ? 0x80000000u : 0u, f1 = (d & 64) ? 0x80000000u : 0u, f2 = (d & 128) ? 0x80000000u : 0u;
+    auto fold = [](float lo, float up, uint32_t flip) { return __fadd_rn(lo, __uint_as_float(__float_as_uint(up) ^ flip)); };
+    #pragma unroll
+    for (int k = 0; k < 8; k += 2) t[k] = fold(t[k], t[k + 1], f0);
+    t[0] = fold(t[0], t[2], f1); t[4] = fold(t[4], t[6], f1);
+    y = __fmul_rn(fold(t[0], t[4], f2), 0.0625f);
+    if ((c_signs.w[d >> 5] >> (d & 31)) & 1u) y = -y;
+  }
+  y = kv8_round(DT, y);
+  if (gate) y = kv8_gated<DT>(y, gt);
+  o16[e] = act_store16<DT>(y);
+}
+
+// One to four splits (prefill): eight lanes per row as in the row codec, four rows per warp, no shared memory and no barrier.
+template <int DT>
+__global__ void __launch_bounds__(256) kv8_combine_rows_kernel(const float* pm, const float* pl, const float* pacc, int S, int nh, long long rows,
+                                                               const void* gate, uint16_t* o16, int inverse_rotate) {
+  const int lane = threadIdx.x & 31, ll = lane & 7;
+  const long long row = (long long)blockIdx.x * 32 + (threadIdx.x >> 5) * 4 + (lane >> 3);       // row = token * nh + head
+  const bool live = row < rows;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const long long tok = live ? row / nh : 0;
+  const int head = live ? (int)(row - tok * nh) : 0;
+  auto slot = [&](int s) -> size_t { return ((size_t)tok * S + s) * nh + head; };
+  float M2 = -1e30f, L2 = 0.f, v[32];
+  #pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = 0.f;
+  for (int s = 0; s < S; ++s) M2 = fmaxf(M2, __ldcg(pm + slot(s)));
+  for (int s = 0; s < S; ++s) {
+    const float m = __ldcg(pm + slot(s)), w = m > -1e29f ? expf(m - M2) : 0.f;
+    L2 += w * __ldcg(pl + slot(s));
+    const float4* src = reinterpret_cast<const float4*>(pacc + slot(s) * KV8_HD) + ll;
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float4 a = __ldcg(src + 8 * k);
+      v[4 * k] += w * a.x; v[4 * k + 1] += w * a.y; v[4 * k + 2] += w * a.z; v[4 * k + 3] += w * a.w;
+    }
+  }
+  #pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __fdiv_rn(v[i], L2);
+  if (inverse_rotate) { hadamard256(v, ll); apply_signs(v, ll); }
+  if (!live) return;
+  const size_t e0 = (size_t)row * KV8_HD + 4 * ll;
+  #pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    uint2 g = make_uint2(0u, 0u);
+    if (gate) g = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(gate) + e0 + 32 * k));
+    const uint16_t gb[4] = {(uint16_t)g.x, (uint16_t)(g.x >> 16), (uint16_t)g.y, (uint16_t)(g.y >> 16)};
+    uint32_t w[4];
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float y = kv8_round(DT, v[4 * k + i]);
+      if (gate) y = kv8_gated<DT>(y, DT == YSKN_KV4_F16 ? h2f(gb[i]) : bf2f(gb[i]));
+      w[i] = act_store16<DT>(y);
+    }
+    *reinterpret_cast<uint2*>(o16 + e0 + 32 * k) = make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+  }
+}
+
+template <int DT>
+int launch_kv8_combine_dt(const float* pm, const float* pl, const float* pacc, int S, int M, int nh, const void* gate, uint16_t* o16, int inverse_rotate, cudaStream_t st) {
+  // The row form reads 16-byte pieces and wants enough rows to fill the GPU: with up to four splits and at least 2,048 rows (half a
+  // block of 32 rows per SM) it wins; a few long sums want the block form's parallel loads.
+  const long long rows = (long long)M * nh;
+  const bool aligned = !((((uintptr_t)pacc) & 15) | (((uintptr_t)o16 | (uintptr_t)gate) & 7));
+  if (S <= 4 && rows >= 2048 && aligned)
+    return launch_pdl("kv8_combine_rows_kernel", kv8_combine_rows_kernel<DT>, dim3((unsigned)((rows + 31) / 32)), 256, 0, st, pm, pl, pacc, S, nh, rows, gate, o16, inverse_rotate);
+  return launch_pdl("kv8_combine_kernel", kv8_combine_kernel<DT>, dim3(nh, M), KV8_CQ * 256, 0, st, pm, pl, pacc, S, nh, gate, o16, inverse_rotate);
 }
 
 }  // namespace
@@ -247,30 +341,31 @@ int launch_kv8_attention(const yskn_kv8_attn_args& a, int act_dtype, cudaStream_
     KV4_REJECT("yskn_kv8_attention: bad shape (kvh %d, nh %d, M %d, splits %d, max_ctx %d): at most 8 query heads per kv-head, max_ctx a multiple of 64",
                a.kvh, a.nh, a.M, a.splits, a.max_ctx);
   if (((uintptr_t)a.k8 | (uintptr_t)a.v8) & 15) KV4_REJECT("yskn_kv8_attention: k8 and v8 must be 16-byte aligned");
-  const size_t smem = 16 * 32 * 8 + 8 * 4 + (size_t)KV8_WARPS * 8 * 258 * 4;
+  const size_t smem = 16 * 32 * 8 + 32 * 4 + (size_t)KV8_WARPS * 8 * 258 * 4;
   Kv8P P{a, a.nh / a.kvh};
   const dim3 grid(a.splits, a.kvh, a.M);
   if (act_dtype == YSKN_KV4_BF16) {
     static std::atomic<unsigned long long> attr{0};
     if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kv8_decode_kernel<YSKN_KV4_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kv8_decode_kernel<YSKN_KV4_BF16><<<grid, KV8_WARPS * 32, smem, st>>>(P);
-  } else if (act_dtype == YSKN_KV4_F16) {
+    return launch_pdl("kv8_decode_kernel", kv8_decode_kernel<YSKN_KV4_BF16>, grid, KV8_WARPS * 32, smem, st, P);
+  }
+  if (act_dtype == YSKN_KV4_F16) {
     static std::atomic<unsigned long long> attr{0};
     if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kv8_decode_kernel<YSKN_KV4_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kv8_decode_kernel<YSKN_KV4_F16><<<grid, KV8_WARPS * 32, smem, st>>>(P);
-  } else KV4_REJECT("yskn_kv8_attention: q16 is bf16 or fp16 (act_dtype %d)", act_dtype);
-  return launch_status("kv8_decode_kernel");
+    return launch_pdl("kv8_decode_kernel", kv8_decode_kernel<YSKN_KV4_F16>, grid, KV8_WARPS * 32, smem, st, P);
+  }
+  KV4_REJECT("yskn_kv8_attention: q16 is bf16 or fp16 (act_dtype %d)", act_dtype);
 }
 
 int launch_kv8_combine(const float* pm, const float* pl, const float* pacc, int splits, int M, int nh, const void* gate, void* o16,
                        int act_dtype, int inverse_rotate, cudaStream_t st) {
   if (!pm || !pl || !pacc || !o16) KV4_REJECT("yskn_kv8_combine: null buffer");
   if (splits <= 0 || splits > 64 || M <= 0 || nh <= 0) KV4_REJECT("yskn_kv8_combine: bad shape (splits %d of at most 64, M %d, nh %d)", splits, M, nh);
-  const dim3 grid(nh, M);
-  if (act_dtype == YSKN_KV4_BF16) kv8_combine_kernel<YSKN_KV4_BF16><<<grid, 256, 0, st>>>(pm, pl, pacc, splits, M, nh, gate, o16, inverse_rotate);
-  else if (act_dtype == YSKN_KV4_F16) kv8_combine_kernel<YSKN_KV4_F16><<<grid, 256, 0, st>>>(pm, pl, pacc, splits, M, nh, gate, o16, inverse_rotate);
-  else KV4_REJECT("yskn_kv8_combine: o16 is bf16 or fp16 (act_dtype %d)", act_dtype);
-  return launch_status("kv8_combine_kernel");
+  if (M > 65535) KV4_REJECT("yskn_kv8_combine: M %d exceeds the grid limit", M);
+  uint16_t* out = static_cast<uint16_t*>(o16);
+  if (act_dtype == YSKN_KV4_BF16) return launch_kv8_combine_dt<YSKN_KV4_BF16>(pm, pl, pacc, splits, M, nh, gate, out, inverse_rotate, st);
+  if (act_dtype == YSKN_KV4_F16) return launch_kv8_combine_dt<YSKN_KV4_F16>(pm, pl, pacc, splits, M, nh, gate, out, inverse_rotate, st);
+  KV4_REJECT("yskn_kv8_combine: o16 is bf16 or fp16 (act_dtype %d)", act_dtype);
 }
 
 }  // namespace kv4

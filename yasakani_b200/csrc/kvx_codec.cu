@@ -8,63 +8,10 @@
 // butterfly stages pair registers and only three go through shuffles, and every load/store instruction of a row's lanes
 // covers one contiguous run.  The stages run in the reference's order h = 1, 2, ... 128.  HBM-bound byte mover by design
 // (1,284 B per fp32 row in + out, 772 B per fp16 row).
-#include "kv4_common.cuh"
+#include "kvx_rotate.cuh"
 
 namespace kv4 {
 namespace {
-
-// Bit 0 of the reference's 32-bit multiply-xorshift hash of d + 1: set = the element's sign is flipped.
-__host__ __device__ constexpr uint32_t kvx_sign_bit(int d) {
-  uint32_t x = (uint32_t)d + 1u;
-  x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
-  return x & 1u;
-}
-struct SignTable { uint32_t w[8]; };                       // 256 sign bits, bit d of the table = kvx_sign_bit(d)
-constexpr SignTable make_signs() {
-  SignTable t{};
-  for (int d = 0; d < 256; ++d) t.w[d >> 5] |= kvx_sign_bit(d) << (d & 31);
-  return t;
-}
-__constant__ SignTable c_signs = make_signs();
-// Element layout of a row over 8 lanes: lane ll (0..7) holds v[4k + e] = element d = 32k + 4ll + e (k 0..7, e 0..3), so every
-// load and store instruction of the 8 lanes covers one contiguous run of the row.  A warp holds 4 rows (lanes 8s .. 8s+7).
-// Multiplying by +-1 is a sign-bit flip (exact, also for zeros and infinities).
-__device__ __forceinline__ void apply_signs(float (&v)[32], int ll) {
-  #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const uint32_t bits = c_signs.w[k] >> (4 * ll);
-    #pragma unroll
-    for (int e = 0; e < 4; ++e) v[4 * k + e] = __uint_as_float(__float_as_uint(v[4 * k + e]) ^ (((bits >> e) & 1u) << 31));
-  }
-}
-
-// Butterflies + 1/16 in the reference's stage order h = 1, 2, ... 128.  Bits 0-1 of d are register bits (e), bits 2-4 the lane
-// within the row (shuffles), bits 5-7 register bits again (k).  Lower index: a + b; upper: lower - upper.
-__device__ __forceinline__ void hadamard256(float (&v)[32], int ll) {
-  #pragma unroll
-  for (int rb = 1; rb < 4; rb *= 2) {                      // h = 1, 2
-    #pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (!(i & rb)) { const float lo = v[i], up = v[i + rb]; v[i] = __fadd_rn(lo, up); v[i + rb] = __fsub_rn(lo, up); }
-  }
-  #pragma unroll
-  for (int m = 1; m < 8; m *= 2) {                         // h = 4, 8, 16
-    const uint32_t flip = (ll & m) ? 0x80000000u : 0u;     // upper lane: other - self = other + (-self), exactly
-    #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float self = v[i], other = __shfl_xor_sync(0xffffffffu, self, m);
-      v[i] = __fadd_rn(other, __uint_as_float(__float_as_uint(self) ^ flip));
-    }
-  }
-  #pragma unroll
-  for (int rb = 4; rb < 32; rb *= 2) {                     // h = 32, 64, 128
-    #pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (!(i & rb)) { const float lo = v[i], up = v[i + rb]; v[i] = __fadd_rn(lo, up); v[i + rb] = __fsub_rn(lo, up); }
-  }
-  #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __fmul_rn(v[i], 0.0625f);
-}
 
 template <int DT> __device__ __forceinline__ void load_row(const void* base, size_t row, int ll, bool live, float (&v)[32]) {
   #pragma unroll
@@ -175,8 +122,10 @@ __device__ __forceinline__ float rbf(float f) { return bf2f(f2bf(f)); }
 template <int NRH>
 __global__ void __launch_bounds__(256, 4) kvx_attn_post_kernel(yskn_kvx_attn_post_args A) {
   const int lane = threadIdx.x & 31, ll = lane & 7;
+  asm volatile("griddepcontrol.wait;" ::: "memory");           // programmatic dependent launch, both directions
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int per_tok = A.nh + 2 * A.kvh;
-  const long long item = (long long)blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5) * 4 + (lane >> 3);
+  const long long item = (long long)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3);
   const bool live = item < (long long)A.M * per_tok;
   const int tok = live ? (int)(item / per_tok) : 0, u = live ? (int)(item % per_tok) : 0;
   const int kind = u < A.nh ? 0 : (u < A.nh + A.kvh ? 1 : 2);    // query / key / value head
@@ -290,15 +239,18 @@ int launch_kvx_attn_post(const yskn_kvx_attn_post_args& a, cudaStream_t st) {
        (uintptr_t)a.k8 | (uintptr_t)a.v8) & 7)
     KV4_REJECT("yskn_kvx_attn_post: row arrays must be 8-byte aligned");
   if ((uintptr_t)a.rope & 15) KV4_REJECT("yskn_kvx_attn_post: the rope table must be 16-byte aligned");
-  unsigned grid; if (grid_for((long long)a.M * (a.nh + 2 * a.kvh), &grid, "yskn_kvx_attn_post")) return -1;
+  // A few tokens are bound by the latency of one warp's straight-line code: one-warp blocks put every four rows on an SM of their own
+  // (one token of the 27B shape is 32 rows, a single block of 256 threads).  From a block per SM on, blocks of 32 rows.
+  const long long rows = (long long)a.M * (a.nh + 2 * a.kvh);
+  const int threads = rows < 148 * ROWS_PER_BLOCK ? 32 : 256;
+  unsigned grid; if (grid_for(rows * (256 / threads), &grid, "yskn_kvx_attn_post")) return -1;
   switch (a.rd / 64) {
-    case 0: kvx_attn_post_kernel<0><<<grid, 256, 0, st>>>(a); break;
-    case 1: kvx_attn_post_kernel<1><<<grid, 256, 0, st>>>(a); break;
-    case 2: kvx_attn_post_kernel<2><<<grid, 256, 0, st>>>(a); break;
-    case 3: kvx_attn_post_kernel<3><<<grid, 256, 0, st>>>(a); break;
-    default: kvx_attn_post_kernel<4><<<grid, 256, 0, st>>>(a); break;
+    case 0: return launch_pdl("kvx_attn_post_kernel", kvx_attn_post_kernel<0>, dim3(grid), threads, 0, st, a);
+    case 1: return launch_pdl("kvx_attn_post_kernel", kvx_attn_post_kernel<1>, dim3(grid), threads, 0, st, a);
+    case 2: return launch_pdl("kvx_attn_post_kernel", kvx_attn_post_kernel<2>, dim3(grid), threads, 0, st, a);
+    case 3: return launch_pdl("kvx_attn_post_kernel", kvx_attn_post_kernel<3>, dim3(grid), threads, 0, st, a);
+    default: return launch_pdl("kvx_attn_post_kernel", kvx_attn_post_kernel<4>, dim3(grid), threads, 0, st, a);
   }
-  return launch_status("kvx_attn_post_kernel");
 }
 
 }  // namespace kv4
