@@ -9,12 +9,6 @@
 //   payload: the kk new bits of every step, MSB first, 8*kk 32-bit words per row; side words: scale, two fp16 coefficients.
 // Sums over a row follow the reference's order (a xor-butterfly over each run of 32 values, then the eight run sums in
 // order), and every product that feeds a rounding decision is an explicit _rn operation, so no FMA contraction moves a bit.
-//
-// Work split (not the reference's): the reference runs one 256-thread block per (row, multiplier, chain) with a block
-// barrier per trellis step.  Here ONE WARP owns a (row, multiplier, chain) search: a lane owns eight consecutive states,
-// which all share one predecessor set, so a step is one vector read of that set (the costs are kept transposed in the
-// warp's own shared memory so that the set is contiguous), one minimum, eight squared differences and eight stores, with
-// a warp-level barrier only.  A second kernel, one block per row, picks the multiplier, rebuilds the row and packs it.
 #include "kv4_common.cuh"
 #include <cstring>
 
@@ -38,220 +32,220 @@ __device__ __forceinline__ TbGroup tb_group(const uint8_t* b, int g) {
   return P;
 }
 
-// ---- a warp's view of a row: lane holds elements 32*w + lane, w = 0..7 (one per run of the reference's reduction)
-__device__ __forceinline__ float warp_rowsum(const float (&v)[8]) {
-  float t = 0.f;
-  #pragma unroll
-  for (int w = 0; w < 8; ++w) {
-    float a = v[w];
-    #pragma unroll
-    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    t = __fadd_rn(t, a);
-  }
-  return t;
-}
-struct RowPre { float r[8], mud[8], u0[8], u1[8], c0, c1, rms; };
-__device__ __forceinline__ void warp_pre(const uint8_t* b, const TbGroup& P, const float* y, int lane, RowPre& Q) {
-  const uint8_t* mup = b + P.go + 8;
-  const uint8_t* Up = mup + (P.has_mu ? 512 : 0);
-  float tmp[8];
-  Q.c0 = Q.c1 = 0.f;
-  #pragma unroll
-  for (int w = 0; w < 8; ++w) {
-    const int d = 32 * w + lane;
-    Q.mud[w] = P.has_mu ? __half2float(__ushort_as_half((unsigned short)tb_u16(mup + 2 * d))) : 0.f;
-    Q.r[w] = P.has_mu ? __fsub_rn(y[d], Q.mud[w]) : y[d];
-    Q.u0[w] = P.m > 0 ? __half2float(__ushort_as_half((unsigned short)tb_u16(Up + 2 * d))) : 0.f;
-    Q.u1[w] = P.m > 1 ? __half2float(__ushort_as_half((unsigned short)tb_u16(Up + 2 * (256 + d)))) : 0.f;
-  }
-  if (P.m > 0) {
-    #pragma unroll
-    for (int w = 0; w < 8; ++w) tmp[w] = __fmul_rn(Q.r[w], Q.u0[w]);
-    Q.c0 = tb_f16r(warp_rowsum(tmp));
-    #pragma unroll
-    for (int w = 0; w < 8; ++w) Q.r[w] = __fsub_rn(Q.r[w], __fmul_rn(Q.c0, Q.u0[w]));
-  }
-  if (P.m > 1) {
-    #pragma unroll
-    for (int w = 0; w < 8; ++w) tmp[w] = __fmul_rn(Q.r[w], Q.u1[w]);
-    Q.c1 = tb_f16r(warp_rowsum(tmp));
-    #pragma unroll
-    for (int w = 0; w < 8; ++w) Q.r[w] = __fsub_rn(Q.r[w], __fmul_rn(Q.c1, Q.u1[w]));
-  }
-  #pragma unroll
-  for (int w = 0; w < 8; ++w) tmp[w] = __fmul_rn(Q.r[w], Q.r[w]);
-  Q.rms = __fsqrt_rn(__fdiv_rn(warp_rowsum(tmp), 256.f));
-  if (Q.rms == 0.f) Q.rms = 1.f;
-}
-
-constexpr int TB_WARPS = 8;                              // searches per block
-struct alignas(16) TbWarpSmem { int cost[2][256]; uint8_t bp[64][32]; uint8_t st[64]; };
-
-struct TbP {
-  const uint8_t* blob; int nm; const float* x; const int* grp; const int* pos; int rows;
-  float* y; uint8_t* pay; int pay_stride; uint32_t* side; uint8_t* scr_states; float* scr_err;
+// ---- encoder: one block of four warps per row, one warp per chain of 64 values.
+//
+// A step of the search takes new(d) = min over the 2^KK predecessors {j * UU + u}, u = d >> KK, of old(p), plus (x - code[d])^2: every
+// state is a candidate of one group u only, so 256 candidates and 256 costs a step.  What bounds it is instruction issue
+// (integer), so the whole step stays in registers: a lane holds eight states, four values of j for two values of u,
+//   p = jhi << (SH+2) | jlo << SH | umid << 1 | ulo,     registers e = (jlo, ulo), lane = (jhi, umid)     (SH = 8 - KK, UU = 2^SH)
+// the minimum over jlo is in the lane (one fused add-minimum per state), the first exchange over jhi halves the lane's two
+// values of u (each lane of the pair keeps one), the other exchanges are plain; the new states of a lane need 4 (KK = 3, 4) or
+// 1 (KK = 5) of the UU minima, one shuffle each: 6 / 7 / 4 shuffles and about 35 instructions a step, no shared memory on the path and no barrier.
+// x^2 is left out of the costs: it adds the same number to every state of a step.
+// Only the minima M_t[u] are kept (no back pointers): the walk back recomputes the 2^KK candidates of the ONE group it passes
+// through, a lane each, and takes the first that equals the minimum, the reference's tie rule (src/kvq_gpu.cuh:101-102).
+// 4,096 rows, 5 multipliers, on a B200: %BEFORE% -> %AFTER% us (one warp per (row, multiplier, chain) with the costs in shared memory and every
+// lane walking its group's predecessors, then a second kernel for choice and packing).
+constexpr int TB_NM = 16;                                // multipliers at most (the blob's limit)
+struct TbRowSmem {
+  int hist[4][64 * 32];                                  // M_t[u] of each chain: [t][u]
+  short code[256]; float red[8]; uint8_t fld[256];
+  struct Mult { uint8_t st[256]; float err[8]; } mult[1];  // one per multiplier: its states and its error sums
+  static size_t bytes(int nm) { return sizeof(TbRowSmem) + (nm - 1) * sizeof(Mult); }      // five multipliers: six blocks (24 warps) per SM
 };
+struct TbP { const uint8_t* blob; int nm; const float* x; const int* grp; const int* pos; int rows; float* y; uint8_t* pay; int pay_stride; uint32_t* side; };
 
-// One warp per (row, multiplier, chain).  States of the best path -> scr_states[row][mi][64*c ..], the two half-chain error
-// sums -> scr_err[row][mi][2c], [2c+1] (the runs of the reference's error sum, src/kvq_fast.cuh:140-147).
-template <int KK>
-__device__ __forceinline__ void tb_search(TbWarpSmem& S, const uint8_t* b, const TbGroup& P, const RowPre& Q, float s, int c, int lane,
-                                          uint8_t* so, float* wo) {
-  constexpr int KQ = 1 << KK, UU = 256 >> KK, SH = 8 - KK;
-  const unsigned to = tb_u32(b + P.off_t + 4u * (unsigned)P.tix);
-  const float gain = tb_f32(b + to + 4);
-  int ci[8];                                             // codes of this lane's states d = 8*lane + e
+// States of the best path of this warp's chain for the scaled values xa (steps 0-31, a lane each) and xb (steps 32-63): returned
+// as (state of step lane, state of step lane + 32).
+template <int KK> __device__ __forceinline__ int2 tb_search(int* hist, const short* code, int xa, int xb, int lane) {
+  constexpr int KQ = 1 << KK, SH = 8 - KK, UU = 1 << SH, NQ = KK == 5 ? 1 : 4;
+  const int umid = lane & ((1 << (SH - 1)) - 1), jhi = lane >> (SH - 1);
+  int m2c[8], c2[8], src[NQ];
   #pragma unroll
-  for (int e = 0; e < 8; ++e) ci[e] = (int)(short)tb_u16(b + to + 12 + 2 * (8 * lane + e));
-  // this chain's 64 scaled values: lane holds steps lane and lane + 32
-  const float ra = Q.r[2 * c], rb = Q.r[2 * c + 1];
-  const int xa = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(ra, s), 256.f)), -2048.f), 2048.f);
-  const int xb = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(rb, s), 256.f)), -2048.f), 2048.f);
-  // transposed cost layout: state p sits at (p % UU) * KQ + p / UU, so the predecessors {j*UU + u} of group u are contiguous
-  const int u = (8 * lane) >> KK;                        // the predecessor group of all eight states of this lane
-  int widx[8];
+  for (int e = 0; e < 8; ++e) {
+    const int c = code[(jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1)];
+    m2c[e] = -2 * c; c2[e] = c * c;
+  }
   #pragma unroll
-  for (int e = 0; e < 8; ++e) { const int d = 8 * lane + e; widx[e] = (d & (UU - 1)) * KQ + (d >> SH); }
-  #pragma unroll
-  for (int e = 0; e < 8; ++e) S.cost[0][widx[e]] = (8 * lane + e == 0) ? 0 : 0x40000000;
-  __syncwarp();
+  for (int q = 0; q < NQ; ++q) {                         // the lane that holds the minimum of group (new state >> KK)
+    const int g = ((jhi << (SH + 2)) | (q << SH) | (umid << 1)) >> KK;
+    src[q] = ((g & 1) << (SH - 1)) | (g >> 1);
+  }
+  const bool upper = (lane >> (SH - 1)) & 1;             // of a pair of lanes the upper one keeps the odd u
+  const int my_u = (umid << 1) | (upper ? 1 : 0);
+  int keep = my_u == 0 ? 0 : 0x40000000;                 // M_0: only state 0 exists
+  auto costs = [&](int x, int (&t)[8], int (&m)[NQ]) {
+    #pragma unroll
+    for (int q = 0; q < NQ; ++q) m[q] = __shfl_sync(0xffffffffu, keep, src[q]);
+    #pragma unroll
+    for (int e = 0; e < 8; ++e) t[e] = x * m2c[e] + c2[e];
+  };
   #pragma unroll 1
-  for (int t = 0; t < 64; ++t) {
-    const int4* cp = reinterpret_cast<const int4*>(&S.cost[t & 1][u * KQ]);
-    int mn = 0x7fffffff, jb = 0;
-    #pragma unroll
-    for (int q = 0; q < KQ / 4; ++q) {                   // first minimum in predecessor order (src/kvq_gpu.cuh:101-102)
-      const int4 v = cp[q];
-      if (v.x < mn) { mn = v.x; jb = 4 * q; }
-      if (v.y < mn) { mn = v.y; jb = 4 * q + 1; }
-      if (v.z < mn) { mn = v.z; jb = 4 * q + 2; }
-      if (v.w < mn) { mn = v.w; jb = 4 * q + 3; }
+  for (int half = 0; half < 2; ++half) {
+    const int xs = half ? xb : xa;
+    #pragma unroll 4
+    for (int i = 0; i < 32; ++i) {
+      const int t = 32 * half + i;
+      if (lane < UU) hist[t * UU + my_u] = keep;         // lanes below UU hold every u once (jhi bits above the first are zero)
+      if (t == 63) break;
+      int ct[8], m[NQ];
+      costs(__shfl_sync(0xffffffffu, xs, i), ct, m);
+      int a = ct[0] + m[0], b = ct[1] + m[0];
+      #pragma unroll
+      for (int q = 1; q < 4; ++q) {
+        a = __viaddmin_s32(ct[2 * q], m[NQ == 1 ? 0 : q], a);
+        b = __viaddmin_s32(ct[2 * q + 1], m[NQ == 1 ? 0 : q], b);
+      }
+      const int other = __shfl_xor_sync(0xffffffffu, upper ? a : b, 1 << (SH - 1));
+      keep = min(upper ? b : a, other);
+      #pragma unroll
+      for (int k = SH; k < 5; ++k) keep = min(keep, __shfl_xor_sync(0xffffffffu, keep, 1 << k));
     }
-    const int xt = __shfl_sync(0xffffffffu, t < 32 ? xa : xb, t & 31);
-    int* cn = S.cost[(t + 1) & 1];
-    #pragma unroll
-    for (int e = 0; e < 8; ++e) { const int dx = xt - ci[e]; cn[widx[e]] = dx * dx + mn; }
-    if (((8 * lane) & (KQ - 1)) == 0) S.bp[t][u] = (uint8_t)jb;
-    __syncwarp();
   }
   // best final state: smallest (cost, state)
-  unsigned long long key = ~0ull;
+  int ct[8], m[NQ];
+  costs(__shfl_sync(0xffffffffu, xb, 31), ct, m);
+  int best = 0x7fffffff, bs = 0;
   #pragma unroll
-  for (int e = 0; e < 8; ++e) { const unsigned long long k = ((unsigned long long)(unsigned)S.cost[0][widx[e]] << 8) | (unsigned long long)(8 * lane + e); key = k < key ? k : key; }
-  #pragma unroll
-  for (int o = 16; o; o >>= 1) { const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, key, o); key = k2 < key ? k2 : key; }
-  if (lane == 0) {
-    int st = (int)(key & 255ull);
-    for (int t = 63; t >= 0; --t) { S.st[t] = (uint8_t)st; const int j = S.bp[t][st >> KK]; st = (j << SH) | (st >> KK); }
+  for (int e = 0; e < 8; ++e) {                          // a lane's states grow with jlo, then ulo
+    const int c = ct[e] + m[NQ == 1 ? 0 : e >> 1], p = (jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1);
+    if (c < best) { best = c; bs = p; }
   }
-  __syncwarp();
-  #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int stt = S.st[lane + 32 * h];
-    const int cs = (int)(short)tb_u16(b + to + 12 + 2 * stt);
-    const float rec = __fmul_rn(__fmul_rn(__fmul_rn((float)cs, 0.00390625f), gain), s);
-    const float dd = __fsub_rn(h ? rb : ra, rec);
-    float v = __fmul_rn(dd, dd);
-    #pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) wo[h] = v;
-    so[lane + 32 * h] = (uint8_t)stt;
+  const int all = __reduce_min_sync(0xffffffffu, best);
+  int st = (int)__reduce_min_sync(0xffffffffu, best == all ? (unsigned)bs : 0xffffffffu);
+  __syncwarp();                                          // the history is complete
+  int2 out = make_int2(0, 0);
+  #pragma unroll 1
+  for (int half = 1; half >= 0; --half) {
+    int mine = 0;
+    #pragma unroll 1
+    for (int i = 31; i >= 0; --i) {
+      const int t = 32 * half + i;
+      if (lane == i) mine = st;
+      if (t == 0) break;
+      const int u = st >> KK, p = ((lane << SH) | u) & 255, c = code[p];
+      const int x = __shfl_sync(0xffffffffu, i > 0 ? (half ? xb : xa) : xa, (i - 1) & 31);      // x of step t - 1
+      const int cost = hist[(t - 1) * UU + (p >> KK)] + c * (c - 2 * x);
+      const unsigned hit = __ballot_sync(0xffffffffu, lane < KQ && cost == hist[t * UU + u]);
+      st = ((__ffs(hit) - 1) << SH) | u;
+    }
+    if (half) out.y = mine; else out.x = mine;
   }
-  __syncwarp();
+  __syncwarp();                                          // the history may be overwritten
+  return out;
 }
 
-__global__ void __launch_bounds__(TB_WARPS * 32) tb_search_kernel(TbP A) {
-  __shared__ TbWarpSmem S[TB_WARPS];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long job = (long long)blockIdx.x * TB_WARPS + warp;
-  if (job >= (long long)A.rows * A.nm * 4) return;
-  const int row = (int)(job / (A.nm * 4)), rem = (int)(job - (long long)row * (A.nm * 4)), mi = rem >> 2, c = rem & 3;
-  const TbGroup P = tb_group(A.blob, A.grp[row]);
-  if (!P.ok || A.pos[row] < P.guard || P.mode != 0) return;           // stored as is, or flat codes: no search
-  RowPre Q;
-  warp_pre(A.blob, P, A.x + (size_t)row * 256, lane, Q);
-  float s = tb_f16r(__fmul_rn(Q.rms, tb_f32(A.blob + P.off_m + 4u * (unsigned)mi)));
-  if (s == 0.f) s = 1.f;
-  uint8_t* so = A.scr_states + ((size_t)row * A.nm + mi) * 256 + 64 * c;
-  float* wo = A.scr_err + ((size_t)row * A.nm + mi) * 8 + 2 * c;
-  if (P.kk == 3) tb_search<3>(S[warp], A.blob, P, Q, s, c, lane, so, wo);
-  else if (P.kk == 4) tb_search<4>(S[warp], A.blob, P, Q, s, c, lane, so, wo);
-  else if (P.kk == 5) tb_search<5>(S[warp], A.blob, P, Q, s, c, lane, so, wo);
-  else { so[lane] = 0; so[lane + 32] = 0; if (lane == 0) { wo[0] = 3.0e38f; wo[1] = 3.0e38f; } }   // a step width the code does not have: never the best
-}
-
-// One block per row: pick the multiplier, rebuild the row, pack fields and side words.
-__global__ void __launch_bounds__(256) tb_select_kernel(TbP A) {
-  __shared__ uint8_t fld[256];
-  __shared__ float red[8];
-  const int row = blockIdx.x, d = threadIdx.x, warp = d >> 5, lane = d & 31;
+__global__ void __launch_bounds__(128, 6) tb_encode_kernel(TbP A) {
+  extern __shared__ __align__(16) unsigned char tbe_smem[];
+  TbRowSmem& S = *reinterpret_cast<TbRowSmem*>(tbe_smem);
+  const int row = blockIdx.x, c = threadIdx.x >> 5, lane = threadIdx.x & 31, d0 = 64 * c + lane, d1 = d0 + 32;     // this thread's two values
   const uint8_t* b = A.blob;
   const TbGroup P = tb_group(b, A.grp[row]);
-  const float yv = A.x[(size_t)row * 256 + d];
-  if (!P.ok || A.pos[row] < P.guard) { if (A.y) A.y[(size_t)row * 256 + d] = yv; return; }
-  auto bsum = [&](float v) -> float {                    // the reference's block sum (src/kvq_fast.cuh:33-43)
+  const int words = A.pay_stride / 4;
+  unsigned* pay = A.pay ? reinterpret_cast<unsigned*>(A.pay + (size_t)row * A.pay_stride) : nullptr;
+  float ra = A.x[(size_t)row * 256 + d0], rb = A.x[(size_t)row * 256 + d1];
+  if (!P.ok || A.pos[row] < P.guard) {                   // stored as it is: the payload and the side words are zero
+    if (A.y) { A.y[(size_t)row * 256 + d0] = ra; A.y[(size_t)row * 256 + d1] = rb; }
+    if (pay) for (int w = threadIdx.x; w < words; w += 128) pay[w] = 0u;
+    if (A.side && threadIdx.x < 2) A.side[2 * row + threadIdx.x] = 0u;
+    return;
+  }
+  // the reference's row sum: a xor-butterfly over each run of 32 values, then the eight runs in order (src/kvq_fast.cuh:33-43)
+  auto runs = [&](float va, float vb, float* out) {
     #pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp] = v;
+    for (int o = 16; o; o >>= 1) { va += __shfl_xor_sync(0xffffffffu, va, o); vb += __shfl_xor_sync(0xffffffffu, vb, o); }
+    if (lane == 0) { out[2 * c] = va; out[2 * c + 1] = vb; }
+  };
+  auto rowsum = [&](float va, float vb) -> float {
+    runs(va, vb, S.red);
     __syncthreads();
     float t = 0.f;
     #pragma unroll
-    for (int w = 0; w < 8; ++w) t = __fadd_rn(t, red[w]);
+    for (int w = 0; w < 8; ++w) t = __fadd_rn(t, S.red[w]);
     __syncthreads();
     return t;
   };
   const uint8_t* mup = b + P.go + 8;
   const uint8_t* Up = mup + (P.has_mu ? 512 : 0);
-  float r = yv, mud = 0.f, u0 = 0.f, u1 = 0.f, c0 = 0.f, c1 = 0.f;
-  if (P.has_mu) { mud = __half2float(__ushort_as_half((unsigned short)tb_u16(mup + 2 * d))); r = __fsub_rn(yv, mud); }
-  if (P.m > 0) { u0 = __half2float(__ushort_as_half((unsigned short)tb_u16(Up + 2 * d))); c0 = tb_f16r(bsum(__fmul_rn(r, u0))); r = __fsub_rn(r, __fmul_rn(c0, u0)); }
-  if (P.m > 1) { u1 = __half2float(__ushort_as_half((unsigned short)tb_u16(Up + 2 * (256 + d)))); c1 = tb_f16r(bsum(__fmul_rn(r, u1))); r = __fsub_rn(r, __fmul_rn(c1, u1)); }
-  float rms = __fsqrt_rn(__fdiv_rn(bsum(__fmul_rn(r, r)), 256.f)); if (rms == 0.f) rms = 1.f;
-  float xq, psc; int field, kb;
+  auto f16at = [&](const uint8_t* p, int d) { return __half2float(__ushort_as_half((unsigned short)tb_u16(p + 2 * d))); };
+  float mua = 0.f, mub = 0.f, u0a = 0.f, u0b = 0.f, u1a = 0.f, u1b = 0.f, c0 = 0.f, c1 = 0.f;
+  if (P.has_mu) { mua = f16at(mup, d0); mub = f16at(mup, d1); ra = __fsub_rn(ra, mua); rb = __fsub_rn(rb, mub); }
+  if (P.m > 0) {
+    u0a = f16at(Up, d0); u0b = f16at(Up, d1);
+    c0 = tb_f16r(rowsum(__fmul_rn(ra, u0a), __fmul_rn(rb, u0b)));
+    ra = __fsub_rn(ra, __fmul_rn(c0, u0a)); rb = __fsub_rn(rb, __fmul_rn(c0, u0b));
+  }
+  if (P.m > 1) {
+    u1a = f16at(Up + 512, d0); u1b = f16at(Up + 512, d1);
+    c1 = tb_f16r(rowsum(__fmul_rn(ra, u1a), __fmul_rn(rb, u1b)));
+    ra = __fsub_rn(ra, __fmul_rn(c1, u1a)); rb = __fsub_rn(rb, __fmul_rn(c1, u1b));
+  }
+  float xqa, xqb, psc; int fa, fb, kb;
   if (P.mode == 1) {                                     // flat 4-bit codes (src/kvq_fast.cuh:193-198)
-    float am = fabsf(r);
+    float am = fmaxf(fabsf(ra), fabsf(rb));
     #pragma unroll
     for (int o = 16; o; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-    if (lane == 0) red[warp] = am;
+    if (lane == 0) S.red[c] = am;
     __syncthreads();
-    am = 0.f;
-    #pragma unroll
-    for (int w = 0; w < 8; ++w) am = fmaxf(am, red[w]);
-    __syncthreads();
+    am = fmaxf(fmaxf(S.red[0], S.red[1]), fmaxf(S.red[2], S.red[3]));
     float s7 = __fdiv_rn(am, 7.f); if (s7 == 0.f) s7 = 1.f;
-    float q = rintf(__fdiv_rn(r, s7)); q = fminf(fmaxf(q, -7.f), 7.f);
-    xq = __fmul_rn(q, s7); field = (int)q + 8; psc = s7; kb = 4;
+    const float qa = fminf(fmaxf(rintf(__fdiv_rn(ra, s7)), -7.f), 7.f), qb = fminf(fmaxf(rintf(__fdiv_rn(rb, s7)), -7.f), 7.f);
+    xqa = __fmul_rn(qa, s7); xqb = __fmul_rn(qb, s7); fa = (int)qa + 8; fb = (int)qb + 8; psc = s7; kb = 4;
   } else {
-    const float* W = A.scr_err + (size_t)row * A.nm * 8;
-    float best_e = 0.f; int best = 0; bool have = false;
-    for (int mi = 0; mi < A.nm; ++mi) {
-      float e = 0.f;
-      #pragma unroll
-      for (int w = 0; w < 8; ++w) e = __fadd_rn(e, W[mi * 8 + w]);
-      if (!have || e < best_e) { have = true; best_e = e; best = mi; }
-    }
-    float s = tb_f16r(__fmul_rn(rms, tb_f32(b + P.off_m + 4u * (unsigned)best))); if (s == 0.f) s = 1.f;
     const unsigned to = tb_u32(b + P.off_t + 4u * (unsigned)P.tix);
     const float gain = tb_f32(b + to + 4);
-    const int st = A.scr_states[((size_t)row * A.nm + best) * 256 + d];
-    const int cs = (int)(short)tb_u16(b + to + 12 + 2 * st);
-    xq = __fmul_rn(__fmul_rn(__fmul_rn((float)cs, 0.00390625f), gain), s);
-    field = st & ((1 << P.kk) - 1); psc = s; kb = P.kk;
-  }
-  float x = xq;
-  if (P.m > 0) x = __fadd_rn(x, __fmul_rn(c0, u0));
-  if (P.m > 1) x = __fadd_rn(x, __fmul_rn(c1, u1));
-  if (P.has_mu) x = __fadd_rn(x, mud);
-  if (A.y) A.y[(size_t)row * 256 + d] = x;
-  if (A.pay) {
-    fld[d] = (uint8_t)field;
-    __syncthreads();
-    if (d < 8 * kb) {                                    // MSB-first bit stream, 32 bits per word (src/kvq_fast.cuh:228-232)
-      unsigned w = 0u;
-      for (int i = 0; i < 32; ++i) { const int gbit = 32 * d + i, e = gbit / kb, jb = gbit - e * kb; w |= (((unsigned)fld[e] >> (kb - 1 - jb)) & 1u) << (31 - i); }
-      reinterpret_cast<unsigned*>(A.pay + (size_t)row * A.pay_stride)[d] = w;
+    for (int i = threadIdx.x; i < 256; i += 128) S.code[i] = (short)tb_u16(b + to + 12 + 2 * i);
+    float rms = __fsqrt_rn(__fdiv_rn(rowsum(__fmul_rn(ra, ra), __fmul_rn(rb, rb)), 256.f));     // its barriers also publish the codes
+    if (rms == 0.f) rms = 1.f;
+    auto scale = [&](int mi) { const float s = tb_f16r(__fmul_rn(rms, tb_f32(b + P.off_m + 4u * (unsigned)mi))); return s == 0.f ? 1.f : s; };
+    auto value = [&](int st, float s) { return __fmul_rn(__fmul_rn(__fmul_rn((float)(int)S.code[st], 0.00390625f), gain), s); };
+    #pragma unroll 1
+    for (int mi = 0; mi < A.nm; ++mi) {
+      const float s = scale(mi);
+      const int xa = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(ra, s), 256.f)), -2048.f), 2048.f);
+      const int xb = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(rb, s), 256.f)), -2048.f), 2048.f);
+      int2 st = make_int2(0, 0);
+      if (P.kk == 3) st = tb_search<3>(S.hist[c], S.code, xa, xb, lane);
+      else if (P.kk == 4) st = tb_search<4>(S.hist[c], S.code, xa, xb, lane);
+      else if (P.kk == 5) st = tb_search<5>(S.hist[c], S.code, xa, xb, lane);
+      const float da = __fsub_rn(ra, value(st.x, s)), db = __fsub_rn(rb, value(st.y, s));
+      runs(__fmul_rn(da, da), __fmul_rn(db, db), S.mult[mi].err);
+      S.mult[mi].st[d0] = (uint8_t)st.x; S.mult[mi].st[d1] = (uint8_t)st.y;
     }
-    if (d == 0 && A.side) {
+    __syncthreads();
+    float best_e = 0.f; int best = 0;
+    for (int mi = 0; mi < A.nm; ++mi) {                  // the smallest squared error, the first on ties
+      float e = 0.f;
+      #pragma unroll
+      for (int w = 0; w < 8; ++w) e = __fadd_rn(e, S.mult[mi].err[w]);
+      if (mi == 0 || e < best_e) { best_e = e; best = mi; }
+    }
+    const float s = scale(best);
+    const int sa = S.mult[best].st[d0], sb = S.mult[best].st[d1];
+    xqa = value(sa, s); xqb = value(sb, s);
+    fa = sa & ((1 << P.kk) - 1); fb = sb & ((1 << P.kk) - 1); psc = s; kb = P.kk;
+  }
+  if (A.y) {
+    if (P.m > 0) { xqa = __fadd_rn(xqa, __fmul_rn(c0, u0a)); xqb = __fadd_rn(xqb, __fmul_rn(c0, u0b)); }
+    if (P.m > 1) { xqa = __fadd_rn(xqa, __fmul_rn(c1, u1a)); xqb = __fadd_rn(xqb, __fmul_rn(c1, u1b)); }
+    if (P.has_mu) { xqa = __fadd_rn(xqa, mua); xqb = __fadd_rn(xqb, mub); }
+    A.y[(size_t)row * 256 + d0] = xqa; A.y[(size_t)row * 256 + d1] = xqb;
+  }
+  if (pay) {
+    S.fld[d0] = (uint8_t)fa; S.fld[d1] = (uint8_t)fb;
+    __syncthreads();
+    for (int w = threadIdx.x; w < words; w += 128) {     // MSB-first bit stream, 32 bits per word (src/kvq_fast.cuh:228-232)
+      unsigned v = 0u;
+      if (w < 8 * kb) {
+        const int e0 = 32 * w / kb;                      // the field that holds the word's first bit
+        for (int e = e0; e * kb < 32 * w + 32; ++e) {
+          const int sh = 32 - (e + 1) * kb + 32 * w;     // where the field's last bit sits in the word; negative: it runs into the next word
+          v |= sh >= 0 ? (unsigned)S.fld[e] << sh : (unsigned)S.fld[e] >> -sh;
+        }
+      }
+      pay[w] = v;
+    }
+    if (A.side && threadIdx.x == 0) {
       A.side[2 * row] = __float_as_uint(psc);
       A.side[2 * row + 1] = (unsigned)__half_as_ushort(__float2half_rn(c0)) | ((unsigned)__half_as_ushort(__float2half_rn(c1)) << 16);
     }
@@ -548,7 +542,7 @@ int launch_tb_decode(const uint8_t* blob, const int* grp, const int* pos, const 
   return launch_status("tb_unpack_kernel");
 }
 
-size_t tb_scratch_bytes(int rows, int nm) { return rows > 0 && nm > 0 ? (size_t)rows * nm * (256 + 8 * sizeof(float)) : 0; }
+size_t tb_scratch_bytes(int, int) { return 0; }              // the encoder keeps everything on chip
 
 // Host-side check of a "KVQP v1" blob, the reference loader's (src/engine35.cpp:50-53) plus its table checks
 // (src/kvq_fast.hpp:66-69); *nm = number of scale multipliers.
@@ -578,18 +572,14 @@ int tb_blob_info(const uint8_t* b, size_t n, int* nm) {
 
 int launch_tb_encode(const uint8_t* blob, int nm, const float* x, const int* grp, const int* pos, int rows, float* y, uint8_t* pay, int pay_stride,
                      uint32_t* side, void* scratch, size_t scratch_bytes, cudaStream_t st) {
-  if (!blob || !x || !grp || !pos || !scratch) KV4_REJECT("yskn_tb_encode: null buffer");
-  if (rows <= 0 || nm < 1 || nm > 16) KV4_REJECT("yskn_tb_encode: bad shape (rows %d, multipliers %d)", rows, nm);
+  (void)scratch; (void)scratch_bytes;
+  if (!blob || !x || !grp || !pos) KV4_REJECT("yskn_tb_encode: null buffer");
+  if (rows <= 0 || nm < 1 || nm > TB_NM) KV4_REJECT("yskn_tb_encode: bad shape (rows %d, multipliers %d)", rows, nm);
   if (pay && (pay_stride < 160 || pay_stride % 4 || ((uintptr_t)pay & 3))) KV4_REJECT("yskn_tb_encode: payload rows need a stride of at least 160 bytes, a multiple of 4");
-  if (scratch_bytes < tb_scratch_bytes(rows, nm) || ((uintptr_t)scratch & 3)) KV4_REJECT("yskn_tb_encode: scratch of %zu bytes needed", tb_scratch_bytes(rows, nm));
-  TbP A{blob, nm, x, grp, pos, rows, y, pay, pay_stride, side, nullptr, nullptr};
-  A.scr_err = static_cast<float*>(scratch);
-  A.scr_states = static_cast<uint8_t*>(scratch) + (size_t)rows * nm * 8 * sizeof(float);
-  const long long jobs = (long long)rows * nm * 4;
-  tb_search_kernel<<<(unsigned)((jobs + TB_WARPS - 1) / TB_WARPS), TB_WARPS * 32, 0, st>>>(A);
-  if (int rc = launch_status("tb_search_kernel")) return rc;
-  tb_select_kernel<<<rows, 256, 0, st>>>(A);
-  return launch_status("tb_select_kernel");
+  static std::atomic<unsigned long long> attr{0};
+  if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(tb_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TbRowSmem::bytes(TB_NM)));
+  tb_encode_kernel<<<rows, 128, TbRowSmem::bytes(nm), st>>>(TbP{blob, nm, x, grp, pos, rows, y, pay, pay_stride, side});
+  return launch_status("tb_encode_kernel");
 }
 
 int launch_tb_attention(const yskn_tb_attn_args& a, int act_dtype, cudaStream_t st) {

@@ -103,13 +103,11 @@ def tb_encode(profile: TrellisProfile, x: torch.Tensor, grp: torch.Tensor, pos: 
     side int32-bits [rows][2]); grp, pos int32 device tensors [rows]."""
     rows = _rows(x)
     assert x.dtype == torch.float32 and grp.dtype == torch.int32 and pos.dtype == torch.int32
-    L = _lib.load()
     y = torch.empty_like(x)
-    pay = torch.zeros((rows, pay_stride), dtype=torch.uint8, device=x.device)
-    side = torch.zeros((rows, 2), dtype=torch.int32, device=x.device)
-    scratch = torch.empty(int(L.yskn_tb_scratch_bytes(rows, profile.nm)), dtype=torch.uint8, device=x.device)
-    check(L.yskn_tb_encode(_ptr(profile.dev), profile.nm, _ptr(x), _ptr(grp), _ptr(pos), rows, _ptr(y), _ptr(pay), pay_stride, _ptr(side),
-                           _ptr(scratch), scratch.numel(), _stream(stream)), "yskn_tb_encode")
+    pay = torch.empty((rows, pay_stride), dtype=torch.uint8, device=x.device)
+    side = torch.empty((rows, 2), dtype=torch.int32, device=x.device)
+    check(_lib.load().yskn_tb_encode(_ptr(profile.dev), profile.nm, _ptr(x), _ptr(grp), _ptr(pos), rows, _ptr(y), _ptr(pay), pay_stride, _ptr(side),
+                                     None, 0, _stream(stream)), "yskn_tb_encode")
     return y, pay, side
 
 
