@@ -41,30 +41,41 @@ __device__ __forceinline__ TbGroup tb_group(const uint8_t* b, int g) {
 // the minimum over jlo is in the lane (one fused add-minimum per state), the first exchange over jhi halves the lane's two
 // values of u (each lane of the pair keeps one), the other exchanges are plain; the new states of a lane need 4 (KK = 3, 4) or
 // 1 (KK = 5) of the UU minima, one shuffle each: 6 / 7 / 4 shuffles and about 35 instructions a step, no shared memory on the path and no barrier.
-// x^2 is left out of the costs: it adds the same number to every state of a step.
-// Only the minima M_t[u] are kept (no back pointers): the walk back recomputes the 2^KK candidates of the ONE group it passes
-// through, a lane each, and takes the first that equals the minimum, the reference's tie rule (src/kvq_gpu.cuh:101-102).
-// 4,096 rows, 5 multipliers, on a B200: %BEFORE% -> %AFTER% us (one warp per (row, multiplier, chain) with the costs in shared memory and every
-// lane walking its group's predecessors, then a second kernel for choice and packing).
+// x^2 is left out of the costs: it adds the same number to every state of a step.  A cost travels as a key, cost << 5 | j, whose j is part
+// of the state's own constant: the minimum over keys is the minimum cost with the first j on ties (the reference's rule,
+// src/kvq_gpu.cuh:101-102) and carries its back pointer, one byte per group and step.
+// Width of the keys: |f| = |c^2 - 2xc| <= F = C^2 + 4096 C with C = max |code| and |x| <= 2048, and f differs by at most D = 8192 C between
+// two states; any state is reached from any other in three steps, so the costs of a step spread over at most 3 D.  They are
+// brought back to one of them every four steps: |cost| <= 3 D + 4 F < 2^26 for C <= 1400, and a key fits 32 bits.  Profiles with larger codes
+// take 64-bit keys (the same code, no bringing back).
+// 4,096 rows, 5 multipliers, on a B200: 1,335 us (one warp per (row, multiplier, chain), costs in shared memory, every lane walking its
+// group's predecessors; a second kernel for choice and packing) -> 448 (minima kept instead of back pointers, candidates recomputed on
+// the way back: 76 instructions a step) -> 321 (55 a step; issue slots 77 % busy, integer ALU 65 %, the
+// multiply pipe 53 %).
 constexpr int TB_NM = 16;                                // multipliers at most (the blob's limit)
 struct TbRowSmem {
-  int hist[4][64 * 32];                                  // M_t[u] of each chain: [t][u]
-  short code[256]; float red[8]; uint8_t fld[256];
+  uint8_t bp[4][64 * 32];                                // back pointers of each chain: [t][u], the low five bits
+  short code[256]; float red[8]; int cmax[4]; uint8_t fld[256];
   struct Mult { uint8_t st[256]; float err[8]; } mult[1];  // one per multiplier: its states and its error sums
-  static size_t bytes(int nm) { return sizeof(TbRowSmem) + (nm - 1) * sizeof(Mult); }      // five multipliers: six blocks (24 warps) per SM
+  static size_t bytes(int nm) { return sizeof(TbRowSmem) + (nm - 1) * sizeof(Mult); }
 };
 struct TbP { const uint8_t* blob; int nm; const float* x; const int* grp; const int* pos; int rows; float* y; uint8_t* pay; int pay_stride; uint32_t* side; };
 
+__device__ __forceinline__ int tb_addmin(int a, int b, int c) { return __viaddmin_s32(a, b, c); }
+__device__ __forceinline__ long long tb_addmin(long long a, long long b, long long c) { return min(a + b, c); }
+
 // States of the best path of this warp's chain for the scaled values xa (steps 0-31, a lane each) and xb (steps 32-63): returned
-// as (state of step lane, state of step lane + 32).
-template <int KK> __device__ __forceinline__ int2 tb_search(int* hist, const short* code, int xa, int xb, int lane) {
-  constexpr int KQ = 1 << KK, SH = 8 - KK, UU = 1 << SH, NQ = KK == 5 ? 1 : 4;
+// as (state of step lane, state of step lane + 32).  K = int or long long, the type of the keys.
+template <int KK, class K> __device__ __forceinline__ int2 tb_search(uint8_t* bp, const short* code, int xa, int xb, int lane) {
+  constexpr int SH = 8 - KK, UU = 1 << SH, NQ = KK == 5 ? 1 : 4;
+  constexpr bool NARROW = sizeof(K) == 4;
   const int umid = lane & ((1 << (SH - 1)) - 1), jhi = lane >> (SH - 1);
-  int m2c[8], c2[8], src[NQ];
+  K m2c[8], c2[8];
+  int src[NQ];
   #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    const int c = code[(jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1)];
-    m2c[e] = -2 * c; c2[e] = c * c;
+    const int p = (jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1), c = code[p];
+    m2c[e] = (K)(-2 * c) * 32; c2[e] = (K)c * c * 32 + (p >> SH);
   }
   #pragma unroll
   for (int q = 0; q < NQ; ++q) {                         // the lane that holds the minimum of group (new state >> KK)
@@ -73,69 +84,74 @@ template <int KK> __device__ __forceinline__ int2 tb_search(int* hist, const sho
   }
   const bool upper = (lane >> (SH - 1)) & 1;             // of a pair of lanes the upper one keeps the odd u
   const int my_u = (umid << 1) | (upper ? 1 : 0);
-  int keep = my_u == 0 ? 0 : 0x40000000;                 // M_0: only state 0 exists
-  auto costs = [&](int x, int (&t)[8], int (&m)[NQ]) {
+  // Only state 0 exists at first.  Every state is reachable after three steps, so the others have to stay behind by more than 6 F
+  // (5e7 for C = 1400) until then, and within the width of a key.
+  K keep = my_u == 0 ? (K)(-(1 << 25)) * 32 : (K)(NARROW ? (1 << 24) + (1 << 23) : 0x40000000) * 32;
+  uint8_t* mine = bp + (lane < UU ? my_u : 0);           // lanes below UU hold every u once (the jhi bits above the first are zero)
+  auto costs = [&](int x, K (&t)[8], K (&m)[NQ]) {
+    keep &= ~(K)31;
     #pragma unroll
     for (int q = 0; q < NQ; ++q) m[q] = __shfl_sync(0xffffffffu, keep, src[q]);
     #pragma unroll
     for (int e = 0; e < 8; ++e) t[e] = x * m2c[e] + c2[e];
   };
-  #pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    const int xs = half ? xb : xa;
-    #pragma unroll 4
-    for (int i = 0; i < 32; ++i) {
-      const int t = 32 * half + i;
-      if (lane < UU) hist[t * UU + my_u] = keep;         // lanes below UU hold every u once (jhi bits above the first are zero)
-      if (t == 63) break;
-      int ct[8], m[NQ];
-      costs(__shfl_sync(0xffffffffu, xs, i), ct, m);
-      int a = ct[0] + m[0], b = ct[1] + m[0];
-      #pragma unroll
-      for (int q = 1; q < 4; ++q) {
-        a = __viaddmin_s32(ct[2 * q], m[NQ == 1 ? 0 : q], a);
-        b = __viaddmin_s32(ct[2 * q + 1], m[NQ == 1 ? 0 : q], b);
-      }
-      const int other = __shfl_xor_sync(0xffffffffu, upper ? a : b, 1 << (SH - 1));
-      keep = min(upper ? b : a, other);
-      #pragma unroll
-      for (int k = SH; k < 5; ++k) keep = min(keep, __shfl_xor_sync(0xffffffffu, keep, 1 << k));
+  auto step = [&](int x, int t) {                        // the minima of step t + 1 from those of step t
+    K ct[8], m[NQ];
+    costs(x, ct, m);
+    K a = ct[0] + m[0], b = ct[1] + m[0];
+    #pragma unroll
+    for (int q = 1; q < 4; ++q) {
+      a = tb_addmin(ct[2 * q], m[NQ == 1 ? 0 : q], a);
+      b = tb_addmin(ct[2 * q + 1], m[NQ == 1 ? 0 : q], b);
     }
+    const K other = __shfl_xor_sync(0xffffffffu, upper ? a : b, 1 << (SH - 1));
+    keep = min(upper ? b : a, other);
+    #pragma unroll
+    for (int k = SH; k < 5; ++k) keep = min(keep, __shfl_xor_sync(0xffffffffu, keep, 1 << k));
+    if (lane < UU) mine[(t + 1) * UU] = (uint8_t)keep;
+  };
+  #pragma unroll 1
+  for (int t = 0; t < 60; t += 4) {
+    const int xs = t < 32 ? xa : xb;
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) step(__shfl_sync(0xffffffffu, xs, (t + i) & 31), t + i);
+    if (NARROW) keep -= __shfl_sync(0xffffffffu, keep, 0) & ~(K)31;
   }
+  #pragma unroll
+  for (int t = 60; t < 63; ++t) step(__shfl_sync(0xffffffffu, xb, t - 32), t);
   // best final state: smallest (cost, state)
-  int ct[8], m[NQ];
+  K ct[8], m[NQ];
   costs(__shfl_sync(0xffffffffu, xb, 31), ct, m);
-  int best = 0x7fffffff, bs = 0;
+  K best = 0; int bs = 0;
   #pragma unroll
   for (int e = 0; e < 8; ++e) {                          // a lane's states grow with jlo, then ulo
-    const int c = ct[e] + m[NQ == 1 ? 0 : e >> 1], p = (jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1);
-    if (c < best) { best = c; bs = p; }
+    const K c = (ct[e] + m[NQ == 1 ? 0 : e >> 1]) & ~(K)31;
+    if (e == 0 || c < best) { best = c; bs = (jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1); }
   }
-  const int all = __reduce_min_sync(0xffffffffu, best);
-  int st = (int)__reduce_min_sync(0xffffffffu, best == all ? (unsigned)bs : 0xffffffffu);
-  __syncwarp();                                          // the history is complete
+  #pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const K c = __shfl_xor_sync(0xffffffffu, best, o); const int b2 = __shfl_xor_sync(0xffffffffu, bs, o);
+    if (c < best || (c == best && b2 < bs)) { best = c; bs = b2; }
+  }
+  __syncwarp();                                          // the back pointers are complete
   int2 out = make_int2(0, 0);
+  int st = bs;
   #pragma unroll 1
   for (int half = 1; half >= 0; --half) {
-    int mine = 0;
-    #pragma unroll 1
+    int keep_st = 0;
+    #pragma unroll 8
     for (int i = 31; i >= 0; --i) {
-      const int t = 32 * half + i;
-      if (lane == i) mine = st;
-      if (t == 0) break;
-      const int u = st >> KK, p = ((lane << SH) | u) & 255, c = code[p];
-      const int x = __shfl_sync(0xffffffffu, i > 0 ? (half ? xb : xa) : xa, (i - 1) & 31);      // x of step t - 1
-      const int cost = hist[(t - 1) * UU + (p >> KK)] + c * (c - 2 * x);
-      const unsigned hit = __ballot_sync(0xffffffffu, lane < KQ && cost == hist[t * UU + u]);
-      st = ((__ffs(hit) - 1) << SH) | u;
+      if (lane == i) keep_st = st;
+      const int u = st >> KK;
+      st = ((bp[(32 * half + i) * UU + u] & 31) << SH) | u;      // (the row of step 0 is read but never used)
     }
-    if (half) out.y = mine; else out.x = mine;
+    if (half) out.y = keep_st; else out.x = keep_st;
   }
-  __syncwarp();                                          // the history may be overwritten
+  __syncwarp();                                          // they may be overwritten
   return out;
 }
 
-__global__ void __launch_bounds__(128, 6) tb_encode_kernel(TbP A) {
+__global__ void __launch_bounds__(128, 7) tb_encode_kernel(TbP A) {
   extern __shared__ __align__(16) unsigned char tbe_smem[];
   TbRowSmem& S = *reinterpret_cast<TbRowSmem*>(tbe_smem);
   const int row = blockIdx.x, c = threadIdx.x >> 5, lane = threadIdx.x & 31, d0 = 64 * c + lane, d1 = d0 + 32;     // this thread's two values
@@ -194,9 +210,13 @@ __global__ void __launch_bounds__(128, 6) tb_encode_kernel(TbP A) {
   } else {
     const unsigned to = tb_u32(b + P.off_t + 4u * (unsigned)P.tix);
     const float gain = tb_f32(b + to + 4);
-    for (int i = threadIdx.x; i < 256; i += 128) S.code[i] = (short)tb_u16(b + to + 12 + 2 * i);
+    int cm = 0;
+    for (int i = threadIdx.x; i < 256; i += 128) { const int v = (short)tb_u16(b + to + 12 + 2 * i); S.code[i] = (short)v; cm = max(cm, abs(v)); }
+    cm = __reduce_max_sync(0xffffffffu, cm);
+    if (lane == 0) S.cmax[c] = cm;
     float rms = __fsqrt_rn(__fdiv_rn(rowsum(__fmul_rn(ra, ra), __fmul_rn(rb, rb)), 256.f));     // its barriers also publish the codes
     if (rms == 0.f) rms = 1.f;
+    const bool narrow = max(max(S.cmax[0], S.cmax[1]), max(S.cmax[2], S.cmax[3])) <= 1400;
     auto scale = [&](int mi) { const float s = tb_f16r(__fmul_rn(rms, tb_f32(b + P.off_m + 4u * (unsigned)mi))); return s == 0.f ? 1.f : s; };
     auto value = [&](int st, float s) { return __fmul_rn(__fmul_rn(__fmul_rn((float)(int)S.code[st], 0.00390625f), gain), s); };
     #pragma unroll 1
@@ -205,9 +225,9 @@ __global__ void __launch_bounds__(128, 6) tb_encode_kernel(TbP A) {
       const int xa = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(ra, s), 256.f)), -2048.f), 2048.f);
       const int xb = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(rb, s), 256.f)), -2048.f), 2048.f);
       int2 st = make_int2(0, 0);
-      if (P.kk == 3) st = tb_search<3>(S.hist[c], S.code, xa, xb, lane);
-      else if (P.kk == 4) st = tb_search<4>(S.hist[c], S.code, xa, xb, lane);
-      else if (P.kk == 5) st = tb_search<5>(S.hist[c], S.code, xa, xb, lane);
+      if (P.kk == 3) st = narrow ? tb_search<3, int>(S.bp[c], S.code, xa, xb, lane) : tb_search<3, long long>(S.bp[c], S.code, xa, xb, lane);
+      else if (P.kk == 4) st = narrow ? tb_search<4, int>(S.bp[c], S.code, xa, xb, lane) : tb_search<4, long long>(S.bp[c], S.code, xa, xb, lane);
+      else if (P.kk == 5) st = narrow ? tb_search<5, int>(S.bp[c], S.code, xa, xb, lane) : tb_search<5, long long>(S.bp[c], S.code, xa, xb, lane);
       const float da = __fsub_rn(ra, value(st.x, s)), db = __fsub_rn(rb, value(st.y, s));
       runs(__fmul_rn(da, da), __fmul_rn(db, db), S.mult[mi].err);
       S.mult[mi].st[d0] = (uint8_t)st.x; S.mult[mi].st[d1] = (uint8_t)st.y;
