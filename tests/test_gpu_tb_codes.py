@@ -40,3 +40,38 @@ def test_encoder_key_widths(oracle, top):
     got = pay.cpu().numpy().view(np.uint32).reshape(n, 41)
     assert np.array_equal(got[:, :40], want["pay"]) and not got[:, 40].any()      # what a row does not use is zero
     assert np.array_equal(side.cpu().numpy().view(np.uint32), want["side"])
+
+
+@pytest.mark.parametrize("top,ctx,M,splits,stride", [
+    (1100, 1000, 1, 3, 160), (1100, 1000, 2, 1, 164),               # many tiles per warp, rows that are not 16-byte aligned
+    (1100, 40, 1, 37, 160), (1100, 15, 1, 1, 176),                  # splits of one or two tokens, a single ragged tile
+    (2048, 200, 1, 2, 160), (2500, 200, 1, 2, 160),                 # the last table the tile path takes, the first it does not
+])
+def test_attention_tiles(oracle, top, ctx, M, splits, stride):
+    """Attention over packed rows against the exact oracle over the oracle's unpacked rows; every code width for keys and values."""
+    from yasakani_b200 import kvx
+    blob = _with_largest_code(make_blob(), top)
+    prof, kvh, nh, n = kvx.TrellisProfile(blob), 4, 32, ctx + M
+    max_ctx = (n + 63) // 64 * 64
+    rng = np.random.default_rng(top + ctx)
+    x = np.zeros((2, kvh, max_ctx, 256), np.float32)
+    x[:, :, :n] = rng.standard_normal((2, kvh, n, 256))
+    grp = np.array([[10, 8, 0, 15], [3, 9, 5, 31]], np.int32)       # 3 / 4 / 5 bits and flat records, ranks 0 - 2
+    rows_pos = np.tile(np.arange(max_ctx, dtype=np.int32), kvh)
+    dev, rows = [], []
+    for i in range(2):
+        gr = np.repeat(grp[i], max_ctx).astype(np.int32)
+        _, pay, side = kvx.tb_encode(prof, *(torch.from_numpy(a).cuda() for a in (x[i].reshape(-1, 256), gr, rows_pos)), pay_stride=stride)
+        p40 = np.ascontiguousarray(pay.cpu().numpy().view(np.uint32).reshape(-1, stride // 4)[:, :40])
+        rows.append(oracle.tb_unpack(blob, gr, rows_pos, p40, side.cpu().numpy().view(np.uint32), x[i].reshape(-1, 256)).reshape(kvh, max_ctx, 256))
+        dev += [pay.view(kvh, max_ctx, stride), side.view(kvh, max_ctx, 2)]
+    q = torch.from_numpy(rng.standard_normal((M, nh, 256)).astype(np.float32)).half()
+    pm = torch.full((M, splits, nh), float("nan"), device="cuda"); pl = pm.clone(); pacc = torch.full((M, splits, nh, 256), float("nan"), device="cuda")
+    kvx.launch_tb_attention(prof, q.cuda(), *dev, *(torch.from_numpy(a).cuda() for a in grp), M, torch.tensor([ctx], dtype=torch.int32, device="cuda"), splits,
+                            pm, pl, pacc, nh, *(torch.from_numpy(a).cuda() for a in x))
+    o16 = torch.empty((M, nh, 256), dtype=torch.float16, device="cuda")
+    kvx.launch_kv8_combine(pm, pl, pacc, splits, M, nh, o16, inverse_rotate=False)
+    want = oracle.rows_attention_exact(q.float().numpy(), rows[0], rows[1], ctx)
+    err = np.abs(o16.float().cpu().numpy() - want)
+    # two fp16 parts carry 22 bits of queries and weights; what remains is fp32 sums (2e-5 here) and the fp16 rounding of the row (2^-11)
+    assert (err <= 5e-5 + 2.0 ** -10 * np.abs(want)).all(), err.max()

@@ -24,6 +24,8 @@ namespace {
 
 constexpr int KV8_HD = 256;
 constexpr int KV8_WARPS = 8;
+constexpr int KV8_MS = 260;                               // words of a merge entry
+static_assert(KV8_WARPS == 8, "one group of eight lanes holds a head's weights");
 constexpr float KV8_LOG2E = 1.4426950408889634f, KV8_LN2 = 0.6931471805599453f;
 constexpr uint32_t C64 = 0x64646464u;                      // high bytes of the fp16 pattern 0x64xx = 1024 + xx
 constexpr float KV8_OFF = 1152.f;                          // 1024 + 128: a byte b is read as 1152 + b
@@ -42,10 +44,11 @@ __device__ __forceinline__ uint4 ldg16(const void* p) { return __ldcs(reinterpre
 template <int DT>
 __global__ void __launch_bounds__(KV8_WARPS * 32, 1) kv8_decode_kernel(const Kv8P P) {
   extern __shared__ __align__(16) uint8_t smem[];
-  // [16 k-steps][32 lanes] uint2 Q fragments | q sums [4][8] | merge area [warps][8 heads][258]
+  // [16 k-steps][32 lanes] uint2 Q fragments | q sums [4][8] | weights | merge area [warps][8 heads][260]
   uint2* s_q = reinterpret_cast<uint2*>(smem);
   float* s_bias = reinterpret_cast<float*>(smem + 16 * 32 * 8);
-  float* s_merge = s_bias + 32;
+  float* s_wgt = s_bias + 32;                              // [8 heads][warps]
+  float* s_merge = s_wgt + 64;
   const yskn_kv8_attn_args& A = P.a;
   const int split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z, G = P.g;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
@@ -171,33 +174,40 @@ __global__ void __launch_bounds__(KV8_WARPS * 32, 1) kv8_decode_kernel(const Kv8
     l[0] += __shfl_xor_sync(0xffffffffu, l[0], o); l[1] += __shfl_xor_sync(0xffffffffu, l[1], o);
     zs[0] += __shfl_xor_sync(0xffffffffu, zs[0], o); zs[1] += __shfl_xor_sync(0xffffffffu, zs[1], o);
   }
+  // Merge entry of a (warp, head): m, l, -, -, then channel d at slot (d & 31) * 8 + d / 32: the lanes of a store (channels 32g + c, heads 2j)
+  // fall into 32 different banks (channels in order gave 8-way conflicts).
   {
-    float* mine = s_merge + (size_t)warp * 8 * 258;
+    float* mine = s_merge + (size_t)warp * 8 * KV8_MS;
     #pragma unroll
     for (int mt = 0; mt < 16; ++mt) {
-      const int c = 32 * g + 2 * mt;
-      mine[(2 * j) * 258 + 2 + c] = acc[mt][0] - KV8_OFF * zs[0]; mine[(2 * j + 1) * 258 + 2 + c] = acc[mt][1] - KV8_OFF * zs[1];
-      mine[(2 * j) * 258 + 2 + c + 1] = acc[mt][2] - KV8_OFF * zs[0]; mine[(2 * j + 1) * 258 + 2 + c + 1] = acc[mt][3] - KV8_OFF * zs[1];
+      const int c = 4 + 16 * mt + g;                       // channel 32g + 2mt; the next one is 8 further on
+      mine[(2 * j) * KV8_MS + c] = acc[mt][0] - KV8_OFF * zs[0]; mine[(2 * j + 1) * KV8_MS + c] = acc[mt][1] - KV8_OFF * zs[1];
+      mine[(2 * j) * KV8_MS + c + 8] = acc[mt][2] - KV8_OFF * zs[0]; mine[(2 * j + 1) * KV8_MS + c + 8] = acc[mt][3] - KV8_OFF * zs[1];
     }
-    if (g == 0) { mine[(2 * j) * 258] = m[0]; mine[(2 * j) * 258 + 1] = l[0]; mine[(2 * j + 1) * 258] = m[1]; mine[(2 * j + 1) * 258 + 1] = l[1]; }
+    if (g == 0) { mine[(2 * j) * KV8_MS] = m[0]; mine[(2 * j) * KV8_MS + 1] = l[0]; mine[(2 * j + 1) * KV8_MS] = m[1]; mine[(2 * j + 1) * KV8_MS + 1] = l[1]; }
   }
   __syncthreads();
   // ---- merge the warps and store the split's partial (m in the natural-log domain, as the reference's partials)
-  for (int e = threadIdx.x; e < G * KV8_HD; e += KV8_WARPS * 32) {
-    const int hh = e / KV8_HD, d = e % KV8_HD;
-    float M2 = -1e30f;
+  if (threadIdx.x < 8 * KV8_WARPS) {                       // the warps' weights, once per head
+    const int hh = threadIdx.x / KV8_WARPS, w = threadIdx.x % KV8_WARPS;
+    float M2 = -1e30f, L2 = 0.f;
     #pragma unroll
-    for (int w = 0; w < KV8_WARPS; ++w) M2 = fmaxf(M2, s_merge[((size_t)w * 8 + hh) * 258]);
-    float L2 = 0.f, o = 0.f;
+    for (int k = 0; k < KV8_WARPS; ++k) M2 = fmaxf(M2, s_merge[((size_t)k * 8 + hh) * KV8_MS]);
+    const float mw = s_merge[((size_t)w * 8 + hh) * KV8_MS], f = mw > -1e29f ? ex2(mw - M2) : 0.f;
+    s_wgt[hh * KV8_WARPS + w] = f;
+    L2 = f * s_merge[((size_t)w * 8 + hh) * KV8_MS + 1];
     #pragma unroll
-    for (int w = 0; w < KV8_WARPS; ++w) {
-      const float* src = s_merge + ((size_t)w * 8 + hh) * 258;
-      const float sc = src[0] > -1e29f ? ex2(src[0] - M2) : 0.f;
-      L2 += sc * src[1]; o += sc * src[2 + d];
-    }
+    for (int o = 1; o < KV8_WARPS; o <<= 1) L2 += __shfl_xor_sync(0xffffffffu, L2, o);
     const size_t pidx = ((size_t)r * A.splits + split) * A.nh + kvh * G + hh;
-    if (d == 0) { A.pm[pidx] = M2 > -1e29f ? M2 * KV8_LN2 : -1e30f; A.pl[pidx] = L2; }
-    A.pacc[pidx * KV8_HD + d] = o;
+    if (w == 0 && hh < G) { A.pm[pidx] = M2 > -1e29f ? M2 * KV8_LN2 : -1e30f; A.pl[pidx] = L2; }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < G * KV8_HD; e += KV8_WARPS * 32) {
+    const int hh = e / KV8_HD, i = e % KV8_HD, d = (i & 7) * 32 + (i >> 3);
+    float o = 0.f;
+    #pragma unroll
+    for (int w = 0; w < KV8_WARPS; ++w) o += s_wgt[hh * KV8_WARPS + w] * s_merge[((size_t)w * 8 + hh) * KV8_MS + 4 + i];
+    A.pacc[(((size_t)r * A.splits + split) * A.nh + kvh * G + hh) * KV8_HD + d] = o;
   }
 }
 
@@ -341,7 +351,7 @@ int launch_kv8_attention(const yskn_kv8_attn_args& a, int act_dtype, cudaStream_
     KV4_REJECT("yskn_kv8_attention: bad shape (kvh %d, nh %d, M %d, splits %d, max_ctx %d): at most 8 query heads per kv-head, max_ctx a multiple of 64",
                a.kvh, a.nh, a.M, a.splits, a.max_ctx);
   if (((uintptr_t)a.k8 | (uintptr_t)a.v8) & 15) KV4_REJECT("yskn_kv8_attention: k8 and v8 must be 16-byte aligned");
-  const size_t smem = 16 * 32 * 8 + 32 * 4 + (size_t)KV8_WARPS * 8 * 258 * 4;
+  const size_t smem = 16 * 32 * 8 + 32 * 4 + 64 * 4 + (size_t)KV8_WARPS * 8 * KV8_MS * 4;
   Kv8P P{a, a.nh / a.kvh};
   const dim3 grid(a.splits, a.kvh, a.M);
   if (act_dtype == YSKN_KV4_BF16) {

@@ -321,232 +321,385 @@ __global__ void __launch_bounds__(256) tb_unpack_kernel(TbDecP A) {
 // ---------------------------------------------------------------------------------------------------------------------
 // Decode attention straight over packed rows: every key and value row is unpacked inside the kernel by tb_unpack_kernel's
 // rule and consumed at once; nothing unpacked is written to memory.  The counterpart of the reference's attention over packed
-// rows (launch_q35_atxpk, src/q35_atxpk3.cuh / q35_atxpk4.cuh) for passes of a few rows, on CUDA cores.  Row r at *d_pos + r
-// sees keys 0 .. *d_pos + r; grid (splits, kvh, M); a warp takes every eighth run of 32 keys of the split.  Online softmax in
-// the exp2 domain, one rescale per 32 keys.  Partials in the layout of yskn_kv8_attention.
-constexpr int TBA_WARPS = 8;
+// rows (launch_q35_atxpk, src/q35_atxpk3.cuh / q35_atxpk4.cuh) for passes of a few rows.  Row r at *d_pos + r sees keys
+// 0 .. *d_pos + r; grid (splits, kvh, M).  Partials in the layout of yskn_kv8_attention.
+//
+// A packed token is 264 bytes for its key and value together (4 bits), but 512 table look-ups: shared-memory wavefronts and issue
+// slots bound this kernel, not HBM.  So
+//   * the code table is replicated per lane (256 x 32 words, 32 KB for keys and 32 KB for values, at addresses that are a multiple of their
+//     size): a look-up is one funnel shift, one AND-OR that yields the address, one conflict-free load; the words carry the code as
+//     an fp16 in both halves, so two of them become an operand register by one byte permute.  Codes are integers up to 2,048 in
+//     size, exact in fp16 (a table with larger ones takes the row path below); the gain and the row's scale stay outside in fp32;
+//   * products run on mma.sync m16n8k16, tokens x heads for the scores, channels x heads for the values.  The contraction order
+//     of the scores is free, so lane (g, j) reads chain j of tokens g and g + 8, and for the values half a chain of four tokens: every
+//     window offset is a compile-time constant per code width;
+//   * queries and weights enter as sums of two fp16 numbers (two MMAs), which keeps the fp32 accuracy of a scalar loop;
+//   * the row terms of the unpack rule leave the loops: q.x = s * gain / 256 * sum_d q_d code_d + c0 (q.U0) + c1 (q.U1) + q.mu, and
+//     O = sum_t p_t s_t code_t + (sum p_t c0_t) U0 + (sum p_t c1_t) U1 + (sum p_t) mu.
+// Rows that the profile leaves unpacked (positions below the guard, at most 255; a group without packed rows) take the row path, a warp
+// per token in fp32.  30,011 tokens of 4 kv-heads on a B200: 152 us (32 keys per warp step in scalar fp32, tables in shared memory with
+// bank conflicts) -> 31 us, of which 14 are set-up, merge and the launch.
+constexpr int TBA_WARPS = 12;                                        // 3 per scheduler at up to 168 registers
 struct TbAttnP { yskn_tb_attn_args a; int G; };
-struct TbTab { float cg[256], mu[256], u0[256], u1[256]; };          // one group's code table (x gain / 256) and row terms
+constexpr uint32_t TBA_TAB = 32768;                                  // bytes of a replicated table, and the alignment of its shared-memory address
+struct TbAttnSm {                                                    // in front of the tables
+  uint4 qf[16][32];                                                  // Q as B fragments: {hi b0, hi b1, lo b0, lo b1} of k-step s, lane
+  float q[8][260];                                                   // q * qscale * log2(e) in fp32 (row path, row terms)
+  float cg[2][256];                                                  // codes of the key and of the value group (row path: x gain)
+  float term[2][3][256];                                             // row terms U0, U1, mu of both groups, channel d at tba_slot(d)
+  float kq[3][8];                                                    // q.U0, q.U1, q.mu of the key group
+  int big;                                                           // some code does not fit fp16 exactly
+};
+constexpr int TBA_MS = 260;                                          // merge entry of a (warp, head): m, l, -, -, then channel d at tba_slot(d)
+constexpr uint32_t TBA_MERGE = TBA_WARPS * 8 * TBA_MS * 4;           // merge area: takes the tables' place after the loop
+constexpr uint32_t TBA_SMEM = sizeof(TbAttnSm) + TBA_TAB + (TBA_MERGE > 2 * TBA_TAB ? TBA_MERGE : 2 * TBA_TAB);     // one TBA_TAB for the alignment
 
-// per-group constants of the unpack rule
-struct TbRule { int packed_ok, mode, kb, guard, m, has_mu; };
-__device__ __forceinline__ TbRule tb_stage_group(const uint8_t* b, int g, TbTab& T) {   // all threads of the CTA
-  const TbGroup P = tb_group(b, g);
-  TbRule R{P.ok && P.mode <= 1, P.mode, P.mode == 1 ? 4 : P.kk, P.guard, P.m, P.has_mu};
-  const unsigned to = tb_u32(b + P.off_t + 4u * (unsigned)P.tix);
-  const float gain = P.mode == 0 ? tb_f32(b + to + 4) : 1.f;
-  const uint8_t* mup = b + P.go + 8;
-  const uint8_t* Up = mup + (P.has_mu ? 512 : 0);
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    T.cg[i] = !R.packed_ok ? 0.f : (P.mode == 1 ? (float)(i - 8) : __fmul_rn(__fmul_rn((float)(int)(short)tb_u16(b + to + 12 + 2 * i), 0.00390625f), gain));
-    T.mu[i] = R.packed_ok && P.has_mu ? __half2float(__ushort_as_half((unsigned short)tb_u16(mup + 2 * i))) : 0.f;
-    T.u0[i] = R.packed_ok && P.m > 0 ? __half2float(__ushort_as_half((unsigned short)tb_u16(Up + 2 * i))) : 0.f;
-    T.u1[i] = R.packed_ok && P.m > 1 ? __half2float(__ushort_as_half((unsigned short)tb_u16(Up + 2 * (256 + i)))) : 0.f;
-  }
-  return R;
+struct TbRule { int packed_ok, mode, kb, guard, m, has_mu; float gain; };     // per-group constants of the unpack rule
+
+__device__ __forceinline__ uint32_t tba_lds(uint32_t a) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ void tba_sts(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ uint32_t tba_pack(float lo, float hi) { uint32_t d; asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo)); return d; }
+__device__ __forceinline__ void tba_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// ---- 32 keys per warp step.  Scores: a lane takes one key and walks its 256 fields (the window offsets
-// are then the same in every lane and known at compile time per code width); the row terms of the unpack rule leave the inner
-// loop: q.x = s * sum_d q_d cg[v_d] + c0 (q.U0) + c1 (q.U1) + q.mu, with the three dot products formed once per CTA.  Values: a
-// lane takes eight channels of every key, O = sum_t p_t s_t cg[v_td] + (sum p_t c0_t) U0 + (sum p_t c1_t) U1 + (sum p_t) mu.
-// The unpacked values themselves are those of tb_unpack_kernel; only the order of the fp32 sums differs (tolerance parity).
-constexpr int TBA_PW = 41;                                           // staged payload row: 40 words + 1 (conflict-free lane stride)
-struct TbWarpSm { unsigned kp[2][32 * TBA_PW]; unsigned vp[2][32 * TBA_PW]; float pw[32][8]; int vplain[32]; };   // two staging buffers: the next 32 keys arrive while these are used
-__device__ __forceinline__ void tb_cp4(unsigned* dst, const unsigned* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+__device__ __forceinline__ uint32_t tba_transpose(uint32_t a) { uint32_t d; asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a)); return d; }
+
+// Where channel d sits in a merge entry and in the row terms: the eight lanes g of an access (channels 32g + c) fall into eight banks, the
+// four lanes j of a merge store (heads 2j, 520 words apart) into four groups of eight.  (Channels in order: 8-way conflicts, 10 us.)
+__device__ __forceinline__ int tba_slot(int d) { return (d & 31) * 8 + (d >> 5); }
+
+// The window of value i of a run of fields that starts at word 0 (`prev` = the word in front, zero at the start of a chain), at bits
+// 7 .. 14: the byte offset of its table row.
+template <int KB, int NWORD> __device__ __forceinline__ uint32_t tba_window(const uint32_t (&w)[NWORD], uint32_t prev, int i) {
+  const int lo = KB * (i + 1) - 8;                                   // first bit of the window in the MSB-first stream; negative: in `prev`
+  const int k = lo >> 5, o = lo & 31;                                // floor
+  const uint32_t hi = k < 0 ? prev : w[k < 0 ? 0 : k];
+  if (o > 24) return __funnelshift_r(w[k + 1 < NWORD ? k + 1 : NWORD - 1], hi, 49 - o);
+  return o <= 17 ? hi >> (17 - o) : hi << (o - 17);
 }
 
-template <int KB, bool FLAT>
-__device__ __forceinline__ void tb_scores32(const unsigned* row, const float* cg, const float (*q)[8], float (&dot)[8]) {
-  #pragma unroll 1
-  for (int c = 0; c < 4; ++c) {                                      // chains of 64 fields: same bit offsets, 2*KB words further
-    const unsigned* wr = row + 2 * KB * c;
+// Words of a run of fields: NWORD consecutive 32-bit words.  v16: rows are 16-byte aligned (then so are the runs of 4-bit codes).
+template <int NWORD> __device__ __forceinline__ void tba_words(const uint32_t* p, bool v16, uint32_t (&w)[NWORD]) {
+  if (NWORD % 4 == 0 && v16) {
     #pragma unroll
-    for (int i = 0; i < 64; ++i) {
-      constexpr int dummy = 0; (void)dummy;
-      const int endb = KB * (i + 1), lo = FLAT ? endb - 4 : (endb - 8 > 0 ? endb - 8 : 0), len = endb - lo;
-      const unsigned v = __funnelshift_l(wr[(lo >> 5) + 1], wr[lo >> 5], lo & 31) >> (32 - len);
-      const float cv = cg[v];
-      const float4 qa = *reinterpret_cast<const float4*>(&q[64 * c + i][0]), qb = *reinterpret_cast<const float4*>(&q[64 * c + i][4]);
-      dot[0] = fmaf(cv, qa.x, dot[0]); dot[1] = fmaf(cv, qa.y, dot[1]); dot[2] = fmaf(cv, qa.z, dot[2]); dot[3] = fmaf(cv, qa.w, dot[3]);
-      dot[4] = fmaf(cv, qb.x, dot[4]); dot[5] = fmaf(cv, qb.y, dot[5]); dot[6] = fmaf(cv, qb.z, dot[6]); dot[7] = fmaf(cv, qb.w, dot[7]);
+    for (int k = 0; k < NWORD / 4; ++k) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + k);
+      w[(4 * k) % NWORD] = u.x; w[(4 * k + 1) % NWORD] = u.y; w[(4 * k + 2) % NWORD] = u.z; w[(4 * k + 3) % NWORD] = u.w;
     }
+  } else {
+    #pragma unroll
+    for (int k = 0; k < NWORD; ++k) w[k] = __ldg(p + k);
   }
 }
 
-template <int KB, bool FLAT>
-__device__ __forceinline__ void tb_values32(const TbWarpSm& W, const unsigned* vp, const float* cg, const float* plain, int lane, int nk, float (&acc)[8][8]) {
-  int wi[8], sh[8], ln[8];
+// Raw scores of a tile's 16 tokens: rows g and g + 8 of the tile, heads 2j and 2j + 1 (c[0] c[1] | c[2] c[3]).
+template <int KB>
+__device__ __forceinline__ void tba_scores(const uint32_t* ra, const uint32_t* rb, bool v16, uint32_t tab, const uint4* qf, float (&s)[4]) {
+  uint32_t wa[2 * KB], wb[2 * KB];
+  tba_words(ra, v16, wa); tba_words(rb, v16, wb);
+  float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
   #pragma unroll
-  for (int w = 0; w < 8; ++w) {
-    const int d = 32 * w + lane, endb = KB * (d + 1), first = KB * (d & ~63), lo = FLAT ? endb - 4 : max(endb - 8, first);
-    wi[w] = lo >> 5; sh[w] = lo & 31; ln[w] = 32 - (endb - lo);
-  }
-  #pragma unroll 2
-  for (int j = 0; j < nk; ++j) {
-    const float4 pa = *reinterpret_cast<const float4*>(&W.pw[j][0]), pb = *reinterpret_cast<const float4*>(&W.pw[j][4]);
-    const float pg[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
-    const unsigned* row = vp + j * TBA_PW;
-    const bool pl = W.vplain[j] != 0;                                // warp-uniform: a row the profile leaves unpacked
+  for (int k = 0; k < 16; ++k) {                                     // k-step: values 4k .. 4k+3 of the chain
+    uint32_t a[4], b[4];
     #pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      float x;
-      if (pl) x = plain ? __ldg(plain + (size_t)j * 256 + 32 * w + lane) : 0.f;
-      else x = cg[__funnelshift_l(row[wi[w] + 1], row[wi[w]], sh[w]) >> ln[w]];
-      #pragma unroll
-      for (int g = 0; g < 8; ++g) acc[g][w] = fmaf(pg[g], x, acc[g][w]);
+    for (int e = 0; e < 4; ++e) {
+      a[e] = tba_lds((tba_window<KB>(wa, 0u, 4 * k + e) & 0x7F80u) | tab);
+      b[e] = tba_lds((tba_window<KB>(wb, 0u, 4 * k + e) & 0x7F80u) | tab);
     }
+    const uint4 q = qf[k * 32];
+    const uint32_t a0 = __byte_perm(a[0], a[1], 0x5410), a1 = __byte_perm(b[0], b[1], 0x5410), a2 = __byte_perm(a[2], a[3], 0x5410),
+                   a3 = __byte_perm(b[2], b[3], 0x5410);
+    tba_mma(hi, a0, a1, a2, a3, q.x, q.y);
+    tba_mma(lo, a0, a1, a2, a3, q.z, q.w);
   }
+  #pragma unroll
+  for (int e = 0; e < 4; ++e) s[e] = hi[e] + lo[e];
+}
+
+// O^T += V^T P^T over a tile: this lane's 32 channels (half a chain) of tokens 2j, 2j+1, 2j+8, 2j+9 (rows r[0..3]).
+template <int KB>
+__device__ __forceinline__ void tba_values(const uint32_t* const (&r)[4], bool odd, bool v16, uint32_t tab, const uint32_t (&ph)[2], const uint32_t (&pl)[2],
+                                           float (&acc)[16][4]) {
+  uint32_t w[4][KB], prev[4];
+  #pragma unroll
+  for (int t = 0; t < 4; ++t) { tba_words(r[t], v16, w[t]); prev[t] = odd ? __ldg(r[t] - 1) : 0u; }
+  #pragma unroll
+  for (int mt = 0; mt < 16; ++mt) {                                  // m-tile: channels 2 mt and 2 mt + 1 of the run as rows g and g + 8
+    uint32_t x[2][4];
+    #pragma unroll
+    for (int c = 0; c < 2; ++c)
+      #pragma unroll
+      for (int t = 0; t < 4; ++t) x[c][t] = tba_lds((tba_window<KB>(w[t], prev[t], 2 * mt + c) & 0x7F80u) | tab);
+    const uint32_t a0 = __byte_perm(x[0][0], x[0][1], 0x5410), a1 = __byte_perm(x[1][0], x[1][1], 0x5410), a2 = __byte_perm(x[0][2], x[0][3], 0x5410),
+                   a3 = __byte_perm(x[1][2], x[1][3], 0x5410);
+    tba_mma(acc[mt], a0, a1, a2, a3, ph[0], ph[1]);
+    tba_mma(acc[mt], a0, a1, a2, a3, pl[0], pl[1]);
+  }
+}
+
+// Value d of a row on its own (tb_unpack_kernel's rule), as its code.
+__device__ __forceinline__ float tba_value(const uint32_t* row, const float* cg, int kb, int d) {
+  const int endb = kb * (d + 1), lo = max(endb - 8, kb * (d & ~63));
+  const uint32_t w0 = __ldg(row + (lo >> 5)), w1 = (lo & 31) + (endb - lo) > 32 ? __ldg(row + (lo >> 5) + 1) : 0u;
+  return cg[__funnelshift_l(w1, w0, lo & 31) >> (32 - (endb - lo))];
 }
 
 template <int DT>
-__global__ void __launch_bounds__(TBA_WARPS * 32) tb_attn32_kernel(TbAttnP P) {
+__global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
   extern __shared__ __align__(16) unsigned char tba_smem[];
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(tba_smem);
+  const uint32_t TK = (base + (uint32_t)sizeof(TbAttnSm) + TBA_TAB - 1) & ~(TBA_TAB - 1), TV = TK + TBA_TAB;
   const yskn_tb_attn_args& A = P.a;
-  const int G = P.G, split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  TbTab* tk = reinterpret_cast<TbTab*>(tba_smem); TbTab* tv = tk + 1;
-  float (*q)[8] = reinterpret_cast<float (*)[8]>(tv + 1);            // [256][8]: q * qscale * log2(e), heads past G are zero
-  float (*kq)[8] = q + 256;                                           // [3][8]: q.U0, q.U1, q.mu of the key group
-  TbWarpSm* Wall = reinterpret_cast<TbWarpSm*>(kq + 4);
-  TbWarpSm& W = Wall[warp];
-  float* mbuf = reinterpret_cast<float*>(Wall);                       // [warp][8][258], takes the staging area's place after the loop
-  const TbRule rk = tb_stage_group(A.blob, __ldg(A.grp_k + kvh), *tk), rv = tb_stage_group(A.blob, __ldg(A.grp_v + kvh), *tv);
+  const int G = P.G, split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+  TbAttnSm& S = *reinterpret_cast<TbAttnSm*>(tba_smem);
+  float* mbuf = reinterpret_cast<float*>(tba_smem + (TK - base));          // [warp][8][258]
+  asm volatile("griddepcontrol.wait;" ::: "memory");                 // programmatic dependent launch, both directions
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const float qs = A.qscale * 1.4426950408889634f;
-  for (int e = threadIdx.x; e < 256 * 8; e += TBA_WARPS * 32) {
-    const int d = e >> 3, g = e & 7;
-    q[d][g] = g < G ? act_load<DT>(A.q16, ((size_t)r * A.nh + kvh * G + g) * 256 + d) * qs : 0.f;
-  }
-  __syncthreads();
-  if (threadIdx.x < 24) {
-    const int which = threadIdx.x >> 3, g = threadIdx.x & 7;
-    const float* vec = which == 0 ? tk->u0 : (which == 1 ? tk->u1 : tk->mu);
-    float a = 0.f;
-    for (int d = 0; d < 256; ++d) a = fmaf(q[d][g], vec[d], a);
-    kq[which][g] = a;
-  }
-  __syncthreads();
   const int pos = __ldg(A.d_pos) + r, len = max(0, min(pos + 1, A.max_ctx));
   const int per = (len + (int)gridDim.x - 1) / (int)gridDim.x, t0 = min(len, split * per), t1 = min(len, t0 + per);
   const size_t row0 = (size_t)kvh * A.max_ctx;
-  const int psw = A.pay_stride / 4, nwk = 8 * rk.kb, nwv = 8 * rv.kb;
-  float acc[8][8], m[8], l[8], a0[8], a1[8], am[8];
-  #pragma unroll
-  for (int g = 0; g < 8; ++g) {
-    m[g] = -1e30f; l[g] = a0[g] = a1[g] = am[g] = 0.f;
-    #pragma unroll
-    for (int w = 0; w < 8; ++w) acc[g][w] = 0.f;
-  }
-  // payload rows of 32 keys into staging buffer `b`, asynchronously (4-byte copies: the padded row stride is not a multiple of 16)
-  auto stage = [&](int tc, int b) {
-    const int nk = min(32, t1 - tc);
-    const unsigned* kw = reinterpret_cast<const unsigned*>(A.k_pay) + (row0 + tc) * psw;
-    const unsigned* vw = reinterpret_cast<const unsigned*>(A.v_pay) + (row0 + tc) * psw;
-    for (int idx = lane; idx < nk * 40; idx += 32) {
-      const int rr = idx / 40, i = idx - 40 * rr;
-      if (i < nwk) tb_cp4(&W.kp[b][rr * TBA_PW + i], kw + (size_t)rr * psw + i); else W.kp[b][rr * TBA_PW + i] = 0u;
-      if (i < nwv) tb_cp4(&W.vp[b][rr * TBA_PW + i], vw + (size_t)rr * psw + i); else W.vp[b][rr * TBA_PW + i] = 0u;
-    }
-    if (lane < nk) { W.kp[b][lane * TBA_PW + 40] = 0u; W.vp[b][lane * TBA_PW + 40] = 0u; }
+  const int psw = A.pay_stride / 4;
+  const uint32_t *kpay = reinterpret_cast<const uint32_t*>(A.k_pay) + row0 * psw, *vpay = reinterpret_cast<const uint32_t*>(A.v_pay) + row0 * psw;
+  auto prefetch = [&](int tc) {                                      // the rows of a tile into L2: a row per lane, keys 0-15, values 16-31
+    const int t = tc + (lane & 15);
+    if (t >= t1) return;
+    const uint32_t* p = (lane < 16 ? kpay : vpay) + (size_t)t * psw;
+    asm volatile("prefetch.global.L2 [%0];\n prefetch.global.L2 [%1];" ::"l"(p), "l"(p + 31));
+    if (!(lane & 15)) asm volatile("prefetch.global.L2 [%0];" ::"l"((lane < 16 ? A.k_side : A.v_side) + 2 * (row0 + t)));
   };
-  int buf = 0;
-  if (t0 + 32 * warp < t1) stage(t0 + 32 * warp, 0);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int tc = t0 + 32 * warp; tc < t1; tc += 32 * TBA_WARPS, buf ^= 1) {
-    const int nk = min(32, t1 - tc);
-    __syncwarp();                                                    // every lane is done with the other buffer
-    if (tc + 32 * TBA_WARPS < t1) stage(tc + 32 * TBA_WARPS, buf ^ 1);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");           // this step's rows have landed (this lane's copies)
-    __syncwarp();                                                    // ... and every other lane's
-    const int t = tc + lane;
-    const bool live = lane < nk, kpk = rk.packed_ok && t >= rk.guard, vpk = rv.packed_ok && t >= rv.guard;
-    float sk = 0.f, c0k = 0.f, c1k = 0.f, sv = 1.f, c0v = 0.f, c1v = 0.f;
-    if (live && kpk) {
-      sk = __uint_as_float(__ldg(A.k_side + 2 * (row0 + t))); const unsigned pc = __ldg(A.k_side + 2 * (row0 + t) + 1);
-      c0k = rk.m > 0 ? __half2float(__ushort_as_half((unsigned short)(pc & 0xffffu))) : 0.f;
-      c1k = rk.m > 1 ? __half2float(__ushort_as_half((unsigned short)(pc >> 16))) : 0.f;
+  prefetch(t0 + 16 * warp);
+  // ---- set-up.  The profile is a chain of five dependent reads (header, group offset, record, table offset, table); both groups walk it side by
+  //      side and everything at its end is requested at once (one group after the other, entry by entry, took 20 us).
+  constexpr int NQ = (256 * 8 + TBA_WARPS * 32 - 1) / (TBA_WARPS * 32);
+  float qv[NQ];                                                      // on their way while the chain is walked
+  #pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    const int e = threadIdx.x + k * TBA_WARPS * 32, h = e >> 8, d = e & 255;
+    qv[k] = h < G ? act_load<DT>(A.q16, ((size_t)r * A.nh + kvh * G + h) * 256 + d) : 0.f;
+  }
+  if (threadIdx.x == 0) S.big = 0;
+  TbRule rk, rv;
+  {
+    const TbGroup Pg[2] = {tb_group(A.blob, __ldg(A.grp_k + kvh)), tb_group(A.blob, __ldg(A.grp_v + kvh))};
+    unsigned to[2];
+    #pragma unroll
+    for (int w = 0; w < 2; ++w) to[w] = tb_u32(A.blob + Pg[w].off_t + 4u * (unsigned)Pg[w].tix);
+    float gain[2];
+    #pragma unroll
+    for (int w = 0; w < 2; ++w) gain[w] = tb_f32(A.blob + to[w] + 4);
+    const int i = threadIdx.x;
+    float x[2][4];                                                   // code, U0, U1, mu of entry / channel i
+    #pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const TbGroup& R = Pg[w];
+      const uint8_t* mup = A.blob + R.go + 8;
+      const uint8_t* Up = mup + (R.has_mu ? 512 : 0);
+      const bool pk = R.ok && R.mode <= 1 && i < 256;
+      auto f16at = [&](const uint8_t* p) { return __half2float(__ushort_as_half((unsigned short)tb_u16(p))); };
+      // a flat code of 4 bits is the low half of the 8-bit window: flat groups use the same windows with a periodic table
+      x[w][0] = !pk ? 0.f : R.mode == 1 ? (float)((i & 15) - 8) : (float)(short)tb_u16(A.blob + to[w] + 12 + 2 * i);
+      x[w][1] = pk && R.m > 0 ? f16at(Up + 2 * i) : 0.f;
+      x[w][2] = pk && R.m > 1 ? f16at(Up + 512 + 2 * i) : 0.f;
+      x[w][3] = pk && R.has_mu ? f16at(mup + 2 * i) : 0.f;
     }
-    if (live && vpk) {
-      sv = __uint_as_float(__ldg(A.v_side + 2 * (row0 + t))); const unsigned pc = __ldg(A.v_side + 2 * (row0 + t) + 1);
-      c0v = rv.m > 0 ? __half2float(__ushort_as_half((unsigned short)(pc & 0xffffu))) : 0.f;
-      c1v = rv.m > 1 ? __half2float(__ushort_as_half((unsigned short)(pc >> 16))) : 0.f;
+    #pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      const int e = threadIdx.x + k * TBA_WARPS * 32;
+      if (e < 256 * 8) S.q[e >> 8][e & 255] = qv[k] * qs;
     }
-    float dot[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const unsigned* myrow = W.kp[buf] + lane * TBA_PW;
-    if (rk.mode == 1) tb_scores32<4, true>(myrow, tk->cg, q, dot);
-    else if (rk.kb == 3) tb_scores32<3, false>(myrow, tk->cg, q, dot);
-    else if (rk.kb == 4) tb_scores32<4, false>(myrow, tk->cg, q, dot);
-    else tb_scores32<5, false>(myrow, tk->cg, q, dot);
+    __syncthreads();                                                 // S.big is cleared
+    if (i < 256)
+      #pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        S.cg[w][i] = x[w][0];
+        #pragma unroll
+        for (int k = 0; k < 3; ++k) S.term[w][k][tba_slot(i)] = x[w][1 + k];
+        if (fabsf(x[w][0]) > 2048.f) S.big = 1;
+      }
+    rk = TbRule{Pg[0].ok && Pg[0].mode <= 1, Pg[0].mode, Pg[0].mode == 1 ? 4 : Pg[0].kk, Pg[0].guard, Pg[0].m, Pg[0].has_mu, Pg[0].mode == 0 ? gain[0] * 0.00390625f : 1.f};
+    rv = TbRule{Pg[1].ok && Pg[1].mode <= 1, Pg[1].mode, Pg[1].mode == 1 ? 4 : Pg[1].kk, Pg[1].guard, Pg[1].m, Pg[1].has_mu, Pg[1].mode == 0 ? gain[1] * 0.00390625f : 1.f};
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 2 * 256 * 8; e += TBA_WARPS * 32) {  // thread = (table, state, four lanes)
+    const int w = e >> 11, st = (e >> 3) & 255, l4 = (e & 7) * 4;
+    const uint32_t h = __half_as_ushort(__float2half_rn(S.cg[w][st])), v = h | (h << 16);
+    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"((w ? TV : TK) + st * 128 + l4 * 4), "r"(v) : "memory");
+  }
+  for (int i = warp; i < 24; i += TBA_WARPS) {                       // q.U0, q.U1, q.mu of each head, a warp per product
+    const int which = i >> 3, h = i & 7;
+    float a = 0.f;
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) a = fmaf(S.q[h][32 * k + lane], S.term[0][which][tba_slot(32 * k + lane)], a);
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) S.kq[which][h] = a;
+  }
+  for (int e = threadIdx.x; e < 16 * 32; e += TBA_WARPS * 32) {      // k-slots (2j, 2j+1, 2j+8, 2j+9) of step s = channels 64j + 4s .. + 3
+    const int s = e >> 5, ln = e & 31, h = ln >> 2, c = 64 * (ln & 3) + 4 * s;
+    float v[4], hi[4];
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) { v[k] = S.q[h][c + k]; hi[k] = __half2float(__float2half_rn(v[k])); }
+    S.qf[s][ln] = make_uint4(tba_pack(hi[0], hi[1]), tba_pack(hi[2], hi[3]), tba_pack(v[0] - hi[0], v[1] - hi[1]), tba_pack(v[2] - hi[2], v[3] - hi[3]));
+  }
+  __syncthreads();
+  // tokens below tf take the row path: either side unpacked there, or codes that fp16 does not hold
+  const int tf = rk.packed_ok && rv.packed_ok && !S.big ? min(t1, max(t0, max(rk.guard, rv.guard))) : t1;
+  const bool v16 = !((A.pay_stride | (int)((uintptr_t)A.k_pay | (uintptr_t)A.v_pay)) & 15);
+  const uint4* qf = &S.qf[0][lane];
+  const uint32_t tabk = TK | (lane * 4), tabv = TV | (lane * 4);
+
+  float acc[16][4];                                                  // O^T: [m-tile][(channel 32g + 2 mt | + 1) x (head 2j | 2j + 1)]
+  #pragma unroll
+  for (int mt = 0; mt < 16; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
+  // heads 2j, 2j+1 (log2 domain); l and the sums of p, p c0, p c1 over packed values are this lane's share of the tokens
+  float m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f}, a0[2] = {0.f, 0.f}, a1[2] = {0.f, 0.f}, am[2] = {0.f, 0.f};
+  const float kq0[2] = {S.kq[0][2 * j], S.kq[0][2 * j + 1]}, kq1[2] = {S.kq[1][2 * j], S.kq[1][2 * j + 1]}, kqm[2] = {S.kq[2][2 * j], S.kq[2][2 * j + 1]};
+  auto side = [&](const uint32_t* sd, int t, int mm, float& s, float& c0, float& c1) {
+    s = __uint_as_float(__ldg(sd + 2 * (row0 + t)));
+    const uint32_t pc = __ldg(sd + 2 * (row0 + t) + 1);
+    c0 = mm > 0 ? __half2float(__ushort_as_half((unsigned short)(pc & 0xffffu))) : 0.f;
+    c1 = mm > 1 ? __half2float(__ushort_as_half((unsigned short)(pc >> 16))) : 0.f;
+  };
+  for (int tc = tf + 16 * warp; tc < t1; tc += 16 * TBA_WARPS) {
+    prefetch(tc + 16 * TBA_WARPS);
+    const bool live0 = tc + g < t1, live1 = tc + g + 8 < t1;
+    const int ta = min(tc + g, t1 - 1), tb = min(tc + g + 8, t1 - 1);  // tokens past the end repeat the last one with weight zero
+    float ks[2], kc0[2], kc1[2], vs[2], vc0[2], vc1[2];
+    side(A.k_side, ta, rk.m, ks[0], kc0[0], kc1[0]); side(A.k_side, tb, rk.m, ks[1], kc0[1], kc1[1]);
+    side(A.v_side, ta, rv.m, vs[0], vc0[0], vc1[0]); side(A.v_side, tb, rv.m, vs[1], vc0[1], vc1[1]);
+    float s[4];
+    {
+      const uint32_t *pa = kpay + (size_t)ta * psw + j * 2 * rk.kb, *pb = kpay + (size_t)tb * psw + j * 2 * rk.kb;
+      if (rk.kb == 4) tba_scores<4>(pa, pb, v16, tabk, qf, s);
+      else if (rk.kb == 5) tba_scores<5>(pa, pb, v16, tabk, qf, s);
+      else tba_scores<3>(pa, pb, v16, tabk, qf, s);
+    }
+    float p[2][2];                                                   // [row g | g + 8][head]
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float sa = fmaf(ks[0] * rk.gain, s[h], fmaf(kc0[0], kq0[h], fmaf(kc1[0], kq1[h], kqm[h])));
+      const float sb = fmaf(ks[1] * rk.gain, s[2 + h], fmaf(kc0[1], kq0[h], fmaf(kc1[1], kq1[h], kqm[h])));
+      p[0][h] = live0 ? sa : -INFINITY; p[1][h] = live1 ? sb : -INFINITY;
+    }
+    float x0 = fmaxf(p[0][0], p[1][0]), x1 = fmaxf(p[0][1], p[1][1]);
+    if (__any_sync(0xffffffffu, x0 > m[0] + 8.f || x1 > m[1] + 8.f)) {     // lazy rescale: the running max may lag by 2^8
+      #pragma unroll
+      for (int o = 4; o <= 16; o <<= 1) { x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, o)); x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o)); }
+      const float n0 = fmaxf(m[0], x0), n1 = fmaxf(m[1], x1), f0 = exp2f(m[0] - n0), f1 = exp2f(m[1] - n1);
+      m[0] = n0; m[1] = n1;
+      l[0] *= f0; a0[0] *= f0; a1[0] *= f0; am[0] *= f0; l[1] *= f1; a0[1] *= f1; a1[1] *= f1; am[1] *= f1;
+      #pragma unroll
+      for (int mt = 0; mt < 16; ++mt) { acc[mt][0] *= f0; acc[mt][1] *= f1; acc[mt][2] *= f0; acc[mt][3] *= f1; }
+    }
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      p[0][h] = exp2f(p[0][h] - m[h]); p[1][h] = exp2f(p[1][h] - m[h]);
+      l[h] += p[0][h] + p[1][h];
+      a0[h] = fmaf(p[0][h], vc0[0], fmaf(p[1][h], vc0[1], a0[h])); a1[h] = fmaf(p[0][h], vc1[0], fmaf(p[1][h], vc1[1], a1[h]));
+      am[h] += p[0][h] + p[1][h];
+    }
+    uint32_t ph[2], pl[2];                                           // weights x scale as two fp16 numbers, transposed into B registers
+    #pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float w0 = p[q][0] * vs[q] * rv.gain, w1 = p[q][1] * vs[q] * rv.gain;
+      const float h0 = __half2float(__float2half_rn(w0)), h1 = __half2float(__float2half_rn(w1));
+      ph[q] = tba_transpose(tba_pack(h0, h1)); pl[q] = tba_transpose(tba_pack(w0 - h0, w1 - h1));
+    }
+    const int tv[4] = {min(tc + 2 * j, t1 - 1), min(tc + 2 * j + 1, t1 - 1), min(tc + 2 * j + 8, t1 - 1), min(tc + 2 * j + 9, t1 - 1)};
+    const uint32_t* vr[4];
+    #pragma unroll
+    for (int q = 0; q < 4; ++q) vr[q] = vpay + (size_t)tv[q] * psw + g * rv.kb;
+    if (rv.kb == 4) tba_values<4>(vr, g & 1, v16, tabv, ph, pl, acc);
+    else if (rv.kb == 5) tba_values<5>(vr, g & 1, v16, tabv, ph, pl, acc);
+    else tba_values<3>(vr, g & 1, v16, tabv, ph, pl, acc);
+  }
+  // ---- this warp's (m, l, O) per head into the merge area (the tables' place); the row terms of the value group added
+  #pragma unroll
+  for (int o = 4; o <= 16; o <<= 1)
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      l[h] += __shfl_xor_sync(0xffffffffu, l[h], o); a0[h] += __shfl_xor_sync(0xffffffffu, a0[h], o);
+      a1[h] += __shfl_xor_sync(0xffffffffu, a1[h], o); am[h] += __shfl_xor_sync(0xffffffffu, am[h], o);
+    }
+  __syncthreads();
+  float* wb = mbuf + (size_t)warp * 8 * TBA_MS;
+  #pragma unroll
+  for (int mt = 0; mt < 16; ++mt)
+    #pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int h = e & 1, d = 32 * g + 2 * mt + (e >> 1);
+      wb[(2 * j + h) * TBA_MS + 4 + tba_slot(d)] = fmaf(a0[h], S.term[1][0][tba_slot(d)], fmaf(a1[h], S.term[1][1][tba_slot(d)], fmaf(am[h], S.term[1][2][tba_slot(d)], acc[mt][e])));
+    }
+  if (g == 0) {
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) { wb[(2 * j + h) * TBA_MS] = m[h]; wb[(2 * j + h) * TBA_MS + 1] = l[h]; }
+  }
+  __syncwarp();
+  // ---- the row path: a token per warp step, lane = channels 32 k + lane, fp32 throughout, straight into the warp's merge entry
+  for (int t = t0 + warp; t < tf; t += TBA_WARPS) {
+    const bool kpk = rk.packed_ok && t >= rk.guard, vpk = rv.packed_ok && t >= rv.guard;
+    float s0, c0, c1, x[8];
+    if (kpk) side(A.k_side, t, rk.m, s0, c0, c1);
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int d = 32 * k + lane;
+      x[k] = kpk ? tba_value(kpay + (size_t)t * psw, S.cg[0], rk.kb, d) * rk.gain * s0 : (A.k_plain ? __ldg(A.k_plain + (row0 + t) * 256 + d) : 0.f);
+    }
     float sc[8];
     #pragma unroll
-    for (int g = 0; g < 8; ++g) sc[g] = fmaf(sk, dot[g], fmaf(c0k, kq[0][g], fmaf(c1k, kq[1][g], kq[2][g])));
-    if (live && !kpk) {                                              // a key row the profile leaves unpacked: the plain row
+    for (int h = 0; h < 8; ++h) {
+      float a = 0.f;
       #pragma unroll
-      for (int g = 0; g < 8; ++g) sc[g] = 0.f;
-      if (A.k_plain) {
-        const float* pr = A.k_plain + (row0 + t) * 256;
-        for (int d = 0; d < 256; ++d) {
-          const float x = __ldg(pr + d);
-          #pragma unroll
-          for (int g = 0; g < 8; ++g) sc[g] = fmaf(q[d][g], x, sc[g]);
-        }
-      }
+      for (int k = 0; k < 8; ++k) a = fmaf(S.q[h][32 * k + lane], x[k], a);
+      #pragma unroll
+      for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      sc[h] = kpk ? a + fmaf(c0, S.kq[0][h], fmaf(c1, S.kq[1][h], S.kq[2][h])) : a;
     }
-    W.vplain[lane] = vpk ? 0 : 1;
+    if (vpk) side(A.v_side, t, rv.m, s0, c0, c1);
     #pragma unroll
-    for (int g = 0; g < 8; ++g) {
-      if (g >= G) { W.pw[lane][g] = 0.f; continue; }
-      float mx = live ? sc[g] : -1e30f;
-      #pragma unroll
-      for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float mn = fmaxf(m[g], mx), al = exp2f(m[g] - mn), p = live ? exp2f(sc[g] - mn) : 0.f;
-      float s0 = p, s1 = p * c0v, s2 = p * c1v, s3 = vpk ? p : 0.f;
-      #pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o); s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, o); s3 += __shfl_xor_sync(0xffffffffu, s3, o);
-      }
-      l[g] = fmaf(l[g], al, s0); a0[g] = fmaf(a0[g], al, s1); a1[g] = fmaf(a1[g], al, s2); am[g] = fmaf(am[g], al, s3); m[g] = mn;
-      #pragma unroll
-      for (int w = 0; w < 8; ++w) acc[g][w] *= al;
-      W.pw[lane][g] = p * sv;
+    for (int k = 0; k < 8; ++k) {
+      const int d = 32 * k + lane, i = tba_slot(d);
+      x[k] = vpk ? fmaf(c0, S.term[1][0][i], fmaf(c1, S.term[1][1][i], fmaf(tba_value(vpay + (size_t)t * psw, S.cg[1], rv.kb, d) * rv.gain, s0, S.term[1][2][i])))
+                 : (A.v_plain ? __ldg(A.v_plain + (row0 + t) * 256 + d) : 0.f);
     }
-    __syncwarp();
-    const float* vpl = A.v_plain ? A.v_plain + (row0 + tc) * 256 : nullptr;
-    if (rv.mode == 1) tb_values32<4, true>(W, W.vp[buf], tv->cg, vpl, lane, nk, acc);
-    else if (rv.kb == 3) tb_values32<3, false>(W, W.vp[buf], tv->cg, vpl, lane, nk, acc);
-    else if (rv.kb == 4) tb_values32<4, false>(W, W.vp[buf], tv->cg, vpl, lane, nk, acc);
-    else tb_values32<5, false>(W, W.vp[buf], tv->cg, vpl, lane, nk, acc);
+    #pragma unroll
+    for (int h = 0; h < 8; ++h) {
+      if (h >= G) break;
+      float* e = wb + h * TBA_MS;
+      const float mo = e[0], lo = e[1], mn = fmaxf(mo, sc[h]), f = exp2f(mo - mn), pw = exp2f(sc[h] - mn);
+      __syncwarp();
+      if (lane == 0) { e[0] = mn; e[1] = fmaf(lo, f, pw); }
+      #pragma unroll
+      for (int k = 0; k < 8; ++k) e[4 + tba_slot(32 * k + lane)] = fmaf(e[4 + tba_slot(32 * k + lane)], f, pw * x[k]);
+      __syncwarp();
+    }
   }
-  // ---- the row terms of the value group, then the merge of the warps (natural-log m, as the merge kernel expects)
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();                                                   // the staging area becomes the merge buffer
-  #pragma unroll
-  for (int g = 0; g < 8; ++g) {
-    if (g >= G) continue;
-    float* wb = mbuf + ((size_t)warp * 8 + g) * 258;
-    if (lane == 0) { wb[0] = m[g]; wb[1] = l[g]; }
+  // ---- the merge of the warps (natural-log m, as the merge kernel expects)
+  __syncthreads();
+  if (threadIdx.x < 8 * TBA_WARPS) {                                 // the warps' weights, and the row's m and l
+    const int h = threadIdx.x / TBA_WARPS, w = threadIdx.x % TBA_WARPS;
+    float M2 = -1e30f;
     #pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      const int d = 32 * w + lane;
-      wb[2 + d] = fmaf(a0[g], tv->u0[d], fmaf(a1[g], tv->u1[d], fmaf(am[g], tv->mu[d], acc[g][w])));
-    }
+    for (int k = 0; k < TBA_WARPS; ++k) M2 = fmaxf(M2, mbuf[((size_t)k * 8 + h) * TBA_MS]);
+    const float mw = mbuf[((size_t)w * 8 + h) * TBA_MS];
+    S.q[h][w] = mw > -1e29f ? exp2f(mw - M2) : 0.f;                  // the queries are done with
+    if (w == 0) S.q[h][TBA_WARPS] = M2;
   }
   __syncthreads();
   for (int e = threadIdx.x; e < G * 256; e += TBA_WARPS * 32) {
-    const int g = e >> 8, d = e & 255;
-    float M2 = -1e30f;
-    #pragma unroll
-    for (int w = 0; w < TBA_WARPS; ++w) M2 = fmaxf(M2, mbuf[((size_t)w * 8 + g) * 258]);
+    const int h = e >> 8, i = e & 255, d = (i & 7) * 32 + (i >> 3);  // entries in their order: tba_slot(d) = i
     float L2 = 0.f, o = 0.f;
     #pragma unroll
     for (int w = 0; w < TBA_WARPS; ++w) {
-      const float* wb = mbuf + ((size_t)w * 8 + g) * 258;
-      const float f = wb[0] > -1e29f ? exp2f(wb[0] - M2) : 0.f;
-      L2 += f * wb[1]; o += f * wb[2 + d];
+      const float* src = mbuf + ((size_t)w * 8 + h) * TBA_MS;
+      const float f = S.q[h][w];
+      L2 += f * src[1]; o += f * src[4 + i];
     }
-    const size_t pidx = ((size_t)r * A.splits + split) * A.nh + kvh * G + g;
-    if (d == 0) { A.pm[pidx] = M2 > -1e29f ? M2 * 0.6931471805599453f : -1e30f; A.pl[pidx] = L2; }
+    const size_t pidx = ((size_t)r * A.splits + split) * A.nh + kvh * G + h;
+    const float M2 = S.q[h][TBA_WARPS];
+    if (i == 0) { A.pm[pidx] = M2 > -1e29f ? M2 * 0.6931471805599453f : -1e30f; A.pl[pidx] = L2; }
     A.pacc[pidx * 256 + d] = o;
   }
 }
@@ -608,20 +761,20 @@ int launch_tb_attention(const yskn_tb_attn_args& a, int act_dtype, cudaStream_t 
   if (a.kvh <= 0 || a.nh <= 0 || a.nh % a.kvh || a.nh / a.kvh > 8 || a.M <= 0 || a.M > 65535 || a.kvh > 65535 || a.splits <= 0 || a.max_ctx <= 0)
     KV4_REJECT("yskn_tb_attention: bad shape (kvh %d, nh %d, M %d, splits %d, max_ctx %d): at most 8 query heads per kv-head", a.kvh, a.nh, a.M, a.splits, a.max_ctx);
   if (a.pay_stride < 160 || a.pay_stride % 4 || (((uintptr_t)a.k_pay | (uintptr_t)a.v_pay) & 3)) KV4_REJECT("yskn_tb_attention: bad payload stride %d or alignment", a.pay_stride);
-  const size_t stage = sizeof(TbWarpSm) * TBA_WARPS, merge = (size_t)TBA_WARPS * 8 * 258 * 4;
-  const size_t smem = 2 * sizeof(TbTab) + (256 + 4) * 8 * 4 + (stage > merge ? stage : merge);
+  const int smem = (int)TBA_SMEM;
   TbAttnP P{a, a.nh / a.kvh};
   const dim3 grid(a.splits, a.kvh, a.M);
   if (act_dtype == YSKN_KV4_BF16) {
     static std::atomic<unsigned long long> attr{0};
-    if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(tb_attn32_kernel<YSKN_KV4_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    tb_attn32_kernel<YSKN_KV4_BF16><<<grid, TBA_WARPS * 32, smem, st>>>(P);
-  } else if (act_dtype == YSKN_KV4_F16) {
+    if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(tb_attn_kernel<YSKN_KV4_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return launch_pdl("tb_attn_kernel", tb_attn_kernel<YSKN_KV4_BF16>, grid, TBA_WARPS * 32, smem, st, P);
+  }
+  if (act_dtype == YSKN_KV4_F16) {
     static std::atomic<unsigned long long> attr{0};
-    if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(tb_attn32_kernel<YSKN_KV4_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    tb_attn32_kernel<YSKN_KV4_F16><<<grid, TBA_WARPS * 32, smem, st>>>(P);
-  } else KV4_REJECT("yskn_tb_attention: q16 is bf16 or fp16 (act_dtype %d)", act_dtype);
-  return launch_status("tb_attn32_kernel");
+    if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(tb_attn_kernel<YSKN_KV4_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return launch_pdl("tb_attn_kernel", tb_attn_kernel<YSKN_KV4_F16>, grid, TBA_WARPS * 32, smem, st, P);
+  }
+  KV4_REJECT("yskn_tb_attention: q16 is bf16 or fp16 (act_dtype %d)", act_dtype);
 }
 
 }  // namespace kv4
