@@ -287,18 +287,26 @@ __device__ __forceinline__ uint32_t tc_pack(float lo, float hi) { uint32_t d; as
 __device__ __forceinline__ uint32_t tc_hadd2(uint32_t a, uint32_t b) { uint32_t d; asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 __device__ __forceinline__ uint32_t tc_hfma2(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
 __device__ __forceinline__ uint32_t tc_hmul2(uint32_t a, uint32_t b) { uint32_t d; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
-__device__ __forceinline__ void tc_nibs(uint32_t w, uint32_t (&n)[4]) {
-  const uint32_t w8 = w >> 8;
-  n[0] = tc_hadd2((w & 0x000F000Fu) | 0x64006400u, 0xE400E400u); n[1] = tc_hadd2((w & 0x00F000F0u) | 0x54005400u, 0xD400D400u);
-  n[2] = tc_hadd2((w8 & 0x000F000Fu) | 0x64006400u, 0xE400E400u); n[3] = tc_hadd2((w8 & 0x00F000F0u) | 0x54005400u, 0xD400D400u);
+// (a & m) | c as ONE logic op: it takes a single immediate, so the masks and offsets live in registers the compiler cannot fold.
+__device__ __forceinline__ uint32_t tc_and_or(uint32_t a, uint32_t m, uint32_t c) { uint32_t d; asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(m), "r"(c)); return d; }
+struct TcNib { uint32_t m0, m1, e, o; };
+__device__ __forceinline__ TcNib tc_nib_consts() {
+  TcNib k;
+  asm volatile("mov.u32 %0, 0x000F000F;\n mov.u32 %1, 0x00F000F0;\n mov.u32 %2, 0x64006400;\n mov.u32 %3, 0x54005400;" : "=r"(k.m0), "=r"(k.m1), "=r"(k.e), "=r"(k.o));
+  return k;
 }
-// eight consecutive fp16 (v.x = (e0, e1) .. v.w = (e6, e7)) <-> registers o[x] = (e_x, e_{x+4})
+__device__ __forceinline__ void tc_nibs(uint32_t w, uint32_t (&n)[4], const TcNib& c) {
+  const uint32_t w8 = w >> 8;
+  n[0] = tc_hadd2(tc_and_or(w, c.m0, c.e), 0xE400E400u); n[1] = tc_hadd2(tc_and_or(w, c.m1, c.o), 0xD400D400u);
+  n[2] = tc_hadd2(tc_and_or(w8, c.m0, c.e), 0xE400E400u); n[3] = tc_hadd2(tc_and_or(w8, c.m1, c.o), 0xD400D400u);
+}
+// eight consecutive fp16 (v.x = (e0, e1) .. v.w = (e6, e7)) -> registers o[x] = (e_x, e_{x+4}).  The converting form over the int4 cache keeps
+// every 16-byte operand chunk in this order (channels 0 4 1 5 2 6 3 7): what the nibble reads yield is stored without a byte permute.  The order
+// of the contraction is free as long as Q follows it (tc_stage_q), and the columns of O are put back by the epilogue (tc_col).
 __device__ __forceinline__ void tc_row_to_pairs(const uint4& v, uint32_t (&o)[4]) {
   o[0] = __byte_perm(v.x, v.z, 0x5410); o[1] = __byte_perm(v.x, v.z, 0x7632); o[2] = __byte_perm(v.y, v.w, 0x5410); o[3] = __byte_perm(v.y, v.w, 0x7632);
 }
-__device__ __forceinline__ uint4 tc_pairs_to_row(const uint32_t (&r)[4]) {
-  return make_uint4(__byte_perm(r[0], r[1], 0x5410), __byte_perm(r[2], r[3], 0x5410), __byte_perm(r[0], r[1], 0x7632), __byte_perm(r[2], r[3], 0x7632));
-}
+__host__ __device__ constexpr int tc_col(int c) { return (c & ~7) | ((c & 3) << 1) | ((c >> 2) & 1); }     // operand column that holds channel c
 // Global loads as ordered asm statements: the compiler keeps them where they are written, ahead of the arithmetic.
 __device__ __forceinline__ uint32_t tc_ldg32(const void* p) { uint32_t v; asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
 __device__ __forceinline__ uint32_t tc_ldg16(const void* p) { unsigned short v; asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p)); return v; }
@@ -309,12 +317,13 @@ __device__ __forceinline__ void tc_prefetch_l2(const void* p) { asm volatile("pr
 __device__ __forceinline__ void tc_sts128(uint32_t a, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-// bf16 queries of one CTA (128 operand rows = (token, head) pairs) as fp16 rows in the swizzled Q blocks; rows without a
-// query are zero.  Thread t of nt; eight 16-byte loads are in flight per thread before the first one is converted.
-template <int HD>
-__device__ __forceinline__ void tc_stage_q_bf16(uint32_t sq, int q_block, const uint16_t* q16, int tok0, int G, int TOK, int M, int nh, int head0,
-                                                int t, int nt) {
+// Queries of one CTA (128 operand rows = (token, head) pairs) as fp16 rows in the swizzled Q blocks; rows without a query are zero.
+// PAIRS: chunks in the order of tc_row_to_pairs.  Thread t of nt; eight 16-byte loads are in flight per thread before the first one is converted.
+template <int HD, bool PAIRS>
+__device__ __forceinline__ void tc_stage_q(uint32_t sq, int q_block, const uint16_t* q16, bool bf16, int tok0, int G, int TOK, int M, int nh, int head0,
+                                           int t, int nt) {
   constexpr int NW = HD / 8, B = 8;
+  #pragma unroll 1
   for (int base = t; base < 128 * NW; base += B * nt) {
     uint4 u[B];
     #pragma unroll
@@ -327,10 +336,12 @@ __device__ __forceinline__ void tc_stage_q_bf16(uint32_t sq, int q_block, const 
     for (int b = 0; b < B; ++b) {
       const int it = base + b * nt, row = it / NW, w = it % NW;
       if (it >= 128 * NW) break;
-      const uint32_t uu[4] = {u[b].x, u[b].y, u[b].z, u[b].w};
-      uint32_t o4[4];
-      #pragma unroll
-      for (int e = 0; e < 4; ++e) o4[e] = tc_pack(__uint_as_float(uu[e] << 16), __uint_as_float(uu[e] & 0xffff0000u));
+      uint32_t o4[4] = {u[b].x, u[b].y, u[b].z, u[b].w};
+      if (bf16) {
+        #pragma unroll
+        for (int e = 0; e < 4; ++e) o4[e] = tc_pack(__uint_as_float(o4[e] << 16), __uint_as_float(o4[e] & 0xffff0000u));
+      }
+      if (PAIRS) tc_row_to_pairs(make_uint4(o4[0], o4[1], o4[2], o4[3]), o4);
       tc_sts128(sq + (w >> 3) * q_block + row * 128 + (((w & 7) ^ (row & 7)) << 4), make_uint4(o4[0], o4[1], o4[2], o4[3]));
     }
   }
@@ -400,6 +411,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   using L = TcLay<HD>;
   constexpr bool FUSED = FORM == 1 || FORM == 2, I8 = FORM == 2;
   const bool act_bf16 = FUSED ? P.bf16 != 0 : FORM == 3;              // a compile-time constant in the workspace forms
+  constexpr bool STAGED_Q = FORM != 0;
   static_assert(!I8 || HD == 256, "INT8 rows have 256 channels");
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sb = s_u32(smem);
@@ -419,7 +431,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     for (int i = 0; i < L::NK; ++i) { bar_init(b_kfull + 8 * i, FUSED ? 2 * TC_KW : 1); bar_init(b_kempty + 8 * i, 1); }
     for (int i = 0; i < L::NV; ++i) { bar_init(b_vfull + 8 * i, FUSED ? 2 * TC_VW : 1); bar_init(b_vempty + 8 * i, 1); }
     for (int i = 0; i < 2; ++i) { bar_init(b_sready + 8 * i, 1); bar_init(b_pready + 8 * i, 2 * TC_SW); bar_init(b_pvdone + 8 * i, 1); }
-    bar_init(b_q, act_bf16 ? (FUSED ? 2 * TC_KW : 2 * TC_SW) : 1);   // bf16 queries are staged by warps, not by TMA
+    bar_init(b_q, STAGED_Q ? 2 * TC_SW : 1);                         // queries that are converted or reordered are staged by the softmax warps
     *s_abort = 0;
     for (int i = 0; i < 128; ++i) reinterpret_cast<volatile uint32_t*>(smem + L::OFF_XCH + 2 * 2 * 128 * 4)[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -461,13 +473,13 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     // ======================================================================= TMA producer (one per CTA)
     // Q once, then two rings: K halves are free again as soon as their S MMAs are done, V halves only after P.V.
     // Every copy reports to the leader's "full" barrier; the leader posts the byte count of both CTAs' parts.
-    if (lane == 0 && n > 0 && !(FUSED && act_bf16)) {
-      if (!act_bf16) {                                                 // bf16 queries are converted and written by warps instead
+    if (lane == 0 && n > 0) {
+      if (!STAGED_Q) {
         if (rank == 0) bar_expect_tx(b_q, 2 * L::KBLK * G * TOK * 128);
         for (int kb = 0; kb < L::KBLK; ++kb) tma_load_4d_pair(sb + L::OFF_Q + kb * L::Q_BLOCK, &mapQ, 64 * kb, 0, kvh, tok0, lead_q);
       }
       int kit = 0; bool ok = true;
-      for (int i = 0; i < n && ok && !FUSED; ++i) {
+      for (int i = 0; i < n && ok; ++i) {
         const int j = j0 + i;
         for (int half = 0; half < (i >= nbulk ? 2 : 1) && ok; ++half, ++kit) {      // Kd; edge tiles: then Ks
           const int st = kit % L::NK;
@@ -485,7 +497,6 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       }
     }
   };
-  // the converting forms have no K / V copies to issue: the warp that requested Q goes on to issue the MMAs
   constexpr int CONV0 = TC_SW + 1;
   auto role_mma = [&]() {
     // ======================================================================= MMA issuer (one thread of the leader CTA)
@@ -622,10 +633,6 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       // ------------------------------------------------------------------- K role
       if constexpr (I8) {
         constexpr int NKI = ((TC_BN / 2) * 16 + NKT - 1) / NKT;      // 64 keys x 16 chunks over the K threads
-        if (P.bf16) {
-          tc_stage_q_bf16<HD>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, tok0, G, TOK, P.M, P.nh, kvh * G, ct, NKT);
-          publish(lead_q);
-        }
         // The items of all tiles form one stream (NKI per tile); two are in flight ahead of the one being converted.  Rolled
         // loops: the kernel's code has to stay inside the instruction cache.
         auto k8_load = [&](int q, I8In& I) {                         // q-th item of this thread's stream
@@ -670,43 +677,48 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       const int npl = NWD - nrw;                                     // plain word columns
       const uint32_t* kq32 = reinterpret_cast<const uint32_t*>(P.kv.kq);
       auto k_addr = [&](uint32_t sk, int w, int k) { return sk + (w >> 3) * L::K_BLOCK + k * 128 + (((w & 7) ^ (k & 7)) << 4); };
-      // Plain items: (word column, octet of keys); item x of a tile = column nrw + x % npl, keys 8 (x / npl) .. +7, so that
-      // consecutive lanes take consecutive columns of one octet.  A thread's items of all tiles form one stream (NPI per tile).
-      constexpr int NPI = (NWD * 8 + NKT - 1) / NKT;
-      const int np1 = npl > 0 ? npl : 1, nplain = npl * 8;
+      const TcNib nk = tc_nib_consts();
+      // Work of a tile in warp items.  Plain: 32 (word column, octet of keys) pairs, x = col + npl * octet, so that consecutive lanes take
+      // consecutive columns; warp w takes items w, w + 4.  Rotary (up to four word pairs per key): nrp pairs x 32 / nrp keys of one group, nrp items
+      // per group; for a 64-channel rotary part six plain and eight rotary items share out as 2 + 1, 2 + 1, 1 + 3, 1 + 3.
+      const int wq = ct >> 5, np1 = npl > 0 ? npl : 1, nplain = npl * 8;
       struct PlainIn { uint32_t w[8]; uint4 s, z; };
-      auto plain_load = [&](int q, PlainIn& I) {                     // q-th item of the stream
-        const int x = ct + NKT * (q % NPI), tk = (j0 + q / NPI) * TC_BN + (TC_BN / 2) * (int)rank;
-        if (q < n * NPI && x < nplain && tk < P.max_ctx) {
-          const int col = nrw + x % np1, key = 8 * (x / np1);
-          const uint32_t* src = kq32 + (row0 + tk + key) * (HD / 8) + col;
+      int pg[2], ps[2], pd[2];                                       // a lane's two items: word offset, scale offset, stage offset
+      #pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int x = 32 * (wq + TC_KW * u) + lane, col = nrw + x % np1, key = 8 * (x / np1);
+        pg[u] = x < nplain ? key * (HD / 8) + col : -1; ps[u] = (key >> 5) * HD + 8 * col;
+        pd[u] = (col >> 3) * L::K_BLOCK + key * 128 + ((col & 7) << 4);
+      }
+      const int pn = 32 * wq >= nplain ? 0 : (32 * (wq + TC_KW) < nplain ? 2 : 1);       // items of this warp
+      static_assert(NWD * 8 <= 32 * TC_KW * 2, "two plain items per warp cover a half tile");
+      auto tile_key = [&](int i) { return (j0 + i) * TC_BN + (TC_BN / 2) * (int)rank; };   // first key of this CTA's half of K tile i
+      auto plain_load = [&](int i, int u, PlainIn& I) {
+        const int tk = tile_key(i), off = u ? pg[1] : pg[0];
+        if (i < n && off >= 0 && tk < P.max_ctx) {
+          const uint32_t* src = kq32 + (row0 + tk) * (HD / 8) + off;
           #pragma unroll
           for (int e = 0; e < 8; ++e) I.w[e] = tc_ldg32(src + e * (HD / 8));
-          const size_t gb = (grp0 + (tk + key) / 32) * HD + 8 * col;
+          const size_t gb = (grp0 + tk / 32) * HD + (u ? ps[1] : ps[0]);
           I.s = tc_ldg128(P.kv.kscale + gb); I.z = tc_ldg128(P.kv.kzero + gb);
         }
       };
       auto plain_store = [&](int u, uint32_t sk, const PlainIn& I) {
-        const int x = ct + NKT * u;
-        if (x >= nplain) return;
-        const int col = nrw + x % np1, key = 8 * (x / np1);
+        if ((u ? pg[1] : pg[0]) < 0) return;
+        const uint32_t base = sk + (u ? pd[1] : pd[0]);                // keys are a multiple of 8 further on: key e swizzles by e
         uint32_t sc[4], zz[4];
         tc_row_to_pairs(I.s, sc); tc_row_to_pairs(I.z, zz);
-        const uint32_t base = sk + (col >> 3) * L::K_BLOCK + key * 128;      // key is a multiple of 8: (key + e) & 7 = e
-        const uint32_t cx = (uint32_t)(col & 7);
         #pragma unroll
         for (int h = 0; h < 8; h += 4) {                               // four words converted, then four stores: independent chains interleave
           uint4 out[4];
           #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            uint32_t nb[4], r[4];
-            tc_nibs(I.w[h + e], nb);
-            #pragma unroll
-            for (int x2 = 0; x2 < 4; ++x2) r[x2] = tc_hfma2(nb[x2], sc[x2], zz[x2]);
-            out[e] = tc_pairs_to_row(r);
+            uint32_t nb[4];
+            tc_nibs(I.w[h + e], nb, nk);
+            out[e] = make_uint4(tc_hfma2(nb[0], sc[0], zz[0]), tc_hfma2(nb[1], sc[1], zz[1]), tc_hfma2(nb[2], sc[2], zz[2]), tc_hfma2(nb[3], sc[3], zz[3]));
           }
           #pragma unroll
-          for (int e = 0; e < 4; ++e) tc_sts128(base + (h + e) * 128 + ((cx ^ (uint32_t)(h + e)) << 4), out[e]);
+          for (int e = 0; e < 4; ++e) tc_sts128((base ^ (uint32_t)((h + e) << 4)) + (h + e) * 128, out[e]);
         }
       };
       struct RotIn { uint32_t wa, wb; uint4 sa, za, sb, zb; uint4 r[4]; };   // shadow items keep their two fp16 rows in sa, za
@@ -735,7 +747,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           if (t >= end) { a[0] = a[1] = a[2] = a[3] = 0u; b[0] = b[1] = b[2] = b[3] = 0u; }
         } else {
           uint32_t na[4], nb[4], sa[4], za[4], sb4[4], zb[4];
-          tc_nibs(R.wa, na); tc_nibs(R.wb, nb);
+          tc_nibs(R.wa, na, nk); tc_nibs(R.wb, nb, nk);
           tc_row_to_pairs(R.sa, sa); tc_row_to_pairs(R.za, za); tc_row_to_pairs(R.sb, sb4); tc_row_to_pairs(R.zb, zb);
           #pragma unroll
           for (int x = 0; x < 4; ++x) { a[x] = tc_hfma2(na[x], sa[x], za[x]); b[x] = tc_hfma2(nb[x], sb4[x], zb[x]); }
@@ -751,24 +763,18 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           lo[x] = tc_hfma2(a[x], C[x], tc_hmul2(b[x], S[x]) ^ 0x80008000u);      // a cos - b sin
           hi[x] = tc_hfma2(a[x], S[x], tc_hmul2(b[x], C[x]));                    // a sin + b cos
         }
-        tc_sts128(k_addr(sk, p, k), tc_pairs_to_row(lo));
-        tc_sts128(k_addr(sk, q, k), tc_pairs_to_row(hi));
+        tc_sts128(k_addr(sk, p, k), make_uint4(lo[0], lo[1], lo[2], lo[3]));
+        tc_sts128(k_addr(sk, q, k), make_uint4(hi[0], hi[1], hi[2], hi[3]));
       };
       auto zero_k = [&](uint32_t sk) {                               // a half tile past max_ctx: nothing to read
         for (int it = ct; it < (TC_BN / 2) * NWD; it += NKT) tc_sts128(k_addr(sk, it % NWD, it / NWD), make_uint4(0u, 0u, 0u, 0u));
       };
-      if (P.bf16) {
-        // bf16 activations: this CTA's query rows (token, head) as fp16 operand rows; rows without a query are zero
-        tc_stage_q_bf16<HD>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, tok0, G, TOK, P.M, P.nh, kvh * G, ct, NKT);
-        publish(lead_q);
-      }
-      // Rotary items in the compact mapping (rotary width of at most 64 channels): a thread owns one word pair (p, p + nrp) of
-      // one 32-key group and up to two keys of it, so the group's scale / zero chunks are loaded once per tile; its items of
-      // all tiles form one stream (RCI per tile).  Wider rotary parts take the items one after the other (rot_load / rot_store).
+      // Rotary items in the compact mapping (rotary width of at most 64 channels): a warp stays in one 32-key group, so the group's scale / zero
+      // chunks are loaded once per tile.  Wider rotary parts take the items one after the other (rot_load / rot_store).
       const bool compact = nrp >= 1 && nrp <= 4;
-      constexpr int RCI = 2;                                         // keys per thread: 32 / tpc <= 2 with 128 K threads
-      const int tpc = compact ? NKT / (2 * nrp) : 1;                 // threads per (pair, group); keys c and c + tpc of the group
-      const int cp = ct & (nrp - 1), cg = compact ? (ct >> lp) & 1 : 0, cc = compact ? ct / (2 * nrp) : 0;
+      const int rlight = nrp == 4 ? 1 : nrp >> 1;                    // rotary items of warps 0 and 1 (group = warp & 1); 2 and 3 take the rest
+      const int r0 = wq < 2 ? 0 : rlight, rn = !compact ? 0 : (wq < 2 ? rlight : nrp - rlight);
+      const int cp = lane & (nrp - 1), cg = wq & 1, cstep = compact ? 32 >> lp : 0, cc = compact ? cstep * r0 + (lane >> lp) : 0;
       struct RotS { uint4 sa, za, sb, zb; };                         // the group's scale / zero chunks of the two words
       struct RotI { uint32_t wa, wb; uint4 r[4]; };                  // one key: the two words and the 8 (cos, sin) pairs
       auto rots_load = [&](int tk0, RotS& R) {
@@ -776,10 +782,10 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         R.sa = tc_ldg128(P.kv.kscale + gb + 8 * cp); R.za = tc_ldg128(P.kv.kzero + gb + 8 * cp);
         R.sb = tc_ldg128(P.kv.kscale + gb + 8 * (cp + nrp)); R.zb = tc_ldg128(P.kv.kzero + gb + 8 * (cp + nrp));
       };
-      auto roti_load = [&](int q, RotI& R) {                         // q-th item of the stream
-        const int kk = cc + tpc * (q % RCI), tk = (j0 + q / RCI) * TC_BN + (TC_BN / 2) * (int)rank;
-        if (q < n * RCI && kk < 32 && tk < P.max_ctx) {
-          const int t = tk + 32 * cg + kk;
+      auto roti_load = [&](int i, int u, RotI& R) {                  // item u of this warp in tile i
+        const int tk = tile_key(i);
+        if (i < n && u < rn && tk < P.max_ctx) {
+          const int t = tk + 32 * cg + cc + cstep * u;
           const uint32_t* rowp = kq32 + (row0 + t) * (HD / 8);
           R.wa = tc_ldg32(rowp + cp); R.wb = tc_ldg32(rowp + cp + nrp);
           const float* rp = P.rope + ((size_t)t * half + 8 * cp) * 2;
@@ -788,12 +794,10 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         }
       };
       auto roti_store = [&](int u, uint32_t sk, const RotS& Sc, const RotI& R) {
-        const int kk = cc + tpc * u;
-        if (kk >= 32) return;
-        const int p = cp, q = cp + nrp, k = 32 * cg + kk;
+        const int p = cp, q = cp + nrp, k = 32 * cg + cc + cstep * u;
         uint32_t sa[4], za[4], sb4[4], zb[4], na[4], nb[4], a[4], b[4], lo[4], hi[4];
         tc_row_to_pairs(Sc.sa, sa); tc_row_to_pairs(Sc.za, za); tc_row_to_pairs(Sc.sb, sb4); tc_row_to_pairs(Sc.zb, zb);
-        tc_nibs(R.wa, na); tc_nibs(R.wb, nb);
+        tc_nibs(R.wa, na, nk); tc_nibs(R.wb, nb, nk);
         #pragma unroll
         for (int x = 0; x < 4; ++x) { a[x] = tc_hfma2(na[x], sa[x], za[x]); b[x] = tc_hfma2(nb[x], sb4[x], zb[x]); }
         const uint4* r = R.r;                                        // r[e/2] = (cos e, sin e, cos e+1, sin e+1) as fp32 bits
@@ -806,14 +810,14 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           lo[x] = tc_hfma2(a[x], C[x], tc_hmul2(b[x], S[x]) ^ 0x80008000u);      // a cos - b sin
           hi[x] = tc_hfma2(a[x], S[x], tc_hmul2(b[x], C[x]));                    // a sin + b cos
         }
-        tc_sts128(k_addr(sk, p, k), tc_pairs_to_row(lo));
-        tc_sts128(k_addr(sk, q, k), tc_pairs_to_row(hi));
+        tc_sts128(k_addr(sk, p, k), make_uint4(lo[0], lo[1], lo[2], lo[3]));
+        tc_sts128(k_addr(sk, q, k), make_uint4(hi[0], hi[1], hi[2], hi[3]));
       };
-      PlainIn pc, pn;                                                // plain stream: current item, next item
-      RotI rc, rn;                                                   // rotary stream (compact mapping)
-      plain_load(0, pc);
-      if (compact) roti_load(0, rc);
-      int pq = 0, rq = 0, kit = 0;
+      PlainIn pc, pnx;                                               // plain stream: current item, next item
+      RotI rc, rcn;                                                  // rotary stream (compact mapping)
+      plain_load(0, 0, pc);
+      roti_load(0, 0, rc);
+      int kit = 0;
       // L2 prefetch of a half tile two tiles ahead (64 packed rows, the scale and zero rows of its two groups; one line per
       // thread), so that the register loads a phase ahead find their lines in L2
       auto k_prefetch = [&](int tk) {
@@ -827,7 +831,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       if (n > 1) k_prefetch(j0 * TC_BN + TC_BN + (TC_BN / 2) * (int)rank);
       for (int i = 0; i < n && ok; ++i) {
         const int j = j0 + i;
-        const int tk0 = j * TC_BN + (TC_BN / 2) * (int)rank;         // first key of this CTA's half of the K tile
+        const int tk0 = tile_key(i);
         const bool kin = tk0 < P.max_ctx;                            // max_ctx is a multiple of 64: the half tile is inside or outside as a whole
         if (i + 2 < n) k_prefetch(tk0 + 2 * TC_BN);
         // ---- item 1: the int4 keys.  The converters never idle, so a request must be made a whole phase before its data
@@ -842,20 +846,22 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           if (kin && compact) rots_load(tk0, RS);
           stage_wait(b_kempty + 8 * st, kit, L::NK);
           if (!ok) break;
-          if (!kin) { zero_k(sk); pq += NPI; rq += RCI; plain_load(pq, pc); if (compact) roti_load(rq, rc); }
+          if (!kin) zero_k(sk);                                      // only the last tile of the last split can lie outside: nothing is loaded after it
           else {
             #pragma unroll 1
-            for (int u = 0; u < NPI; ++u, ++pq) {
-              plain_load(pq + 1, pn);
+            for (int u = 0; u < pn; ++u) {
+              const bool more = u + 1 < pn;
+              plain_load(more ? i : i + 1, more ? 1 : 0, pnx);
               plain_store(u, sk, pc);
-              pc = pn;
+              pc = pnx;
             }
             if (compact) {
               #pragma unroll 1
-              for (int u = 0; u < RCI; ++u, ++rq) {
-                roti_load(rq + 1, rn);
+              for (int u = 0; u < rn; ++u) {
+                const bool more = u + 1 < rn;
+                roti_load(more ? i : i + 1, more ? u + 1 : 0, rcn);
                 roti_store(u, sk, RS, rc);
-                rc = rn;
+                rc = rcn;
               }
             } else {
               RotIn R1;
@@ -882,7 +888,9 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
               if (w < nrw) continue;
               uint4 x = make_uint4(0u, 0u, 0u, 0u);
               if (tk0 + k < end) x = tc_ldg128(P.kv.kshadow + (row0 + tk0 + k) * HD + 8 * w);
-              tc_sts128(k_addr(sk, w, k), x);
+              uint32_t o4[4];
+              tc_row_to_pairs(x, o4);
+              tc_sts128(k_addr(sk, w, k), make_uint4(o4[0], o4[1], o4[2], o4[3]));
             }
             RotIn R1;
             #pragma unroll 1
@@ -935,38 +943,43 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         }
       } else {
       // Item = (key, 16-byte part of the key's half row = 32 channels); tokens that do not exist yet read as zero.
-      constexpr int PARTS = NWV / 4, NVI = (TC_BN * PARTS + NVT - 1) / NVT;
-      const int vt = ct - NKT;
+      constexpr int PARTS = NWV / 4, NVI = (TC_BN * PARTS + NVT - 1) / NVT, VSTEP = NVT / PARTS;
+      static_assert(NVT % PARTS == 0, "a thread keeps its part of the half row");
+      const int vt = ct - NKT, part = vt % PARTS, vk0 = vt / PARTS;  // item u of this thread in a tile: key vk0 + VSTEP u, its part of the half row
+      const TcNib nk = tc_nib_consts();
       struct VIn { uint4 w; uint32_t s, z; };
       // The items of all tiles form one stream (tile by tile, NVI items each); two items are in flight ahead of the one being
       // converted.  A rolled loop: the lines are in L2 already (prefetched two tiles ahead), and small code matters more
       // here than the last cycles of latency.
-      auto v_item_load = [&](int q, VIn& I) {                        // q-th item of this thread's stream
-        const int j = j0 + q / NVI, it = vt + NVT * (q % NVI), t = j * TC_BN + it / PARTS;
-        if (q < n * NVI && it < TC_BN * PARTS && t < end) {
-          I.w = tc_ldg128(P.kv.vq + (row0 + t) * (HD / 2) + (HD / 4) * (int)rank + 16 * (it % PARTS));
+      const uint8_t* vsrc = P.kv.vq + row0 * (HD / 2) + (HD / 4) * (int)rank + 16 * part;
+      int li = 0, lu = 0;                                            // tile and item of the next load
+      auto v_item_load = [&](VIn& I) {
+        const int k = vk0 + VSTEP * lu, t = (j0 + li) * TC_BN + k;
+        if (li < n && k < TC_BN && t < end) {
+          I.w = tc_ldg128(vsrc + (size_t)t * (HD / 2));
           I.s = tc_ldg16(P.kv.vscale + row0 + t); I.z = tc_ldg16(P.kv.vzero + row0 + t);
         }
+        if (++lu == NVI) { lu = 0; ++li; }
       };
       auto v_prefetch = [&](int j) {                                 // L2 prefetch of a tile's half rows and per-token scales
         for (int x = vt; x < TC_BN; x += NVT) if (j * TC_BN + x < end) tc_prefetch_l2(P.kv.vq + (row0 + j * TC_BN + x) * (HD / 2) + (HD / 4) * (int)rank);
         if (vt < 4 && j * TC_BN + 64 * (vt & 1) < end) tc_prefetch_l2((vt & 2 ? P.kv.vzero : P.kv.vscale) + row0 + j * TC_BN + 64 * (vt & 1));
       };
       VIn cur, n1, n2;
-      v_item_load(0, cur); v_item_load(1, n1);
+      v_item_load(cur); v_item_load(n1);
       if (n > 1) v_prefetch(j0 + 1);
-      int q = 0;
+      const uint32_t vdst = (part >> 1) * L::V_BLOCK + (4 * (part & 1) << 4);     // chunk 4*part + e of the half row = chunk (4 (part & 1)) ^ e of its block
       for (int i = 0; i < n && ok; ++i) {
         const int j = j0 + i, st = i % L::NV;
-        const uint32_t sv = sb + L::OFF_V + st * L::V_HALF;
+        const uint32_t sv = sb + L::OFF_V + st * L::V_HALF + vdst;
         if (i + 2 < n) v_prefetch(j + 2);
         stage_wait(b_vempty + 8 * st, i, L::NV);
         if (!ok) break;
         #pragma unroll 1
-        for (int u = 0; u < NVI; ++u, ++q) {
-          v_item_load(q + 2, n2);
-          const int it = vt + NVT * u, k = it / PARTS, part = it % PARTS;
-          if (it < TC_BN * PARTS) {
+        for (int u = 0; u < NVI; ++u) {
+          v_item_load(n2);
+          const int k = vk0 + VSTEP * u;
+          if (k < TC_BN) {
             // no branches inside an item: a token that does not exist yet gets scale = zero = 0 (nibbles are finite whatever
             // the word holds), and the four words are converted before the four stores, so their chains interleave
             const bool live = j * TC_BN + k < end;
@@ -975,15 +988,13 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
             uint4 out[4];
             #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              uint32_t nb[4], r[4];
-              tc_nibs(ww[e], nb);
-              #pragma unroll
-              for (int x = 0; x < 4; ++x) r[x] = tc_hfma2(nb[x], s2, z2);
-              out[e] = tc_pairs_to_row(r);
+              uint32_t nb[4];
+              tc_nibs(ww[e], nb, nk);
+              out[e] = make_uint4(tc_hfma2(nb[0], s2, z2), tc_hfma2(nb[1], s2, z2), tc_hfma2(nb[2], s2, z2), tc_hfma2(nb[3], s2, z2));
             }
-            const uint32_t base = sv + (part >> 1) * L::V_BLOCK + k * 128, kx = (uint32_t)(k & 7), c0 = 4 * (part & 1);   // chunk 4*part + e of the half row
+            const uint32_t base = (sv + k * 128) ^ (uint32_t)((k & 7) << 4);
             #pragma unroll
-            for (int e = 0; e < 4; ++e) tc_sts128(base + (((c0 + e) ^ kx) << 4), out[e]);
+            for (int e = 0; e < 4; ++e) tc_sts128(base ^ (uint32_t)(e << 4), out[e]);
           }
           cur = n1; n1 = n2;
         }
@@ -1001,11 +1012,10 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     const int pr = pos0 + tok, cr = pr / 32;                         // row position and its own group
     const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16);
     const float cs = P.qscale * TC_LOG2E;
-    if constexpr (FORM == 3) {
+    if constexpr (STAGED_Q) {
       if (n > 0) {
-        // bf16 activations in the workspace form: these eight warps write this CTA's query rows as fp16 operand rows
-        // (the converting forms leave that to their K converters); rows without a query are zero
-        tc_stage_q_bf16<HD>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, tok0, G, TOK, P.M, P.nh, kvh * G, threadIdx.x, 32 * TC_SW);
+        // bf16 activations, or the chunk order of the int4 form: these eight warps write this CTA's query rows (there is no Q copy)
+        tc_stage_q<HD, FORM == 1>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, act_bf16, tok0, G, TOK, P.M, P.nh, kvh * G, threadIdx.x, 32 * TC_SW);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) bar_arrive_cluster(lead_q);
@@ -1108,6 +1118,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     if (ok && !*s_abort) {
       const size_t pidx = ((size_t)tok * S + split) * P.nh + kvh * G + head;
       const bool direct = P.o16 != nullptr && S == 1;                // one split: this CTA holds the whole row, finish it here
+      auto ocol = [](int c) { return FORM == 1 ? tc_col(c) : c; };   // the int4 form's V chunks keep their channels in pair order
       if (valid && !direct && hf == 0) { P.pm[pidx] = (n > 0 && m > -1e29f) ? m * TC_LN2 : -1e30f; P.pl[pidx] = n > 0 ? l : 0.f; }
       #pragma unroll 1
       for (int c = hf; c < HD / 32; c += 2) {
@@ -1122,7 +1133,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           uint32_t w[16];
           #pragma unroll
           for (int k = 0; k < 32; k += 2) {
-            float y0 = round_f16(o[k] / l), y1 = round_f16(o[k + 1] / l);
+            float y0 = round_f16(o[ocol(k)] / l), y1 = round_f16(o[ocol(k + 1)] / l);
             if (act_bf16) {
               if (P.bv) { y0 = __fadd_rn(y0, bf2f(P.bv[kvh * HD + 32 * c + k])); y1 = __fadd_rn(y1, bf2f(P.bv[kvh * HD + 32 * c + k + 1])); }
               w[k / 2] = (uint32_t)f2bf(y0) | ((uint32_t)f2bf(y1) << 16);
@@ -1137,7 +1148,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         } else if (valid) {
           float4* dst = reinterpret_cast<float4*>(P.pacc + pidx * HD + 32 * c);
           #pragma unroll
-          for (int k = 0; k < 8; ++k) dst[k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+          for (int k = 0; k < 8; ++k) dst[k] = make_float4(o[ocol(4 * k)], o[ocol(4 * k + 1)], o[ocol(4 * k + 2)], o[ocol(4 * k + 3)]);
         }
       }
     }
@@ -1148,7 +1159,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     if (warp < TC_SW) { asm volatile("setmaxnreg.dec.sync.aligned.u32 120;"); role_softmax(); }
     else if (warp < TC_SW + 4) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
-      if (warp == TC_SW) { role_producer(); role_mma(); } else role_conv(false);
+      if (warp == TC_SW) role_mma(); else role_conv(false);
     } else { asm volatile("setmaxnreg.inc.sync.aligned.u32 160;"); role_conv(true); }
   } else {
     if (warp == TC_SW) role_producer();
@@ -1279,9 +1290,8 @@ int launch_tc_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, const TcWs&
 template <int HD>
 int launch_tc_fused_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, uint16_t* o16, const uint16_t* bv, cudaStream_t st) {
   using L = TcLay<HD>;
-  CUtensorMap mq;
-  if (bf16) memset(&mq, 0, sizeof(mq));                               // the converter warps stage Q
-  else if (!tc_map_q(&mq, a.q16, a.M, a.kvh, g, HD)) KV4_REJECT("yskn_kv4_attention: cuTensorMapEncodeTiled failed or is unavailable");
+  CUtensorMap mq;                                                     // unused: the softmax warps stage Q
+  memset(&mq, 0, sizeof(mq));
   auto kern = kv4_tc_attn_kernel<HD, 1>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
@@ -1342,9 +1352,8 @@ int launch_kv8_attention_tc(const yskn_kv8_attn_args& a, int act_dtype, cudaStre
   if (((uintptr_t)a.k8 | (uintptr_t)a.v8 | (uintptr_t)a.q16 | (uintptr_t)a.pacc) & 15) KV4_REJECT("yskn_kv8_attention_tc: k8, v8, q16 and pacc must be 16-byte aligned");
   using L = TcLay<256>;
   const int g = a.nh / a.kvh, bf16 = act_dtype == YSKN_KV4_BF16;
-  CUtensorMap mq;
-  if (bf16) memset(&mq, 0, sizeof(mq));
-  else if (!tc_map_q(&mq, a.q16, a.M, a.kvh, g, 256)) KV4_REJECT("yskn_kv8_attention_tc: cuTensorMapEncodeTiled failed or is unavailable");
+  CUtensorMap mq;                                                     // unused: the softmax warps stage Q
+  memset(&mq, 0, sizeof(mq));
   auto kern = kv4_tc_attn_kernel<256, 2>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
