@@ -182,6 +182,9 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {       
   for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) if (bar_try(bar, parity)) return true;
   return false;
 }
+__device__ __forceinline__ bool elect_one() {                         // true in one lane of a converged warp
+  uint32_t p; asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p)); return p != 0;
+}
 __device__ __forceinline__ uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 // Address of the leader CTA's copy (rank 0 of the pair) of a shared-memory location, in the cluster window.
 __device__ __forceinline__ uint32_t leader_addr(uint32_t local) { uint32_t r; asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(local)); return r; }
@@ -444,7 +447,9 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   __syncthreads();
   cluster_sync_all();                                                // both CTAs' barriers exist before anyone signals the other
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  // An allocation of all 512 columns starts at column 0, so the tensor-memory addresses below are compile-time constants.
+  constexpr uint32_t tmem = 0;
+  if (*tmem_slot != 0) { if (threadIdx.x == 0) { atomicExch(&g_tc_status, 5); *s_abort = 1; } }
   // Programmatic dependent launch: the grid may be scheduled while its predecessor in the stream drains, and everything above
   // (barriers, tensor memory, the cluster handshake) touches nothing the predecessor wrote.  From here on the position, the
   // queries and the cache (or the workspace the prep kernel fills) are read; the merge kernel that follows may be scheduled
@@ -499,93 +504,64 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   };
   constexpr int CONV0 = TC_SW + 1;
   auto role_mma = [&]() {
-    // ======================================================================= MMA issuer (one thread of the leader CTA)
-    // The tensor pipe runs this thread's MMAs in issue order, so S of tile i+2, issued after P.V of tile i, may
+    // ======================================================================= MMA issuer (one warp of the leader CTA, one elected thread)
+    // The tensor pipe runs the elected thread's MMAs in issue order, so S of tile i+2, issued after P.V of tile i, may
     // overwrite the TMEM buffer that P.V reads P from without a barrier in between.
-    if (lane == 0 && n > 0 && rank == 0) {
+    // The whole warp walks the loop and only the tcgen05 instructions are predicated: descriptors and addresses are then warp-uniform
+    // values and need no move from a thread's registers before every MMA (under "if (lane == 0)", in a rolled loop, an MMA cost
+    // 140-230 cycles to issue and the issue paced the converting forms: 4.1 k cycles a tile for 2.06 k of tensor work).
+    if (n > 0 && rank == 0) {
       constexpr uint32_t ID_S = instr_desc(256, TC_BN, false), ID_PV = instr_desc(256, HD, true);
       bool ok = true;
-      auto fail = [&]() { atomicExch(&g_tc_status, 5); *s_abort = 1; ok = false; };
+      const bool leader = elect_one();
+      auto fail = [&]() { if (leader) { atomicExch(&g_tc_status, 5); *s_abort = 1; } ok = false; };
       const uint64_t qdesc0 = smem_desc(sb + L::OFF_Q, 16, 1024), kdesc0 = smem_desc(sb + L::OFF_K, 16, 1024),
                      vdesc0 = smem_desc(sb + L::OFF_V, L::V_BLOCK, 1024);
       auto issue_s = [&](int item, int buf) {                        // S[buf] = Q . K(item)^T
         const int st = item % L::NK;
-        if (!bar_wait(b_kfull + 8 * st, (item / L::NK) & 1)) { fail(); return; }
+        if (!__all_sync(0xffffffffu, bar_wait(b_kfull + 8 * st, (item / L::NK) & 1))) { fail(); return; }
         tc_fence_after();
         const uint64_t kd = kdesc0 + (uint64_t)((st * L::K_HALF) >> 4);
-        // The workspace form (prefill) lives on this thread's issue rate: everything unrolled.  The converting forms keep
-        // their code inside the instruction cache: one expansion per lambda and a rolled loop, whose iteration is kept to a
-        // handful of instructions by stepping the two descriptors (an MMA cost this thread ~220 cycles with the
-        // descriptors recomputed in every iteration, and the thread then paced the whole kernel).
-        if constexpr (FUSED) {
-          const uint32_t dcol = tmem + (buf ? L::TM_S1 : L::TM_S0);
-          uint64_t qd = qdesc0, kdd = kd;
-          #pragma unroll 1
-          for (int t = 0; t < 4 * L::KBLK; ++t) {
-            umma2_ss(dcol, qd, kdd, ID_S, t ? 1u : 0u);
-            const bool last = (t & 3) == 3;                          // next 64-channel block: the next operand block of Q and of K
-            qd += last ? (uint64_t)((L::Q_BLOCK - 96) >> 4) : 2ull;
-            kdd += last ? (uint64_t)((L::K_BLOCK - 96) >> 4) : 2ull;
-          }
-        } else {
-        #pragma unroll
-        for (int kb = 0; kb < L::KBLK; ++kb)
+        const uint32_t dcol = buf ? L::TM_S1 : L::TM_S0;
+        if (leader) {
           #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma2_ss(tmem + (buf ? L::TM_S1 : L::TM_S0), qdesc0 + (uint64_t)((kb * L::Q_BLOCK + ks * 32) >> 4),
-                     kd + (uint64_t)((kb * L::K_BLOCK + ks * 32) >> 4), ID_S, (kb | ks) ? 1u : 0u);
+          for (int kb = 0; kb < L::KBLK; ++kb)
+            #pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+              umma2_ss(dcol, qdesc0 + (uint64_t)((kb * L::Q_BLOCK + ks * 32) >> 4), kd + (uint64_t)((kb * L::K_BLOCK + ks * 32) >> 4), ID_S, (kb | ks) ? 1u : 0u);
+          umma2_commit(b_sready + 8 * buf);
+          umma2_commit(b_kempty + 8 * st);                           // the K halves may be overwritten once these MMAs are done
         }
-        umma2_commit(b_sready + 8 * buf);
-        umma2_commit(b_kempty + 8 * st);                             // the K halves may be overwritten once these MMAs are done
+        __syncwarp();
       };
       auto issue_pv = [&](int tile_i, int buf) {                     // O (+)= P . V(tile_i), P from TMEM (over S[buf])
         const int st = tile_i % L::NV;
-        if (!bar_wait(b_pready + 8 * (tile_i & 1), (tile_i >> 1) & 1)) { fail(); return; }
-        if (!bar_wait(b_vfull + 8 * st, (tile_i / L::NV) & 1)) { fail(); return; }
+        if (!__all_sync(0xffffffffu, bar_wait(b_pready + 8 * (tile_i & 1), (tile_i >> 1) & 1))) { fail(); return; }
+        if (!__all_sync(0xffffffffu, bar_wait(b_vfull + 8 * st, (tile_i / L::NV) & 1))) { fail(); return; }
         tc_fence_after();
         const uint64_t vd = vdesc0 + (uint64_t)((st * L::V_HALF) >> 4);
-        const uint32_t pcol = tmem + (buf ? L::TM_S1 : L::TM_S0);
-        if constexpr (FUSED) {
-          uint32_t pa = pcol; uint64_t vdd = vd;
-          #pragma unroll 1
-          for (int ks = 0; ks < TC_BN / 16; ++ks) {                  // P columns: keys 0-63 at +0.., keys 64-127 at +64..
-            umma2_ts(tmem + L::TM_O, pa, vdd, ID_PV, (tile_i | ks) ? 1u : 0u);
-            pa += ks == 3 ? 64u - 24u : 8u; vdd += 128ull;
-          }
-        } else {
-        #pragma unroll
-        for (int ks = 0; ks < TC_BN / 16; ++ks)                      // P columns: keys 0-63 at +0.., keys 64-127 at +64..
-          umma2_ts(tmem + L::TM_O, pcol + 64 * (ks >> 2) + 8 * (ks & 3), vd + (uint64_t)((ks * 2048) >> 4), ID_PV, (tile_i | ks) ? 1u : 0u);
+        const uint32_t pcol = buf ? L::TM_S1 : L::TM_S0;
+        if (leader) {
+          #pragma unroll
+          for (int ks = 0; ks < TC_BN / 16; ++ks)                    // P columns: keys 0-63 at +0.., keys 64-127 at +64..
+            umma2_ts(L::TM_O, pcol + 64 * (ks >> 2) + 8 * (ks & 3), vd + (uint64_t)((ks * 2048) >> 4), ID_PV, (tile_i | ks) ? 1u : 0u);
+          umma2_commit(b_pvdone + 8 * (tile_i & 1));                 // O may be rescaled
+          umma2_commit(b_vempty + 8 * st);                           // the V halves may be overwritten
         }
-        umma2_commit(b_pvdone + 8 * (tile_i & 1));                   // O may be rescaled
-        umma2_commit(b_vempty + 8 * st);                             // the V halves may be overwritten
+        __syncwarp();
       };
-      if (!bar_wait(b_q, 0)) fail();
+      if (!__all_sync(0xffffffffu, bar_wait(b_q, 0))) fail();
       tc_fence_after();
       // Bulk tiles: S(0), S(1), then P.V(i), S(i+2), ...: S of the next two tiles is done or in flight while the softmax
       // warps work on this one.  Edge tiles: S from the int4 keys, S from the shadow keys, then P.V.
-      if constexpr (FUSED) {                                         // the same order as one loop with a single expansion of each lambda
-        int s_next = 0, pv_next = 0;
-        const int s_total = npipe + 2 * (n - npipe);
-        while (ok && pv_next < n) {
-          bool do_s = false; int buf = 0;
-          if (s_next < npipe) { do_s = s_next < pv_next + 2; buf = s_next & 1; }
-          else if (pv_next >= npipe) { const int e = s_next - (npipe + 2 * (pv_next - npipe)); do_s = s_next < s_total && e < 2; buf = e; }
-          if (do_s) { issue_s(s_next, buf); ++s_next; }
-          else { issue_pv(pv_next, pv_next < npipe ? (pv_next & 1) : 0); ++pv_next; }
-        }
-      } else {
-        if (ok && npipe > 0) issue_s(0, 0);
-        if (ok && npipe > 1) issue_s(1, 1);
-        for (int i = 0; i < npipe && ok; ++i) {
-          issue_pv(i, i & 1);
-          if (ok && i + 2 < npipe) issue_s(i + 2, i & 1);
-        }
-        for (int i = npipe, kit = npipe; i < n && ok; ++i, kit += 2) {
-          issue_s(kit, 0); if (!ok) break;
-          issue_s(kit + 1, 1); if (!ok) break;
-          issue_pv(i, 0);
-        }
+      int s_next = 0, pv_next = 0;                                   // one loop with a single expansion of each lambda (code size)
+      const int s_total = npipe + 2 * (n - npipe);
+      while (ok && pv_next < n) {
+        bool do_s = false; int buf = 0;
+        if (s_next < npipe) { do_s = s_next < pv_next + 2; buf = s_next & 1; }
+        else if (pv_next >= npipe) { const int e = s_next - (npipe + 2 * (pv_next - npipe)); do_s = s_next < s_total && e < 2; buf = e; }
+        if (do_s) { issue_s(s_next, buf); ++s_next; }
+        else { issue_pv(pv_next, pv_next < npipe ? (pv_next & 1) : 0); ++pv_next; }
       }
     }
   };
