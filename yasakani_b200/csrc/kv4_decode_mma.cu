@@ -60,17 +60,15 @@ namespace {
 #ifndef KV4_DECODE_NCW
 #define KV4_DECODE_NCW 7                     // consumer warps per CTA
 #endif
-#ifndef KV4_DECODE_MAXREG
-#define KV4_DECODE_MAXREG 255                // 2 warps per SM sub-partition, one CTA of 8 warps per SM.  Measured at 262,144 tokens:
-                                             // 4 / 6 / 8 / 12 / 16 warps (255 / 255 / 255 / 168 / 128 registers) = 127 / 111 / 83.5 / 90.2 / 107 us per step
-#endif
-constexpr int NSTAGE = 5;                    // ring depth (128-token units in flight per CTA)
+// 8 warps = 2 per SM sub-partition, one CTA per SM, up to 255 registers a thread.  Measured at 262,144 tokens:
+// 4 / 6 / 8 / 12 / 16 warps (255 / 255 / 255 / 168 / 128 registers) = 127 / 111 / 83.5 / 90.2 / 107 us per step
 constexpr int NCW = KV4_DECODE_NCW;
 constexpr int NTHREADS = (NCW + 1) * 32;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;    // polls of try_wait before giving up (each poll suspends up to ~us)
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
-template <int HD, int RD> struct Lay {
+constexpr int NSTAGE = 5;                    // ring depth (128-token units in flight per CTA); with four, rows of a batch took 15-20 % longer
+template <int HD, int RD, bool Q> struct Lay {
   static constexpr int UG = 4;                             // groups per unit (one ring stage)
   static constexpr int ROWB = HD / 2;                      // bytes of one packed row
   static constexpr int KB = 32 * ROWB;                     // packed K (or V) bytes of one group
@@ -89,10 +87,16 @@ template <int HD, int RD> struct Lay {
   static constexpr int OFF_QFRAG = NSTAGE * STAGE;
   static constexpr int OFF_RELT = OFF_QFRAG + QFRAG;
   static constexpr int OFF_BARS = OFF_RELT + RELT;         // full[NSTAGE], empty[NSTAGE]
-  static constexpr int OFF_MISC = OFF_BARS + 2 * NSTAGE * 8;
-  static constexpr int TOTAL = OFF_MISC + 64;
-  static constexpr int MERGE = NCW * 8 * (HD + 2) * 4;     // aliases the stage ring after the loop
-  static_assert(MERGE <= NSTAGE * STAGE, "merge buffer must fit in the ring");
+  static constexpr int OFF_MISC = OFF_BARS + 2 * NSTAGE * 8;   // abort flag
+  static constexpr int OFF_RESP = (OFF_MISC + 4 + 15) / 16 * 16, OFF_CLC = OFF_RESP + 32;   // queue: two cancel responses, their full / empty barriers
+  static constexpr int OFF_ORDER = OFF_CLC + 32, OFF_POS = OFF_ORDER + 64;                   // queue: rows by length; their positions
+  static constexpr int OFF_ML = (OFF_POS + 256 + 15) / 16 * 16;                              // (m, l) of heads 2j, 2j+1 per (warp, j)
+  static constexpr int NH = HD / 32;                       // m-tiles of one half
+  // O of all warps, half of the m-tiles at a time: [warp][m-tile][lane] x 16 bytes.  Without the queue it aliases the ring, which is empty by
+  // then: the block then leaves room on its SM for a block of the merge kernel, which starts ahead of its end.
+  static constexpr int OFF_MERGE = Q ? OFF_ML + NCW * 4 * 16 : 0, MERGE = NCW * NH * 512;
+  static constexpr int TOTAL = Q ? OFF_MERGE + MERGE : OFF_ML + NCW * 4 * 16;
+  static_assert(Q || MERGE <= NSTAGE * STAGE, "merge buffer must fit in the ring");
   static_assert(SHADOW == UG * KB, "the open group's fp16 rows take the place of the unit's packed K");
   static_assert(NR % 2 == 0 && NR <= NW, "rotary width must be a multiple of 64 and at most head_dim");
   static_assert(TOTAL <= 227 * 1024, "shared memory budget of one CTA");
@@ -109,6 +113,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// Ask the hardware for a block of this grid that has not started: its index (or "none left") arrives in 16 bytes of shared memory.
+__device__ __forceinline__ void cancel_next(uint32_t resp, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(resp), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool cancel_result(uint32_t resp, int& x, int& y, int& z) {
+  uint32_t ok;
+  asm volatile("{\n .reg .b128 h;\n .reg .pred p;\n .reg .b32 w;\n ld.shared.b128 h, [%4];\n"
+               " clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n selp.u32 %0, 1, 0, p;\n"
+               " mov.u32 %1, 0;\n mov.u32 %2, 0;\n mov.u32 %3, 0;\n"
+               " @p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, w}, h;\n}"
+               : "=r"(ok), "=r"(x), "=r"(y), "=r"(z) : "r"(resp) : "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the next response into these bytes is ordered behind this read
   return ok != 0;
 }
 // Bounded wait; false when the limit ran out.
@@ -185,16 +203,22 @@ struct DecodeP {
   yskn_kv4_ms_rows ms;  // rows of several sequences (ms.pos != nullptr): row r reads the cache ms.layers[ms.slot[r]] at position ms.pos[r]
 };
 
-template <int HD, int RD, int DT>
-__global__ void __maxnreg__(KV4_DECODE_MAXREG)
+// Q ("queue"): for grids of more blocks than the GPU holds at once (several rows, or several sequences).  A CTA that has
+// issued the last copy of its item cancels a block that has not started (clusterlaunchcontrol) and takes over its indexes, so
+// the ring fills with the next item's keys while the consumers finish, merge and store this one.  Rows of several
+// sequences are taken longest first: the last blocks to start are then the shortest.  What each (split, kv-head, row) computes, and so every
+// bit of it, does not depend on Q.  Before, each item paid its launch, set-up, first-copy latency and merge by itself, and the longest
+// rows of a batch came last: eight sequences of 2,048 .. 131,072 tokens 171 -> 124 us with their merge, five rows over 20,011 tokens 67.6 ->
+// 55.6 us with their append and merge, eight rows over 172 tokens 48.8 -> 38 us.
+template <int HD, int RD, int DT, bool Q>
+__global__ void __launch_bounds__(NTHREADS, 1)
 kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV,
                       const __grid_constant__ CUtensorMap mapR, const DecodeP P) {
-  using L = Lay<HD, RD>;
+  using L = Lay<HD, RD, Q>;
   constexpr int NW = L::NW, NR = L::NR, NP = L::NP, NRd = NR > 0 ? NR : 1;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const yskn_attn_g_args& A = P.A;
-  const int split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   const int G = P.g;
   // Programmatic dependent launch in both directions (src/pdl.cuh:15-30 is the reference's form of this): this grid may be
@@ -209,56 +233,89 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
 
-  // ---- which groups this CTA owns (local token indices of this shard)
   const bool multi = P.ms.pos != nullptr;                       // rows of several sequences: per-row position and cache
-  const int base_local = multi ? P.ms.pos[r] : *A.d_pos - P.sh.start;   // row 0's local position: rows below it are never written again
-  const int pos = multi ? base_local : base_local + r;
-  const int len = max(0, min(pos + 1, P.sh.len));
-  const int cg = pos >= 0 ? pos / 32 : 0;                       // first group that is not read as int4
-  const int nq = min(cg, len / 32);                             // int4 groups, all fully visible
-  const bool has_tail = len > nq * 32;                          // the open group lives in this shard
-  const int nu4 = (nq + L::UG - 1) / L::UG;                     // int4 units of four groups (the last may hold fewer)
-  const int units = nu4 + (has_tail ? 1 : 0);                   // the open group is a unit of its own, the last one
-  const int per = (units + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int u0 = min(units, split * per), u1 = min(units, u0 + per), nu = u1 - u0;
+  // ---- which groups an item (split, kv-head, row) covers (local token indices of this shard)
+  struct Item { int split, kvh, r, base_local, len, nq, nu4, u0, nu; bool has_tail; };
+  auto item_at = [&](int x, int y, int z) {
+    Item t;
+    t.split = x; t.kvh = y;
+    t.r = Q && multi ? smem[L::OFF_ORDER + z] : z;              // Q: rows by length
+    t.base_local = multi ? P.ms.pos[t.r] : *A.d_pos - P.sh.start;   // row 0's local position: rows below it are never written again
+    const int pos = multi ? t.base_local : t.base_local + t.r;
+    t.len = max(0, min(pos + 1, P.sh.len));
+    const int cg = pos >= 0 ? pos / 32 : 0;                     // first group that is not read as int4
+    t.nq = min(cg, t.len / 32);                                 // int4 groups, all fully visible
+    t.has_tail = t.len > t.nq * 32;                             // the open group lives in this shard
+    t.nu4 = (t.nq + L::UG - 1) / L::UG;                         // int4 units of four groups (the last may hold fewer)
+    const int units = t.nu4 + (t.has_tail ? 1 : 0);             // the open group is a unit of its own, the last one
+    const int per = (units + (int)gridDim.x - 1) / (int)gridDim.x;
+    t.u0 = min(units, x * per); t.nu = min(units, t.u0 + per) - t.u0;
+    return t;
+  };
 
   const uint32_t bar_full = sbase + L::OFF_BARS, bar_empty = bar_full + NSTAGE * 8;
+  const uint32_t bar_clc = sbase + L::OFF_CLC, resp = sbase + L::OFF_RESP;       // Q: full[2], empty[2]; two responses
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + L::OFF_MISC);
   if (sbase & 1023u) { if (threadIdx.x == 0) atomicExch(&g_decode_status, 3); return; }   // the swizzled tiles need a 1 KB base
   if (threadIdx.x == 0) {
-    // a stage is free again once the consumers of its four groups have arrived (units with fewer groups are never reused)
+    // a stage is free again once the consumers of its four groups have arrived (without Q units with fewer groups are never reused)
     for (int s = 0; s < NSTAGE; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, L::UG); }
+    if (Q) for (int s = 0; s < 2; ++s) { mbar_init(bar_clc + 8 * s, 1); mbar_init(bar_clc + 16 + 8 * s, NCW); }
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (Q && multi) {                                             // rows by falling length, ties by index (at most 64 rows)
+    int* s_pos = reinterpret_cast<int*>(smem + L::OFF_POS);
+    if (threadIdx.x < A.M) s_pos[threadIdx.x] = P.ms.pos[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x < A.M) {
+      const int mine = s_pos[threadIdx.x];
+      int rank = 0;
+      for (int i = 0; i < A.M; ++i) rank += s_pos[i] > mine || (s_pos[i] == mine && i < (int)threadIdx.x);
+      smem[L::OFF_ORDER + rank] = (uint8_t)threadIdx.x;
+    }
+  }
   __syncthreads();
 
-  float* mbuf = reinterpret_cast<float*>(smem);                 // merge buffer, aliases the ring after the loop
+  Item it = item_at(blockIdx.x, blockIdx.y, blockIdx.z);
 
   if (warp == NCW) {
     // =========================================================== producer warp
-    if (nu > 0) {
+    int k = 0;                                                  // units issued by this CTA so far
+    bool waited = !early, go = true, asked = false;
+    // The next item is claimed when a ring's worth of this one's units is still to be issued.  Claimed always at the start of this one,
+    // every second item was bound to a CTA at once and the lengths no longer evened out (five sequences of 1,204 .. 57,119 tokens:
+    // 58 -> 70 us); claimed after the last unit, the answer came too late for short items (five rows over 20,011 tokens: 57.5 -> 61 us).
+    auto claim = [&](int n) {
+      if (lane != 0 || *s_abort) return;
+      if (n >= 2 && !mbar_wait(bar_clc + 16 + 8 * (n & 1), ((n >> 1) - 1) & 1)) { atomicExch(&g_decode_status, 2); *s_abort = 1; return; }
+      mbar_expect_tx(bar_clc + 8 * (n & 1), 16);
+      cancel_next(resp + 16 * (n & 1), bar_clc + 8 * (n & 1));
+      asked = true;
+    };
+    for (int n = 0; ; ++n) {                                    // items
+      const int nq = it.nq, nu4 = it.nu4, kvh = it.kvh;
+      const bool has_tail = it.has_tail;
       const size_t row0 = (size_t)kvh * A.max_ctx;              // first row of this kv-head in the [Hkv*max_ctx] arrays
-      const int slot = multi ? P.ms.slot[r] : 0;
+      const int slot = multi ? P.ms.slot[it.r] : 0;
       const yskn_kv_layer kvl = multi ? P.ms.layers[slot] : A.kv;
       const CUtensorMap* const mk = multi ? static_cast<const CUtensorMap*>(P.ms.maps) + 2 * slot : &mapK;
       const CUtensorMap* const mv = multi ? static_cast<const CUtensorMap*>(P.ms.maps) + 2 * slot + 1 : &mapV;
-      int issued = 0;
-      bool waited = !early;
-      for (int k = 0; k < nu; ++k) {
-        const int s = k % NSTAGE, u = u0 + k;
+      for (int u = it.u0; u < it.u0 + it.nu; ++u) {
+        const int s = k % NSTAGE;
         // an early unit: one of the first ring fills, int4 only, every token below the base position
-        if (!waited && (k >= NSTAGE || (has_tail && u == nu4) || min(nq, (u + 1) * L::UG) * 32 > max(0, min(base_local, P.sh.len)))) {
+        if (!waited && (k >= NSTAGE || (has_tail && u == nu4) || min(nq, (u + 1) * L::UG) * 32 > max(0, min(it.base_local, P.sh.len)))) {
           asm volatile("griddepcontrol.wait;" ::: "memory");
           asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
           waited = true;
         }
-        int go = 1;
+        if (Q && u == max(it.u0, it.u0 + it.nu - NSTAGE)) claim(n);
+        int ok = 1;
         if (lane == 0) {
           if (k >= NSTAGE && !mbar_wait(bar_empty + 8 * s, ((k / NSTAGE) - 1) & 1)) { atomicExch(&g_decode_status, 2); *s_abort = 1; }
-          if (*s_abort) go = 0;
+          if (*s_abort) ok = 0;
         }
-        go = __shfl_sync(0xffffffffu, go, 0);
+        go = __shfl_sync(0xffffffffu, ok, 0) != 0;
         if (!go) break;
         const bool tail = has_tail && u == nu4;
         const int ngr = tail ? 1 : min(L::UG, nq - u * L::UG);   // groups in this unit
@@ -278,16 +335,26 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
           case 6: if (RD > 0) tma_2d(st + L::OFF_ROPE, &mapR, 0, g0 + P.sh.start / 32, bar); break;   // rows 32*(g0..g0+3) of the table
           default: break;
         }
-        issued = k + 1;
+        ++k;
       }
-      if (!waited) { asm volatile("griddepcontrol.wait;" ::: "memory"); asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-      // After an abort nobody may have consumed the last copies: wait (bounded) until they have landed before the CTA ends.
-      if (lane == 0 && *s_abort)
-        for (int k = max(0, issued - NSTAGE); k < issued; ++k) mbar_wait(bar_full + 8 * (k % NSTAGE), (k / NSTAGE) & 1);
-    } else if (early) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+      if (!Q) break;
+      if (!waited) { asm volatile("griddepcontrol.wait;" ::: "memory"); asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); waited = true; }
+      if (it.nu == 0) claim(n);
+      int x = 0, y = 0, z = 0, more = 0;
+      if (lane == 0 && asked) {                                  // also after an abort: the answer has landed before the CTA ends
+        if (!mbar_wait(bar_clc + 8 * (n & 1), (n >> 1) & 1)) { atomicExch(&g_decode_status, 2); *s_abort = 1; }
+        else more = cancel_result(resp + 16 * (n & 1), x, y, z) ? 1 : 0;
+        if (*s_abort) more = 0;
+        asked = false;
+      }
+      more = __shfl_sync(0xffffffffu, more, 0);
+      if (!more) break;
+      it = item_at(__shfl_sync(0xffffffffu, x, 0), __shfl_sync(0xffffffffu, y, 0), __shfl_sync(0xffffffffu, z, 0));
     }
+    if (!waited) { asm volatile("griddepcontrol.wait;" ::: "memory"); asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+    // After an abort nobody may have consumed the last copies: wait (bounded) until they have landed before the CTA ends.
+    if (lane == 0 && *s_abort)
+      for (int i = max(0, k - NSTAGE); i < k; ++i) mbar_wait(bar_full + 8 * (i % NSTAGE), (i / NSTAGE) & 1);
   } else {
     // =========================================================== consumer warps
     if (early) {                                                // q16 and the partial buffers belong to the predecessor until here
@@ -296,18 +363,21 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
     }
     // ---- one-time set-up, spread over the consumer threads
     const int ct = threadIdx.x;                                 // 0..NCW*32-1
-    {
-      // Q as B fragments, pre-scaled by qscale*log2(e): entry [i][lane'] = 4 regs x, reg x = (q[g'][8w+x], q[g'][8w+x+4]), w = 4i+j'
-      const float qs = A.qscale * LOG2E;
-      for (int e = ct; e < NW * 32 * 4; e += NCW * 32) {
-        const int x = e & 3, ln = (e >> 2) & 31, i = e >> 7, gg = ln >> 2, jj = ln & 3, c = 8 * (4 * i + jj) + x;
-        float lo = 0.f, hi = 0.f;
-        if (gg < G) {
-          const size_t qb = ((size_t)r * A.nh + kvh * G + gg) * HD;
-          lo = act_load<DT>(A.q16, qb + c) * qs; hi = act_load<DT>(A.q16, qb + c + 4) * qs;
-        }
-        reinterpret_cast<uint32_t*>(smem + L::OFF_QFRAG)[e] = pack_h2(lo, hi);
+    constexpr int NQE = (NW * 32 * 4 + NCW * 32 - 1) / (NCW * 32);   // Q entries per thread
+    // Q as B fragments, pre-scaled by qscale*log2(e): entry [i][lane'] = 4 regs x, reg x = (q[g'][8w+x], q[g'][8w+x+4]), w = 4i+j'
+    const float qs = A.qscale * LOG2E;
+    auto q_entry = [&](int e, const Item& t) -> uint32_t {
+      const int x = e & 3, ln = (e >> 2) & 31, i = e >> 7, gg = ln >> 2, jj = ln & 3, c = 8 * (4 * i + jj) + x;
+      float lo = 0.f, hi = 0.f;
+      if (gg < G) {
+        const size_t qb = ((size_t)t.r * A.nh + t.kvh * G + gg) * HD;
+        lo = act_load<DT>(A.q16, qb + c) * qs; hi = act_load<DT>(A.q16, qb + c + 4) * qs;
       }
+      return pack_h2(lo, hi);
+    };
+    {
+      #pragma unroll
+      for (int n = 0; n < NQE; ++n) { const int e = ct + n * NCW * 32; if (e < NW * 32 * 4) reinterpret_cast<uint32_t*>(smem + L::OFF_QFRAG)[e] = q_entry(e, it); }
       // relative rotation by dt = 0..31 tokens, from the table's rows 0..31: entry [tile][half][i][xp][lane'] =
       // {cd_{2xp}, sd_{2xp}, cd_{2xp+1}, sd_{2xp+1}}, each a half2 over frequencies (8w+x, 8w+x+4), w = 4i+j'
       if (RD > 0) {
@@ -512,58 +582,121 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
     };
 
     bool ok = true;
+    int k0 = 0;                                                  // units of the items before this one
+    for (int n = 0; ; ++n) {                                     // items
+    const int nq = it.nq, nu4 = it.nu4, u0 = it.u0, nu = it.nu, len = it.len, r = it.r, kvh = it.kvh, split = it.split;
+    const bool has_tail = it.has_tail;
     // Slot kk = (unit kk/4 of this CTA, group kk%4 of the unit), round-robin over the consumer warps: a fixed assignment, so
     // the summation order and with it every bit of the result is the same from run to run (handing slots out from a shared
     // counter was measured: no faster with two warps per scheduler, and not reproducible).
     for (int kk = warp; kk < nu * L::UG && ok; kk += NCW) {
-      const int k = kk / L::UG, sub = kk % L::UG, u = u0 + k, s = k % NSTAGE;
-      const bool tail = has_tail && u == nu4;
-      if (tail ? sub != 0 : u * L::UG + sub >= nq) continue;     // the unit holds fewer than four groups
+      const int sub = kk % L::UG, u = u0 + kk / L::UG, k = k0 + kk / L::UG, s = k % NSTAGE;
+      const bool tail = has_tail && u == nu4, none = tail ? sub != 0 : u * L::UG + sub >= nq;   // the unit holds fewer than four groups
+      if (!Q && none) continue;
       const uint32_t st = sbase + L::OFF_STAGES + s * L::STAGE;
       if (!mbar_wait(bar_full + 8 * s, (k / NSTAGE) & 1)) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; break; }
-      if (tail) group(std::true_type{}, st, 0, len - nq * 32);
-      else group(std::false_type{}, st, sub, 32);
+      if (!none) {
+        if (tail) group(std::true_type{}, st, 0, len - nq * 32);
+        else group(std::false_type{}, st, sub, 32);
+      }
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_empty + 8 * s);             // one of the four arrivals that free the stage
     }
 
-    // ---- all consumers done with the ring: publish per-warp (m, l, O) into the merge buffer
+    // Q: the item after this one, and its queries on their way while this one is merged
+    bool more = false;
+    uint32_t qnext[Q ? NQE : 1];
+    if (Q) {
+      int x = 0, y = 0, z = 0;
+      if (*s_abort) ok = false;
+      if (ok && !mbar_wait(bar_clc + 8 * (n & 1), (n >> 1) & 1)) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; }
+      if (ok) more = cancel_result(resp + 16 * (n & 1), x, y, z);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_clc + 16 + 8 * (n & 1));
+      if (more) {
+        it = item_at(x, y, z);
+        #pragma unroll
+        for (int i = 0; i < NQE; ++i) qnext[i] = ct + i * NCW * 32 < NW * 32 * 4 ? q_entry(ct + i * NCW * 32, it) : 0u;
+      }
+    }
+    // ---- all consumers done with the item: publish per-warp (m, l, O) into the merge buffer
     #pragma unroll
     for (int o = 4; o <= 16; o <<= 1) {
       l[0] += __shfl_xor_sync(0xffffffffu, l[0], o); l[1] += __shfl_xor_sync(0xffffffffu, l[1], o);
       zacc[0] += __shfl_xor_sync(0xffffffffu, zacc[0], o); zacc[1] += __shfl_xor_sync(0xffffffffu, zacc[1], o);
     }
     const float ze[2] = {zacc[0], zacc[1]}, zo[2] = {zacc[0] - 64.f * zs[0], zacc[1] - 64.f * zs[1]};
-    asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");  // nobody still reads a stage
-    if (!*s_abort) {
-      float* wb = mbuf + (size_t)warp * 8 * (HD + 2);
-      if (g == 0) { wb[(2 * j) * (HD + 2)] = m[0]; wb[(2 * j) * (HD + 2) + 1] = l[0]; wb[(2 * j + 1) * (HD + 2)] = m[1]; wb[(2 * j + 1) * (HD + 2) + 1] = l[1]; }
-      #pragma unroll
-      for (int mt = 0; mt < HD / 16; ++mt) {
-        const int c = 32 * (mt >> 1) + 4 * g + 2 * (mt & 1);           // even channel of the m-tile; the odd one is c + 1
-        wb[(2 * j) * (HD + 2) + 2 + c] = acc[mt][0] + ze[0]; wb[(2 * j + 1) * (HD + 2) + 2 + c] = acc[mt][1] + ze[1];
-        wb[(2 * j) * (HD + 2) + 2 + c + 1] = acc[mt][2] + zo[0]; wb[(2 * j + 1) * (HD + 2) + 2 + c + 1] = acc[mt][3] + zo[1];
-      }
+    // ---- merge the consumer warps and store this split's partial (natural-log m, as the merge kernel expects).  Every warp
+    //      scales its own sums by the weight of its maximum and leaves them as they lie in its registers (16 bytes per lane, no bank
+    //      conflicts), half of the m-tiles at a time; the sum over the warps runs in warp order.
+    if (g == 0) *reinterpret_cast<float4*>(smem + L::OFF_ML + (warp * 4 + j) * 16) = make_float4(m[0], l[0], m[1], l[1]);
+    bool bad;                                                    // an abort is seen by all threads or by none
+    {
+      uint32_t any; const uint32_t mine = !ok || *s_abort;
+      asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}" : "=r"(any) : "r"(mine), "n"(NCW * 32) : "memory");
+      bad = any != 0;
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
-    // ---- merge the consumer warps and store this split's partial (natural-log m, as the merge kernel expects)
-    if (!*s_abort) {
-      for (int e = ct; e < G * HD; e += NCW * 32) {
-        const int h = e / HD, c = e % HD;
-        float M2 = -1e30f;
-        #pragma unroll
-        for (int w = 0; w < NCW; ++w) M2 = fmaxf(M2, mbuf[((size_t)w * 8 + h) * (HD + 2)]);
-        float L2 = 0.f, o = 0.f;
+    if (!bad) {
+      float M2[2] = {-1e30f, -1e30f}, L2[2] = {0.f, 0.f};
+      float4 ml[NCW];
+      #pragma unroll
+      for (int w = 0; w < NCW; ++w) {
+        ml[w] = *reinterpret_cast<const float4*>(smem + L::OFF_ML + (w * 4 + j) * 16);
+        M2[0] = fmaxf(M2[0], ml[w].x); M2[1] = fmaxf(M2[1], ml[w].z);
+      }
+      const float sc0 = m[0] > -1e29f ? ex2(m[0] - M2[0]) : 0.f, sc1 = m[1] > -1e29f ? ex2(m[1] - M2[1]) : 0.f;
+      const size_t p0 = ((size_t)r * A.splits + split) * A.nh + kvh * G;
+      if (warp == NCW - 1 && g == 0) {
         #pragma unroll
         for (int w = 0; w < NCW; ++w) {
-          const float* wb = mbuf + ((size_t)w * 8 + h) * (HD + 2);
-          const float sc = wb[0] > -1e29f ? ex2(wb[0] - M2) : 0.f;
-          L2 += sc * wb[1]; o += sc * wb[2 + c];
+          L2[0] += (ml[w].x > -1e29f ? ex2(ml[w].x - M2[0]) : 0.f) * ml[w].y;
+          L2[1] += (ml[w].z > -1e29f ? ex2(ml[w].z - M2[1]) : 0.f) * ml[w].w;
         }
-        const size_t p = ((size_t)r * A.splits + split) * A.nh + kvh * G + h;
-        if (c == 0) { A.pm[p] = M2 > -1e29f ? M2 * LN2 : -1e30f; A.pl[p] = L2; }
-        A.pacc[p * HD + c] = o;
+        #pragma unroll
+        for (int x = 0; x < 2; ++x)
+          if (2 * j + x < G) { A.pm[p0 + 2 * j + x] = M2[x] > -1e29f ? M2[x] * LN2 : -1e30f; A.pl[p0 + 2 * j + x] = L2[x]; }
       }
+      const bool wide = !((uintptr_t)A.pacc & 15);
+      float4* mbuf = reinterpret_cast<float4*>(smem + L::OFF_MERGE);
+      #pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (half) asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
+        #pragma unroll
+        for (int t = 0; t < L::NH; ++t) {                        // m-tile: (even | odd channel) x (head 2j | 2j+1)
+          const int mt = half * L::NH + t;
+          mbuf[(warp * L::NH + t) * 32 + lane] = make_float4((acc[mt][0] + ze[0]) * sc0, (acc[mt][1] + ze[1]) * sc1,
+                                                             (acc[mt][2] + zo[0]) * sc0, (acc[mt][3] + zo[1]) * sc1);
+        }
+        if (Q && more && half == 0) {                            // nobody still reads the Q fragments of this item
+          #pragma unroll
+          for (int i = 0; i < NQE; ++i) if (ct + i * NCW * 32 < NW * 32 * 4) reinterpret_cast<uint32_t*>(smem + L::OFF_QFRAG)[ct + i * NCW * 32] = qnext[i];
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
+        if (warp < L::NH / 2) {                                  // a warp per pair of m-tiles: a lane has four channels of two heads
+          float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+          #pragma unroll
+          for (int w = 0; w < NCW; ++w) {
+            const float4 x = mbuf[(w * L::NH + 2 * warp) * 32 + lane], y = mbuf[(w * L::NH + 2 * warp + 1) * 32 + lane];
+            a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w; b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
+          }
+          const int c = 32 * (half * (L::NH / 2) + warp) + 4 * g;
+          float* o0 = A.pacc + (p0 + 2 * j) * HD + c;
+          if (wide) {
+            if (2 * j < G) *reinterpret_cast<float4*>(o0) = make_float4(a.x, a.z, b.x, b.z);
+            if (2 * j + 1 < G) *reinterpret_cast<float4*>(o0 + HD) = make_float4(a.y, a.w, b.y, b.w);
+          } else {
+            if (2 * j < G) { o0[0] = a.x; o0[1] = a.z; o0[2] = b.x; o0[3] = b.z; }
+            if (2 * j + 1 < G) { o0[HD] = a.y; o0[HD + 1] = a.w; o0[HD + 2] = b.y; o0[HD + 3] = b.w; }
+          }
+        }
+      }
+    }
+    if (!Q || !more || bad) break;
+    k0 += nu;
+    #pragma unroll
+    for (int mt = 0; mt < HD / 16; ++mt) { acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f; }
+    m[0] = m[1] = -1e30f;
+    l[0] = l[1] = zacc[0] = zacc[1] = zs[0] = zs[1] = zs[2] = zs[3] = 0.f;
     }
   }
 }
@@ -623,10 +756,10 @@ bool make_rope_map(CUtensorMap* out, const float* rope, int rd, uint64_t groups)
   return true;
 }
 
-template <int HD, int RD, int DT>
-int launch_t(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, cudaStream_t st) {
-  using L = Lay<HD, RD>;
-  auto kern = kv4_decode_mma_kernel<HD, RD, DT>;
+template <int HD, int RD, int DT, bool Q>
+int launch_q(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, cudaStream_t st) {
+  using L = Lay<HD, RD, Q>;
+  auto kern = kv4_decode_mma_kernel<HD, RD, DT, Q>;
   static std::atomic<unsigned long long> attr{0};               // once per device, like the reference's launchers once per process
   if (first_use_on_device(attr)) {
     KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
@@ -640,6 +773,16 @@ int launch_t(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_k
   cfg.attrs = at; cfg.numAttrs = 1;
   KV4_CUDA(cudaLaunchKernelEx(&cfg, kern, mk, mv, mr, P));
   return launch_status("kv4_decode_mma_kernel");
+}
+
+// One CTA fills an SM, so a grid of up to one block per SM starts at once and has nothing to take over; a larger one runs as a queue.
+template <int HD, int RD, int DT>
+int launch_t(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, cudaStream_t st) {
+  int dev = 0, sms = 0;
+  KV4_CUDA(cudaGetDevice(&dev));
+  KV4_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if ((long long)a.splits * a.kvh * a.M > sms) return launch_q<HD, RD, DT, true>(a, g, sh, early, ms, mk, mv, mr, st);
+  return launch_q<HD, RD, DT, false>(a, g, sh, early, ms, mk, mv, mr, st);
 }
 
 template <int HD, int RD>
