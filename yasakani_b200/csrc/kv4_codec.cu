@@ -22,6 +22,14 @@ __device__ __forceinline__ int quant4(float v, float lo, float inv) {
   return q < 0 ? 0 : (q > 15 ? 15 : q);
 }
 
+// Programmatic dependent launch: a decode pass is three short launches, and the start of each is hidden behind the one before.  The
+// successor is let in only behind the wait, so what it reads ahead of its own wait (yskn_kv4_attn_ext.early) is
+// no newer than the launch before this one.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // The 32-token group `gi` of kv-head `head`, by one warp: per channel min / max over the 32 shadow rows, fp16 scale and zero,
 // int4 codes (src/attention_gqa.cu:143-154).  A lane touches only its own HD/32 channels of every row.
 template <int HD>
@@ -81,6 +89,7 @@ template <int HD, int DT, bool FUSE>
 __global__ void __launch_bounds__(128) kv4_append_rows_kernel(yskn_kv_append_args A) {
   constexpr int CPL = HD / 32;                       // channels per lane (2, 4 or 8)
   const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  pdl_enter();
   if (w >= A.M * A.kvh) return;
   const int r = w / A.kvh, head = w % A.kvh, pos = *A.d_pos + r;
   if (pos < 0 || pos >= A.max_ctx) return;
@@ -121,6 +130,7 @@ template <int HD>
 __global__ void __launch_bounds__(128) kv4_group_quant_kernel(yskn_kv_quant_args A, int kvh) {
   const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int ncand = (A.M + 31) / 32 + 1;
+  pdl_enter();
   if (w >= ncand * kvh) return;
   const int pos0 = *A.d_pos, last = pos0 + A.M - 1;
   const int gi = pos0 / 32 + w / kvh, head = w % kvh, gend = gi * 32 + 31;
@@ -143,14 +153,14 @@ __global__ void kv4_rope_table_kernel(float2* out, int max_ctx, float theta, int
 }
 
 template <int HD, bool FUSE> int append_dt(const yskn_kv_append_args& a, cudaStream_t st) {
-  const int blocks = (a.M * a.kvh + 3) / 4;
+  const dim3 blocks((unsigned)((a.M * a.kvh + 3) / 4));
+  const char* who = "kv4_append_rows_kernel";
   switch (a.in_dtype) {
-    case YSKN_KV4_F16: kv4_append_rows_kernel<HD, YSKN_KV4_F16, FUSE><<<blocks, 128, 0, st>>>(a); break;
-    case YSKN_KV4_BF16: kv4_append_rows_kernel<HD, YSKN_KV4_BF16, FUSE><<<blocks, 128, 0, st>>>(a); break;
-    case YSKN_KV4_F32: kv4_append_rows_kernel<HD, YSKN_KV4_F32, FUSE><<<blocks, 128, 0, st>>>(a); break;
+    case YSKN_KV4_F16: return launch_pdl(who, kv4_append_rows_kernel<HD, YSKN_KV4_F16, FUSE>, blocks, 128, 0, st, a);
+    case YSKN_KV4_BF16: return launch_pdl(who, kv4_append_rows_kernel<HD, YSKN_KV4_BF16, FUSE>, blocks, 128, 0, st, a);
+    case YSKN_KV4_F32: return launch_pdl(who, kv4_append_rows_kernel<HD, YSKN_KV4_F32, FUSE>, blocks, 128, 0, st, a);
     default: KV4_REJECT("yskn_kv4_append: unknown in_dtype %d", a.in_dtype);
   }
-  return launch_status("kv4_append_rows_kernel");
 }
 
 // A copy by a kernel, for the few kilobytes a decode step exchanges with the host: either side may be pinned (mapped) host
@@ -182,12 +192,12 @@ int launch_rope_table(float* d_out, int max_ctx, float theta, int rd, cudaStream
 
 int launch_group_quant(const yskn_kv_quant_args& a, int kvh, int hd, cudaStream_t st) {
   if (a.M <= 0 || kvh <= 0 || !a.d_pos || a.max_ctx % 32) KV4_REJECT("yskn_kv4_group_quant: bad arguments (M %d, kvh %d, max_ctx %d)", a.M, kvh, a.max_ctx);
-  const int blocks = (((a.M + 31) / 32 + 1) * kvh + 3) / 4;
-  if (hd == 256) kv4_group_quant_kernel<256><<<blocks, 128, 0, st>>>(a, kvh);
-  else if (hd == 128) kv4_group_quant_kernel<128><<<blocks, 128, 0, st>>>(a, kvh);
-  else if (hd == 64) kv4_group_quant_kernel<64><<<blocks, 128, 0, st>>>(a, kvh);
-  else KV4_REJECT("yskn_kv4_group_quant: unsupported head_dim %d (64, 128, 256)", hd);   // src/attention_gqa.cu:186
-  return launch_status("kv4_group_quant_kernel");
+  const dim3 blocks((unsigned)((((a.M + 31) / 32 + 1) * kvh + 3) / 4));
+  const char* who = "kv4_group_quant_kernel";
+  if (hd == 256) return launch_pdl(who, kv4_group_quant_kernel<256>, blocks, 128, 0, st, a, kvh);
+  if (hd == 128) return launch_pdl(who, kv4_group_quant_kernel<128>, blocks, 128, 0, st, a, kvh);
+  if (hd == 64) return launch_pdl(who, kv4_group_quant_kernel<64>, blocks, 128, 0, st, a, kvh);
+  KV4_REJECT("yskn_kv4_group_quant: unsupported head_dim %d (64, 128, 256)", hd);   // src/attention_gqa.cu:186
 }
 
 int launch_append(const yskn_kv_append_args& a, cudaStream_t st) {
