@@ -397,6 +397,12 @@ YSKN_KV4_API int yskn_kv8_attention(const yskn_kv8_attn_args* a, int act_dtype, 
  * fp16 operand tiles (byte times scale, rounded once to fp16); q16 fp16 or bf16; q16 and pacc 16-byte aligned; `splits`
  * partitions the 128-key tiles below *d_pos.  yskn_kv8_attention takes this route by itself for M > 8. */
 YSKN_KV4_API int yskn_kv8_attention_tc(const yskn_kv8_attn_args* a, int act_dtype, void* cuda_stream);
+/* yskn_kv8_attention_tc over a caller-owned workspace of 1,024 * kvh * max_ctx bytes (16-byte aligned; its contents need not survive the
+ * call's work on the stream): the visible keys become fp16 rows once, in a launch of their own, instead of once per 256 query
+ * rows.  Same operands bit for bit, same partials.  yskn_kv8_workspace_bytes: that size where the pass is the faster for it (more than
+ * 64 rows, and at most 1 GiB), 0 where yskn_kv8_attention is to be called as it is. */
+YSKN_KV4_API size_t yskn_kv8_workspace_bytes(const yskn_kv8_attn_args* a);
+YSKN_KV4_API int yskn_kv8_attention_ws(const yskn_kv8_attn_args* a, int act_dtype, void* d_workspace, size_t workspace_bytes, void* cuda_stream);
 
 /* Merge of the splits as launch_q35_combine does up to the gated row (src/q35_kernels.cu:1400-1424): y = o / L, inverse
  * rotation if inverse_rotate != 0, rounding to the activation dtype, then y * sigmoid(gate) with the reference's roundings

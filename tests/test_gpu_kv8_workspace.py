@@ -1,0 +1,62 @@
+"""Long passes over INT8 rows from fp16 rows written once (yskn_kv8_attention_ws) against the converting form: equal partials bit for
+bit, at the edges of the row tiles and key tiles, and where no memory may be taken (a stream under capture)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+NH, KVH = 24, 4
+
+
+def _case(ctx, M, dtype, seed, max_ctx=None):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    max_ctx = max_ctx or (ctx + M + 63) // 64 * 64
+    k8, v8 = (torch.randint(-127, 128, (KVH, max_ctx, 256), generator=g, device="cuda", dtype=torch.int8) for _ in range(2))
+    ks, vs = (torch.rand((KVH, max_ctx), generator=g, device="cuda") * 0.02 + 1e-3 for _ in range(2))
+    ks[:, ctx + M:], vs[:, ctx + M:] = float("nan"), float("nan")          # rows that do not exist yet
+    q = torch.randn((M, NH, 256), generator=g, device="cuda").to(dtype)
+    return q, k8, v8, ks, vs, torch.tensor([ctx], dtype=torch.int32, device="cuda")
+
+
+def _converting(c, M, S, out):
+    """The C entry without a workspace."""
+    import ctypes as C
+    from yasakani_b200 import _lib
+    q, k8, v8, ks, vs, pos = c
+    a = _lib.Kv8AttnArgsC(q.data_ptr(), k8.data_ptr(), v8.data_ptr(), ks.data_ptr(), vs.data_ptr(), k8.shape[1], M, pos.data_ptr(), S, *(t.data_ptr() for t in out),
+                          KVH, NH, 0.0625)
+    dt = {torch.float16: 0, torch.bfloat16: 1}[q.dtype]
+    assert _lib.load().yskn_kv8_attention_tc(C.byref(a), dt, torch.cuda.current_stream().cuda_stream) == 0
+
+
+@pytest.mark.parametrize("ctx,M,S", [(0, 65, 1), (0, 128, 2), (63, 65, 3), (127, 85, 1), (1000, 169, 1), (3001, 300, 2), (4096, 64, 5), (640, 8, 3)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_partials_equal_the_converting_form(ctx, M, S, dtype):
+    from yasakani_b200 import kv4, kvx
+    c = _case(ctx, M, dtype, seed=ctx + M)
+    outs = []
+    for f in (lambda o: kvx.launch_kv8_attention_tc(*c[:5], M, c[5], S, *o, NH), lambda o: _converting(c, M, S, o)):
+        out = [torch.full_like(t, float("nan")) for t in kv4.attn_scratch(M, S, NH, 256)]
+        f(out)
+        outs.append([t.view(torch.int32) for t in out])
+    assert torch.isfinite(outs[0][2].view(torch.float32)).all()
+    assert all(torch.equal(a, b) for a, b in zip(*outs)) and kv4.device_status() == 0
+
+
+def test_other_stream_and_capture_give_the_same_rows():
+    from yasakani_b200 import kv4, kvx
+    M, S, c = 100, 1, _case(500, 100, torch.bfloat16, seed=3)
+    want = kv4.attn_scratch(M, S, NH, 256)
+    kvx.launch_kv8_attention(*c[:5], M, c[5], S, *want, NH)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    got = kv4.attn_scratch(M, S, NH, 256)
+    kvx.launch_kv8_attention(*c[:5], M, c[5], S, *got, NH, stream=side)
+    side.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+    graphed = kv4.attn_scratch(M, S, NH, 256)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        kvx.launch_kv8_attention(*c[:5], M, c[5], S, *graphed, NH)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, graphed))

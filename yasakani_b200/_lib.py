@@ -123,6 +123,8 @@ PROTOTYPES = {
                                  C.c_void_p, C.c_size_t, C.c_void_p]),
     "yskn_kv8_attention": (C.c_int, [C.POINTER(Kv8AttnArgsC), C.c_int, C.c_void_p]),
     "yskn_kv8_attention_tc": (C.c_int, [C.POINTER(Kv8AttnArgsC), C.c_int, C.c_void_p]),
+    "yskn_kv8_workspace_bytes": (C.c_size_t, [C.POINTER(Kv8AttnArgsC)]),
+    "yskn_kv8_attention_ws": (C.c_int, [C.POINTER(Kv8AttnArgsC), C.c_int, C.c_void_p, C.c_size_t, C.c_void_p]),
     "yskn_kv8_combine": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p]),
     "yskn_kv4_attention_host": (C.c_int, [C.c_void_p, C.POINTER(KvLayerC), C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p,
                                           C.c_int, C.c_int, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p, C.c_int,

@@ -26,8 +26,9 @@
 //     Tiles that contain a row's own group ("edge" tiles) get S twice, from Kd and from Ks, and each row picks per
 //     32-key group: int4 keys for groups before its own, shadow keys (causally masked) for its own.
 //
-//  The attention kernel has four forms (template FORM): 0 = operand tiles by TMA from the workspace, as above (3 = the same
-//  with bf16 queries and output rows: the softmax warps convert the queries, there is no Q copy); 1 = no
+//  The attention kernel has five forms (template FORM): 0 = operand tiles by TMA from the workspace, as above (3 = the same
+//  with bf16 queries and output rows: the softmax warps convert the queries, there is no Q copy; 4 = the same over a workspace of
+//  Family-B INT8 rows); 1 = no
 //  workspace and no prep launch, converter warps build the tiles from the packed KV4 cache inside the kernel; 2 = the same over
 //  Family-B INT8 rows.  The converting forms run 16 warps: 0-7 softmax, 8 Q copy + MMA issue, 9-11 V tiles, 12-15 K tiles.
 //
@@ -310,6 +311,23 @@ __device__ __forceinline__ void tc_row_to_pairs(const uint4& v, uint32_t (&o)[4]
   o[0] = __byte_perm(v.x, v.z, 0x5410); o[1] = __byte_perm(v.x, v.z, 0x7632); o[2] = __byte_perm(v.y, v.w, 0x5410); o[3] = __byte_perm(v.y, v.w, 0x7632);
 }
 __host__ __device__ constexpr int tc_col(int c) { return (c & ~7) | ((c & 3) << 1) | ((c >> 2) & 1); }     // operand column that holds channel c
+// 16 INT8 bytes of a row times its scale as 16 fp16 operands (channels 0-7 and 8-15 of the chunk); zero when not live.
+__device__ __forceinline__ void tc_i8_chunk(const uint4& w, float sf, bool live, uint4& lo, uint4& hi) {
+  // the row's scale as a sum of two fp16 numbers: b * scale = fma(b, hi, b * lo) is then rounded once, without the
+  // per-row relative error of up to 2^-11 that a scale rounded to fp16 alone would put on all 256 channels of the row
+  const float sh = __half2float(__float2half_rn(sf));
+  const uint32_t s_hi = tc_pack(sh, sh), s_lo = tc_pack(sf - sh, sf - sh);
+  const uint32_t ww[4] = {w.x ^ 0x80808080u, w.y ^ 0x80808080u, w.z ^ 0x80808080u, w.w ^ 0x80808080u};
+  uint32_t r[8];
+  #pragma unroll
+  for (int e = 0; e < 4; ++e) {                                      // byte b -> 0x64bb = 1152 + b (b two's complement, top bit flipped)
+    const uint32_t n0 = tc_hadd2(__byte_perm(ww[e], 0x64646464u, 0x4140), 0xE480E480u), n1 = tc_hadd2(__byte_perm(ww[e], 0x64646464u, 0x4342), 0xE480E480u);
+    r[2 * e] = tc_hfma2(n0, s_hi, tc_hmul2(n0, s_lo));
+    r[2 * e + 1] = tc_hfma2(n1, s_hi, tc_hmul2(n1, s_lo));
+  }
+  lo = live ? make_uint4(r[0], r[1], r[2], r[3]) : make_uint4(0u, 0u, 0u, 0u);
+  hi = live ? make_uint4(r[4], r[5], r[6], r[7]) : make_uint4(0u, 0u, 0u, 0u);
+}
 // Global loads as ordered asm statements: the compiler keeps them where they are written, ahead of the arithmetic.
 __device__ __forceinline__ uint32_t tc_ldg32(const void* p) { uint32_t v; asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
 __device__ __forceinline__ uint32_t tc_ldg16(const void* p) { unsigned short v; asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p)); return v; }
@@ -349,6 +367,27 @@ __device__ __forceinline__ void tc_stage_q(uint32_t sq, int q_block, const uint1
     }
   }
 }
+// ------------------------------------------------------------------------------------------------ INT8 rows -> fp16 workspace
+// K and V rows of every visible key as fp16 operand rows, by the very rule of the converting form (tc_i8_chunk: the two forms' operands
+// are equal bit for bit); zero rows up to the tile boundary.  HBM-bound byte mover (260 bytes in, 512 out per row): a thread takes
+// 16 channels of one row; rows past the last tile return at once.
+__global__ void __launch_bounds__(256) kv8_tc_prep_kernel(const int8_t* k8, const int8_t* v8, const float* ks, const float* vs, const int* d_pos, int M,
+                                                          int max_ctx, uint16_t* kd, uint16_t* vd) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int t = (int)blockIdx.x * 16 + (int)(threadIdx.x >> 4), c = (int)(threadIdx.x & 15);     // grid (max_ctx / 16, kv-heads, K | V)
+  const int end = min(max_ctx, *d_pos + M), end_tile = min(max_ctx, (end + TC_BN - 1) / TC_BN * TC_BN);
+  if (t >= end_tile) return;
+  const size_t row = (size_t)blockIdx.y * max_ctx + t;
+  const bool is_v = blockIdx.z != 0;
+  const uint4 w = __ldg(reinterpret_cast<const uint4*>((is_v ? v8 : k8) + row * 256) + c);
+  const float sf = __ldg((is_v ? vs : ks) + row);
+  uint4 lo, hi;
+  tc_i8_chunk(w, sf, t < end, lo, hi);
+  uint4* dst = reinterpret_cast<uint4*>((is_v ? vd : kd) + row * 256) + 2 * c;
+  dst[0] = lo; dst[1] = hi;
+}
+
 // ------------------------------------------------------------------------------------------------ attention kernel
 constexpr int TC_SW = 8;                                   // softmax warps: warp w owns rows 32*(w%4).., key columns 64*(w/4)..
 constexpr int TC_KW = 4, TC_VW = 3, TC_CW = TC_KW + TC_VW;  // converter warps of the fused forms: K half tiles, V half tiles
@@ -407,13 +446,15 @@ struct TcP {
 // nothing is rotated at read time and there is no shadow, so every tile has one K item and the tiles that hold the new
 // rows are masked causally.  A byte is read as the fp16 number 1152 + b by one byte permute, the offset leaves by an exact
 // subtraction, and the row's scale (rounded to fp16) is multiplied in.
+// FORM 4: FORM 3 over INT8 rows: kv8_tc_prep_kernel has written K and V as fp16 rows.  Long passes convert every key once instead of once per
+// 256 query rows.
 template <int HD, int FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc_threads(FORM == 1 || FORM == 2), 1)
 kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapKd,
                    const __grid_constant__ CUtensorMap mapVd, const __grid_constant__ CUtensorMap mapKs, const TcP P) {
   using L = TcLay<HD>;
-  constexpr bool FUSED = FORM == 1 || FORM == 2, I8 = FORM == 2;
-  const bool act_bf16 = FUSED ? P.bf16 != 0 : FORM == 3;              // a compile-time constant in the workspace forms
+  constexpr bool FUSED = FORM == 1 || FORM == 2, I8 = FORM == 2 || FORM == 4;
+  const bool act_bf16 = FUSED || FORM == 4 ? P.bf16 != 0 : FORM == 3; // a compile-time constant in the workspace forms over the int4 cache
   constexpr bool STAGED_Q = FORM != 0;
   static_assert(!I8 || HD == 256, "INT8 rows have 256 channels");
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -486,7 +527,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       int kit = 0; bool ok = true;
       for (int i = 0; i < n && ok; ++i) {
         const int j = j0 + i;
-        for (int half = 0; half < (i >= nbulk ? 2 : 1) && ok; ++half, ++kit) {      // Kd; edge tiles: then Ks
+        for (int half = 0; half < (i >= npipe ? 2 : 1) && ok; ++half, ++kit) {      // Kd; edge tiles: then Ks
           const int st = kit % L::NK;
           if (kit >= L::NK && !bar_wait(b_kempty + 8 * st, (kit / L::NK - 1) & 1)) { atomicExch(&g_tc_status, 6); *s_abort = 1; ok = false; break; }
           if (*s_abort) { ok = false; break; }
@@ -589,22 +630,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     // INT8 rows: item = (key, 16-byte chunk = 16 channels) -> two 16-byte chunks of fp16; cur holds this tile's items, each
     // next-tile item is requested right before the same item of this tile is converted
     struct I8In { uint4 w; uint32_t s; };
-    auto i8_convert = [&](const I8In& I, bool live, uint4& lo, uint4& hi) {      // channels 0-7 and 8-15 of the chunk
-      // the row's scale as a sum of two fp16 numbers: b * scale = fma(b, hi, b * lo) is then rounded once, without the
-      // per-row relative error of up to 2^-11 that a scale rounded to fp16 alone would put on all 256 channels of the row
-      const float sf = __uint_as_float(I.s), sh = __half2float(__float2half_rn(sf));
-      const uint32_t s_hi = tc_pack(sh, sh), s_lo = tc_pack(sf - sh, sf - sh);
-      const uint32_t ww[4] = {I.w.x ^ 0x80808080u, I.w.y ^ 0x80808080u, I.w.z ^ 0x80808080u, I.w.w ^ 0x80808080u};
-      uint32_t r[8];
-      #pragma unroll
-      for (int e = 0; e < 4; ++e) {                                  // byte b -> 0x64bb = 1152 + b (b two's complement, top bit flipped)
-        const uint32_t n0 = tc_hadd2(__byte_perm(ww[e], 0x64646464u, 0x4140), 0xE480E480u), n1 = tc_hadd2(__byte_perm(ww[e], 0x64646464u, 0x4342), 0xE480E480u);
-        r[2 * e] = tc_hfma2(n0, s_hi, tc_hmul2(n0, s_lo));
-        r[2 * e + 1] = tc_hfma2(n1, s_hi, tc_hmul2(n1, s_lo));
-      }
-      lo = live ? make_uint4(r[0], r[1], r[2], r[3]) : make_uint4(0u, 0u, 0u, 0u);
-      hi = live ? make_uint4(r[4], r[5], r[6], r[7]) : make_uint4(0u, 0u, 0u, 0u);
-    };
+    auto i8_convert = [&](const I8In& I, bool live, uint4& lo, uint4& hi) { tc_i8_chunk(I.w, __uint_as_float(I.s), live, lo, hi); };
     if (n > 0 && is_k) {
       // ------------------------------------------------------------------- K role
       if constexpr (I8) {
@@ -1318,14 +1344,19 @@ int launch_attention_tc_fused(const yskn_attn_g_args& a, int g, int hd, int rd, 
   return hd == 256 ? launch_tc_fused_hd<256>(a, g, rd, bf16, o16_direct, bv, st) : launch_tc_fused_hd<128>(a, g, rd, bf16, o16_direct, bv, st);
 }
 
-// Many-row attention over Family-B INT8 rows on the tcgen05 kernel (FORM 2): partials in the layout of yskn_kv8_attention.
-int launch_kv8_attention_tc(const yskn_kv8_attn_args& a, int act_dtype, cudaStream_t st) {
+static int check_kv8_tc(const yskn_kv8_attn_args& a, int act_dtype) {
   if (!a.q16 || !a.k8 || !a.v8 || !a.ks || !a.vs || !a.d_pos || !a.pm || !a.pl || !a.pacc) KV4_REJECT("yskn_kv8_attention_tc: null buffer");
   if (a.kvh <= 0 || a.nh <= 0 || a.nh % a.kvh || a.nh / a.kvh > 8 || a.M <= 0 || a.M > 65535 || a.kvh > 65535 || a.splits <= 0 || a.splits > 65535 ||
       a.max_ctx <= 0 || a.max_ctx % 64)
     KV4_REJECT("yskn_kv8_attention_tc: bad shape (kvh %d, nh %d, M %d, splits %d, max_ctx %d)", a.kvh, a.nh, a.M, a.splits, a.max_ctx);
   if (act_dtype != YSKN_KV4_F16 && act_dtype != YSKN_KV4_BF16) KV4_REJECT("yskn_kv8_attention_tc: q16 is fp16 or bf16 (act_dtype %d)", act_dtype);
   if (((uintptr_t)a.k8 | (uintptr_t)a.v8 | (uintptr_t)a.q16 | (uintptr_t)a.pacc) & 15) KV4_REJECT("yskn_kv8_attention_tc: k8, v8, q16 and pacc must be 16-byte aligned");
+  return 0;
+}
+
+// Many-row attention over Family-B INT8 rows on the tcgen05 kernel (FORM 2): partials in the layout of yskn_kv8_attention.
+int launch_kv8_attention_tc(const yskn_kv8_attn_args& a, int act_dtype, cudaStream_t st) {
+  if (int rc = check_kv8_tc(a, act_dtype)) return rc;
   using L = TcLay<256>;
   const int g = a.nh / a.kvh, bf16 = act_dtype == YSKN_KV4_BF16;
   CUtensorMap mq;                                                     // unused: the softmax warps stage Q
@@ -1338,6 +1369,33 @@ int launch_kv8_attention_tc(const yskn_kv8_attn_args& a, int act_dtype, cudaStre
         a.q16, bf16, a.k8, a.v8, a.ks, a.vs};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), tc_threads(true), L::TOTAL, st, mq, mq, mq, mq, P)) return rc;
   return launch_status("kv4_tc_attn_kernel (INT8 rows)");
+}
+
+size_t kv8_tc_workspace_bytes(int kvh, int max_ctx) { return (size_t)2 * kvh * max_ctx * 512; }
+
+// The same over a caller's workspace: one launch that writes the fp16 rows of all visible keys, then FORM 4.
+int launch_kv8_attention_tc_ws(const yskn_kv8_attn_args& a, int act_dtype, void* ws, size_t ws_bytes, cudaStream_t st) {
+  if (int rc = check_kv8_tc(a, act_dtype)) return rc;
+  if (!ws || ws_bytes < kv8_tc_workspace_bytes(a.kvh, a.max_ctx)) KV4_REJECT("yskn_kv8_attention_ws: workspace of %zu bytes needed, %zu given",
+                                                                           kv8_tc_workspace_bytes(a.kvh, a.max_ctx), ws ? ws_bytes : (size_t)0);
+  if ((uintptr_t)ws & 15) KV4_REJECT("yskn_kv8_attention_ws: the workspace must be 16-byte aligned");
+  using L = TcLay<256>;
+  uint16_t* kd = static_cast<uint16_t*>(ws); uint16_t* vd = kd + (size_t)a.kvh * a.max_ctx * 256;
+  if (int rc = launch_pdl("kv8_tc_prep_kernel", kv8_tc_prep_kernel, dim3((unsigned)(a.max_ctx / 16), (unsigned)a.kvh, 2), 256, 0, st,
+                          a.k8, a.v8, a.ks, a.vs, a.d_pos, a.M, a.max_ctx, kd, vd)) return rc;
+  CUtensorMap mq, mkd, mvd;
+  memset(&mq, 0, sizeof(mq));                                         // unused: the softmax warps stage Q
+  const uint64_t rows = (uint64_t)a.kvh * a.max_ctx;
+  if (!tc_map_rows(&mkd, kd, rows, 256, TC_BN / 2, L::KBLK) || !tc_map_rows(&mvd, vd, rows, 256, TC_BN, L::KBLK / 2))
+    KV4_REJECT("yskn_kv8_attention_ws: cuTensorMapEncodeTiled failed or is unavailable");
+  auto kern = kv4_tc_attn_kernel<256, 4>;
+  static std::atomic<unsigned long long> attr{0};
+  if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+  const int g = a.nh / a.kvh, tok = 128 / g, qtiles = ((a.M + tok - 1) / tok + 1) & ~1;
+  TcP P{a.d_pos, a.M, a.splits, g, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, nullptr, nullptr, yskn_kv_layer{}, nullptr, 0,
+        a.q16, act_dtype == YSKN_KV4_BF16, nullptr, nullptr, nullptr, nullptr};
+  if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), TC_THREADS, L::TOTAL, st, mq, mkd, mvd, mq, P)) return rc;
+  return launch_status("kv4_tc_attn_kernel (INT8 rows, workspace)");
 }
 
 int tc_status_fetch(int* out) {
