@@ -19,8 +19,8 @@
 //       warp 9      (leader CTA only) one thread issues every tcgen05.mma of the pair: S = Q.K^T (M256 N128 K16 steps, Q and
 //                   K from shared memory, K-major, 128-byte swizzle) into one of two TMEM buffers, and O += P.V (M256
 //                   N=HD, P from tensor memory, V as MN-major operand); commits arrive on both CTAs' barriers
-//       warps 0-7   two threads per query row (64 of the tile's 128 keys each): tcgen05.ld of the S row, masks, online
-//                   softmax in the log2 domain with a lazy rescale of O, P -> fp16 -> tensor memory over the S columns
+//       warps 0-7   two threads per query row (tiles in turn; in the converting forms 64 of each tile's 128 keys): tcgen05.ld
+//                   of the S row, masks, online softmax in the log2 domain with a lazy rescale of O, P -> fp16 -> tensor memory over the S columns
 //                   just read; final (m, l, O) store, or the finished fp16 row when there is a single split
 //     S of tile i+2 is issued right after P.V of tile i, so the tensor pipe works while the softmax warps run.
 //     Tiles that contain a row's own group ("edge" tiles) get S twice, from Kd and from Ks, and each row picks per
@@ -280,6 +280,24 @@ __device__ __forceinline__ void tmem_st32u(uint32_t taddr, const uint32_t (&v)[3
                  "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
                  "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
 }
+__device__ __forceinline__ void tmem_st16u(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+                 "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+// Two fp32 operations in one instruction, each rounded as the single one.
+__device__ __forceinline__ float2 tc_fma2(float2 a, float b, float c) {
+  float2 d;
+  asm("{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %4};\n mov.b64 c, {%5, %5};\n fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float2 tc_add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float tc_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ uint32_t tc_pack(float lo, float hi) { uint32_t d; asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo)); return d; }
@@ -393,7 +411,9 @@ constexpr int TC_SW = 8;                                   // softmax warps: war
 constexpr int TC_KW = 4, TC_VW = 3, TC_CW = TC_KW + TC_VW;  // converter warps of the fused forms: K half tiles, V half tiles
 // + producer warp, + MMA issuer warp; the fused form adds the converter warps and fills up to four warpgroups (16 warps x 128
 // registers at launch), so that setmaxnreg can move registers from the softmax warps (120 each) and the V converters (112) to the K converters (160)
-constexpr int tc_threads(bool fused) { return fused ? 512 : (TC_SW + 2) * 32; }
+// The workspace forms launch three warpgroups of 168 registers a thread (504 per scheduler lane): 208 for the two of softmax warps, whose threads hold
+// a whole row of a tile, 88 for producer and MMA issuer (two of its four warps have no role).
+constexpr int tc_threads(bool fused) { return fused ? 512 : 384; }
 static_assert(TC_SW == 8 && TC_SW + 1 + TC_CW <= 16, "warpgroups 0-1 = softmax warps, warpgroups 2-3 = Q copy + MMA issuer (one warp), converters");
 constexpr int TC_THREADS = tc_threads(false);
 
@@ -462,19 +482,22 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();                           // 0 = leader: issues the MMAs, owns the "full"/"ready" barriers
   // barriers (8 bytes each), same offsets in both CTAs:
-  //   leader's copy only: kfull[NK] vfull[NV] pready[2] qfull     each CTA's copy: kempty[NK] vempty[NV] sready[2] pvdone[2]
+  //   leader's copy only: kfull[NK] vfull[NV] pready[2] phalf[2] qfull     each CTA's copy: kempty[NK] vempty[NV] sready[2] pvdone[2]
   const uint32_t B0 = sb + L::OFF_BAR;
   const uint32_t b_kfull = B0, b_kempty = B0 + 32, b_vfull = B0 + 64, b_vempty = B0 + 96, b_sready = B0 + 128, b_pready = B0 + 144,
-                 b_pvdone = B0 + 160, b_q = B0 + 176;
+                 b_pvdone = B0 + 160, b_q = B0 + 176, b_phalf = B0 + 192;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + L::OFF_BAR + 184);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + L::OFF_BAR + 188);
-  const uint32_t lead_kfull = leader_addr(b_kfull), lead_vfull = leader_addr(b_vfull), lead_pready = leader_addr(b_pready), lead_q = leader_addr(b_q);
+  const uint32_t lead_kfull = leader_addr(b_kfull), lead_vfull = leader_addr(b_vfull), lead_pready = leader_addr(b_pready), lead_q = leader_addr(b_q),
+                 lead_phalf = leader_addr(b_phalf);
 
   if (sb & 1023u) { if (threadIdx.x == 0) atomicExch(&g_tc_status, 3); return; }   // same in both CTAs: nobody is left waiting
   if (threadIdx.x == 0) {
     for (int i = 0; i < L::NK; ++i) { bar_init(b_kfull + 8 * i, FUSED ? 2 * TC_KW : 1); bar_init(b_kempty + 8 * i, 1); }
     for (int i = 0; i < L::NV; ++i) { bar_init(b_vfull + 8 * i, FUSED ? 2 * TC_VW : 1); bar_init(b_vempty + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { bar_init(b_sready + 8 * i, 1); bar_init(b_pready + 8 * i, 2 * TC_SW); bar_init(b_pvdone + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) { bar_init(b_sready + 8 * i, 1); bar_init(b_pvdone + 8 * i, 1); }
+    // P of a tile: all softmax warps of both CTAs in the converting forms; the four of the tile's warpgroup otherwise, half of the keys at a time
+    for (int i = 0; i < 2; ++i) { bar_init(b_pready + 8 * i, FUSED ? 2 * TC_SW : TC_SW); bar_init(b_phalf + 8 * i, TC_SW); }
     bar_init(b_q, STAGED_Q ? 2 * TC_SW : 1);                         // queries that are converted or reordered are staged by the softmax warps
     *s_abort = 0;
     for (int i = 0; i < 128; ++i) reinterpret_cast<volatile uint32_t*>(smem + L::OFF_XCH + 2 * 2 * 128 * 4)[i] = 0;
@@ -577,14 +600,23 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       };
       auto issue_pv = [&](int tile_i, int buf) {                     // O (+)= P . V(tile_i), P from TMEM (over S[buf])
         const int st = tile_i % L::NV;
-        if (!__all_sync(0xffffffffu, bar_wait(b_pready + 8 * (tile_i & 1), (tile_i >> 1) & 1))) { fail(); return; }
+        if (!__all_sync(0xffffffffu, bar_wait((FUSED ? b_pready : b_phalf) + 8 * (tile_i & 1), (tile_i >> 1) & 1))) { fail(); return; }
         if (!__all_sync(0xffffffffu, bar_wait(b_vfull + 8 * st, (tile_i / L::NV) & 1))) { fail(); return; }
         tc_fence_after();
         const uint64_t vd = vdesc0 + (uint64_t)((st * L::V_HALF) >> 4);
         const uint32_t pcol = buf ? L::TM_S1 : L::TM_S0;
+        if constexpr (!FUSED) {                                      // keys 0-63 while the softmax warps work on the rest
+          if (leader) {
+            #pragma unroll
+            for (int ks = 0; ks < TC_BN / 32; ++ks) umma2_ts(L::TM_O, pcol + 8 * ks, vd + (uint64_t)((ks * 2048) >> 4), ID_PV, (tile_i | ks) ? 1u : 0u);
+          }
+          __syncwarp();
+          if (!__all_sync(0xffffffffu, bar_wait(b_pready + 8 * (tile_i & 1), (tile_i >> 1) & 1))) { fail(); return; }
+          tc_fence_after();
+        }
         if (leader) {
           #pragma unroll
-          for (int ks = 0; ks < TC_BN / 16; ++ks)                    // P columns: keys 0-63 at +0.., keys 64-127 at +64..
+          for (int ks = FUSED ? 0 : TC_BN / 32; ks < TC_BN / 16; ++ks)   // P columns: keys 0-63 at +0.., keys 64-127 at +64..
             umma2_ts(L::TM_O, pcol + 64 * (ks >> 2) + 8 * (ks & 3), vd + (uint64_t)((ks * 2048) >> 4), ID_PV, (tile_i | ks) ? 1u : 0u);
           umma2_commit(b_pvdone + 8 * (tile_i & 1));                 // O may be rescaled
           umma2_commit(b_vempty + 8 * st);                           // the V halves may be overwritten
@@ -1037,9 +1069,121 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       atomicExch(&g_tc_status, 4); *s_abort = 1;
       return v;
     };
-    float m = -1e30f, l = 0.f;                                       // m is common to the row's two threads, l is this half's sum
-    int srd[2] = {0, 0};                                             // how often each S buffer has been read
+    float m = -1e30f, l = 0.f;                                       // m is common to the row's two threads, l is this thread's share of the sum
     bool ok = true;
+    if constexpr (!FUSED) {
+      // Workspace forms: the two warpgroups take the tiles in turn, a thread takes all 128 keys of its row.  A scheduler has one warp of each, so
+      // the loads, the maximum and the stores of one tile run under the exponentials of the other (1,024 cycles a tile at 16 per clock and SM, which the
+      // tensor pipe's 2,057 leave room for).  What passes from tile to tile is the running maximum, known well before the
+      // exponentials: tile i waits for m of tile i-1 from the other warpgroup.  P of keys 0-63 is published before the rest is computed.
+      // With both warpgroups on the same tile (64 keys a thread, maxima swapped) the chain S -> softmax -> P.V was the pace: 8,192 causal rows
+      // with their append 815-839 -> 798 us, 1,000 INT8 rows behind 3,001 tokens 152 -> 149 us.
+      float mown = -1e30f;                                           // the maximum that l refers to
+      auto wait_tag = [&](int slot, int tag) {                       // bounded; slot = the warpgroup that publishes
+        for (uint32_t it = 0; it < TC_WAIT_LIMIT; ++it)
+          if ((uint16_t)(xseq[slot * 128 + rho] - (uint16_t)tag) < 0x8000u) { __threadfence_block(); return true; }
+        atomicExch(&g_tc_status, 4); *s_abort = 1;
+        return false;
+      };
+      // Edge tiles, which use both S buffers, all belong to warpgroup 0: it has seen every earlier phase of buffer 0, and S in buffer 0 being
+      // ready implies that every earlier S of buffer 1 is, so no parity is ever waited for two phases ahead.
+      const int i0 = hf < npipe ? hf : hf == 0 ? npipe : n;
+      #pragma unroll 1
+      for (int i = i0; i < n && ok; i = i >= npipe ? i + 1 : i + 2 < npipe ? i + 2 : hf == 0 ? npipe : n) {
+        const int j = j0 + i;
+        const bool edge = i >= npipe;
+        const int buf = edge ? 0 : hf, e = i - npipe;                // edge tile e uses both buffers once
+        const uint32_t scol = trow + (buf ? L::TM_S1 : L::TM_S0);
+        float x[128];
+        float (&x0)[64] = *reinterpret_cast<float (*)[64]>(x); float (&x1)[64] = *reinterpret_cast<float (*)[64]>(x + 64);
+        if (!bar_wait(b_sready + 8 * buf, (edge ? (npipe + 1) / 2 + e : i >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
+        tc_fence_after();
+        tmem_ld64(scol, x0); tmem_ld64(scol + 64, x1);
+        if (edge) {
+          if (!bar_wait(b_sready + 8, (npipe / 2 + e) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
+          tc_fence_after();
+          // each 32-key quarter is one group: before the row's own -> int4 keys; own group -> shadow keys up to the row; later -> nothing
+          #pragma unroll
+          for (int h4 = 0; h4 < 4; ++h4) {
+            float a[32];
+            tmem_ld32(trow + L::TM_S1 + 32 * h4, a);
+            const int gk = 4 * j + h4, tb = j * TC_BN + 32 * h4;
+            #pragma unroll
+            for (int k = 0; k < 32; ++k) x[32 * h4 + k] = gk < cr ? x[32 * h4 + k] : (gk == cr && tb + k <= pr) ? a[k] : -INFINITY;
+          }
+        }
+        if (I8 && i >= nbulk) {                                      // INT8 rows: the tiles that hold the new rows are masked causally
+          const int tb = j * TC_BN;
+          #pragma unroll
+          for (int k = 0; k < 128; ++k) x[k] = tb + k <= pr ? x[k] : -INFINITY;
+        }
+        // ---- online softmax in the log2 domain on p = 2^(x*cs - m); lazy rescale (the running max may lag by up to 2^8)
+        float tm4[4] = {x[0], x[1], x[2], x[3]};
+        #pragma unroll
+        for (int k = 4; k < 128; k += 8)
+          #pragma unroll
+          for (int q = 0; q < 4; ++q) tm4[q] = k + 4 + q < 128 ? fmaxf(tm4[q], fmaxf(x[k + q], x[k + 4 + q])) : fmaxf(tm4[q], x[k + q]);
+        const float tmax = fmaxf(fmaxf(tm4[0], tm4[1]), fmaxf(tm4[2], tm4[3])) * cs;
+        if (i > 0 && (i > npipe ? 0 : (i - 1) & 1) != hf) {          // the tile before this one is the other warpgroup's
+          if (!__all_sync(0xffffffffu, wait_tag(hf ^ 1, i))) { ok = false; break; }
+          m = xval[(hf ^ 1) * 128 + rho];
+        }
+        const bool bump = valid && tmax > m + 8.f;
+        const float alpha = bump ? tc_ex2(m - tmax) : 1.f;
+        if (bump) m = tmax;
+        xval[hf * 128 + rho] = m;                                    // read by the other warpgroup before this one's next tile can publish
+        __threadfence_block();
+        xseq[hf * 128 + rho] = (uint16_t)(i + 1);
+        if (mown != m) { l *= tc_ex2(mown - m); mown = m; }
+        // ---- O may be rescaled once P.V of tile i-1 is done (P.V of this tile waits for the signals below)
+        if (i > 0 && __any_sync(0xffffffffu, bump)) {                // rows that did not bump multiply by exactly 1
+          if (!bar_wait(b_pvdone + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
+          tc_fence_after();
+          #pragma unroll 1
+          for (int c = 0; c < HD / 32; ++c) {
+            float o[32];
+            tmem_ld32(trow + L::TM_O + 32 * c, o);
+            #pragma unroll
+            for (int k = 0; k < 32; ++k) o[k] *= alpha;
+            tmem_st32(trow + L::TM_O + 32 * c, o);
+          }
+        }
+        const float nm = -m;
+        float2 ls0 = make_float2(0.f, 0.f), ls1 = ls0;
+        #pragma unroll
+        for (int c = 0; c < 4; ++c) {                                // 32 keys: P as the A operand of P.V, over S columns this thread has read
+          uint32_t pk[16];
+          #pragma unroll
+          for (int k = 0; k < 32; k += 4) {
+            float2 a = tc_fma2(make_float2(x[32 * c + k], x[32 * c + k + 1]), cs, nm), b = tc_fma2(make_float2(x[32 * c + k + 2], x[32 * c + k + 3]), cs, nm);
+            a.x = tc_ex2(a.x); a.y = tc_ex2(a.y); b.x = tc_ex2(b.x); b.y = tc_ex2(b.y);          // exp2(-inf) = 0 for masked keys
+            ls0 = tc_add2(ls0, a); ls1 = tc_add2(ls1, b);
+            pk[k / 2] = valid ? tc_pack(a.x, a.y) : 0u; pk[k / 2 + 1] = valid ? tc_pack(b.x, b.y) : 0u;   // rows of the tile that hold no query: P = 0
+          }
+          tmem_st16u(scol + 64 * (c >> 1) + 16 * (c & 1), pk);
+          if (c & 1) {
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) bar_arrive_cluster((c == 1 ? lead_phalf : lead_pready) + 8 * (i & 1));
+          }
+        }
+        l = valid ? l + ((ls0.x + ls0.y) + (ls1.x + ls1.y)) : 0.f;
+      }
+      if (ok && n > 0) {                                             // the row's maximum and the sum of both shares
+        if ((n > npipe ? 0 : (n - 1) & 1) != hf) {
+          ok = __all_sync(0xffffffffu, wait_tag(hf ^ 1, n));
+          if (ok) m = xval[(hf ^ 1) * 128 + rho];
+        }
+        if (mown != m) l *= tc_ex2(mown - m);
+        xval[256 + hf * 128 + rho] = l;
+        __threadfence_block();
+        xseq[hf * 128 + rho] = (uint16_t)(n + 1);
+        if (ok) ok = __all_sync(0xffffffffu, wait_tag(hf ^ 1, n + 1));
+        if (ok) l = hf == 0 ? l + xval[256 + 128 + rho] : xval[256 + rho] + l;
+      }
+    } else {
+    int srd[2] = {0, 0};                                             // how often each S buffer has been read
     for (int i = 0; i < n && ok; ++i) {
       const int j = j0 + i;
       const bool edge = i >= npipe;
@@ -1113,10 +1257,11 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       __syncwarp();
       if (lane == 0) bar_arrive_cluster(lead_pready + 8 * (i & 1));
     }
+    }
     // ---- this split's result per (row, head): (m, l, O) partial, or the finished row when there is one split
     if (ok && n > 0 && !bar_wait(b_pvdone + 8 * ((n - 1) & 1), ((n - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; }
     tc_fence_after();
-    if (ok) l += swap_with_partner(l, n + 1);                        // the row's sum = the two halves' sums
+    if constexpr (FUSED) { if (ok) l += swap_with_partner(l, n + 1); }   // the row's sum = the two halves' sums
     if (ok && !*s_abort) {
       const size_t pidx = ((size_t)tok * S + split) * P.nh + kvh * G + head;
       const bool direct = P.o16 != nullptr && S == 1;                // one split: this CTA holds the whole row, finish it here
@@ -1164,9 +1309,12 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       if (warp == TC_SW) role_mma(); else role_conv(false);
     } else { asm volatile("setmaxnreg.inc.sync.aligned.u32 160;"); role_conv(true); }
   } else {
-    if (warp == TC_SW) role_producer();
-    else if (warp == TC_SW + 1) role_mma();
-    else role_softmax();
+    if (warp < TC_SW) { asm volatile("setmaxnreg.inc.sync.aligned.u32 208;"); role_softmax(); }
+    else {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+      if (warp == TC_SW) role_producer();
+      else if (warp == TC_SW + 1) role_mma();
+    }
   }
   tc_fence_before();
   __syncthreads();
