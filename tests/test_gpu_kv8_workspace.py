@@ -17,15 +17,19 @@ def _case(ctx, M, dtype, seed, max_ctx=None):
     return q, k8, v8, ks, vs, torch.tensor([ctx], dtype=torch.int32, device="cuda")
 
 
-def _converting(c, M, S, out):
-    """The C entry without a workspace."""
+def _entry(c, M, S, out, ws=None):
+    """The C entries: over a workspace, or converting without one."""
     import ctypes as C
     from yasakani_b200 import _lib
+    lib = _lib.load()
     q, k8, v8, ks, vs, pos = c
     a = _lib.Kv8AttnArgsC(q.data_ptr(), k8.data_ptr(), v8.data_ptr(), ks.data_ptr(), vs.data_ptr(), k8.shape[1], M, pos.data_ptr(), S, *(t.data_ptr() for t in out),
                           KVH, NH, 0.0625)
-    dt = {torch.float16: 0, torch.bfloat16: 1}[q.dtype]
-    assert _lib.load().yskn_kv8_attention_tc(C.byref(a), dt, torch.cuda.current_stream().cuda_stream) == 0
+    dt, st = {torch.float16: 0, torch.bfloat16: 1}[q.dtype], torch.cuda.current_stream().cuda_stream
+    assert lib.yskn_kv8_workspace_bytes(C.byref(a)) == (1024 * KVH * k8.shape[1] if M >= 384 else 0)
+    if ws is None:
+        return lib.yskn_kv8_attention_tc(C.byref(a), dt, st)
+    return lib.yskn_kv8_attention_ws(C.byref(a), dt, ws.data_ptr(), ws.numel(), st)
 
 
 def _assert_same(a, b, keys):
@@ -35,23 +39,25 @@ def _assert_same(a, b, keys):
     assert ((l0 - l1).abs() <= 2 * keys * 2.0 ** -24 * l1).all()
 
 
-@pytest.mark.parametrize("ctx,M,S", [(0, 65, 1), (0, 128, 2), (63, 65, 3), (127, 85, 1), (1000, 169, 1), (3001, 300, 2), (4096, 64, 5), (640, 8, 3)])
+@pytest.mark.parametrize("ctx,M,S", [(0, 65, 1), (0, 128, 2), (63, 65, 3), (127, 85, 1), (1000, 169, 1), (3001, 400, 2), (4096, 64, 5), (640, 8, 3)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_partials_equal_the_converting_form(ctx, M, S, dtype):
-    from yasakani_b200 import kv4, kvx
+    from yasakani_b200 import kv4
     c = _case(ctx, M, dtype, seed=ctx + M)
+    ws = torch.full((1024 * KVH * c[1].shape[1],), 0xFF, dtype=torch.uint8, device="cuda")     # fp16 NaN wherever nothing is written
     outs = []
-    for f in (lambda o: kvx.launch_kv8_attention_tc(*c[:5], M, c[5], S, *o, NH), lambda o: _converting(c, M, S, o)):
+    for w in (ws, None):
         out = [torch.full_like(t, float("nan")) for t in kv4.attn_scratch(M, S, NH, 256)]
-        f(out)
+        assert _entry(c, M, S, out, w) == 0
         outs.append(out)
     assert torch.isfinite(outs[0][2]).all() and kv4.device_status() == 0
     _assert_same(*outs, ctx + M)
+    assert _entry(c, M, S, outs[0], ws[:-16]) == -1 and _entry(c, M, S, outs[0], ws[8:]) == -1
 
 
 def test_other_stream_and_capture_give_the_same_rows():
     from yasakani_b200 import kv4, kvx
-    M, S, c = 100, 1, _case(500, 100, torch.bfloat16, seed=3)
+    M, S, c = 400, 1, _case(500, 400, torch.bfloat16, seed=3)
     want = kv4.attn_scratch(M, S, NH, 256)
     kvx.launch_kv8_attention(*c[:5], M, c[5], S, *want, NH)
     torch.cuda.synchronize()
@@ -66,4 +72,4 @@ def test_other_stream_and_capture_give_the_same_rows():
         kvx.launch_kv8_attention(*c[:5], M, c[5], S, *graphed, NH)
     graph.replay()
     torch.cuda.synchronize()
-    _assert_same(want, graphed, 600)                                       # the converting form
+    _assert_same(want, graphed, 900)                                       # the converting form

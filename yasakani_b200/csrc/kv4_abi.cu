@@ -74,7 +74,7 @@ static int attention_dispatch(const yskn_attn_g_args* a, int g, int hd, int rd, 
 
 using namespace kv4;
 
-constexpr int KV8_WS_MIN_ROWS = 64;
+constexpr int KV8_WS_MIN_ROWS = 384;
 constexpr size_t KV8_WS_MAX_BYTES = (size_t)1 << 30;
 
 extern "C" {
@@ -370,10 +370,12 @@ int yskn_kv8_attention_tc(const yskn_kv8_attn_args* a, int act_dtype, void* cuda
   return launch_kv8_attention_tc(*a, act_dtype, (cudaStream_t)cuda_stream);
 }
 // Converting inside the kernel costs every pair of 128-row tiles its own pass over the keys (4.0 us per 128 keys, against 1.5 from
-// fp16 rows); writing the rows first costs one pass over them.  1,000 rows
-// behind 3,001 tokens, with row epilogue and merge: 264 -> 152 us.
+// fp16 rows); writing the rows first costs a launch and one pass over them.  The host does not know how many keys are visible, so
+// the line lies where the written rows win for any number of them.  Attention alone, converting / written rows, in us, behind
+// 0 and 8,000 tokens: 127 rows 14.9 / 16.4 and 58 / 43; 300 rows 17.0 / 18.7 and 109 / 65; 500 rows 21.9 / 20.3 and 213 / 102; 1,000 rows
+// 48 / 39 and 416 / 197.  1,000 rows behind 3,001 tokens, with row epilogue and merge: 264 -> 149 us.
 size_t yskn_kv8_workspace_bytes(const yskn_kv8_attn_args* a) {
-  if (!a || a->M <= KV8_WS_MIN_ROWS || a->kvh <= 0 || a->max_ctx <= 0 || current_algo() == ALGO_SCALAR) return 0;
+  if (!a || a->M < KV8_WS_MIN_ROWS || a->kvh <= 0 || a->max_ctx <= 0 || current_algo() == ALGO_SCALAR) return 0;
   if (!a->q16 || !a->pacc || (((uintptr_t)a->q16 | (uintptr_t)a->pacc) & 15)) return 0;
   const size_t n = kv8_tc_workspace_bytes(a->kvh, a->max_ctx);
   return n <= KV8_WS_MAX_BYTES ? n : 0;
