@@ -80,6 +80,9 @@ template <int CPL> __device__ __forceinline__ void load_halves(const uint16_t* p
 template <int HD>
 __global__ void __launch_bounds__(128) kv4_tc_prep_kernel(PrepP P) {
   constexpr int CPL = HD / 32;
+  // programmatic dependent launch: the start is hidden behind the append's end, and the attention kernel's set-up behind this kernel's last blocks
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31;
   const int t = P.t_begin + (int)blockIdx.x * 4 + (int)(threadIdx.x >> 5), head = blockIdx.y;   // grid (tokens / 4, kv-heads)
   const int pos0 = *P.d_pos, end = pos0 + P.M;                      // tokens [0, end) exist
@@ -1418,8 +1421,7 @@ int launch_tc_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, const TcWs&
   PrepP pp{a.kv, a.d_pos, a.M, a.max_ctx, a.kvh, a.rope, rd, w.kd, w.vd, w.ks, w.ks_rows, valid_tokens, t_begin};
   const int span = a.max_ctx - t_begin;
   if (span <= 0) KV4_REJECT("yskn_kv4_attention_tc: valid_tokens %d is beyond max_ctx %d", valid_tokens, a.max_ctx);
-  kv4_tc_prep_kernel<HD><<<dim3((unsigned)((span + 3) / 4), (unsigned)a.kvh), 128, 0, st>>>(pp);
-  if (int rc = launch_status("kv4_tc_prep_kernel")) return rc;
+  if (int rc = launch_pdl("kv4_tc_prep_kernel", kv4_tc_prep_kernel<HD>, dim3((unsigned)((span + 3) / 4), (unsigned)a.kvh), 128, 0, st, pp)) return rc;
   CUtensorMap mq, mkd, mvd, mks;
   const uint64_t rows = (uint64_t)a.kvh * a.max_ctx;
   if (bf16) memset(&mq, 0, sizeof(mq));                               // the softmax warps stage Q
