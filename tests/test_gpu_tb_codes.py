@@ -25,6 +25,16 @@ def _with_largest_code(blob, top):
     return bytes(b)
 
 
+def _plain_groups(blob):
+    """The profile without mean rows, low-rank rows and guards."""
+    b = bytearray(blob)
+    off_g, = struct.unpack_from("<I", b, 40)
+    for g in range(128):
+        o, = struct.unpack_from("<I", b, off_g + 4 * g)
+        b[o + 3:o + 6] = bytes(3)
+    return bytes(b)
+
+
 @pytest.mark.parametrize("top", [1400, 1401, 2200])
 def test_encoder_key_widths(oracle, top):
     from yasakani_b200 import kvx
@@ -73,5 +83,70 @@ def test_attention_tiles(oracle, top, ctx, M, splits, stride):
     kvx.launch_kv8_combine(pm, pl, pacc, splits, M, nh, o16, inverse_rotate=False)
     want = oracle.rows_attention_exact(q.float().numpy(), rows[0], rows[1], ctx)
     err = np.abs(o16.float().cpu().numpy() - want)
-    # two fp16 parts carry 22 bits of queries and weights; what remains is fp32 sums (2e-5 here) and the fp16 rounding of the row (2^-11)
+    # queries and weights in fp32 accuracy: what remains is fp32 sums (2e-5 here) and the fp16 rounding of the row (2^-11)
     assert (err <= 5e-5 + 2.0 ** -10 * np.abs(want)).all(), err.max()
+
+
+def _packed_case(oracle, blob, scale, grp, ctx, M, q, seed, stride=160):
+    """Encoded rows (values times `scale`, an array that broadcasts over [key | value][kv-head][token]) with the oracle's unpacked rows; the
+    kernel's partials merged in 64 bits and the exact rows."""
+    from yasakani_b200 import kvx
+    prof, kvh, nh, n, splits = kvx.TrellisProfile(blob), 4, q.shape[1], ctx + M, 3
+    max_ctx = (n + 63) // 64 * 64
+    rng = np.random.default_rng(seed)
+    x = np.zeros((2, kvh, max_ctx, 256), np.float32)
+    x[:, :, :n] = rng.standard_normal((2, kvh, n, 256)) * np.broadcast_to(scale, (2, kvh, n))[..., None]
+    rows_pos = np.tile(np.arange(max_ctx, dtype=np.int32), kvh)
+    dev, rows = [], []
+    for i in range(2):
+        gr = np.repeat(grp[i], max_ctx).astype(np.int32)
+        _, pay, side = kvx.tb_encode(prof, *(torch.from_numpy(a).cuda() for a in (x[i].reshape(-1, 256), gr, rows_pos)), pay_stride=stride)
+        p40 = np.ascontiguousarray(pay.cpu().numpy().view(np.uint32).reshape(-1, stride // 4)[:, :40])
+        rows.append(oracle.tb_unpack(blob, gr, rows_pos, p40, side.cpu().numpy().view(np.uint32), x[i].reshape(-1, 256)).reshape(kvh, max_ctx, 256))
+        dev += [pay.view(kvh, max_ctx, stride), side.view(kvh, max_ctx, 2)]
+    pm = torch.full((M, splits, nh), float("nan"), device="cuda"); pl = pm.clone(); pacc = torch.full((M, splits, nh, 256), float("nan"), device="cuda")
+    kvx.launch_tb_attention(prof, q.cuda(), *dev, *(torch.from_numpy(a).cuda() for a in grp), M, torch.tensor([ctx], dtype=torch.int32, device="cuda"), splits,
+                            pm, pl, pacc, nh, *(torch.from_numpy(a).cuda() for a in x))
+    m, l, o = (t.double().cpu().numpy() for t in (pm, pl, pacc))
+    w = np.exp(m - m.max(1, keepdims=True))
+    got = (w[..., None] * o).sum(1) / (w * l).sum(1)[..., None]
+    return got, oracle.rows_attention_exact(q.float().numpy(), rows[0], rows[1], ctx).astype(np.float64)
+
+
+@pytest.mark.parametrize("values", [1e-6, 1e-3, 1e-2, 1.0, 1e3, "flat 1e4", "mixed", "outlier"])
+def test_attention_is_fp32_at_every_scale_of_the_values(oracle, values):
+    """Weights (probability x row scale x gain) and queries keep fp32 accuracy and range whatever the rows' scale: tiny and large values, scales
+    that differ by 2^30 inside a sequence, a large row that the softmax leaves out, and large flat rows (whose gain is 1, not 1 / 256)."""
+    ctx, M, nh = 900, 1, 24
+    rng = np.random.default_rng(7)
+    scale = np.ones((2, 1, ctx + M), np.float32)
+    grp = np.array([[10, 8, 0, 12], [3, 9, 5, 7]], np.int32)        # value groups of 5 / 3 / 5 / 4 bits, no flat one
+    q = torch.from_numpy(rng.standard_normal((M, nh, 256)).astype(np.float32)).bfloat16()
+    if values == "flat 1e4":
+        grp[1] = [15, 31, 47, 63]
+        scale[1] = 1e4
+    elif values == "mixed":
+        scale[1] = 2.0 ** rng.integers(-20, 11, ctx + M)
+    elif values == "outlier":                                       # a large value under a weight of about 2^-38
+        q = q * 8
+        scale[1, 0, 5], scale[0, 0, 5] = 2.0 ** 12, 1e-3
+    else:
+        scale[1] = values
+    # a profile without mean rows or low-rank rows: they do not scale with the values and would hide the codes' part
+    got, want = _packed_case(oracle, _plain_groups(make_blob()), scale, grp, ctx, M, q, 3)
+    rel = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
+    # An fp32 sum of 900 terms in runs of 16 (8 of them per warp) and 25 partial sums: at most 16 + 33 roundings of 2^-23 of the sum of
+    # magnitudes, which is up to 8 times the result here; scores of up to 2^5 carry 2^-24 x 24 roundings of the dot product.
+    assert (rel < 2e-5).all(), rel.max()
+
+
+@pytest.mark.parametrize("size", [1e-6, 1.0, 1e6])
+def test_attention_queries_of_any_size(oracle, size):
+    """bf16 queries beyond the range of fp16 and far below it, against keys that bring the scores back to ordinary size."""
+    ctx, M, nh = 300, 2, 32
+    scale = np.ones((2, 1, ctx + M), np.float32)
+    scale[0] = 1.0 / size if size > 1 else 1.0
+    q = torch.from_numpy((np.random.default_rng(11).standard_normal((M, nh, 256)) * size).astype(np.float32)).bfloat16()
+    got, want = _packed_case(oracle, _plain_groups(make_blob()), scale, np.array([[10, 8, 0, 12], [3, 9, 5, 7]], np.int32), ctx, M, q, 5)
+    rel = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
+    assert (rel < 2e-5).all(), rel.max()

@@ -333,7 +333,16 @@ __global__ void __launch_bounds__(256) tb_unpack_kernel(TbDecP A) {
 //   * products run on mma.sync m16n8k16, tokens x heads for the scores, channels x heads for the values.  The contraction order
 //     of the scores is free, so lane (g, j) reads chain j of tokens g and g + 8, and for the values half a chain of four tokens: every
 //     window offset is a compile-time constant per code width;
-//   * queries and weights enter as sums of two fp16 numbers (two MMAs), which keeps the fp32 accuracy of a scalar loop;
+//   * a query row is bf16 or fp16: brought to a maximum of 2^13 .. 2^14 by a power of two it is exact in fp16 (what lies 2^38 below that maximum
+//     apart), and power, qscale and log2(e) are put on the fp32 score;
+//   * a weight (probability x row scale x gain) enters as two fp16 numbers (two MMAs), an integer of up to 2^11 and the rest, after a power of two
+//     of its head (and warp) that keeps the largest weight of the sum between 2^9 and 2^11; an error of at most 2^-13 of that unit.  The power moves with
+//     the running maximum, and when a weight outgrows it, and leaves the sums in the merge entry.  Without it small values (row scale 0.01: 4e-3
+//     of the result) sat among fp16's subnormals and large flat ones overflowed;
+//   * the tensor core's accumulators truncate: a tile's products are summed on their own and added in rounded fp32, and the integer part of the weights makes its
+//     sum exact (below 2^24).  Carried from tile to tile the error grew with their number (2.3e-6 of a row at 30,011 tokens in 37 splits, 1e-4 in
+//     one), with a rounded fp16 in the place of the integer a bias of half a unit was left.  Error of a row against 64 bits, rms over 500 .. 32,768
+//     tokens in 37 splits: 2.9e-7 .. 4.6e-7, of a scalar fp32 loop over the same rows 4.9e-7 .. 7.1e-7;
 //   * the row terms of the unpack rule leave the loops: q.x = s * gain / 256 * sum_d q_d code_d + c0 (q.U0) + c1 (q.U1) + q.mu, and
 //     O = sum_t p_t s_t code_t + (sum p_t c0_t) U0 + (sum p_t c1_t) U1 + (sum p_t) mu.
 // Rows that the profile leaves unpacked (positions below the guard, at most 255; a group without packed rows) take the row path, a warp
@@ -343,11 +352,12 @@ constexpr int TBA_WARPS = 12;                                        // 3 per sc
 struct TbAttnP { yskn_tb_attn_args a; int G; };
 constexpr uint32_t TBA_TAB = 32768;                                  // bytes of a replicated table, and the alignment of its shared-memory address
 struct TbAttnSm {                                                    // in front of the tables
-  uint4 qf[16][32];                                                  // Q as B fragments: {hi b0, hi b1, lo b0, lo b1} of k-step s, lane
-  float q[8][260];                                                   // q * qscale * log2(e) in fp32 (row path, row terms)
+  uint2 qf[16][32];                                                  // Q x its head's power of two as B fragments of k-step s, lane
+  float q[8][260];                                                   // q in fp32 (row path, row terms)
   float cg[2][256];                                                  // codes of the key and of the value group (row path: x gain)
   float term[2][3][256];                                             // row terms U0, U1, mu of both groups, channel d at tba_slot(d)
-  float kq[3][8];                                                    // q.U0, q.U1, q.mu of the key group
+  float kq[4][8];                                                    // q.U0, q.U1, q.mu of the key group, x qscale * log2(e); that over the power of two in qf
+  int qmax[8];                                                       // largest |q| of a head, as bits
   int big;                                                           // some code does not fit fp16 exactly
 };
 constexpr int TBA_MS = 260;                                          // merge entry of a (warp, head): m, l, -, -, then channel d at tba_slot(d)
@@ -363,6 +373,11 @@ __device__ __forceinline__ void tba_mma(float (&c)[4], uint32_t a0, uint32_t a1,
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// Powers of two from 2^-120 to 2^120 by exponent; the exponent of a number (zero and subnormals: -127, infinities: 128).
+constexpr int TBA_EXP = 120;
+__device__ __forceinline__ int tba_exponent(float x) { return (int)((__float_as_uint(x) >> 23) & 255u) - 127; }
+__device__ __forceinline__ float tba_pow2(int e) { return __uint_as_float((unsigned)(min(max(e, -TBA_EXP), TBA_EXP) + 127) << 23); }
+__device__ __forceinline__ float tba_inverse(float pow2) { return __uint_as_float((254u << 23) - __float_as_uint(pow2)); }
 __device__ __forceinline__ uint32_t tba_transpose(uint32_t a) { uint32_t d; asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a)); return d; }
 
 // Where channel d sits in a merge entry and in the row terms: the eight lanes g of an access (channels 32g + c) fall into eight banks, the
@@ -395,10 +410,10 @@ template <int NWORD> __device__ __forceinline__ void tba_words(const uint32_t* p
 
 // Raw scores of a tile's 16 tokens: rows g and g + 8 of the tile, heads 2j and 2j + 1 (c[0] c[1] | c[2] c[3]).
 template <int KB>
-__device__ __forceinline__ void tba_scores(const uint32_t* ra, const uint32_t* rb, bool v16, uint32_t tab, const uint4* qf, float (&s)[4]) {
+__device__ __forceinline__ void tba_scores(const uint32_t* ra, const uint32_t* rb, bool v16, uint32_t tab, const uint2* qf, float (&s)[4]) {
   uint32_t wa[2 * KB], wb[2 * KB];
   tba_words(ra, v16, wa); tba_words(rb, v16, wb);
-  float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+  float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};      // two chains
   #pragma unroll
   for (int k = 0; k < 16; ++k) {                                     // k-step: values 4k .. 4k+3 of the chain
     uint32_t a[4], b[4];
@@ -407,14 +422,12 @@ __device__ __forceinline__ void tba_scores(const uint32_t* ra, const uint32_t* r
       a[e] = tba_lds((tba_window<KB>(wa, 0u, 4 * k + e) & 0x7F80u) | tab);
       b[e] = tba_lds((tba_window<KB>(wb, 0u, 4 * k + e) & 0x7F80u) | tab);
     }
-    const uint4 q = qf[k * 32];
-    const uint32_t a0 = __byte_perm(a[0], a[1], 0x5410), a1 = __byte_perm(b[0], b[1], 0x5410), a2 = __byte_perm(a[2], a[3], 0x5410),
-                   a3 = __byte_perm(b[2], b[3], 0x5410);
-    tba_mma(hi, a0, a1, a2, a3, q.x, q.y);
-    tba_mma(lo, a0, a1, a2, a3, q.z, q.w);
+    const uint2 q = qf[k * 32];
+    tba_mma(c[k & 1], __byte_perm(a[0], a[1], 0x5410), __byte_perm(b[0], b[1], 0x5410), __byte_perm(a[2], a[3], 0x5410), __byte_perm(b[2], b[3], 0x5410),
+            q.x, q.y);
   }
   #pragma unroll
-  for (int e = 0; e < 4; ++e) s[e] = hi[e] + lo[e];
+  for (int e = 0; e < 4; ++e) s[e] = c[0][e] + c[1][e];
 }
 
 // O^T += V^T P^T over a tile: this lane's 32 channels (half a chain) of tokens 2j, 2j+1, 2j+8, 2j+9 (rows r[0..3]).
@@ -433,8 +446,11 @@ __device__ __forceinline__ void tba_values(const uint32_t* const (&r)[4], bool o
       for (int t = 0; t < 4; ++t) x[c][t] = tba_lds((tba_window<KB>(w[t], prev[t], 2 * mt + c) & 0x7F80u) | tab);
     const uint32_t a0 = __byte_perm(x[0][0], x[0][1], 0x5410), a1 = __byte_perm(x[1][0], x[1][1], 0x5410), a2 = __byte_perm(x[0][2], x[0][3], 0x5410),
                    a3 = __byte_perm(x[1][2], x[1][3], 0x5410);
-    tba_mma(acc[mt], a0, a1, a2, a3, ph[0], ph[1]);
-    tba_mma(acc[mt], a0, a1, a2, a3, pl[0], pl[1]);
+    float ch[4] = {0.f, 0.f, 0.f, 0.f}, cl[4] = {0.f, 0.f, 0.f, 0.f};
+    tba_mma(ch, a0, a1, a2, a3, ph[0], ph[1]);
+    tba_mma(cl, a0, a1, a2, a3, pl[0], pl[1]);
+    #pragma unroll
+    for (int e = 0; e < 4; ++e) acc[mt][e] += ch[e] + cl[e];
   }
 }
 
@@ -453,7 +469,7 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
   const yskn_tb_attn_args& A = P.a;
   const int G = P.G, split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   TbAttnSm& S = *reinterpret_cast<TbAttnSm*>(tba_smem);
-  float* mbuf = reinterpret_cast<float*>(tba_smem + (TK - base));          // [warp][8][258]
+  float* mbuf = reinterpret_cast<float*>(tba_smem + (TK - base));          // [warp][8][TBA_MS]
   asm volatile("griddepcontrol.wait;" ::: "memory");                 // programmatic dependent launch, both directions
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const float qs = A.qscale * 1.4426950408889634f;
@@ -480,6 +496,7 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     qv[k] = h < G ? act_load<DT>(A.q16, ((size_t)r * A.nh + kvh * G + h) * 256 + d) : 0.f;
   }
   if (threadIdx.x == 0) S.big = 0;
+  if (threadIdx.x < 8) S.qmax[threadIdx.x] = 0;
   TbRule rk, rv;
   {
     const TbGroup Pg[2] = {tb_group(A.blob, __ldg(A.grp_k + kvh)), tb_group(A.blob, __ldg(A.grp_v + kvh))};
@@ -507,9 +524,14 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     #pragma unroll
     for (int k = 0; k < NQ; ++k) {
       const int e = threadIdx.x + k * TBA_WARPS * 32;
-      if (e < 256 * 8) S.q[e >> 8][e & 255] = qv[k] * qs;
+      if (e < 256 * 8) S.q[e >> 8][e & 255] = qv[k];
     }
-    __syncthreads();                                                 // S.big is cleared
+    __syncthreads();                                                 // S.big and S.qmax are cleared
+    #pragma unroll
+    for (int k = 0; k < NQ; ++k) {                                   // a warp's 32 entries are of one head
+      const int h = (threadIdx.x + k * TBA_WARPS * 32) >> 8, top = __reduce_max_sync(0xffffffffu, __float_as_int(qv[k]) & 0x7fffffff);
+      if (h < 8 && lane == 0) atomicMax(&S.qmax[h], top);
+    }
     if (i < 256)
       #pragma unroll
       for (int w = 0; w < 2; ++w) {
@@ -527,6 +549,7 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     const uint32_t h = __half_as_ushort(__float2half_rn(S.cg[w][st])), v = h | (h << 16);
     asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"((w ? TV : TK) + st * 128 + l4 * 4), "r"(v) : "memory");
   }
+  if (threadIdx.x < 8) S.kq[3][threadIdx.x] = qs * tba_inverse(tba_pow2(13 - tba_exponent(__int_as_float(S.qmax[threadIdx.x]))));
   for (int i = warp; i < 24; i += TBA_WARPS) {                       // q.U0, q.U1, q.mu of each head, a warp per product
     const int which = i >> 3, h = i & 7;
     float a = 0.f;
@@ -534,28 +557,26 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     for (int k = 0; k < 8; ++k) a = fmaf(S.q[h][32 * k + lane], S.term[0][which][tba_slot(32 * k + lane)], a);
     #pragma unroll
     for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) S.kq[which][h] = a;
+    if (lane == 0) S.kq[which][h] = a * qs;
   }
   for (int e = threadIdx.x; e < 16 * 32; e += TBA_WARPS * 32) {      // k-slots (2j, 2j+1, 2j+8, 2j+9) of step s = channels 64j + 4s .. + 3
     const int s = e >> 5, ln = e & 31, h = ln >> 2, c = 64 * (ln & 3) + 4 * s;
-    float v[4], hi[4];
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) { v[k] = S.q[h][c + k]; hi[k] = __half2float(__float2half_rn(v[k])); }
-    S.qf[s][ln] = make_uint4(tba_pack(hi[0], hi[1]), tba_pack(hi[2], hi[3]), tba_pack(v[0] - hi[0], v[1] - hi[1]), tba_pack(v[2] - hi[2], v[3] - hi[3]));
+    const float f = tba_pow2(13 - tba_exponent(__int_as_float(S.qmax[h])));
+    S.qf[s][ln] = make_uint2(tba_pack(S.q[h][c] * f, S.q[h][c + 1] * f), tba_pack(S.q[h][c + 2] * f, S.q[h][c + 3] * f));
   }
   __syncthreads();
   // tokens below tf take the row path: either side unpacked there, or codes that fp16 does not hold
   const int tf = rk.packed_ok && rv.packed_ok && !S.big ? min(t1, max(t0, max(rk.guard, rv.guard))) : t1;
   const bool v16 = !((A.pay_stride | (int)((uintptr_t)A.k_pay | (uintptr_t)A.v_pay)) & 15);
-  const uint4* qf = &S.qf[0][lane];
+  const uint2* qf = &S.qf[0][lane];
   const uint32_t tabk = TK | (lane * 4), tabv = TV | (lane * 4);
 
   float acc[16][4];                                                  // O^T: [m-tile][(channel 32g + 2 mt | + 1) x (head 2j | 2j + 1)]
   #pragma unroll
   for (int mt = 0; mt < 16; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
-  // heads 2j, 2j+1 (log2 domain); l and the sums of p, p c0, p c1 over packed values are this lane's share of the tokens
-  float m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f}, a0[2] = {0.f, 0.f}, a1[2] = {0.f, 0.f}, am[2] = {0.f, 0.f};
-  const float kq0[2] = {S.kq[0][2 * j], S.kq[0][2 * j + 1]}, kq1[2] = {S.kq[1][2 * j], S.kq[1][2 * j + 1]}, kqm[2] = {S.kq[2][2 * j], S.kq[2][2 * j + 1]};
+  // heads 2j, 2j+1 (log2 domain); l (of packed values: the mean row's weight too) and the sums of p c0, p c1 are this lane's share of the tokens
+  float m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f}, a0[2] = {0.f, 0.f}, a1[2] = {0.f, 0.f};
+  float u[2] = {tba_pow2(TBA_EXP), tba_pow2(TBA_EXP)};               // acc holds sum x u
   auto side = [&](const uint32_t* sd, int t, int mm, float& s, float& c0, float& c1) {
     s = __uint_as_float(__ldg(sd + 2 * (row0 + t)));
     const uint32_t pc = __ldg(sd + 2 * (row0 + t) + 1);
@@ -569,6 +590,8 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     float ks[2], kc0[2], kc1[2], vs[2], vc0[2], vc1[2];
     side(A.k_side, ta, rk.m, ks[0], kc0[0], kc1[0]); side(A.k_side, tb, rk.m, ks[1], kc0[1], kc1[1]);
     side(A.v_side, ta, rv.m, vs[0], vc0[0], vc1[0]); side(A.v_side, tb, rv.m, vs[1], vc0[1], vc1[1]);
+    if (!live0) vs[0] = vc0[0] = vc1[0] = 0.f;
+    if (!live1) vs[1] = vc0[1] = vc1[1] = 0.f;
     float s[4];
     {
       const uint32_t *pa = kpay + (size_t)ta * psw + j * 2 * rk.kb, *pb = kpay + (size_t)tb * psw + j * 2 * rk.kb;
@@ -579,33 +602,51 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     float p[2][2];                                                   // [row g | g + 8][head]
     #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const float sa = fmaf(ks[0] * rk.gain, s[h], fmaf(kc0[0], kq0[h], fmaf(kc1[0], kq1[h], kqm[h])));
-      const float sb = fmaf(ks[1] * rk.gain, s[2 + h], fmaf(kc0[1], kq0[h], fmaf(kc1[1], kq1[h], kqm[h])));
+      const volatile float* kq = &S.kq[0][2 * j + h];                // read per tile: the registers are needed for the sums
+      const float kq0 = kq[0], kq1 = kq[8], kqm = kq[16], qu = kq[24];
+      const float sa = fmaf(ks[0] * rk.gain, s[h] * qu, fmaf(kc0[0], kq0, fmaf(kc1[0], kq1, kqm)));
+      const float sb = fmaf(ks[1] * rk.gain, s[2 + h] * qu, fmaf(kc0[1], kq0, fmaf(kc1[1], kq1, kqm)));
       p[0][h] = live0 ? sa : -INFINITY; p[1][h] = live1 ? sb : -INFINITY;
     }
-    float x0 = fmaxf(p[0][0], p[1][0]), x1 = fmaxf(p[0][1], p[1][1]);
-    if (__any_sync(0xffffffffu, x0 > m[0] + 8.f || x1 > m[1] + 8.f)) {     // lazy rescale: the running max may lag by 2^8
+    float x0 = fmaxf(p[0][0], p[1][0]), x1 = fmaxf(p[0][1], p[1][1]), f0 = 1.f, f1 = 1.f;
+    const bool bump = __any_sync(0xffffffffu, x0 > m[0] + 8.f || x1 > m[1] + 8.f);     // lazy rescale: the running max may lag by 2^8
+    if (bump) {
       #pragma unroll
       for (int o = 4; o <= 16; o <<= 1) { x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, o)); x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o)); }
-      const float n0 = fmaxf(m[0], x0), n1 = fmaxf(m[1], x1), f0 = exp2f(m[0] - n0), f1 = exp2f(m[1] - n1);
+      const float n0 = fmaxf(m[0], x0), n1 = fmaxf(m[1], x1);
+      f0 = exp2f(m[0] - n0); f1 = exp2f(m[1] - n1);
       m[0] = n0; m[1] = n1;
-      l[0] *= f0; a0[0] *= f0; a1[0] *= f0; am[0] *= f0; l[1] *= f1; a0[1] *= f1; a1[1] *= f1; am[1] *= f1;
-      #pragma unroll
-      for (int mt = 0; mt < 16; ++mt) { acc[mt][0] *= f0; acc[mt][1] *= f1; acc[mt][2] *= f0; acc[mt][3] *= f1; }
+      l[0] *= f0; a0[0] *= f0; a1[0] *= f0; l[1] *= f1; a0[1] *= f1; a1[1] *= f1;
     }
     #pragma unroll
     for (int h = 0; h < 2; ++h) {
       p[0][h] = exp2f(p[0][h] - m[h]); p[1][h] = exp2f(p[1][h] - m[h]);
       l[h] += p[0][h] + p[1][h];
       a0[h] = fmaf(p[0][h], vc0[0], fmaf(p[1][h], vc0[1], a0[h])); a1[h] = fmaf(p[0][h], vc1[0], fmaf(p[1][h], vc1[1], a1[h]));
-      am[h] += p[0][h] + p[1][h];
     }
-    uint32_t ph[2], pl[2];                                           // weights x scale as two fp16 numbers, transposed into B registers
+    float w[2][2];                                                   // weights
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) { w[0][h] = p[0][h] * (vs[0] * rv.gain); w[1][h] = p[1][h] * (vs[1] * rv.gain); }
+    float w0 = fmaxf(fabsf(w[0][0]), fabsf(w[1][0])), w1 = fmaxf(fabsf(w[0][1]), fabsf(w[1][1]));
+    if (bump || __any_sync(0xffffffffu, w0 * u[0] > 2048.f || w1 * u[1] > 2048.f)) {       // the powers of two follow the largest weight of the sum
+      #pragma unroll
+      for (int o = 4; o <= 16; o <<= 1) { w0 = fmaxf(w0, __shfl_xor_sync(0xffffffffu, w0, o)); w1 = fmaxf(w1, __shfl_xor_sync(0xffffffffu, w1, o)); }
+      const float b0 = 512.f * tba_inverse(u[0]) * f0, b1 = 512.f * tba_inverse(u[1]) * f1;  // the weight u was made for, under the new maximum
+      const float n0 = tba_pow2(9 - tba_exponent(fmaxf(w0, b0))), n1 = tba_pow2(9 - tba_exponent(fmaxf(w1, b1)));
+      f0 *= tba_inverse(u[0]); f1 *= tba_inverse(u[1]);
+      u[0] = n0; u[1] = n1;
+      #pragma unroll
+      for (int mt = 0; mt < 16; ++mt) {                              // two factors: their product may leave the range of a float
+        acc[mt][0] = acc[mt][0] * f0 * n0; acc[mt][1] = acc[mt][1] * f1 * n1; acc[mt][2] = acc[mt][2] * f0 * n0; acc[mt][3] = acc[mt][3] * f1 * n1;
+      }
+    }
+    uint32_t ph[2], pl[2];                                           // weights x u, whole part and rest, transposed into B registers
     #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const float w0 = p[q][0] * vs[q] * rv.gain, w1 = p[q][1] * vs[q] * rv.gain;
-      const float h0 = __half2float(__float2half_rn(w0)), h1 = __half2float(__float2half_rn(w1));
-      ph[q] = tba_transpose(tba_pack(h0, h1)); pl[q] = tba_transpose(tba_pack(w0 - h0, w1 - h1));
+      const float y0 = w[q][0] * u[0], y1 = w[q][1] * u[1];
+      const float h0 = rintf(y0), h1 = rintf(y1);
+      ph[q] = tba_transpose(tba_pack(h0, h1));
+      pl[q] = tba_transpose(tba_pack(isinf(h0) ? 0.f : y0 - h0, isinf(h1) ? 0.f : y1 - h1));      // an infinite row scale stays infinite
     }
     const int tv[4] = {min(tc + 2 * j, t1 - 1), min(tc + 2 * j + 1, t1 - 1), min(tc + 2 * j + 8, t1 - 1), min(tc + 2 * j + 9, t1 - 1)};
     const uint32_t* vr[4];
@@ -621,7 +662,7 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     #pragma unroll
     for (int h = 0; h < 2; ++h) {
       l[h] += __shfl_xor_sync(0xffffffffu, l[h], o); a0[h] += __shfl_xor_sync(0xffffffffu, a0[h], o);
-      a1[h] += __shfl_xor_sync(0xffffffffu, a1[h], o); am[h] += __shfl_xor_sync(0xffffffffu, am[h], o);
+      a1[h] += __shfl_xor_sync(0xffffffffu, a1[h], o);
     }
   __syncthreads();
   float* wb = mbuf + (size_t)warp * 8 * TBA_MS;
@@ -630,7 +671,8 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int h = e & 1, d = 32 * g + 2 * mt + (e >> 1);
-      wb[(2 * j + h) * TBA_MS + 4 + tba_slot(d)] = fmaf(a0[h], S.term[1][0][tba_slot(d)], fmaf(a1[h], S.term[1][1][tba_slot(d)], fmaf(am[h], S.term[1][2][tba_slot(d)], acc[mt][e])));
+      wb[(2 * j + h) * TBA_MS + 4 + tba_slot(d)] =
+          fmaf(a0[h], S.term[1][0][tba_slot(d)], fmaf(a1[h], S.term[1][1][tba_slot(d)], fmaf(l[h], S.term[1][2][tba_slot(d)], acc[mt][e] * tba_inverse(u[h]))));
     }
   if (g == 0) {
     #pragma unroll
@@ -655,6 +697,7 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
       for (int k = 0; k < 8; ++k) a = fmaf(S.q[h][32 * k + lane], x[k], a);
       #pragma unroll
       for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      a *= qs;
       sc[h] = kpk ? a + fmaf(c0, S.kq[0][h], fmaf(c1, S.kq[1][h], S.kq[2][h])) : a;
     }
     if (vpk) side(A.v_side, t, rv.m, s0, c0, c1);
