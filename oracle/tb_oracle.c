@@ -155,7 +155,7 @@ void ysko_tb_decode_fields(const uint8_t* blob, int g, const uint32_t* pay, floa
   const unsigned off_t = u32(blob + 36), off_g = u32(blob + 40);
   const unsigned go = u32(blob + off_g + 4u * (unsigned)g);
   const int mode = blob[go], kk = blob[go + 1], tix = blob[go + 2], kb = mode == 1 ? 4 : kk;
-  const unsigned to = u32(blob + off_t + 4u * (unsigned)tix);
+  const unsigned to = mode == 1 ? 0u : u32(blob + off_t + 4u * (unsigned)tix);
   const float gain = mode == 0 ? f32(blob + to + 4) : 1.f;
   int st = 0;
   for (int e = 0; e < 256; ++e) {
@@ -187,7 +187,7 @@ void ysko_tb_unpack(const uint8_t* blob, const int* grp, const int* pos, const u
     float s; memcpy(&s, &side[2 * r], 4);
     const unsigned pc = side[2 * r + 1];
     const int kb = mode == 1 ? 4 : kk;
-    const unsigned to = u32(blob + off_t + 4u * (unsigned)tix);
+    const unsigned to = mode == 1 ? 0u : u32(blob + off_t + 4u * (unsigned)tix);
     const uint8_t* mup = blob + go + 8; const uint8_t* Up = mup + (has_mu ? 512 : 0);
     for (int d = 0; d < 256; ++d) {
       const int endb = kb * (d + 1), first = kb * (d & ~63), lo = mode == 1 ? endb - 4 : (endb - 8 > first ? endb - 8 : first);

@@ -150,3 +150,31 @@ def test_attention_queries_of_any_size(oracle, size):
     got, want = _packed_case(oracle, _plain_groups(make_blob()), scale, np.array([[10, 8, 0, 12], [3, 9, 5, 7]], np.int32), ctx, M, q, 5)
     rel = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
     assert (rel < 2e-5).all(), rel.max()
+
+
+@pytest.mark.parametrize("tables", [3, 0])
+def test_flat_groups_have_no_table(oracle, tables):
+    """The loader does not check a flat group's table index: profiles whose flat groups name a table that does not exist, with and without tables."""
+    from yasakani_b200 import kvx
+    b = bytearray(_plain_groups(make_blob()))
+    off_g, = struct.unpack_from("<I", b, 40)
+    for g in range(128):
+        o, = struct.unpack_from("<I", b, off_g + 4 * g)
+        if tables == 0 or b[o] == 1:
+            b[o:o + 3] = bytes((1, 200, 255))                       # flat, no step width, table 255
+    if tables == 0:
+        struct.pack_into("<H", b, 22, 0)
+        struct.pack_into("<I", b, 36, len(b))                       # the list of tables is empty: it ends with the blob
+    blob = bytes(b)
+    assert oracle.tb_check_blob(blob) == 0
+    ctx, M, nh = 100, 1, 32
+    q = torch.from_numpy(np.random.default_rng(2).standard_normal((M, nh, 256)).astype(np.float32)).half()
+    got, want = _packed_case(oracle, blob, np.ones((2, 1, ctx + M), np.float32), np.array([[15, 31, 47, 63], [79, 15, 95, 31]], np.int32), ctx, M, q, 5)
+    assert (np.linalg.norm(got - want, axis=-1) < 2e-5 * np.linalg.norm(want, axis=-1)).all()
+    x = np.random.default_rng(3).standard_normal((8, 256)).astype(np.float32)
+    grp, pos = np.full(8, 15, np.int32), np.arange(8, dtype=np.int32)
+    want = oracle.tb_encode(blob, x, grp, pos)
+    dev = [torch.from_numpy(a).cuda() for a in (x, grp, pos)]
+    y, pay, side = kvx.tb_encode(kvx.TrellisProfile(blob), *dev)
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want["y"].view(np.uint32))
+    assert np.array_equal(kvx.tb_decode(kvx.TrellisProfile(blob), pay, side, dev[1], dev[2]).cpu().numpy(), want["y"])      # (by value: -0 decodes to +0)

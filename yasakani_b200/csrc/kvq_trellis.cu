@@ -32,6 +32,10 @@ __device__ __forceinline__ TbGroup tb_group(const uint8_t* b, int g) {
   return P;
 }
 
+// Offset of a trellis group's code table.  A flat group has none: its table index is not checked by the loader and may lie beyond the blob, so
+// nothing is read through it (0: the header, which every blob has).
+__device__ __forceinline__ unsigned tb_table(const uint8_t* b, const TbGroup& P) { return P.ok && P.mode == 0 ? tb_u32(b + P.off_t + 4u * (unsigned)P.tix) : 0u; }
+
 // ---- encoder: one block of four warps per row, one warp per chain of 64 values.
 //
 // A step of the search takes new(d) = min over the 2^KK predecessors {j * UU + u}, u = d >> KK, of old(p), plus (x - code[d])^2: every
@@ -208,7 +212,7 @@ __global__ void __launch_bounds__(128, 7) tb_encode_kernel(TbP A) {
     const float qa = fminf(fmaxf(rintf(__fdiv_rn(ra, s7)), -7.f), 7.f), qb = fminf(fmaxf(rintf(__fdiv_rn(rb, s7)), -7.f), 7.f);
     xqa = __fmul_rn(qa, s7); xqb = __fmul_rn(qb, s7); fa = (int)qa + 8; fb = (int)qb + 8; psc = s7; kb = 4;
   } else {
-    const unsigned to = tb_u32(b + P.off_t + 4u * (unsigned)P.tix);
+    const unsigned to = tb_table(b, P);
     const float gain = tb_f32(b + to + 4);
     int cm = 0;
     for (int i = threadIdx.x; i < 256; i += 128) { const int v = (short)tb_u16(b + to + 12 + 2 * i); S.code[i] = (short)v; cm = max(cm, abs(v)); }
@@ -295,7 +299,7 @@ __global__ void __launch_bounds__(256) tb_unpack_kernel(TbDecP A) {
   __syncwarp();
   const float s = __uint_as_float(A.side[2 * (size_t)row]);
   const unsigned pc = A.side[2 * (size_t)row + 1];
-  const unsigned to = tb_u32(b + P.off_t + 4u * (unsigned)P.tix);
+  const unsigned to = tb_table(b, P);
   const float gain = P.mode == 0 ? tb_f32(b + to + 4) : 1.f;
   const uint8_t* mup = b + P.go + 8;
   const uint8_t* Up = mup + (P.has_mu ? 512 : 0);
@@ -502,10 +506,10 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     const TbGroup Pg[2] = {tb_group(A.blob, __ldg(A.grp_k + kvh)), tb_group(A.blob, __ldg(A.grp_v + kvh))};
     unsigned to[2];
     #pragma unroll
-    for (int w = 0; w < 2; ++w) to[w] = tb_u32(A.blob + Pg[w].off_t + 4u * (unsigned)Pg[w].tix);
+    for (int w = 0; w < 2; ++w) to[w] = tb_table(A.blob, Pg[w]);
     float gain[2];
     #pragma unroll
-    for (int w = 0; w < 2; ++w) gain[w] = tb_f32(A.blob + to[w] + 4);
+    for (int w = 0; w < 2; ++w) gain[w] = tb_f32(A.blob + to[w] + 4);        // (no table: not used)
     const int i = threadIdx.x;
     float x[2][4];                                                   // code, U0, U1, mu of entry / channel i
     #pragma unroll
