@@ -337,10 +337,11 @@ YSKN_KV4_API int yskn_kvx_probe(const float* x, int8_t* q, float* scales, float*
  * kind 0 = K, 1 = V), d_pos[r] = its position (rows below the group's guard position are passed through and not
  * packed).  Outputs, each optional (NULL): d_y [rows][256] the re-quantised rows; d_pay [rows][pay_stride bytes] the
  * payload, 8*k 32-bit words per row, the k new bits of every value MSB first (pay_stride >= 160, a multiple of 4);
- * d_side [rows][2] = the row's scale (fp32 bits) and its two fp16 low-rank coefficients.  Payload and side words are written
- * whole: what a row does not use is zero, and so are rows that are not packed (side words belong to the payload: they are
- * written only with it, except for rows that are not packed).  d_scratch: yskn_tb_scratch_bytes(rows, nm) bytes, which is none
- * (NULL is fine).  Enqueue-only, nothing allocated. */
+ * d_side [rows][2] = the row's scale (fp32 bits) and its two fp16 low-rank coefficients (written only together with a payload).
+ * Nothing else of the payload and side rows is touched: not the words between 8*k and the stride, and not rows that are not
+ * packed.  d_scratch: yskn_tb_scratch_bytes(rows, nm) bytes, which is none (NULL is fine).  Enqueue-only, nothing allocated.
+ * yskn_tb_encode_whole: the same into fresh payload and side arrays (both needed): whatever a row does not use is written as
+ * zero, and so are rows that are not packed. */
 /* yskn_tb_decode: the packed rows back to fp32 values (tba_unpack_kernel, src/kvq_attn.cuh:39-72): every value's state is
  * the 8-bit window of the row's bit stream that ends with its field, so rows decode without the search; rows that were
  * not packed take d_yin (may be NULL: zeros).  Same d_grp / d_pos / pay_stride as the encoder's. */
@@ -350,6 +351,8 @@ YSKN_KV4_API int yskn_tb_blob_info(const uint8_t* h_blob, size_t blob_len, int* 
 YSKN_KV4_API size_t yskn_tb_scratch_bytes(int rows, int nm);
 YSKN_KV4_API int yskn_tb_encode(const uint8_t* d_blob, int nm, const float* d_x, const int* d_grp, const int* d_pos, int rows, float* d_y,
                                 uint8_t* d_pay, int pay_stride, uint32_t* d_side, void* d_scratch, size_t scratch_bytes, void* cuda_stream);
+YSKN_KV4_API int yskn_tb_encode_whole(const uint8_t* d_blob, int nm, const float* d_x, const int* d_grp, const int* d_pos, int rows, float* d_y,
+                                      uint8_t* d_pay, int pay_stride, uint32_t* d_side, void* cuda_stream);
 
 /* Decode attention straight over packed trellis rows: the counterpart of the reference's attention over packed rows
  * (launch_q35_atxpk, src/q35_atxpk.hpp:14-24, src/q35_atxpk3.cuh / q35_atxpk4.cuh) for passes of a few rows.  Every key and

@@ -52,6 +52,28 @@ def test_encoder_key_widths(oracle, top):
     assert np.array_equal(side.cpu().numpy().view(np.uint32), want["side"])
 
 
+@pytest.mark.parametrize("with_payload", [True, False])
+def test_encoder_leaves_the_callers_other_words_alone(oracle, with_payload):
+    """The C entry writes a packed row's payload words and its side words, nothing else: rows of records that hold other data behind the
+    payload, and rows that are not packed, keep their bytes."""
+    from yasakani_b200 import _lib, kvx
+    prof, n, stride = kvx.TrellisProfile(make_blob()), 48, 320
+    rng = np.random.default_rng(4)
+    x, grp, pos = rng.standard_normal((n, 256)).astype(np.float32), np.arange(n, dtype=np.int32), (np.arange(n) % 6).astype(np.int32)
+    want = oracle.tb_encode(make_blob(), x, grp, pos)
+    assert (want["kb"] == 0).any() and (want["kb"] == 5).any()
+    dx, dg, dp = (torch.from_numpy(a).cuda() for a in (x, grp, pos))
+    y, pay, side = torch.empty_like(dx), torch.full((n, stride), 0xAB, dtype=torch.uint8, device="cuda"), torch.full((n, 2), 0x5A5A5A5A, dtype=torch.int32, device="cuda")
+    assert _lib.load().yskn_tb_encode(prof.dev.data_ptr(), prof.nm, dx.data_ptr(), dg.data_ptr(), dp.data_ptr(), n, y.data_ptr(),
+                                      pay.data_ptr() if with_payload else None, stride, side.data_ptr(), None, 0, torch.cuda.current_stream().cuda_stream) == 0
+    got, gs = pay.cpu().numpy().view(np.uint32), side.cpu().numpy().view(np.uint32)
+    for r in range(n):
+        words = 8 * want["kb"][r] if with_payload else 0
+        assert np.array_equal(got[r, :words], want["pay"][r, :words]) and (got[r, words:] == 0xABABABAB).all(), r
+        assert np.array_equal(gs[r], want["side"][r] if words else np.full(2, 0x5A5A5A5A, np.uint32)), r
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want["y"].view(np.uint32))
+
+
 @pytest.mark.parametrize("top,ctx,M,splits,stride", [
     (1100, 1000, 1, 3, 160), (1100, 1000, 2, 1, 164),               # many tiles per warp, rows that are not 16-byte aligned
     (1100, 40, 1, 37, 160), (1100, 15, 1, 1, 176),                  # splits of one or two tokens, a single ragged tile
@@ -113,7 +135,7 @@ def _packed_case(oracle, blob, scale, grp, ctx, M, q, seed, stride=160):
     return got, oracle.rows_attention_exact(q.float().numpy(), rows[0], rows[1], ctx).astype(np.float64)
 
 
-@pytest.mark.parametrize("values", [1e-6, 1e-3, 1e-2, 1.0, 1e3, "flat 1e4", "mixed", "outlier"])
+@pytest.mark.parametrize("values", [1e-6, 1e-3, 1e-2, 1.0, 1e3, "flat 1e6", "mixed", "outlier"])
 def test_attention_is_fp32_at_every_scale_of_the_values(oracle, values):
     """Weights (probability x row scale x gain) and queries keep fp32 accuracy and range whatever the rows' scale: tiny and large values, scales
     that differ by 2^30 inside a sequence, a large row that the softmax leaves out, and large flat rows (whose gain is 1, not 1 / 256)."""
@@ -122,9 +144,9 @@ def test_attention_is_fp32_at_every_scale_of_the_values(oracle, values):
     scale = np.ones((2, 1, ctx + M), np.float32)
     grp = np.array([[10, 8, 0, 12], [3, 9, 5, 7]], np.int32)        # value groups of 5 / 3 / 5 / 4 bits, no flat one
     q = torch.from_numpy(rng.standard_normal((M, nh, 256)).astype(np.float32)).bfloat16()
-    if values == "flat 1e4":
+    if values == "flat 1e6":
         grp[1] = [15, 31, 47, 63]
-        scale[1] = 1e4
+        scale[1] = 1e6
     elif values == "mixed":
         scale[1] = 2.0 ** rng.integers(-20, 11, ctx + M)
     elif values == "outlier":                                       # a large value under a weight of about 2^-38

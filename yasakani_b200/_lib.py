@@ -121,6 +121,7 @@ PROTOTYPES = {
     "yskn_tb_scratch_bytes": (C.c_size_t, [C.c_int, C.c_int]),
     "yskn_tb_encode": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p,
                                  C.c_void_p, C.c_size_t, C.c_void_p]),
+    "yskn_tb_encode_whole": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "yskn_kv8_attention": (C.c_int, [C.POINTER(Kv8AttnArgsC), C.c_int, C.c_void_p]),
     "yskn_kv8_attention_tc": (C.c_int, [C.POINTER(Kv8AttnArgsC), C.c_int, C.c_void_p]),
     "yskn_kv8_workspace_bytes": (C.c_size_t, [C.POINTER(Kv8AttnArgsC)]),

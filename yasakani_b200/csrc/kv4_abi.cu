@@ -350,7 +350,13 @@ int yskn_tb_blob_info(const uint8_t* h_blob, size_t blob_len, int* nm) { return 
 size_t yskn_tb_scratch_bytes(int rows, int nm) { return tb_scratch_bytes(rows, nm); }
 int yskn_tb_encode(const uint8_t* d_blob, int nm, const float* d_x, const int* d_grp, const int* d_pos, int rows, float* d_y, uint8_t* d_pay,
                    int pay_stride, uint32_t* d_side, void* d_scratch, size_t scratch_bytes, void* cuda_stream) {
-  return launch_tb_encode(d_blob, nm, d_x, d_grp, d_pos, rows, d_y, d_pay, pay_stride, d_side, d_scratch, scratch_bytes, (cudaStream_t)cuda_stream);
+  (void)d_scratch; (void)scratch_bytes;
+  return launch_tb_encode(d_blob, nm, d_x, d_grp, d_pos, rows, d_y, d_pay, pay_stride, d_side, 0, (cudaStream_t)cuda_stream);
+}
+int yskn_tb_encode_whole(const uint8_t* d_blob, int nm, const float* d_x, const int* d_grp, const int* d_pos, int rows, float* d_y, uint8_t* d_pay,
+                         int pay_stride, uint32_t* d_side, void* cuda_stream) {
+  if (!d_pay || !d_side) KV4_REJECT("yskn_tb_encode_whole: null buffer");
+  return launch_tb_encode(d_blob, nm, d_x, d_grp, d_pos, rows, d_y, d_pay, pay_stride, d_side, 1, (cudaStream_t)cuda_stream);
 }
 
 int yskn_tb_decode(const uint8_t* d_blob, const int* d_grp, const int* d_pos, const uint8_t* d_pay, int pay_stride, const uint32_t* d_side,

@@ -116,7 +116,7 @@ size_t tb_scratch_bytes(int rows, int nm);
 int tb_blob_info(const uint8_t* h_blob, size_t n, int* nm);
 int launch_tb_attention(const yskn_tb_attn_args& a, int act_dtype, cudaStream_t st);
 int launch_tb_encode(const uint8_t* blob, int nm, const float* x, const int* grp, const int* pos, int rows, float* y, uint8_t* pay, int pay_stride,
-                     uint32_t* side, void* scratch, size_t scratch_bytes, cudaStream_t st);
+                     uint32_t* side, int whole, cudaStream_t st);
 
 int launch_tb_decode(const uint8_t* blob, const int* grp, const int* pos, const uint8_t* pay, int pay_stride, const uint32_t* side, const float* yin,
                      float* y, int rows, cudaStream_t st);

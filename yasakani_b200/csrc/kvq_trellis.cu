@@ -63,7 +63,7 @@ struct TbRowSmem {
   struct Mult { uint8_t st[256]; float err[8]; } mult[1];  // one per multiplier: its states and its error sums
   static size_t bytes(int nm) { return sizeof(TbRowSmem) + (nm - 1) * sizeof(Mult); }
 };
-struct TbP { const uint8_t* blob; int nm; const float* x; const int* grp; const int* pos; int rows; float* y; uint8_t* pay; int pay_stride; uint32_t* side; };
+struct TbP { const uint8_t* blob; int nm; const float* x; const int* grp; const int* pos; int rows; float* y; uint8_t* pay; int pay_stride; uint32_t* side; int whole; };
 
 __device__ __forceinline__ int tb_addmin(int a, int b, int c) { return __viaddmin_s32(a, b, c); }
 __device__ __forceinline__ long long tb_addmin(long long a, long long b, long long c) { return min(a + b, c); }
@@ -164,10 +164,12 @@ __global__ void __launch_bounds__(128, 7) tb_encode_kernel(TbP A) {
   const int words = A.pay_stride / 4;
   unsigned* pay = A.pay ? reinterpret_cast<unsigned*>(A.pay + (size_t)row * A.pay_stride) : nullptr;
   float ra = A.x[(size_t)row * 256 + d0], rb = A.x[(size_t)row * 256 + d1];
-  if (!P.ok || A.pos[row] < P.guard) {                   // stored as it is: the payload and the side words are zero
+  if (!P.ok || A.pos[row] < P.guard) {                   // stored as it is
     if (A.y) { A.y[(size_t)row * 256 + d0] = ra; A.y[(size_t)row * 256 + d1] = rb; }
-    if (pay) for (int w = threadIdx.x; w < words; w += 128) pay[w] = 0u;
-    if (A.side && threadIdx.x < 2) A.side[2 * row + threadIdx.x] = 0u;
+    if (A.whole) {
+      for (int w = threadIdx.x; w < words; w += 128) pay[w] = 0u;
+      if (threadIdx.x < 2) A.side[2 * row + threadIdx.x] = 0u;
+    }
     return;
   }
   // the reference's row sum: a xor-butterfly over each run of 32 values, then the eight runs in order (src/kvq_fast.cuh:33-43)
@@ -258,7 +260,7 @@ __global__ void __launch_bounds__(128, 7) tb_encode_kernel(TbP A) {
   if (pay) {
     S.fld[d0] = (uint8_t)fa; S.fld[d1] = (uint8_t)fb;
     __syncthreads();
-    for (int w = threadIdx.x; w < words; w += 128) {     // MSB-first bit stream, 32 bits per word (src/kvq_fast.cuh:228-232)
+    for (int w = threadIdx.x; w < (A.whole ? words : 8 * kb); w += 128) {     // MSB-first bit stream, 32 bits per word (src/kvq_fast.cuh:228-232)
       unsigned v = 0u;
       if (w < 8 * kb) {
         const int e0 = 32 * w / kb;                      // the field that holds the word's first bit
@@ -791,14 +793,13 @@ int tb_blob_info(const uint8_t* b, size_t n, int* nm) {
 }
 
 int launch_tb_encode(const uint8_t* blob, int nm, const float* x, const int* grp, const int* pos, int rows, float* y, uint8_t* pay, int pay_stride,
-                     uint32_t* side, void* scratch, size_t scratch_bytes, cudaStream_t st) {
-  (void)scratch; (void)scratch_bytes;
+                     uint32_t* side, int whole, cudaStream_t st) {
   if (!blob || !x || !grp || !pos) KV4_REJECT("yskn_tb_encode: null buffer");
   if (rows <= 0 || nm < 1 || nm > TB_NM) KV4_REJECT("yskn_tb_encode: bad shape (rows %d, multipliers %d)", rows, nm);
   if (pay && (pay_stride < 160 || pay_stride % 4 || ((uintptr_t)pay & 3))) KV4_REJECT("yskn_tb_encode: payload rows need a stride of at least 160 bytes, a multiple of 4");
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(tb_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TbRowSmem::bytes(TB_NM)));
-  tb_encode_kernel<<<rows, 128, TbRowSmem::bytes(nm), st>>>(TbP{blob, nm, x, grp, pos, rows, y, pay, pay_stride, side});
+  tb_encode_kernel<<<rows, 128, TbRowSmem::bytes(nm), st>>>(TbP{blob, nm, x, grp, pos, rows, y, pay, pay_stride, side, whole});
   return launch_status("tb_encode_kernel");
 }
 

@@ -106,8 +106,8 @@ def tb_encode(profile: TrellisProfile, x: torch.Tensor, grp: torch.Tensor, pos: 
     y = torch.empty_like(x)
     pay = torch.empty((rows, pay_stride), dtype=torch.uint8, device=x.device)
     side = torch.empty((rows, 2), dtype=torch.int32, device=x.device)
-    check(_lib.load().yskn_tb_encode(_ptr(profile.dev), profile.nm, _ptr(x), _ptr(grp), _ptr(pos), rows, _ptr(y), _ptr(pay), pay_stride, _ptr(side),
-                                     None, 0, _stream(stream)), "yskn_tb_encode")
+    check(_lib.load().yskn_tb_encode_whole(_ptr(profile.dev), profile.nm, _ptr(x), _ptr(grp), _ptr(pos), rows, _ptr(y), _ptr(pay), pay_stride, _ptr(side),
+                                           _stream(stream)), "yskn_tb_encode")
     return y, pay, side
 
 
