@@ -26,6 +26,10 @@ inline int launch_status(const char* what) {
 }
 
 // Launch with programmatic stream serialization allowed (for kernels that wait in griddepcontrol.wait before they read what a predecessor wrote).
+// Such a kernel is resident while its predecessor still writes, so it reads with plain loads: the read-only path (__ldg, ld.global.nc, const
+// __restrict__) wants bytes that do not change while the kernel runs, and griddepcontrol.wait does not order it.  ld_table is for weights and
+// tables, which no kernel in front of a pass writes.
+template <class T> __device__ __forceinline__ T ld_table(const T* p) { return __ldg(p); }
 template <class K, class... Args>
 inline int launch_pdl(const char* who, K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg{};

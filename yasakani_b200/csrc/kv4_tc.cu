@@ -68,12 +68,12 @@ __device__ __forceinline__ uint32_t tc_pack(float lo, float hi);
 
 // CPL nibbles (CPL/2 bytes) or CPL fp16 values of one lane in a single load
 template <int CPL> __device__ __forceinline__ uint32_t load_packed(const uint8_t* p) {
-  if (CPL == 8) return __ldg(reinterpret_cast<const uint32_t*>(p));
-  return (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(p));
+  if (CPL == 8) return *reinterpret_cast<const uint32_t*>(p);
+  return (uint32_t)*reinterpret_cast<const uint16_t*>(p);
 }
 template <int CPL> __device__ __forceinline__ void load_halves(const uint16_t* p, uint32_t (&o)[CPL / 2]) {
-  if (CPL == 8) { const uint4 u = __ldg(reinterpret_cast<const uint4*>(p)); o[0] = u.x; o[1] = u.y; o[CPL / 2 - 2] = u.z; o[CPL / 2 - 1] = u.w; }
-  else { const uint2 u = __ldg(reinterpret_cast<const uint2*>(p)); o[0] = u.x; o[CPL / 2 - 1] = u.y; }
+  if (CPL == 8) { const uint4 u = *reinterpret_cast<const uint4*>(p); o[0] = u.x; o[1] = u.y; o[CPL / 2 - 2] = u.z; o[CPL / 2 - 1] = u.w; }
+  else { const uint2 u = *reinterpret_cast<const uint2*>(p); o[0] = u.x; o[CPL / 2 - 1] = u.y; }
 }
 
 // One warp per (token t, kv-head); lane owns HD/32 contiguous channels.
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) kv4_tc_prep_kernel(PrepP P) {
     const float4* rp = reinterpret_cast<const float4*>(P.rope + ((size_t)t * half + (rot ? (c0 & (half - 1)) : 0)) * 2);
     float4 cs2[CPL / 2];
     #pragma unroll
-    for (int e = 0; e < CPL / 2; ++e) cs2[e] = __ldg(rp + e);
+    for (int e = 0; e < CPL / 2; ++e) cs2[e] = rp[e];
     #pragma unroll
     for (int e = 0; e < CPL; ++e) {
       const float other = __shfl_xor_sync(0xffffffffu, k[e], lanes_off);
@@ -350,10 +350,10 @@ __device__ __forceinline__ void tc_i8_chunk(const uint4& w, float sf, bool live,
   hi = live ? make_uint4(r[4], r[5], r[6], r[7]) : make_uint4(0u, 0u, 0u, 0u);
 }
 // Global loads as ordered asm statements: the compiler keeps them where they are written, ahead of the arithmetic.
-__device__ __forceinline__ uint32_t tc_ldg32(const void* p) { uint32_t v; asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
-__device__ __forceinline__ uint32_t tc_ldg16(const void* p) { unsigned short v; asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p)); return v; }
+__device__ __forceinline__ uint32_t tc_ldg32(const void* p) { uint32_t v; asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
+__device__ __forceinline__ uint32_t tc_ldg16(const void* p) { unsigned short v; asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p)); return v; }
 __device__ __forceinline__ uint4 tc_ldg128(const void* p) {
-  uint4 v; asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p)); return v;
+  uint4 v; asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p)); return v;
 }
 __device__ __forceinline__ void tc_prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void tc_sts128(uint32_t a, const uint4& v) {
@@ -401,8 +401,8 @@ __global__ void __launch_bounds__(256) kv8_tc_prep_kernel(const int8_t* k8, cons
   if (t >= end_tile) return;
   const size_t row = (size_t)blockIdx.y * max_ctx + t;
   const bool is_v = blockIdx.z != 0;
-  const uint4 w = __ldg(reinterpret_cast<const uint4*>((is_v ? v8 : k8) + row * 256) + c);
-  const float sf = __ldg((is_v ? vs : ks) + row);
+  const uint4 w = reinterpret_cast<const uint4*>((is_v ? v8 : k8) + row * 256)[c];
+  const float sf = (is_v ? vs : ks)[row];
   uint4 lo, hi;
   tc_i8_chunk(w, sf, t < end, lo, hi);
   uint4* dst = reinterpret_cast<uint4*>((is_v ? vd : kd) + row * 256) + 2 * c;

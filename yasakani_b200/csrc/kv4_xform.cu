@@ -12,7 +12,7 @@
 namespace kv4 {
 namespace {
 
-__global__ void __launch_bounds__(512) kv4_xform_a8_kernel(const uint16_t* __restrict__ o16, const int8_t* __restrict__ signs,
+__global__ void __launch_bounds__(512) kv4_xform_a8_kernel(const uint16_t* o16, const int8_t* __restrict__ signs,
                                                            int8_t* __restrict__ qx, float* __restrict__ alpha, int n) {
   __shared__ float b0[512], b1[512];
   __shared__ unsigned s_amax;

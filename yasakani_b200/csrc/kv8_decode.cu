@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(KV8_WARPS * 32, 1) kv8_decode_kernel(const Kv8
       #pragma unroll
       for (int q = 0; q < 4; ++q) { vr[q][0] = ldg16(vbase + tt[q] * KV8_HD); vr[q][1] = ldg16(vbase + tt[q] * KV8_HD + 16); }
     }
-    const float ks0 = v0 ? __ldg(ksb + tg) : 0.f, ks1 = v1 ? __ldg(ksb + tg + 8) : 0.f;
-    const float vs0 = v0 ? __ldg(vsb + tg) : 0.f, vs1 = v1 ? __ldg(vsb + tg + 8) : 0.f;
+    const float ks0 = v0 ? ksb[tg] : 0.f, ks1 = v1 ? ksb[tg + 8] : 0.f;
+    const float vs0 = v0 ? vsb[tg] : 0.f, vs1 = v1 ? vsb[tg + 8] : 0.f;
     // ---- S^T[16 tokens x 8 heads] = K . Q^T, two accumulation chains
     float sa[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     #pragma unroll
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(256) kv8_combine_rows_kernel(const float* pm, 
   #pragma unroll
   for (int k = 0; k < 8; ++k) {
     uint2 g = make_uint2(0u, 0u);
-    if (gate) g = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(gate) + e0 + 32 * k));
+    if (gate) g = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(gate) + e0 + 32 * k);
     const uint16_t gb[4] = {(uint16_t)g.x, (uint16_t)(g.x >> 16), (uint16_t)g.y, (uint16_t)(g.y >> 16)};
     uint32_t w[4];
     #pragma unroll

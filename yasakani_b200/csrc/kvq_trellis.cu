@@ -405,12 +405,12 @@ template <int NWORD> __device__ __forceinline__ void tba_words(const uint32_t* p
   if (NWORD % 4 == 0 && v16) {
     #pragma unroll
     for (int k = 0; k < NWORD / 4; ++k) {
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + k);
+      const uint4 u = reinterpret_cast<const uint4*>(p)[k];
       w[(4 * k) % NWORD] = u.x; w[(4 * k + 1) % NWORD] = u.y; w[(4 * k + 2) % NWORD] = u.z; w[(4 * k + 3) % NWORD] = u.w;
     }
   } else {
     #pragma unroll
-    for (int k = 0; k < NWORD; ++k) w[k] = __ldg(p + k);
+    for (int k = 0; k < NWORD; ++k) w[k] = p[k];
   }
 }
 
@@ -442,7 +442,7 @@ __device__ __forceinline__ void tba_values(const uint32_t* const (&r)[4], bool o
                                            float (&acc)[16][4]) {
   uint32_t w[4][KB], prev[4];
   #pragma unroll
-  for (int t = 0; t < 4; ++t) { tba_words(r[t], v16, w[t]); prev[t] = odd ? __ldg(r[t] - 1) : 0u; }
+  for (int t = 0; t < 4; ++t) { tba_words(r[t], v16, w[t]); prev[t] = odd ? r[t][-1] : 0u; }
   #pragma unroll
   for (int mt = 0; mt < 16; ++mt) {                                  // m-tile: channels 2 mt and 2 mt + 1 of the run as rows g and g + 8
     uint32_t x[2][4];
@@ -463,7 +463,7 @@ __device__ __forceinline__ void tba_values(const uint32_t* const (&r)[4], bool o
 // Value d of a row on its own (tb_unpack_kernel's rule), as its code.
 __device__ __forceinline__ float tba_value(const uint32_t* row, const float* cg, int kb, int d) {
   const int endb = kb * (d + 1), lo = max(endb - 8, kb * (d & ~63));
-  const uint32_t w0 = __ldg(row + (lo >> 5)), w1 = (lo & 31) + (endb - lo) > 32 ? __ldg(row + (lo >> 5) + 1) : 0u;
+  const uint32_t w0 = row[lo >> 5], w1 = (lo & 31) + (endb - lo) > 32 ? row[(lo >> 5) + 1] : 0u;
   return cg[__funnelshift_l(w1, w0, lo & 31) >> (32 - (endb - lo))];
 }
 
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
   asm volatile("griddepcontrol.wait;" ::: "memory");                 // programmatic dependent launch, both directions
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const float qs = A.qscale * 1.4426950408889634f;
-  const int pos = __ldg(A.d_pos) + r, len = max(0, min(pos + 1, A.max_ctx));
+  const int pos = *A.d_pos + r, len = max(0, min(pos + 1, A.max_ctx));
   const int per = (len + (int)gridDim.x - 1) / (int)gridDim.x, t0 = min(len, split * per), t1 = min(len, t0 + per);
   const size_t row0 = (size_t)kvh * A.max_ctx;
   const int psw = A.pay_stride / 4;
@@ -491,7 +491,6 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     asm volatile("prefetch.global.L2 [%0];\n prefetch.global.L2 [%1];" ::"l"(p), "l"(p + 31));
     if (!(lane & 15)) asm volatile("prefetch.global.L2 [%0];" ::"l"((lane < 16 ? A.k_side : A.v_side) + 2 * (row0 + t)));
   };
-  prefetch(t0 + 16 * warp);
   // ---- set-up.  The profile is a chain of five dependent reads (header, group offset, record, table offset, table); both groups walk it side by
   //      side and everything at its end is requested at once (one group after the other, entry by entry, took 20 us).
   constexpr int NQ = (256 * 8 + TBA_WARPS * 32 - 1) / (TBA_WARPS * 32);
@@ -501,11 +500,13 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     const int e = threadIdx.x + k * TBA_WARPS * 32, h = e >> 8, d = e & 255;
     qv[k] = h < G ? act_load<DT>(A.q16, ((size_t)r * A.nh + kvh * G + h) * 256 + d) : 0.f;
   }
+  const int gk = A.grp_k[kvh], gv = A.grp_v[kvh];
+  prefetch(t0 + 16 * warp);                                          // (waits for the position: behind the first loads of the chain)
   if (threadIdx.x == 0) S.big = 0;
   if (threadIdx.x < 8) S.qmax[threadIdx.x] = 0;
   TbRule rk, rv;
   {
-    const TbGroup Pg[2] = {tb_group(A.blob, __ldg(A.grp_k + kvh)), tb_group(A.blob, __ldg(A.grp_v + kvh))};
+    const TbGroup Pg[2] = {tb_group(A.blob, gk), tb_group(A.blob, gv)};
     unsigned to[2];
     #pragma unroll
     for (int w = 0; w < 2; ++w) to[w] = tb_table(A.blob, Pg[w]);
@@ -584,8 +585,8 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
   float m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f}, a0[2] = {0.f, 0.f}, a1[2] = {0.f, 0.f};
   float u[2] = {tba_pow2(TBA_EXP), tba_pow2(TBA_EXP)};               // acc holds sum x u
   auto side = [&](const uint32_t* sd, int t, int mm, float& s, float& c0, float& c1) {
-    s = __uint_as_float(__ldg(sd + 2 * (row0 + t)));
-    const uint32_t pc = __ldg(sd + 2 * (row0 + t) + 1);
+    s = __uint_as_float(sd[2 * (row0 + t)]);
+    const uint32_t pc = sd[2 * (row0 + t) + 1];
     c0 = mm > 0 ? __half2float(__ushort_as_half((unsigned short)(pc & 0xffffu))) : 0.f;
     c1 = mm > 1 ? __half2float(__ushort_as_half((unsigned short)(pc >> 16))) : 0.f;
   };
@@ -693,7 +694,7 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int d = 32 * k + lane;
-      x[k] = kpk ? tba_value(kpay + (size_t)t * psw, S.cg[0], rk.kb, d) * rk.gain * s0 : (A.k_plain ? __ldg(A.k_plain + (row0 + t) * 256 + d) : 0.f);
+      x[k] = kpk ? tba_value(kpay + (size_t)t * psw, S.cg[0], rk.kb, d) * rk.gain * s0 : (A.k_plain ? A.k_plain[(row0 + t) * 256 + d] : 0.f);
     }
     float sc[8];
     #pragma unroll
@@ -711,7 +712,7 @@ __global__ void __launch_bounds__(TBA_WARPS * 32, 1) tb_attn_kernel(TbAttnP P) {
     for (int k = 0; k < 8; ++k) {
       const int d = 32 * k + lane, i = tba_slot(d);
       x[k] = vpk ? fmaf(c0, S.term[1][0][i], fmaf(c1, S.term[1][1][i], fmaf(tba_value(vpay + (size_t)t * psw, S.cg[1], rv.kb, d) * rv.gain, s0, S.term[1][2][i])))
-                 : (A.v_plain ? __ldg(A.v_plain + (row0 + t) * 256 + d) : 0.f);
+                 : (A.v_plain ? A.v_plain[(row0 + t) * 256 + d] : 0.f);
     }
     #pragma unroll
     for (int h = 0; h < 8; ++h) {

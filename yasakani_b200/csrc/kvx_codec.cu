@@ -18,10 +18,10 @@ template <int DT> __device__ __forceinline__ void load_row(const void* base, siz
   for (int k = 0; k < 8; ++k) {
     const size_t d = row * 256 + 32 * k + 4 * ll;
     if (DT == YSKN_KV4_F32) {
-      const float4 a = live ? __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 a = live ? *reinterpret_cast<const float4*>(static_cast<const float*>(base) + d) : make_float4(0.f, 0.f, 0.f, 0.f);
       v[4 * k] = a.x; v[4 * k + 1] = a.y; v[4 * k + 2] = a.z; v[4 * k + 3] = a.w;
     } else {
-      const uint2 u = live ? __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + d)) : make_uint2(0u, 0u);
+      const uint2 u = live ? *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + d) : make_uint2(0u, 0u);
       v[4 * k] = DT == YSKN_KV4_F16 ? h2f((uint16_t)u.x) : bf2f((uint16_t)u.x); v[4 * k + 1] = DT == YSKN_KV4_F16 ? h2f((uint16_t)(u.x >> 16)) : bf2f((uint16_t)(u.x >> 16));
       v[4 * k + 2] = DT == YSKN_KV4_F16 ? h2f((uint16_t)u.y) : bf2f((uint16_t)u.y); v[4 * k + 3] = DT == YSKN_KV4_F16 ? h2f((uint16_t)(u.y >> 16)) : bf2f((uint16_t)(u.y >> 16));
     }
@@ -98,11 +98,11 @@ __global__ void __launch_bounds__(256) kvx_decode_kernel(const int8_t* q8, const
   const int lane = threadIdx.x & 31, ll = lane & 7;
   const long long row = (long long)blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5) * 4 + (lane >> 3);
   const bool live = row < rows;
-  const float sc = live ? __ldg(scales + row) : 0.f;
+  const float sc = live ? scales[row] : 0.f;
   float v[32];
   #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const uint32_t u = live ? __ldg(reinterpret_cast<const uint32_t*>(q8 + (size_t)row * 256 + 32 * k + 4 * ll)) : 0u;
+    const uint32_t u = live ? *reinterpret_cast<const uint32_t*>(q8 + (size_t)row * 256 + 32 * k + 4 * ll) : 0u;
     #pragma unroll
     for (int e = 0; e < 4; ++e) v[4 * k + e] = __fmul_rn((float)(int8_t)(uint8_t)(u >> (8 * e)), sc);
   }
@@ -130,15 +130,17 @@ __global__ void __launch_bounds__(256, 4) kvx_attn_post_kernel(yskn_kvx_attn_pos
   const int tok = live ? (int)(item / per_tok) : 0, u = live ? (int)(item % per_tok) : 0;
   const int kind = u < A.nh ? 0 : (u < A.nh + A.kvh ? 1 : 2);    // query / key / value head
   const int head = kind == 0 ? u : (kind == 1 ? u - A.nh : u - A.nh - A.kvh);
-  const int pos = __ldg(A.d_pos) + tok;
+  const int pos = *A.d_pos + tok;
   const uint16_t* src = kind == 0 ? A.q_rows + ((size_t)tok * A.nh + head) * 512
                                   : (kind == 1 ? A.k_rows : A.v_rows) + ((size_t)tok * A.kvh + head) * 256;
   float v[32];
   load_row<YSKN_KV4_BF16>(src, 0, ll, live, v);
   if (live && kind == 0) {                                       // the gate half of the head's projection, as it is
+    uint2 gate[8];                                               // all loads ahead of the first store
     #pragma unroll
-    for (int k = 0; k < 8; ++k)
-      *reinterpret_cast<uint2*>(A.gate16 + ((size_t)tok * A.nh + head) * 256 + 32 * k + 4 * ll) = __ldg(reinterpret_cast<const uint2*>(src + 256 + 32 * k + 4 * ll));
+    for (int k = 0; k < 8; ++k) gate[k] = *reinterpret_cast<const uint2*>(src + 256 + 32 * k + 4 * ll);
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) *reinterpret_cast<uint2*>(A.gate16 + ((size_t)tok * A.nh + head) * 256 + 32 * k + 4 * ll) = gate[k];
   }
   // ---- RMS norm (all lanes of a warp run the shuffles unless its four rows are all value heads, which keep their rows)
   float tot = 0.f;
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(256, 4) kvx_attn_post_kernel(yskn_kvx_attn_pos
     const uint16_t* wn = kind == 0 ? A.qn_w : A.kn_w;
     #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const uint2 w = __ldg(reinterpret_cast<const uint2*>(wn + 32 * k + 4 * ll));
+      const uint2 w = ld_table(reinterpret_cast<const uint2*>(wn + 32 * k + 4 * ll));
       const uint16_t wb[4] = {(uint16_t)w.x, (uint16_t)(w.x >> 16), (uint16_t)w.y, (uint16_t)(w.y >> 16)};
       #pragma unroll
       for (int e = 0; e < 4; ++e) v[4 * k + e] = rbf(__fmul_rn(__fmul_rn(v[4 * k + e], r), __fadd_rn(1.f, bf2f(wb[e]))));
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(256, 4) kvx_attn_post_kernel(yskn_kvx_attn_pos
     #pragma unroll
     for (int k = 0; k < NRH; ++k) {
       const float4* rr = reinterpret_cast<const float4*>(A.rope + ((size_t)pos * (32 * NRH) + 32 * k + 4 * ll) * 2);
-      const float4 c01 = live ? __ldg(rr) : make_float4(0.f, 0.f, 0.f, 0.f), c23 = live ? __ldg(rr + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 c01 = live ? ld_table(rr) : make_float4(0.f, 0.f, 0.f, 0.f), c23 = live ? ld_table(rr + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
       const float cs[4] = {c01.x, c01.z, c23.x, c23.z}, sn[4] = {c01.y, c01.w, c23.y, c23.w};
       #pragma unroll
       for (int e = 0; e < 4; ++e) {
