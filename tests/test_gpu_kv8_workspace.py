@@ -26,7 +26,8 @@ def _entry(c, M, S, out, ws=None):
     a = _lib.Kv8AttnArgsC(q.data_ptr(), k8.data_ptr(), v8.data_ptr(), ks.data_ptr(), vs.data_ptr(), k8.shape[1], M, pos.data_ptr(), S, *(t.data_ptr() for t in out),
                           KVH, NH, 0.0625)
     dt, st = {torch.float16: 0, torch.bfloat16: 1}[q.dtype], torch.cuda.current_stream().cuda_stream
-    assert lib.yskn_kv8_workspace_bytes(C.byref(a)) == (1024 * KVH * k8.shape[1] if M >= 384 else 0)
+    need = 1024 * KVH * k8.shape[1]
+    assert lib.yskn_kv8_workspace_bytes(C.byref(a)) == (need if M >= 384 and need <= 1 << 28 else 0)
     if ws is None:
         return lib.yskn_kv8_attention_tc(C.byref(a), dt, st)
     return lib.yskn_kv8_attention_ws(C.byref(a), dt, ws.data_ptr(), ws.numel(), st)
@@ -39,11 +40,15 @@ def _assert_same(a, b, keys):
     assert ((l0 - l1).abs() <= 2 * keys * 2.0 ** -24 * l1).all()
 
 
-@pytest.mark.parametrize("ctx,M,S", [(0, 65, 1), (0, 128, 2), (63, 65, 3), (127, 85, 1), (1000, 169, 1), (3001, 400, 2), (4096, 64, 5), (640, 8, 3)])
+# max_ctx None: the cache is full.  Otherwise capacities that the rows leave mostly empty (more and fewer runs of 16 rows than the preparation has
+# blocks), and an odd multiple of 64 that ends inside the last key tile.
+@pytest.mark.parametrize("ctx,M,S,max_ctx", [(0, 65, 1, None), (0, 128, 2, None), (63, 65, 3, None), (127, 85, 1, None), (1000, 169, 1, None), (3001, 400, 2, None),
+                                             (4096, 64, 5, None), (640, 8, 3, None), (100, 400, 1, 65536), (20000, 384, 1, 32832), (0, 384, 1, 448),
+                                             (5, 400, 1, 65600)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_partials_equal_the_converting_form(ctx, M, S, dtype):
+def test_partials_equal_the_converting_form(ctx, M, S, max_ctx, dtype):
     from yasakani_b200 import kv4
-    c = _case(ctx, M, dtype, seed=ctx + M)
+    c = _case(ctx, M, dtype, seed=ctx + M, max_ctx=max_ctx)
     ws = torch.full((1024 * KVH * c[1].shape[1],), 0xFF, dtype=torch.uint8, device="cuda")     # fp16 NaN wherever nothing is written
     outs = []
     for w in (ws, None):
@@ -73,3 +78,33 @@ def test_other_stream_and_capture_give_the_same_rows():
     graph.replay()
     torch.cuda.synchronize()
     _assert_same(want, graphed, 900)                                       # the converting form
+
+
+def test_cost_does_not_grow_with_the_capacity():
+    """400 rows at the start of a cache: time over a workspace in a cache of 65,536 tokens against one that is full (before the preparation's grid was
+    bounded 52 against 19 us), and no memory taken for a cache whose workspace would be larger than 256 MiB."""
+    from yasakani_b200 import kv4, kvx
+    M, times = 400, []
+    for max_ctx in (448, 65536):
+        c = _case(0, M, torch.bfloat16, seed=1, max_ctx=max_ctx)
+        out, ws = kv4.attn_scratch(M, 1, NH, 256), torch.empty(1024 * KVH * max_ctx, dtype=torch.uint8, device="cuda")
+        best = float("inf")
+        for _ in range(10):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(20):
+                _entry(c, M, 1, out, ws)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) / 20)
+        times.append(best)
+    assert times[1] < 1.4 * times[0], times
+    del ws
+    for max_ctx, most in ((65536, 1 << 28), (131072, 0)):
+        c, out = _case(0, M, torch.bfloat16, seed=1, max_ctx=max_ctx), kv4.attn_scratch(M, 1, NH, 256)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        kvx.launch_kv8_attention(*c[:5], M, c[5], 1, *out, NH)
+        assert torch.cuda.max_memory_allocated() - before <= most
+        assert torch.cuda.memory_allocated() == before                     # given back when the call returns

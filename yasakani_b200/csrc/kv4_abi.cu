@@ -75,7 +75,7 @@ static int attention_dispatch(const yskn_attn_g_args* a, int g, int hd, int rd, 
 using namespace kv4;
 
 constexpr int KV8_WS_MIN_ROWS = 384;
-constexpr size_t KV8_WS_MAX_BYTES = (size_t)1 << 30;
+constexpr size_t KV8_WS_MAX_BYTES = (size_t)1 << 28;         // a cache of 65,536 tokens of 4 kv-heads
 
 extern "C" {
 
@@ -377,9 +377,12 @@ int yskn_kv8_attention_tc(const yskn_kv8_attn_args* a, int act_dtype, void* cuda
 }
 // Converting inside the kernel costs every pair of 128-row tiles its own pass over the keys (4.0 us per 128 keys, against 1.5 from
 // fp16 rows); writing the rows first costs a launch and one pass over them.  The host does not know how many keys are visible, so
-// the line lies where the written rows win for any number of them.  Attention alone, converting / written rows, in us, behind
-// 0 and 8,000 tokens: 127 rows 14.9 / 16.4 and 58 / 43; 300 rows 17.0 / 18.7 and 109 / 65; 500 rows 21.9 / 20.3 and 213 / 102; 1,000 rows
-// 48 / 39 and 416 / 197.  1,000 rows behind 3,001 tokens, with row epilogue and merge: 264 -> 149 us.
+// the line lies where the written rows win for any number of them, or lose less than that launch.  Attention alone, converting / written
+// rows, in us, behind 0 and 8,000 tokens: 127 rows 14.9 / 16.4 and 58 / 43; 300 rows 17.0 / 18.7 and 109 / 65; 384 rows 19.2 / 19.1 (in a cache
+// much larger than its contents 20.4) and 212 / 101; 500 rows 21.8 / 20.2 and 208 / 101; 1,000 rows 47.7 / 39 and 414 / 198, whatever the
+// capacity.  1,000 rows behind 3,001 tokens, with row epilogue and merge: 264 -> 149 us.
+// The workspace grows with the capacity, not with the visible keys.  It is taken up to 256 MiB (0.15 % of the GPU's memory); beyond it a
+// pass that needed no memory before would hold as much as several layers' caches, so larger caches keep the converting form.
 size_t yskn_kv8_workspace_bytes(const yskn_kv8_attn_args* a) {
   if (!a || a->M < KV8_WS_MIN_ROWS || a->kvh <= 0 || a->max_ctx <= 0 || current_algo() == ALGO_SCALAR) return 0;
   if (!a->q16 || !a->pacc || (((uintptr_t)a->q16 | (uintptr_t)a->pacc) & 15)) return 0;

@@ -39,6 +39,7 @@
 // Every wait is bounded; a wait that runs out sets the device status word (4/5/6 = softmax / MMA / producer) and the CTA
 // frees its TMEM and returns.
 #include "kv4_common.cuh"
+#include <algorithm>
 #include <cuda.h>
 #include <cstring>
 #include <mutex>
@@ -391,22 +392,34 @@ __device__ __forceinline__ void tc_stage_q(uint32_t sq, int q_block, const uint1
 // ------------------------------------------------------------------------------------------------ INT8 rows -> fp16 workspace
 // K and V rows of every visible key as fp16 operand rows, by the very rule of the converting form (tc_i8_chunk: the two forms' operands
 // are equal bit for bit); zero rows up to the tile boundary.  HBM-bound byte mover (260 bytes in, 512 out per row): a thread takes
-// 16 channels of one row; rows past the last tile return at once.
+// 16 channels of a row.  The grid is bounded and strides over the visible rows, which only the device knows: with a block per 16 rows of the
+// cache's capacity, 384 rows at the start of a cache of 262,144 took 154 us with their attention, nearly all of it blocks without work (now
+// 20.3).  Twelve blocks an SM and a row in flight ahead: 4 / 8 / 12 / 16 blocks took 151.5 / 149.4 / 149.0 / 148.7 us for 1,000 rows behind 3,001 tokens
+// in a cache that is full, and 19.2 / 19.4 / 20.3 / 21.1 us for 384 rows at the start of a large one.
+constexpr int TC_PREP8_BLOCKS = 148 * 12;
 __global__ void __launch_bounds__(256) kv8_tc_prep_kernel(const int8_t* k8, const int8_t* v8, const float* ks, const float* vs, const int* d_pos, int M,
                                                           int max_ctx, uint16_t* kd, uint16_t* vd) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int t = (int)blockIdx.x * 16 + (int)(threadIdx.x >> 4), c = (int)(threadIdx.x & 15);     // grid (max_ctx / 16, kv-heads, K | V)
+  const int c = (int)(threadIdx.x & 15);                             // grid (runs of 16 rows, kv-heads, K | V)
   const int end = min(max_ctx, *d_pos + M), end_tile = min(max_ctx, (end + TC_BN - 1) / TC_BN * TC_BN);
-  if (t >= end_tile) return;
-  const size_t row = (size_t)blockIdx.y * max_ctx + t;
   const bool is_v = blockIdx.z != 0;
-  const uint4 w = reinterpret_cast<const uint4*>((is_v ? v8 : k8) + row * 256)[c];
-  const float sf = (is_v ? vs : ks)[row];
-  uint4 lo, hi;
-  tc_i8_chunk(w, sf, t < end, lo, hi);
-  uint4* dst = reinterpret_cast<uint4*>((is_v ? vd : kd) + row * 256) + 2 * c;
-  dst[0] = lo; dst[1] = hi;
+  const int step = 16 * (int)gridDim.x;
+  const size_t row0 = (size_t)blockIdx.y * max_ctx;
+  const int8_t* src = (is_v ? v8 : k8) + row0 * 256 + 16 * c;
+  const float* scale = (is_v ? vs : ks) + row0;
+  uint16_t* dst = (is_v ? vd : kd) + row0 * 256 + 16 * c;
+  int t = (int)blockIdx.x * 16 + (int)(threadIdx.x >> 4);
+  uint4 w = make_uint4(0u, 0u, 0u, 0u); float sf = 0.f;
+  if (t < end_tile) { w = *reinterpret_cast<const uint4*>(src + (size_t)t * 256); sf = scale[t]; }
+  for (; t < end_tile; t += step) {
+    const uint4 w1 = w; const float s1 = sf;
+    if (t + step < end_tile) { w = *reinterpret_cast<const uint4*>(src + (size_t)(t + step) * 256); sf = scale[t + step]; }   // ahead of this row's stores
+    uint4 lo, hi;
+    tc_i8_chunk(w1, s1, t < end, lo, hi);
+    uint4* d = reinterpret_cast<uint4*>(dst + (size_t)t * 256);
+    d[0] = lo; d[1] = hi;
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ attention kernel
@@ -1531,7 +1544,8 @@ int launch_kv8_attention_tc_ws(const yskn_kv8_attn_args& a, int act_dtype, void*
   if ((uintptr_t)ws & 15) KV4_REJECT("yskn_kv8_attention_ws: the workspace must be 16-byte aligned");
   using L = TcLay<256>;
   uint16_t* kd = static_cast<uint16_t*>(ws); uint16_t* vd = kd + (size_t)a.kvh * a.max_ctx * 256;
-  if (int rc = launch_pdl("kv8_tc_prep_kernel", kv8_tc_prep_kernel, dim3((unsigned)(a.max_ctx / 16), (unsigned)a.kvh, 2), 256, 0, st,
+  const int runs = std::max(1, std::min(a.max_ctx / 16, TC_PREP8_BLOCKS / (2 * a.kvh)));
+  if (int rc = launch_pdl("kv8_tc_prep_kernel", kv8_tc_prep_kernel, dim3((unsigned)runs, (unsigned)a.kvh, 2), 256, 0, st,
                           a.k8, a.v8, a.ks, a.vs, a.d_pos, a.M, a.max_ctx, kd, vd)) return rc;
   CUtensorMap mq, mkd, mvd;
   memset(&mq, 0, sizeof(mq));                                         // unused: the softmax warps stage Q
