@@ -108,3 +108,34 @@ def test_cost_does_not_grow_with_the_capacity():
         kvx.launch_kv8_attention(*c[:5], M, c[5], 1, *out, NH)
         assert torch.cuda.max_memory_allocated() - before <= most
         assert torch.cuda.memory_allocated() == before                     # given back when the call returns
+
+
+def test_scratch_is_no_tensor_and_no_part_of_another_streams_capture():
+    """The scratch of a launch is seen by no dispatch mode (nor filled in deterministic mode), and it may be taken while another stream is under
+    capture in global mode, where an ordinary allocation would end the capture with an error."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from yasakani_b200 import kv4, kvx
+
+    class Ops(TorchDispatchMode):
+        seen = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    M, c = 400, _case(300, 400, torch.bfloat16, seed=5)
+    want, got, x = kv4.attn_scratch(M, 1, NH, 256), kv4.attn_scratch(M, 1, NH, 256), torch.ones(1000, device="cuda")
+    with Ops():
+        kvx.launch_kv8_attention(*c[:5], M, c[5], 1, *want, NH)
+    assert not Ops.seen, Ops.seen
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()                                               # the next scratch is not in the cache
+    other, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):                                          # global mode: the strictest
+        x *= 2
+        kvx.launch_kv8_attention(*c[:5], M, c[5], 1, *got, NH, stream=other)
+    other.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, got)) and kv4.device_status() == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (x == 2).all()

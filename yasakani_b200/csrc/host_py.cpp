@@ -7,10 +7,10 @@
 // TypeError / ValueError for types and shapes, Kv4Error with the library's message for a rejected call.  The library call
 // itself runs without the interpreter lock, as a ctypes call does.
 #include <torch/csrc/autograd/python_variable.h>
-#include <ATen/Functions.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
-#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cstdlib>
 #include "../../include/yskn_kv4_abi.h"
 
 namespace {
@@ -235,18 +235,24 @@ FN(attn_post) {                                          // q_rows, k_rows, v_ro
   });
 }
 
-// Device memory for the work of one call, from torch's allocator for the stream the call runs on: given back when the call returns,
-// and handed out again only behind this work in that stream.  Undefined (the caller's form without it runs) when nothing is asked for, when the
-// stream is being captured (a graph outlives the call) and when there is no memory.
-at::Tensor scratch(size_t bytes, cudaStream_t st) {
-  if (!bytes) return {};
-  const c10::cuda::CUDAStream cur = c10::cuda::getCurrentCUDAStream();
-  c10::cuda::OptionalCUDAStreamGuard on;
-  if (cur.stream() != st) on.reset_stream(c10::cuda::getStreamFromExternal(st, cur.device_index()));
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return {};
-  try { return at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, cur.device_index())); }
-  catch (const c10::OutOfMemoryError&) { return {}; }
-}
+// Device memory for the work of one call, from torch's caching allocator for the stream the call runs on: given back when the call returns,
+// and handed out again only behind this work in that stream.  Straight from the allocator: a tensor would be filled in torch's deterministic mode and
+// seen by dispatch modes.  None (the caller's form without it runs) when nothing is asked for, when the stream is being captured (a
+// graph outlives the call), when there is no memory, and when torch caches none (every call would wait for the GPU).  Another stream may
+// be under capture, in this thread or another: the allocation is no part of it and is made in relaxed mode.
+struct Scratch {
+  void* p = nullptr;
+  size_t bytes = 0;
+  Scratch(size_t n, cudaStream_t st) {
+    if (!n || getenv("PYTORCH_NO_CUDA_MEMORY_CACHING")) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
+    const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+    try { p = c10::cuda::CUDACachingAllocator::raw_alloc_with_stream(n, st); bytes = n; } catch (const c10::OutOfMemoryError&) {}
+  }
+  ~Scratch() { if (p) c10::cuda::CUDACachingAllocator::raw_delete(p); }
+  Scratch(const Scratch&) = delete;
+};
 
 // q16, k8, v8, ks, vs, M, d_pos, splits, pm, pl, pacc, nh, qscale, stream
 PyObject* kv8(PyObject* const* v, Py_ssize_t n, const char* who, int (*entry)(const yskn_kv8_attn_args*, int, void*)) {
@@ -259,8 +265,8 @@ PyObject* kv8(PyObject* const* v, Py_ssize_t n, const char* who, int (*entry)(co
                                int_of(v[11]), float_of(v[12])};
     const int dt = dtype_code(q);
     const cudaStream_t st = stream_of(v[13]);
-    const at::Tensor ws = scratch(yskn_kv8_workspace_bytes(&a), st);
-    if (ws.defined()) return call(who, [&] { return yskn_kv8_attention_ws(&a, dt, ws.data_ptr(), (size_t)ws.numel(), st); });
+    const Scratch ws(yskn_kv8_workspace_bytes(&a), st);
+    if (ws.p) return call(who, [&] { return yskn_kv8_attention_ws(&a, dt, ws.p, ws.bytes, st); });
     return call(who, [&] { return entry(&a, dt, st); });
   });
 }
