@@ -149,7 +149,7 @@ def load():
     if _LIB is None:
         path = _build.LIB
         if not os.path.exists(path) or os.environ.get("YSKN_KV4_REBUILD"):
-            path = _build.build()
+            path = _build.build_lib()
         L = C.CDLL(path)
         for name, (res, args) in PROTOTYPES.items():
             fn = getattr(L, name)          # AttributeError here = header and library disagree
@@ -159,16 +159,17 @@ def load():
 
 
 class _Host:
-    """The extension module `_host` (csrc/host_py.cpp), loaded at the first use of one of its functions."""
+    """The extension module `_host` (csrc/host_py.cpp), loaded at the first use of one of its functions (and compiled first where there is none
+    for this torch, this Python and this ABI header).  It calls the library that load() has loaded, never a second copy of it."""
 
     def __getattr__(self, name):
         import torch  # noqa: F401  (the extension links against torch's libraries)
-        load()
-        if not os.path.exists(_build.HOST):
-            _build.build()
-        spec = importlib.util.spec_from_file_location("yasakani_b200._host", _build.HOST)
+        lib = load()
+        spec = importlib.util.spec_from_file_location("yasakani_b200._host", _build.build_host())
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
+        if mod.library() != C.cast(lib.yskn_kv4_last_error, C.c_void_p).value:
+            raise ImportError("yasakani_b200: another copy of libyskn_kv4.so was built while this one was loaded; start the process again")
         self.__dict__.update({k: v for k, v in vars(mod).items() if not k.startswith("__")})
         return self.__dict__[name]
 

@@ -300,9 +300,13 @@ FN(tb_attention) {  // profile, q16, k_pay, k_side, v_pay, v_side, grp_k, grp_v,
   });
 }
 
+PyObject* library(PyObject*, PyObject* const*, Py_ssize_t) {  // where the library this module calls is loaded
+  return PyLong_FromVoidPtr((void*)yskn_kv4_last_error);
+}
+
 #define M_(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {M_(kv_append), M_(attention), M_(decode), M_(combine), M_(attention_ms), M_(attention_tc), M_(prefill_tc), M_(attn_post),
-                         M_(kv8_attention), M_(kv8_attention_tc), M_(kv8_combine), M_(tb_attention), {nullptr, nullptr, 0, nullptr}};
+                         M_(kv8_attention), M_(kv8_attention_tc), M_(kv8_combine), M_(tb_attention), M_(library), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "argument marshalling of the hot launchers", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
