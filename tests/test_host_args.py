@@ -42,3 +42,19 @@ def test_a_call_the_library_refuses_carries_its_message():
     pm = torch.zeros((1, 2, 16))
     with pytest.raises(Kv4Error, match="unsupported head_dim 24"):
         kv4.launch_attn_combine_gqa(pm, pm, pm, 2, 1, torch.zeros((1, 16, 24), dtype=torch.float16), 16, 8, stream=type("S", (), {"cuda_stream": 0})())
+
+
+@pytest.mark.parametrize("name", ["q16", "d_pos", "pm", "pl", "pacc"])
+@pytest.mark.parametrize("value", [None, 3])
+def test_what_is_no_tensor_raises_attribute_error(name, value):
+    with pytest.raises(AttributeError):
+        kv4.launch_decode(**_decode_args(**{name: value}))
+
+
+@pytest.mark.gpu
+def test_a_missing_buffer_is_the_librarys_to_refuse():
+    o16 = torch.zeros((1, 16, 256), dtype=torch.float16, device="cuda")
+    with pytest.raises(Kv4Error, match="null buffer"):
+        kvx.launch_kv8_combine(None, None, None, 2, 1, 16, o16)
+    with pytest.raises(AttributeError):
+        kvx.launch_kv8_combine(None, None, None, 2, 1, 16, None)

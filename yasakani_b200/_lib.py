@@ -139,6 +139,10 @@ class Kv4Error(RuntimeError):
     pass
 
 
+class NotATensor(AttributeError, TypeError):
+    """An argument that should be a tensor has none of a tensor's attributes."""
+
+
 def lib_path() -> str:
     return _build.LIB
 

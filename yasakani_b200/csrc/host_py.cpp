@@ -3,9 +3,10 @@
 // What bounds it: a decode step of a few microseconds on the GPU is two or three calls from Python.  Building the argument
 // structs through ctypes (attribute look-ups, data_ptr() calls, nested Structure constructors, one checked conversion per
 // argument) took 8-10 us a call; here a call reads the tensors' C++ objects directly and takes about 1 us beside the launch itself.
-// Checks and exception types are those of the Python code it replaces: AssertionError for buffers that do not fit,
-// TypeError / ValueError for types and shapes, Kv4Error with the library's message for a rejected call.  The library call
-// itself runs without the interpreter lock, as a ctypes call does.
+// Checks and exception types are those of the Python code it replaces: AssertionError for buffers that do not fit, AttributeError (NotATensor,
+// also a TypeError) for what is no tensor, TypeError / ValueError for types and shapes, Kv4Error with the library's message for a rejected
+// call, a missing buffer (None) among them where the launcher left that check to the library.  Integers beyond a C int raise OverflowError
+// (ctypes cut them off).  The library call itself runs without the interpreter lock, as a ctypes call does.
 #include <torch/csrc/autograd/python_variable.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -15,14 +16,14 @@
 
 namespace {
 
-PyObject* g_kv4_error = nullptr;
+PyObject *g_kv4_error = nullptr, *g_not_a_tensor = nullptr;
 struct Names { PyObject *kq, *kscale, *kzero, *kshadow, *vq, *vscale, *vzero, *hkv, *hd, *max_ctx, *cuda_stream, *maps_ptr, *d_layers, *n, *dev; } N;
 
 struct PyFail {};                                       // a Python exception is set
 [[noreturn]] void fail(PyObject* type, const char* msg) { PyErr_SetString(type, msg); throw PyFail{}; }
 
 const at::Tensor& tensor(PyObject* o, const char* what) {
-  if (!THPVariable_Check(o)) { PyErr_Format(PyExc_TypeError, "%s: a tensor is needed", what); throw PyFail{}; }
+  if (!THPVariable_Check(o)) { PyErr_Format(g_not_a_tensor, "%s: '%s' object is not a tensor", what, Py_TYPE(o)->tp_name); throw PyFail{}; }
   return THPVariable_Unpack(o);
 }
 void check_dev(const at::Tensor& t, const char* what) {
@@ -204,7 +205,7 @@ FN(prefill_tc) {                                         // the eleven of attn_o
   return guarded(n, 17, [&]() -> PyObject* {
     const Attn A = attn_of(v);
     const int rd = int_of(v[11]), valid = int_of(v[15]);
-    uint16_t* o16 = (uint16_t*)dev_ptr(v[12], "o16");
+    uint16_t* o16 = (uint16_t*)opt_dev(v[12], "o16");
     const uint16_t* bv = (const uint16_t*)opt_raw(v[14], "bv");
     void* ws; size_t wb;
     ws_of(v[13], &ws, &wb);
@@ -227,8 +228,8 @@ FN(attn_post) {                                          // q_rows, k_rows, v_ro
     const int pm = PyObject_IsTrue(v[15]);
     if (pm < 0) throw PyFail{};
     const yskn_kvx_attn_post_args a{u16(0, "q_rows"), u16(1, "k_rows"), u16(2, "v_rows"), u16(3, "qn_w"), u16(4, "kn_w"), float_of(v[5]), M,
-                                    (const int*)dev_ptr(v[6], "d_pos"), (const float*)opt_dev(v[7], "rope"), int_of(v[8]), u16(9, "q16"), u16(10, "gate16"),
-                                    (int8_t*)dev_ptr(v[11], "k8"), (int8_t*)dev_ptr(v[13], "v8"), (float*)dev_ptr(v[12], "ks"), (float*)dev_ptr(v[14], "vs"),
+                                    (const int*)opt_dev(v[6], "d_pos"), (const float*)opt_dev(v[7], "rope"), int_of(v[8]), u16(9, "q16"), u16(10, "gate16"),
+                                    (int8_t*)dev_ptr(v[11], "k8"), (int8_t*)opt_dev(v[13], "v8"), (float*)opt_dev(v[12], "ks"), (float*)opt_dev(v[14], "vs"),
                                     max_ctx, nh, kvh, pm};
     const cudaStream_t st = stream_of(v[16]);
     return call("yskn_kvx_attn_post", [&] { return yskn_kvx_attn_post(&a, st); });
@@ -275,7 +276,7 @@ FN(kv8_attention_tc) { return kv8(v, n, "yskn_kv8_attention_tc", yskn_kv8_attent
 
 FN(kv8_combine) {                                        // pm, pl, pacc, splits, M, nh, o16, gate, inverse_rotate, stream
   return guarded(n, 10, [&]() -> PyObject* {
-    const float *pm = (const float*)dev_ptr(v[0], "pm"), *pl = (const float*)dev_ptr(v[1], "pl"), *pacc = (const float*)dev_ptr(v[2], "pacc");
+    const float *pm = (const float*)opt_dev(v[0], "pm"), *pl = (const float*)opt_dev(v[1], "pl"), *pacc = (const float*)opt_dev(v[2], "pacc");
     const int splits = int_of(v[3]), M = int_of(v[4]), nh = int_of(v[5]), inv = PyObject_IsTrue(v[8]);
     if (inv < 0) throw PyFail{};
     void *o16 = dev_ptr(v[6], "o16"), *gate = opt_dev(v[7], "gate");
@@ -290,10 +291,10 @@ FN(tb_attention) {  // profile, q16, k_pay, k_side, v_pay, v_side, grp_k, grp_v,
     const at::Tensor& kp = tensor(v[2], "k_pay");
     if (kp.dim() != 3) fail(PyExc_ValueError, "k_pay [kvh, max_ctx, stride]");
     const yskn_tb_attn_args a{(const uint16_t*)dev_ptr(v[1], "q16"), (const uint8_t*)dev_ptr(attr(v[0], N.dev).p, "profile"), (const uint8_t*)dev_ptr(v[2], "k_pay"),
-                              (const uint8_t*)dev_ptr(v[4], "v_pay"), (int)kp.size(2), (const uint32_t*)dev_ptr(v[3], "k_side"), (const uint32_t*)dev_ptr(v[5], "v_side"),
-                              (const int*)dev_ptr(v[6], "grp_k"), (const int*)dev_ptr(v[7], "grp_v"), (const float*)opt_dev(v[15], "k_plain"),
-                              (const float*)opt_dev(v[16], "v_plain"), (int)kp.size(1), int_of(v[8]), (const int*)dev_ptr(v[9], "d_pos"), int_of(v[10]),
-                              (float*)dev_ptr(v[11], "pm"), (float*)dev_ptr(v[12], "pl"), (float*)dev_ptr(v[13], "pacc"), (int)kp.size(0), int_of(v[14]), float_of(v[17])};
+                              (const uint8_t*)opt_dev(v[4], "v_pay"), (int)kp.size(2), (const uint32_t*)opt_dev(v[3], "k_side"), (const uint32_t*)opt_dev(v[5], "v_side"),
+                              (const int*)opt_dev(v[6], "grp_k"), (const int*)opt_dev(v[7], "grp_v"), (const float*)opt_dev(v[15], "k_plain"),
+                              (const float*)opt_dev(v[16], "v_plain"), (int)kp.size(1), int_of(v[8]), (const int*)opt_dev(v[9], "d_pos"), int_of(v[10]),
+                              (float*)opt_dev(v[11], "pm"), (float*)opt_dev(v[12], "pl"), (float*)opt_dev(v[13], "pacc"), (int)kp.size(0), int_of(v[14]), float_of(v[17])};
     const int dt = dtype_code(tensor(v[1], "q16"));
     const cudaStream_t st = stream_of(v[18]);
     return call("yskn_tb_attention", [&] { return yskn_tb_attention(&a, dt, st); });
@@ -315,8 +316,9 @@ PyMODINIT_FUNC PyInit__host() {
   PyObject* lib = PyImport_ImportModule("yasakani_b200._lib");
   if (!lib) return nullptr;
   g_kv4_error = PyObject_GetAttrString(lib, "Kv4Error");
+  g_not_a_tensor = PyObject_GetAttrString(lib, "NotATensor");
   Py_DECREF(lib);
-  if (!g_kv4_error) return nullptr;
+  if (!g_kv4_error || !g_not_a_tensor) return nullptr;
   struct { PyObject** p; const char* s; } names[] = {{&N.kq, "kq"}, {&N.kscale, "kscale"}, {&N.kzero, "kzero"}, {&N.kshadow, "kshadow"}, {&N.vq, "vq"},
       {&N.vscale, "vscale"}, {&N.vzero, "vzero"}, {&N.hkv, "hkv"}, {&N.hd, "hd"}, {&N.max_ctx, "max_ctx"}, {&N.cuda_stream, "cuda_stream"},
       {&N.maps_ptr, "maps_ptr"}, {&N.d_layers, "d_layers"}, {&N.n, "n"}, {&N.dev, "dev"}};
