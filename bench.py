@@ -718,7 +718,7 @@ def run_secondary(args):
                             "splits": S, "l2": f"2 cache copies cycled; {byt / 1e6:.1f} MB read per launch: L2-resident, the kernel is latency-bound"},
                     gpu_launches=K,
                     roofline={"bound": "hbm", "achieved": byt / t / 1e9, "peak": hbm, "unit": "GB/s", "frac": byt / t / 1e9 / hbm, "traffic": None,
-                              "kernel": "tb_attn32_kernel", "bytes_per_launch": byt, "peak_kind": f"of {kind}"})
+                              "kernel": "tb_attn_kernel", "bytes_per_launch": byt, "peak_kind": f"of {kind}"})
         print(json.dumps(line), flush=True)
     elif args.workload == "kvx":
         rows = 1 << 20

@@ -363,8 +363,8 @@ YSKN_KV4_API int yskn_tb_encode_whole(const uint8_t* d_blob, int nm, const float
  * of each head's rows; rows the profile leaves unpacked (position below the group's guard, or a group that is not a
  * packed one) are read from k_plain / v_plain fp32 [kvh][max_ctx][256] (NULL: zeros), the `yin` of yskn_tb_decode.
  * q16 [M][nh][256] bf16 or fp16; row r sits at *d_pos + r and sees keys 0 .. *d_pos + r; partials in the layout of
- * yskn_kv8_attention (merge with yskn_kv8_combine).  Warp-level tensor-core tiles over looked-up codes with queries and weights in two fp16
- * parts; rows the profile leaves unpacked, and code tables beyond +-2,048, take a slower fp32 path inside the same launch. */
+ * yskn_kv8_attention (merge with yskn_kv8_combine).  Warp-level tensor-core tiles over looked-up codes, queries and weights in
+ * fp32 accuracy and range; rows the profile leaves unpacked, and code tables beyond +-2,048, take a slower fp32 path inside the same launch. */
 typedef struct {
   const uint16_t* q16; const uint8_t* blob;
   const uint8_t* k_pay; const uint8_t* v_pay; int pay_stride;

@@ -14,7 +14,7 @@
 //     fp32 arithmetic, one rounding to fp16.  HBM-bound byte mover: one warp per (token, kv-head).
 //  2. kv4_tc_attn_kernel: a pair of CTAs (cluster of two, tcgen05 cta_group::2) = 256 query rows ((token, head) pairs
 //     of one kv-head, 128 per CTA) x one split of the keys, in tiles of 128 keys.  Per CTA:
-//       warp 8      TMA producer: its Q rows once, then its half of every K tile (64 keys) and V tile (HD/2 channels)
+//       warp 8      TMA producer: its Q rows once (form 0), then its half of every K tile (64 keys) and V tile (HD/2 channels)
 //                   into two mbarrier rings, one tiled copy each; the copies report to the leader CTA's barriers
 //       warp 9      (leader CTA only) one thread issues every tcgen05.mma of the pair: S = Q.K^T (M256 N128 K16 steps, Q and
 //                   K from shared memory, K-major, 128-byte swizzle) into one of two TMEM buffers, and O += P.V (M256
@@ -26,15 +26,17 @@
 //     Tiles that contain a row's own group ("edge" tiles) get S twice, from Kd and from Ks, and each row picks per
 //     32-key group: int4 keys for groups before its own, shadow keys (causally masked) for its own.
 //
-//  The attention kernel has five forms (template FORM): 0 = operand tiles by TMA from the workspace, as above (3 = the same
-//  with bf16 queries and output rows: the softmax warps convert the queries, there is no Q copy; 4 = the same over a workspace of
-//  Family-B INT8 rows); 1 = no
-//  workspace and no prep launch, converter warps build the tiles from the packed KV4 cache inside the kernel; 2 = the same over
-//  Family-B INT8 rows.  The converting forms run 16 warps: 0-7 softmax, 8 Q copy + MMA issue, 9-11 V tiles, 12-15 K tiles.
+//  The attention kernel has five forms (template FORM): 0 = operand tiles by TMA from the workspace, as above; 3 = the same
+//  with bf16 queries and output rows; 4 = the same over a workspace of Family-B INT8 rows; 1 = no workspace and no prep launch,
+//  converter warps build the tiles from the packed KV4 cache inside the kernel; 2 = the same over Family-B INT8 rows.  Only form 0
+//  copies its queries by TMA, in the others the softmax warps stage them.  The converting forms (1, 2) run 16 warps: 0-7 softmax, 8 MMA
+//  issue, 9-11 V tiles, 12-15 K tiles.
 //
 // Rows are independent of one another inside every step (an MMA output row depends on its own A row only, the lazy
 // rescale multiplies other rows by exactly 1), tiles start at multiples of 128 keys and split boundaries depend on
-// *d_pos and `splits` only, so a row's result does not depend on how many rows the pass holds.
+// *d_pos and `splits` only, so within a form a row's result does not depend on how many rows the pass holds.  Forms differ in the order in
+// which a row's weights are added (pl, and with it the last bit of the row): over INT8 rows a pass takes form 4 from 384 rows on, where its caller
+// lends a workspace, and form 2 otherwise.
 //
 // Every wait is bounded; a wait that runs out sets the device status word (4/5/6 = softmax / MMA / producer) and the CTA
 // frees its TMEM and returns.
@@ -430,7 +432,7 @@ constexpr int TC_KW = 4, TC_VW = 3, TC_CW = TC_KW + TC_VW;  // converter warps o
 // The workspace forms launch three warpgroups of 168 registers a thread (504 per scheduler lane): 208 for the two of softmax warps, whose threads hold
 // a whole row of a tile, 88 for producer and MMA issuer (two of its four warps have no role).
 constexpr int tc_threads(bool fused) { return fused ? 512 : 384; }
-static_assert(TC_SW == 8 && TC_SW + 1 + TC_CW <= 16, "warpgroups 0-1 = softmax warps, warpgroups 2-3 = Q copy + MMA issuer (one warp), converters");
+static_assert(TC_SW == 8 && TC_SW + 1 + TC_CW <= 16, "warpgroups 0-1 = softmax warps, warpgroups 2-3 = MMA issuer (one warp), converters");
 constexpr int TC_THREADS = tc_threads(false);
 
 // A pair of CTAs (a cluster of two, tcgen05 cta_group::2) works on 256 query rows with MMAs of M = 256: each CTA keeps
@@ -466,7 +468,7 @@ struct TcP {
   float* pm; float* pl; float* pacc;
   uint16_t* o16; const uint16_t* bv;                       // splits == 1 and o16 set: store the finished rows, no partials
   yskn_kv_layer kv; const float* rope; int rd;             // the fused form reads the packed cache itself
-  const uint16_t* q16; int bf16;                           // fused form with bf16 activations: the converter warps also stage Q (as fp16)
+  const uint16_t* q16; int bf16;                           // all forms but 0: the softmax warps stage Q (as fp16)
   const int8_t* k8; const int8_t* v8; const float* ks8; const float* vs8;     // FORM 2: INT8 rows and their scales
 };
 
@@ -481,7 +483,7 @@ struct TcP {
 // reference's q35_attention_kernel<KV8> semantics, src/q35_kernels.cu:1176-1281, for many rows): every key is an INT8 row,
 // nothing is rotated at read time and there is no shadow, so every tile has one K item and the tiles that hold the new
 // rows are masked causally.  A byte is read as the fp16 number 1152 + b by one byte permute, the offset leaves by an exact
-// subtraction, and the row's scale (rounded to fp16) is multiplied in.
+// subtraction, and the row's scale (as two fp16 terms) is multiplied in.
 // FORM 4: FORM 3 over INT8 rows: kv8_tc_prep_kernel has written K and V as fp16 rows.  Long passes convert every key once instead of once per
 // 256 query rows.
 template <int HD, int FORM>

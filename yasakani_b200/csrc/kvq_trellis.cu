@@ -352,8 +352,8 @@ __global__ void __launch_bounds__(256) tb_unpack_kernel(TbDecP A) {
 //   * the row terms of the unpack rule leave the loops: q.x = s * gain / 256 * sum_d q_d code_d + c0 (q.U0) + c1 (q.U1) + q.mu, and
 //     O = sum_t p_t s_t code_t + (sum p_t c0_t) U0 + (sum p_t c1_t) U1 + (sum p_t) mu.
 // Rows that the profile leaves unpacked (positions below the guard, at most 255; a group without packed rows) take the row path, a warp
-// per token in fp32.  30,011 tokens of 4 kv-heads on a B200: 152 us (32 keys per warp step in scalar fp32, tables in shared memory with
-// bank conflicts) -> 31 us, of which 14 are set-up, merge and the launch.
+// per token in fp32.  32,768 tokens of 4 kv-heads on a B200: 152 us (32 keys per warp step in scalar fp32, tables in shared memory with
+// bank conflicts) -> 33.9 us, of which 14 are set-up, merge and the launch.
 constexpr int TBA_WARPS = 12;                                        // 3 per scheduler at up to 168 registers
 struct TbAttnP { yskn_tb_attn_args a; int G; };
 constexpr uint32_t TBA_TAB = 32768;                                  // bytes of a replicated table, and the alignment of its shared-memory address
