@@ -247,7 +247,8 @@ struct Scratch {
   Scratch(size_t n, cudaStream_t st) {
     if (!n || getenv("PYTORCH_NO_CUDA_MEMORY_CACHING")) return;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) { (void)cudaGetLastError(); return; }      // the launch itself will tell
+    if (cap != cudaStreamCaptureStatusNone) return;
     const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
     try { p = c10::cuda::CUDACachingAllocator::raw_alloc_with_stream(n, st); bytes = n; } catch (const c10::OutOfMemoryError&) {}
   }
