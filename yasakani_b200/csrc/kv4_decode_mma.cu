@@ -21,17 +21,17 @@
 //   O^T[HD x 8 heads]     += V^T[HD x 16 tok] . P^T[16 tok x 8 heads]    (HD/16 m-tiles)
 // so one K/V tile serves all G <= 8 query heads of the group, and the packed bytes go from shared memory straight
 // into A-fragment registers:
-//   * a 32-bit word holds 8 nibbles; one LOP3 reads nibbles (x, x+4) in place as the half2 (off+n_x, off+n_{x+4}):
-//     bits 0..3 of a half count in steps of 1 under exponent 2^10 (off 1024), bits 4..7 under 2^6 (off 64).  That is
-//     exactly one A register because the contraction order over channels is free.  K's per-channel scale is folded
-//     into Q once per group (q' = q*scale); the zero points and the offsets become a per-head bias,
-//     sum q*zero - sum off*q', formed by two more MMA rows so that the offsets cancel against the rounded q'.
+//   * a 32-bit word holds 8 nibbles; one AND reads nibbles (x, x+4) in place as two fp16 subnormals, n * 2^-24 at bits 0..3 of a
+//     half, n * 2^-20 at bits 4..7: exactly one A register, because the contraction order over channels is free.  The tensor core
+//     multiplies subnormals exactly and sums in fp32, so the factor is taken out of the sum (one accumulator per factor).  K's
+//     per-channel scale is folded into Q once per group (q' = q*scale); the zero points become a per-head bias, sum q*zero, formed
+//     by two more MMA rows.
 //   * for V the contraction runs over tokens: a transposed 8x8 shared-memory load (ldmatrix.trans) hands a lane the same
 //     four channels of two consecutive tokens in one register, which is the pairing an A register wants.  V's per-token
-//     scale is folded into P and its zero point into a per-head scalar.  The even channels' offset of 1024 is removed by
-//     an exact fp16 subtraction before the MMA: the tensor core's fp32 accumulators truncate, and a sum that carries
-//     1024 * sum(p) loses about 2e-3 of the output at 262,144 tokens (measured, on the even channels only); the odd
-//     channels' offset of 64 stays and is cancelled by an MMA row of ones over the same rounded P.
+//     scale is folded into P and its zero point into a per-head scalar.  No offset may ride along in these sums: the tensor
+//     core's fp32 accumulators truncate, and one that carried 1024 * sum(p) lost about 2e-3 of the output at 262,144 tokens.
+//     Before the subnormals, offsets (1024 + n, 64 + n) were added by the logic op and taken out again by subtractions and by MMA rows
+//     of ones: 262,144 tokens 85.6 -> 82.2 us, eight sequences 124.2 -> 116.9 us (both tiles of a group in step, see below, included).
 //   * RoPE: Q is rotated back by the group's first position (one table row per group), the remaining angle
 //     (0..31 tokens) is applied to the rotary channels of K with the table's first 32 rows.  cos/sin of
 //     (t0 + dt) are thereby formed by angle addition from the caller's table entries for t0 and dt.  The table's own
@@ -147,7 +147,7 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v; asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a)); return v;
 }
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void ldmatrix_x4_t(uint32_t a, uint32_t (&r)[4]) {
@@ -159,27 +159,29 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) { uint32_t d; as
 __device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) { uint32_t d; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 __device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
 __device__ __forceinline__ uint32_t hadd2(uint32_t a, uint32_t b) { uint32_t d; asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
-__device__ __forceinline__ uint32_t hneg2(uint32_t a) { return a ^ 0x80008000u; }
-// A 32-bit word of a packed row holds nibbles 0..7.  Register X pairs nibbles (X, X+4) as the two halves of a
-// half2 WITHOUT moving them: nibbles at bits 0..3 of a half read as 1024 + n under exponent 2^10 (0x6400), nibbles at
-// bits 4..7 as 64 + n under exponent 2^6 (0x5400).  One shift (w >> 8) serves X = 2, 3.  The constant offsets are
-// removed exactly: on the Q side by an MMA row of the same constants, on the rotary path by an exact subtraction.
-constexpr uint32_t OFF_E = 0x64006400u, OFF_O = 0x54005400u;       // (1024,1024), (64,64)
-constexpr uint32_t NEG_E = 0xE400E400u, NEG_O = 0xD400D400u;       // their negatives
+__device__ __forceinline__ uint32_t hneg2(uint32_t a) { uint32_t d; asm("neg.f16x2 %0, %1;" : "=r"(d) : "r"(a)); return d; }
+// A 32-bit word of a packed row holds nibbles 0..7.  One AND pairs nibbles (X, X+4) as the two halves of a register
+// WITHOUT moving them (one shift, w >> 8, serves X = 2, 3), and the halves are fp16 subnormals: a nibble at bits 0..3 reads as n * 2^-24, at
+// bits 4..7 as n * 2^-20.  The tensor core multiplies subnormals exactly, so the factor leaves behind the fp32 sum, and nothing is added to the
+// operands.  Rotary words need the value itself: under exponent 2^10 (0x6400) or 2^6 (0x5400) the halves read as 1024 + n or 64 + n, and the
+// constant leaves by an exact subtraction.
+constexpr uint32_t NIB_E = 0x000F000Fu, NIB_O = 0x00F000F0u;
+constexpr float NIB_E_INV = 16777216.f, NIB_O_INV = 1048576.f;     // 2^24, 2^20
+constexpr uint32_t NEG_E = 0xE400E400u, NEG_O = 0xD400D400u;       // -(1024, 1024), -(64, 64)
 // (a & m) | c as ONE LOP3.  LOP3 takes a single immediate, so with two literal constants the compiler emits AND then OR
 // (measured: 562 LOP3 per group instead of ~280); the masks and offsets are therefore kept in registers that the
 // compiler cannot fold (NibK).
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t m, uint32_t c) {
   uint32_t d; asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(m), "r"(c)); return d;
 }
-struct NibK { uint32_t m0, m1, e, o; };                          // 0x000F000F, 0x00F000F0, OFF_E, OFF_O
+struct NibK { uint32_t m0, m1, e, o; };                          // the masks; (1024, 1024), (64, 64)
 __device__ __forceinline__ NibK nib_consts() {
   NibK k;
   asm volatile("mov.u32 %0, 0x000F000F;\n mov.u32 %1, 0x00F000F0;\n mov.u32 %2, 0x64006400;\n mov.u32 %3, 0x54005400;"
                : "=r"(k.m0), "=r"(k.m1), "=r"(k.e), "=r"(k.o));
   return k;
 }
-__device__ __forceinline__ void nib_regs(uint32_t w, uint32_t (&o)[4], const NibK& c) {
+__device__ __forceinline__ void nib_off_regs(uint32_t w, uint32_t (&o)[4], const NibK& c) {
   const uint32_t w8 = w >> 8;
   o[0] = and_or(w, c.m0, c.e); o[1] = and_or(w, c.m1, c.o);
   o[2] = and_or(w8, c.m0, c.e); o[3] = and_or(w8, c.m1, c.o);
@@ -364,14 +366,16 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
     // ---- one-time set-up, spread over the consumer threads
     const int ct = threadIdx.x;                                 // 0..NCW*32-1
     constexpr int NQE = (NW * 32 * 4 + NCW * 32 - 1) / (NCW * 32);   // Q entries per thread
-    // Q as B fragments, pre-scaled by qscale*log2(e): entry [i][lane'] = 4 regs x, reg x = (q[g'][8w+x], q[g'][8w+x+4]), w = 4i+j'
+    // Q as B fragments, pre-scaled by qscale*log2(e): entry [i][lane'] = 4 regs x, w = 4i+j': reg x = (q[g'][8w+x], q[g'][8w+x+4]) of a
+    // rotary word, (q[g'][8w+2x], q[g'][8w+2x+1]) of a plain one (its scale and zero rows lie so, and only the product is put in nibble order)
     const float qs = A.qscale * LOG2E;
     auto q_entry = [&](int e, const Item& t) -> uint32_t {
-      const int x = e & 3, ln = (e >> 2) & 31, i = e >> 7, gg = ln >> 2, jj = ln & 3, c = 8 * (4 * i + jj) + x;
+      const int x = e & 3, ln = (e >> 2) & 31, i = e >> 7, gg = ln >> 2, jj = ln & 3;
+      const int c = 8 * (4 * i + jj) + (i < NR ? x : 2 * x), d = i < NR ? 4 : 1;
       float lo = 0.f, hi = 0.f;
       if (gg < G) {
         const size_t qb = ((size_t)t.r * A.nh + t.kvh * G + gg) * HD;
-        lo = act_load<DT>(A.q16, qb + c) * qs; hi = act_load<DT>(A.q16, qb + c + 4) * qs;
+        lo = act_load<DT>(A.q16, qb + c) * qs; hi = act_load<DT>(A.q16, qb + c + d) * qs;
       }
       return pack_h2(lo, hi);
     };
@@ -403,7 +407,6 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
     #pragma unroll
     for (int mt = 0; mt < HD / 16; ++mt) { acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f; }
     float m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f}, zacc[2] = {0.f, 0.f};   // heads 2j, 2j+1 (log2 domain); zacc = sum p*vzero
-    float zs[4] = {0.f, 0.f, 0.f, 0.f};                         // [0], [1]: sum over ALL tokens of the rounded p*vscale, formed by an MMA against ones
 
     // per-lane constant offsets: K word i of row g (swizzled chunk), V chunk of rows 2j and 2j+1
     const int swz = HD == 256 ? (g & 7) : ((g >> 1) & 3);
@@ -414,44 +417,34 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
     // chunk 2q + (mat>>1) (q = which of the HD/64 loads), XOR-swizzled as the TMA tile is.
     const int vtok = ((lane >> 3) & 1) * 8 + (lane & 7), vch = lane >> 4;
     const uint32_t vrow = vtok * L::ROWB, vsw = HD == 256 ? (vtok & 7) : ((vtok >> 1) & 3);
-    const uint32_t ONE2 = 0x3C003C00u;
     const uint32_t qfrag = sbase + L::OFF_QFRAG + lane * 16;
     const uint32_t relt = sbase + L::OFF_RELT + lane * 16;
     const NibK nk = nib_consts();
 
     // One 32-token group.  TAIL: the open group (fp16 shadow rows, `nvalid` visible tokens); else an int4 group.
     // `st` = stage base, `sub` = which of the unit's four groups (0 for the open group).
-    auto group = [&](auto tail_c, const uint32_t st, const int sub, const int nvalid) {
+    auto group = [&](auto tail_c, const uint32_t st, const uint32_t bar_free, const int sub, const int nvalid) {
       constexpr bool TAIL = decltype(tail_c)::value;
       const uint32_t s_k = st + L::OFF_K + sub * L::KB, s_v = st + L::OFF_V + sub * L::KB, s_ks = st + L::OFF_KS + sub * L::SCB,
                      s_kz = st + L::OFF_KZ + sub * L::SCB, s_vs = st + L::OFF_VS + sub * 64, s_rope = st + L::OFF_ROPE + sub * L::ROPEB;
       // ---- per-group fold: q' = q*scale (plain channels); Q rotated back by the group's first position (rotary
-      //      channels); bias[h] = sum_c q[h][c]*zero[c] - sum_c off[c]*q'[h][c], both sums as MMA rows, so the operand
-      //      offsets cancel exactly against the fp16-rounded q' the tiles really use.  Every A row carries the same
-      //      vector, so every lane ends up with the bias of its own two heads.
+      //      channels); bias[h] = sum_c q[h][c]*zero[c] as MMA rows that all carry the same vector, so every lane ends up
+      //      with the bias of its own two heads.
       uint32_t qf[NW][4], rs[NRd][4], rz[NRd][4];
-      float bz[4] = {0.f, 0.f, 0.f, 0.f}, bo[4] = {0.f, 0.f, 0.f, 0.f};
+      float bias[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
       #pragma unroll
       for (int i = 0; i < NW; ++i) {
         const uint4 q4 = lds128(qfrag + i * 512);
         const uint32_t qv[4] = {q4.x, q4.y, q4.z, q4.w};
-        if (TAIL) {
-          #pragma unroll
-          for (int x = 0; x < 4; ++x) qf[i][x] = qv[x];
-        } else {
-          uint32_t sc[4], zz[4];
-          pair_regs(lds128(s_ks + 16 * (4 * i + j)), sc);
-          pair_regs(lds128(s_kz + 16 * (4 * i + j)), zz);
-          if (i < NR) {
-            #pragma unroll
-            for (int x = 0; x < 4; ++x) { qf[i][x] = qv[x]; rs[i][x] = sc[x]; rz[i][x] = zz[x]; }
-          } else {
-            #pragma unroll
-            for (int x = 0; x < 4; ++x) qf[i][x] = hmul2(qv[x], sc[x]);
-            mma16816(bz, zz[0], 0u, zz[1], 0u, qv[0], qv[1]);
-            mma16816(bz, zz[2], 0u, zz[3], 0u, qv[2], qv[3]);
-            mma16816(bo, OFF_E, 0u, OFF_O, 0u, qf[i][0], qf[i][1]);
-            mma16816(bo, OFF_E, 0u, OFF_O, 0u, qf[i][2], qf[i][3]);
+        #pragma unroll
+        for (int x = 0; x < 4; ++x) qf[i][x] = qv[x];
+        if (!TAIL) {
+          const uint4 sc = lds128(s_ks + 16 * (4 * i + j)), zz = lds128(s_kz + 16 * (4 * i + j));
+          if (i < NR) { pair_regs(sc, rs[i]); pair_regs(zz, rz[i]); }
+          else {
+            pair_regs(make_uint4(hmul2(qv[0], sc.x), hmul2(qv[1], sc.y), hmul2(qv[2], sc.z), hmul2(qv[3], sc.w)), qf[i]);
+            mma16816(bias[0], zz.x, zz.x, zz.y, zz.y, qv[0], qv[1]);
+            mma16816(bias[1], zz.z, zz.z, zz.w, zz.w, qv[2], qv[3]);
           }
         }
       }
@@ -472,43 +465,30 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
           }
         }
       }
-      const float bias0 = bz[0] - bo[0], bias1 = bz[1] - bo[1];
-
-      uint32_t ka[NW];                                           // address of this lane's word i in row g of the current tile
+      // Both 16-token tiles of the group go through each step together: twice the independent work between two dependent steps.
+      constexpr uint32_t ROW8 = TAIL ? 8 * HD * 2 : 8 * L::ROWB;       // eight K rows further down
+      uint32_t ka[NW];                                           // this lane's word i in row g of the group
       #pragma unroll
       for (int i = 0; i < NW; ++i) ka[i] = TAIL ? s_k + g * (HD * 2) + 16 * (4 * i + j) : s_k + koff[i];
-      uint32_t va = s_v + vrow, vsa = s_vs + 2 * g, rta = relt;
-      constexpr uint32_t KROW8 = TAIL ? 8 * HD * 2 : 8 * L::ROWB;      // eight rows further down
-
-      #pragma unroll 1
-      for (int tile = 0; tile < 2; ++tile) {
-        if (TAIL && tile * 16 >= nvalid) break;
-        // The tile's packed words and V rows are requested up front, so their shared-memory latency overlaps the arithmetic
-        // that follows (the loads are ordered asm statements: the compiler will not hoist them by itself).
-        uint32_t kw[2][NW];
-        if (!TAIL) {
-          #pragma unroll
-          for (int h = 0; h < 2; ++h)
-            #pragma unroll
-            for (int i = 0; i < NW; ++i) kw[h][i] = lds32(ka[i] + h * KROW8);
-        }
-        uint32_t vx[HD / 64][4];                                 // [load q][tokens 0-7 | 8-15 of chunk 2q, the same of chunk 2q+1]
+      // ---- S^T[32 tok x 8 heads] = K . Q^T.  Three sums a tile: nibbles read at 2^-24 (E), at 2^-20 (O), and true values (R)
+      float se[2][4], so[2][4], sr[2][4];
+      #pragma unroll
+      for (int t = 0; t < 2; ++t)
         #pragma unroll
-        for (int q = 0; q < HD / 64; ++q) ldmatrix_x4_t(va + 16 * ((2 * q + vch) ^ vsw), vx[q]);
-        auto load_k = [&](int h, int i, uint32_t (&o)[4]) {     // A regs of word w = 4i+j, row g + 8h of the tile
-          if (TAIL) pair_regs(lds128(ka[i] + h * KROW8), o); else nib_regs(kw[h][i], o, nk);
-        };
-        // ---- S^T[16 tok x 8 heads] = K . Q^T, two independent accumulation chains
-        float sa[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        uint32_t kr[2][NRd][4];                                  // rotary words: true value, rotated by dt
-        if (RD > 0) {
+        for (int x = 0; x < 4; ++x) { se[t][x] = so[t][x] = 0.f; sr[t][x] = bias[0][x] + bias[1][x]; }
+      if (RD > 0) {                                              // rotary words: true value, rotated by dt
+        #pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          uint32_t kr[2][NRd][4];
           #pragma unroll
           for (int h = 0; h < 2; ++h)
             #pragma unroll
             for (int i = 0; i < NP; ++i) {
               uint32_t a4[4], b4[4];
-              load_k(h, i, a4); load_k(h, i + NP, b4);
-              const uint4 t0 = lds128(rta + ((h * NP + i) * 2) * 512), t1 = lds128(rta + ((h * NP + i) * 2 + 1) * 512);
+              if (TAIL) { pair_regs(lds128(ka[i] + (2 * t + h) * ROW8), a4); pair_regs(lds128(ka[i + NP] + (2 * t + h) * ROW8), b4); }
+              else { nib_off_regs(lds32(ka[i] + (2 * t + h) * ROW8), a4, nk); nib_off_regs(lds32(ka[i + NP] + (2 * t + h) * ROW8), b4, nk); }
+              const uint32_t ra = relt + (((2 * t + h) * NP + i) * 2) * 512;
+              const uint4 t0 = lds128(ra), t1 = lds128(ra + 512);
               const uint32_t cd[4] = {t0.x, t0.z, t1.x, t1.z}, sd[4] = {t0.y, t0.w, t1.y, t1.w};
               #pragma unroll
               for (int x = 0; x < 4; ++x) {
@@ -521,64 +501,84 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
                 kr[h][i + NP][x] = hfma2(a, sd[x], hmul2(b, cd[x]));          // a*sd + b*cd
               }
             }
+          #pragma unroll
+          for (int i = 0; i < NR; ++i) {
+            mma16816(sr[t], kr[0][i][0], kr[1][i][0], kr[0][i][1], kr[1][i][1], qf[i][0], qf[i][1]);
+            mma16816(sr[t], kr[0][i][2], kr[1][i][2], kr[0][i][3], kr[1][i][3], qf[i][2], qf[i][3]);
+          }
         }
+      }
+      #pragma unroll
+      for (int i = NR; i < NW; ++i)
         #pragma unroll
-        for (int i = 0; i < NW; ++i) {
-          uint32_t k0[4], k1[4];
-          if (i < NR) {
-            #pragma unroll
-            for (int x = 0; x < 4; ++x) { k0[x] = kr[0][i][x]; k1[x] = kr[1][i][x]; }
-          } else { load_k(0, i, k0); load_k(1, i, k1); }
-          mma16816(sa[0], k0[0], k1[0], k0[1], k1[1], qf[i][0], qf[i][1]);
-          mma16816(sa[1], k0[2], k1[2], k0[3], k1[3], qf[i][2], qf[i][3]);
+        for (int t = 0; t < 2; ++t) {
+          if (TAIL) {
+            const uint4 k0 = lds128(ka[i] + 2 * t * ROW8), k1 = lds128(ka[i] + (2 * t + 1) * ROW8);
+            mma16816(sr[t], k0.x, k1.x, k0.y, k1.y, qf[i][0], qf[i][1]);
+            mma16816(sr[t], k0.z, k1.z, k0.w, k1.w, qf[i][2], qf[i][3]);
+          } else {
+            const uint32_t k0 = lds32(ka[i] + 2 * t * ROW8), k1 = lds32(ka[i] + (2 * t + 1) * ROW8), k08 = k0 >> 8, k18 = k1 >> 8;
+            mma16816(se[t], k0 & NIB_E, k1 & NIB_E, k08 & NIB_E, k18 & NIB_E, qf[i][0], qf[i][2]);
+            mma16816(so[t], k0 & NIB_O, k1 & NIB_O, k08 & NIB_O, k18 & NIB_O, qf[i][1], qf[i][3]);
+          }
         }
-        // ---- softmax over the tile (log2 domain); rows rg, rg+8; heads 2j, 2j+1
-        const int rg = tile * 16 + g;
-        const bool v0 = !TAIL || rg < nvalid, v1 = !TAIL || rg + 8 < nvalid;
-        const float s00 = v0 ? sa[0][0] + sa[1][0] + bias0 : -INFINITY, s01 = v0 ? sa[0][1] + sa[1][1] + bias1 : -INFINITY;
-        const float s10 = v1 ? sa[0][2] + sa[1][2] + bias0 : -INFINITY, s11 = v1 ? sa[0][3] + sa[1][3] + bias1 : -INFINITY;
-        float t0 = fmaxf(s00, s10), t1 = fmaxf(s01, s11);
-        if (__any_sync(0xffffffffu, t0 > m[0] + 8.f || t1 > m[1] + 8.f)) {   // lazy rescale: the running max may lag by 2^8; no shuffle unless it must move
-          #pragma unroll
-          for (int o = 4; o <= 16; o <<= 1) { t0 = fmaxf(t0, __shfl_xor_sync(0xffffffffu, t0, o)); t1 = fmaxf(t1, __shfl_xor_sync(0xffffffffu, t1, o)); }
-          const float n0 = fmaxf(m[0], t0), n1 = fmaxf(m[1], t1), a0 = ex2(m[0] - n0), a1 = ex2(m[1] - n1);
-          m[0] = n0; m[1] = n1; l[0] *= a0; l[1] *= a1; zacc[0] *= a0; zacc[1] *= a1; zs[0] *= a0; zs[1] *= a1; zs[2] *= a0; zs[3] *= a1;
-          #pragma unroll
-          for (int mt = 0; mt < HD / 16; ++mt) { acc[mt][0] *= a0; acc[mt][1] *= a1; acc[mt][2] *= a0; acc[mt][3] *= a1; }
+      // V rows of both tiles with their scales and zeros, requested ahead of the softmax
+      uint32_t vx[2][HD / 64][4];                                // [tile][load q][tokens 0-7 | 8-15 of chunk 2q, the same of chunk 2q+1]
+      #pragma unroll
+      for (int t = 0; t < 2; ++t)
+        #pragma unroll
+        for (int q = 0; q < HD / 64; ++q) ldmatrix_x4_t(s_v + vrow + t * 16 * L::ROWB + 16 * ((2 * q + vch) ^ vsw), vx[t][q]);
+      float vs[4], vz[4];                                        // token rows g, g+8, g+16, g+24
+      #pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const bool v = !TAIL || 8 * y + g < nvalid;
+        vs[y] = v ? lds_h(s_vs + 2 * g + 16 * y) : 0.f; vz[y] = v ? lds_h(s_vs + L::UG * 64 + 2 * g + 16 * y) : 0.f;
+      }
+      // All of the group has been read: its part of the stage goes back here, with the softmax and P.V still ahead.
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_free);                      // one of the four arrivals that free the stage
+      // ---- softmax over the group (log2 domain); heads 2j, 2j+1
+      float s[4][2];
+      #pragma unroll
+      for (int y = 0; y < 4; ++y)
+        #pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int t = y >> 1, c = 2 * (y & 1) + x;
+          s[y][x] = NR < NW && !TAIL ? fmaf(se[t][c], NIB_E_INV, fmaf(so[t][c], NIB_O_INV, sr[t][c])) : sr[t][c];
+          if (TAIL && 8 * y + g >= nvalid) s[y][x] = -INFINITY;
         }
-        const float p00 = v0 ? ex2(s00 - m[0]) : 0.f, p01 = v0 ? ex2(s01 - m[1]) : 0.f;
-        const float p10 = v1 ? ex2(s10 - m[0]) : 0.f, p11 = v1 ? ex2(s11 - m[1]) : 0.f;
-        l[0] += p00 + p10; l[1] += p01 + p11;
-        // V per-token scale folded into P (fp16), zero point into a per-head scalar: v = vs*(off+n) + (vz - off*vs), off = 0 for
-        // even channels (1024 subtracted exactly before the MMA) and 64 for odd ones.  The -off*vs*p part uses the sum of the
-        // ROUNDED p*vs the MMA consumes (an MMA row of ones), so the offset cancels exactly; it is subtracted once, after the loop.
-        const float vs0 = v0 ? lds_h(vsa) : 0.f, vz0 = v0 ? lds_h(vsa + L::UG * 64) : 0.f;
-        const float vs1 = v1 ? lds_h(vsa + 16) : 0.f, vz1 = v1 ? lds_h(vsa + L::UG * 64 + 16) : 0.f;
-        const uint32_t pp0 = pack_h2(p00 * vs0, p01 * vs0), pp1 = pack_h2(p10 * vs1, p11 * vs1);
-        zacc[0] += p00 * vz0 + p10 * vz1;
-        zacc[1] += p01 * vz0 + p11 * vz1;
-        const uint32_t pb0 = movmatrix_t(pp0);                   // B regs: (tokens 2j,2j+1 | head g)
-        const uint32_t pb1 = movmatrix_t(pp1);                   //         (tokens 2j+8,2j+9 | head g)
-        mma16816(zs, ONE2, ONE2, ONE2, ONE2, pb0, pb1);          // every row: sum over the tile's tokens of the rounded p*vscale
-        // ---- O^T += V^T P^T.  A transposed 8x8 load hands lane (g, j) the 16-bit element g of token rows 2j and 2j+1 of a
-        //      16-byte chunk: four channels (4g .. 4g+3 of the chunk's 32) of two consecutive tokens, which is the pairing along
-        //      the contraction that an A register wants.  Nibbles are read in place: channel 4g+0 / 4g+2 (after >> 8) as 1024 + n,
-        //      made n by an exact subtraction; 4g+1 / 4g+3 as 64 + n.  MMA row g = the even channel, row g+8 = the odd one.
+      float t0 = fmaxf(fmaxf(s[0][0], s[1][0]), fmaxf(s[2][0], s[3][0])), t1 = fmaxf(fmaxf(s[0][1], s[1][1]), fmaxf(s[2][1], s[3][1]));
+      if (__any_sync(0xffffffffu, t0 > m[0] + 8.f || t1 > m[1] + 8.f)) {   // lazy rescale: the running max may lag by 2^8; no shuffle unless it must move
+        #pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) { t0 = fmaxf(t0, __shfl_xor_sync(0xffffffffu, t0, o)); t1 = fmaxf(t1, __shfl_xor_sync(0xffffffffu, t1, o)); }
+        const float n0 = fmaxf(m[0], t0), n1 = fmaxf(m[1], t1), a0 = ex2(m[0] - n0), a1 = ex2(m[1] - n1);
+        m[0] = n0; m[1] = n1; l[0] *= a0; l[1] *= a1; zacc[0] *= a0; zacc[1] *= a1;
+        #pragma unroll
+        for (int mt = 0; mt < HD / 16; ++mt) { acc[mt][0] *= a0; acc[mt][1] *= a1; acc[mt][2] *= a0; acc[mt][3] *= a1; }
+      }
+      // V's per-token scale is folded into P (fp16), its zero point into a per-head scalar: v = vs*n + vz.
+      uint32_t pb[4];                                            // B regs per tile: (tokens 2j,2j+1 | head g), (tokens 2j+8,2j+9 | head g)
+      #pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const bool v = !TAIL || 8 * y + g < nvalid;
+        const float p0 = v ? ex2(s[y][0] - m[0]) : 0.f, p1 = v ? ex2(s[y][1] - m[1]) : 0.f;
+        l[0] += p0; l[1] += p1;
+        zacc[0] = fmaf(p0, vz[y], zacc[0]); zacc[1] = fmaf(p1, vz[y], zacc[1]);
+        pb[y] = movmatrix_t(pack_h2(p0 * vs[y], p1 * vs[y]));
+      }
+      // ---- O^T += V^T P^T.  A transposed 8x8 load hands lane (g, j) the 16-bit element g of token rows 2j and 2j+1 of a
+      //      16-byte chunk: four channels (4g .. 4g+3 of the chunk's 32) of two consecutive tokens, which is the pairing along
+      //      the contraction that an A register wants.  MMA row g = the channel at bits 0..3 (2^-24), row g+8 = the one at bits 4..7 (2^-20).
+      #pragma unroll
+      for (int t = 0; t < 2; ++t)
         #pragma unroll
         for (int q = 0; q < HD / 64; ++q)
           #pragma unroll
           for (int p = 0; p < 2; ++p) {
-            const uint32_t lo = vx[q][2 * p], hi = vx[q][2 * p + 1], lo8 = lo >> 8, hi8 = hi >> 8;
-            mma16816(acc[(2 * q + p) * 2], hadd2(and_or(lo, nk.m0, nk.e), NEG_E), and_or(lo, nk.m1, nk.o),
-                     hadd2(and_or(hi, nk.m0, nk.e), NEG_E), and_or(hi, nk.m1, nk.o), pb0, pb1);
-            mma16816(acc[(2 * q + p) * 2 + 1], hadd2(and_or(lo8, nk.m0, nk.e), NEG_E), and_or(lo8, nk.m1, nk.o),
-                     hadd2(and_or(hi8, nk.m0, nk.e), NEG_E), and_or(hi8, nk.m1, nk.o), pb0, pb1);
+            const uint32_t lo = vx[t][q][2 * p], hi = vx[t][q][2 * p + 1], lo8 = lo >> 8, hi8 = hi >> 8;
+            mma16816(acc[(2 * q + p) * 2], lo & NIB_E, lo & NIB_O, hi & NIB_E, hi & NIB_O, pb[2 * t], pb[2 * t + 1]);
+            mma16816(acc[(2 * q + p) * 2 + 1], lo8 & NIB_E, lo8 & NIB_O, hi8 & NIB_E, hi8 & NIB_O, pb[2 * t], pb[2 * t + 1]);
           }
-        // next tile: sixteen rows further down
-        #pragma unroll
-        for (int i = 0; i < NW; ++i) ka[i] += 2 * KROW8;
-        va += 16 * L::ROWB; vsa += 32; rta += 2 * NP * 2 * 512;
-      }
     };
 
     bool ok = true;
@@ -595,12 +595,10 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
       if (!Q && none) continue;
       const uint32_t st = sbase + L::OFF_STAGES + s * L::STAGE;
       if (!mbar_wait(bar_full + 8 * s, (k / NSTAGE) & 1)) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; break; }
-      if (!none) {
-        if (tail) group(std::true_type{}, st, 0, len - nq * 32);
-        else group(std::false_type{}, st, sub, 32);
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_empty + 8 * s);             // one of the four arrivals that free the stage
+      const uint32_t bar_free = bar_empty + 8 * s;
+      if (none) { if (lane == 0) mbar_arrive(bar_free); }
+      else if (tail) group(std::true_type{}, st, bar_free, 0, len - nq * 32);
+      else group(std::false_type{}, st, bar_free, sub, 32);
     }
 
     // Q: the item after this one, and its queries on their way while this one is merged
@@ -625,7 +623,6 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
       l[0] += __shfl_xor_sync(0xffffffffu, l[0], o); l[1] += __shfl_xor_sync(0xffffffffu, l[1], o);
       zacc[0] += __shfl_xor_sync(0xffffffffu, zacc[0], o); zacc[1] += __shfl_xor_sync(0xffffffffu, zacc[1], o);
     }
-    const float ze[2] = {zacc[0], zacc[1]}, zo[2] = {zacc[0] - 64.f * zs[0], zacc[1] - 64.f * zs[1]};
     // ---- merge the consumer warps and store this split's partial (natural-log m, as the merge kernel expects).  Every warp
     //      scales its own sums by the weight of its maximum and leaves them as they lie in its registers (16 bytes per lane, no bank
     //      conflicts), half of the m-tiles at a time; the sum over the warps runs in warp order.
@@ -664,8 +661,8 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
         #pragma unroll
         for (int t = 0; t < L::NH; ++t) {                        // m-tile: (even | odd channel) x (head 2j | 2j+1)
           const int mt = half * L::NH + t;
-          mbuf[(warp * L::NH + t) * 32 + lane] = make_float4((acc[mt][0] + ze[0]) * sc0, (acc[mt][1] + ze[1]) * sc1,
-                                                             (acc[mt][2] + zo[0]) * sc0, (acc[mt][3] + zo[1]) * sc1);
+          mbuf[(warp * L::NH + t) * 32 + lane] = make_float4(fmaf(acc[mt][0], NIB_E_INV, zacc[0]) * sc0, fmaf(acc[mt][1], NIB_E_INV, zacc[1]) * sc1,
+                                                             fmaf(acc[mt][2], NIB_O_INV, zacc[0]) * sc0, fmaf(acc[mt][3], NIB_O_INV, zacc[1]) * sc1);
         }
         if (Q && more && half == 0) {                            // nobody still reads the Q fragments of this item
           #pragma unroll
@@ -696,7 +693,7 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
     #pragma unroll
     for (int mt = 0; mt < HD / 16; ++mt) { acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f; }
     m[0] = m[1] = -1e30f;
-    l[0] = l[1] = zacc[0] = zacc[1] = zs[0] = zs[1] = zs[2] = zs[3] = 0.f;
+    l[0] = l[1] = zacc[0] = zacc[1] = 0.f;
     }
   }
 }
