@@ -1,0 +1,31 @@
+"""The KV4 merge against double precision on both sides of the line between its two forms (rows x heads above 296 take a warp each): one split,
+the edges of a batch of loads and of a warp's lanes of weights, empty splits, bias and gate, a partial buffer that is aligned for no wide load."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,nh,g,hd", [(12, 24, 6, 256), (13, 24, 6, 256), (64, 24, 6, 256), (300, 16, 8, 128), (80, 4, 2, 64)])
+@pytest.mark.parametrize("S", [1, 7, 8, 9, 18, 32, 33, 41])
+@pytest.mark.parametrize("dtype,shift", [(torch.bfloat16, 0), (torch.float16, 0), (torch.float16, 1)])
+def test_merge_matches_double_precision(M, nh, g, hd, S, dtype, shift):
+    from yasakani_b200 import kv4
+    gen = torch.Generator(device="cuda").manual_seed(M * 100 + S)
+    pm = torch.randn((M, S, nh), generator=gen, device="cuda") * 3
+    if S > 1:
+        pm[:, S // 2] = -1e30                                  # an empty split
+    pl = torch.rand((M, S, nh), generator=gen, device="cuda") * 50 + 1
+    pacc = torch.randn((M, S, nh, hd), generator=gen, device="cuda") * pl[..., None]
+    gate, bv = (torch.randn(s, generator=gen, device="cuda").to(dtype) for s in ((M, nh, hd), (nh // g, hd)))
+    buf = torch.empty(pacc.numel() + shift, device="cuda")
+    buf[shift:] = pacc.view(-1)
+    o16 = torch.empty((M, nh, hd), dtype=dtype, device="cuda")
+    kv4.launch_attn_combine_gqa(pm, pl, buf[shift:].view(pacc.shape), S, M, o16, nh, g, bv=bv, gate=gate)
+    w = torch.exp(pm.double() - pm.double().amax(1, keepdim=True)) * (pm > -1e29)
+    bare = ((w[..., None] * pacc.double()).sum(1) / (w * pl.double()).sum(1)[..., None]).to(torch.float16).double()
+    want = (bare + bv.double().repeat_interleave(g, 0)) * torch.sigmoid(gate.double())
+    # the row before the bias may fall to the other side of an fp16 tie: one ulp, 2^-10 of it (2^-24 among subnormals); the result is rounded to its own
+    # type: half an ulp, 2^-11 or 2^-8 of the value; fp32 arithmetic between the two is far below either
+    bound = bare.abs() * 2.0 ** -10 + want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.01 + 1e-6
+    assert ((o16.double() - want).abs() <= bound).all()

@@ -8,9 +8,7 @@
 // Every arithmetic step that decides a stored bit uses an explicit round-to-nearest intrinsic, so the
 // result does not depend on the compiler's FMA contraction (the reference relies on --fmad=false).
 //
-// Both kernels are HBM-bound byte movers: one warp owns one (row, kv-head) or one (group, kv-head),
-// each lane owns HD/32 contiguous channels, so every load and store of a warp is one contiguous
-// 128..512-byte segment.
+// Byte movers: every load of a warp is one contiguous 128..512-byte segment.
 #include "kv4_common.cuh"
 #include <cmath>
 
@@ -30,112 +28,166 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The 32-token group `gi` of kv-head `head`, by one warp: per channel min / max over the 32 shadow rows, fp16 scale and zero,
-// int4 codes (src/attention_gqa.cu:143-154).  A lane touches only its own HD/32 channels of every row.
-template <int HD>
-__device__ __forceinline__ void group_quant_warp(const yskn_kv_layer& kv, int max_ctx, int gi, int head, int lane) {
-  constexpr int CPL = HD / 32;
-  const uint16_t* rows = kv.kshadow + ((size_t)head * max_ctx + (size_t)gi * 32) * HD + (size_t)lane * CPL;
+__device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b) { uint32_t d; asm("min.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) { uint32_t d; asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+// Channels i, i + 1 of the key rows: fp32 as fp16, 16-bit types as they are; PAIRS: the array is aligned for one load.
+template <int DT, bool PAIRS> __device__ __forceinline__ uint32_t load_pair(const void* p, size_t i) {
+  if (DT == YSKN_KV4_F32) return (uint32_t)f2h(static_cast<const float*>(p)[i]) | ((uint32_t)f2h(static_cast<const float*>(p)[i + 1]) << 16);
+  const uint16_t* h = static_cast<const uint16_t*>(p) + i;
+  return PAIRS ? *reinterpret_cast<const uint32_t*>(h) : (uint32_t)h[0] | ((uint32_t)h[1] << 16);
+}
+// A pair of them as fp16; fp16 too, so that a NaN has one form (x + -0 is x for every other x).
+template <int DT> __device__ __forceinline__ uint32_t act_pair(uint32_t u) {
+  uint32_t d = u;
+  if (DT == YSKN_KV4_BF16) asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(u & 0xffff0000u)), "f"(__uint_as_float(u << 16)));
+  if (DT == YSKN_KV4_F16) asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(u), "r"(0x80008000u));
+  return d;
+}
 
-  float lo[CPL], hi[CPL];
-  #pragma unroll
-  for (int e = 0; e < CPL; ++e) { lo[e] = 1e30f; hi[e] = -1e30f; }
-  for (int t = 0; t < 32; ++t) {
+constexpr int KB = 8;                                // key rows of a batch: their loads are in flight together
+
+// Keys: 64 channels of a 32-token group by one warp, two channels a lane.  Rows [first, end) of the pass go to the fp16 shadow; a group that this pass
+// completes is quantised: per channel min / max over the 32 rows, fp16 scale and zero, int4 codes (src/attention_gqa.cu:143-154).  The codes
+// are formed from the shadow read a second time (a lane's own stores, and lines that were just read): to keep the first walk's values in registers
+// the loops would be unrolled, and code that runs once per launch comes from memory itself.
+template <int HD, int DT, bool PAIRS>
+__device__ __forceinline__ void keys_warp(const yskn_kv_layer& kv, int max_ctx, const void* k_in, int kvh, int pos0, int first, int end, int gi, int head, int c,
+                                          bool closes) {
+  uint16_t* rows = kv.kshadow + ((size_t)head * max_ctx + (size_t)gi * 32) * HD + c;
+  const int f = first - gi * 32, e = end - gi * 32;  // rows of this pass
+  uint32_t lo2 = 0x7C007C00u, hi2 = 0xFC00FC00u;
+  #pragma unroll 1
+  for (int t0 = closes ? 0 : f & ~(KB - 1); t0 < (closes ? 32 : e); t0 += KB) {
+    uint32_t v[KB];
     #pragma unroll
-    for (int e = 0; e < CPL; e += 2) {
-      const uint32_t u = *reinterpret_cast<const uint32_t*>(rows + (size_t)t * HD + e);
-      const float a = h2f((uint16_t)u), b = h2f((uint16_t)(u >> 16));
-      lo[e] = fminf(lo[e], a); hi[e] = fmaxf(hi[e], a); lo[e + 1] = fminf(lo[e + 1], b); hi[e + 1] = fmaxf(hi[e + 1], b);
+    for (int i = 0; i < KB; ++i) {
+      const int t = t0 + i;
+      const bool mine = t >= f && t < e;
+      v[i] = 0u;
+      if (mine) v[i] = load_pair<DT, PAIRS>(k_in, ((size_t)(gi * 32 + t - pos0) * kvh + head) * HD + c);
+      if (!mine && closes) v[i] = *reinterpret_cast<const uint32_t*>(rows + (size_t)t * HD);
+    }
+    #pragma unroll
+    for (int i = 0; i < KB; ++i) {
+      const int t = t0 + i;
+      if (t >= f && t < e) {
+        v[i] = act_pair<DT>(v[i]);
+        *reinterpret_cast<uint32_t*>(rows + (size_t)t * HD) = v[i];
+      }
+      lo2 = min2(lo2, v[i]); hi2 = max2(hi2, v[i]);
     }
   }
-  float inv[CPL];
+  if (!closes) return;
+  float lo[2], inv[2];
+  uint32_t s2 = 0, z2 = 0;
+  #pragma unroll
+  for (int k = 0; k < 2; ++k) {                      // within the bounds that the reference's search starts from
+    lo[k] = fminf(1e30f, h2f((uint16_t)(lo2 >> (16 * k))));
+    const float hi = fmaxf(-1e30f, h2f((uint16_t)(hi2 >> (16 * k)))), d = __fsub_rn(hi, lo[k]);
+    inv[k] = hi > lo[k] ? __fdiv_rn(15.f, d) : 0.f;
+    s2 |= (uint32_t)f2h(__fdiv_rn(d, 15.f)) << (16 * k);
+    z2 |= (uint32_t)f2h(lo[k]) << (16 * k);
+  }
   const size_t gb = (size_t)head * (max_ctx / 32) + gi;
-  uint16_t* ks = kv.kscale + gb * HD + (size_t)lane * CPL;
-  uint16_t* kz = kv.kzero + gb * HD + (size_t)lane * CPL;
-  #pragma unroll
-  for (int e = 0; e < CPL; e += 2) {
-    uint32_t s2 = 0, z2 = 0;
+  *reinterpret_cast<uint32_t*>(kv.kscale + gb * HD + c) = s2;
+  *reinterpret_cast<uint32_t*>(kv.kzero + gb * HD + c) = z2;
+  uint8_t* kq = kv.kq + gb * 32 * (HD / 2) + c / 2;  // a warp's 32 bytes of a row are one sector
+  #pragma unroll 1
+  for (int t0 = 0; t0 < 32; t0 += KB) {
+    uint32_t v[KB];
     #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const float d = __fsub_rn(hi[e + k], lo[e + k]);
-      inv[e + k] = hi[e + k] > lo[e + k] ? __fdiv_rn(15.f, d) : 0.f;
-      s2 |= (uint32_t)f2h(__fdiv_rn(d, 15.f)) << (16 * k);
-      z2 |= (uint32_t)f2h(lo[e + k]) << (16 * k);
-    }
-    *reinterpret_cast<uint32_t*>(ks + e) = s2;
-    *reinterpret_cast<uint32_t*>(kz + e) = z2;
+    for (int i = 0; i < KB; ++i) v[i] = *reinterpret_cast<const uint32_t*>(rows + (size_t)(t0 + i) * HD);
+    #pragma unroll
+    for (int i = 0; i < KB; ++i)
+      kq[(size_t)(t0 + i) * (HD / 2)] = (uint8_t)(quant4(h2f((uint16_t)v[i]), lo[0], inv[0]) | (quant4(h2f((uint16_t)(v[i] >> 16)), lo[1], inv[1]) << 4));
   }
-  uint8_t* kq = kv.kq + gb * 32 * (HD / 2) + (size_t)lane * (CPL / 2);
-  for (int t = 0; t < 32; ++t) {
+}
+
+// Values: rows first, first + step, .. below end by one warp, each to int4 with its fp16 scale and zero; the next row is on its way meanwhile.
+template <int HD, int DT>
+__device__ __forceinline__ void values_warp(const yskn_kv_layer& kv, int max_ctx, const void* v_in, int kvh, int pos0, int first, int end, int step, int head, int lane,
+                                            bool wide) {
+  constexpr int CPL = HD / 32;                       // channels per lane (2, 4 or 8)
+  struct Row { uint32_t u[DT == YSKN_KV4_F32 ? CPL : CPL / 2]; };
+  auto load = [&](int pos, Row& r) {
+    const size_t i = ((size_t)(pos - pos0) * kvh + head) * HD + (size_t)lane * CPL;
+    if constexpr (DT == YSKN_KV4_F32) {
+      #pragma unroll
+      for (int e = 0; e < CPL; ++e) r.u[e] = __float_as_uint(static_cast<const float*>(v_in)[i + e]);
+    } else {
+      const uint16_t* p = static_cast<const uint16_t*>(v_in) + i;
+      if (!wide) {
+        #pragma unroll
+        for (int e = 0; e < CPL; e += 2) r.u[e / 2] = (uint32_t)p[e] | ((uint32_t)p[e + 1] << 16);
+      } else if constexpr (CPL == 8) { const uint4 u = *reinterpret_cast<const uint4*>(p); r.u[0] = u.x; r.u[1] = u.y; r.u[2] = u.z; r.u[3] = u.w; }
+      else if constexpr (CPL == 4) { const uint2 u = *reinterpret_cast<const uint2*>(p); r.u[0] = u.x; r.u[1] = u.y; }
+      else r.u[0] = *reinterpret_cast<const uint32_t*>(p);
+    }
+  };
+  Row next;
+  if (first < end) load(first, next);
+  #pragma unroll 1
+  for (int pos = first; pos < end; pos += step) {
+    const Row row = next;
+    if (pos + step < end) load(pos + step, next);
+    float y[CPL];
+    #pragma unroll
+    for (int e = 0; e < CPL; ++e) {
+      if (DT == YSKN_KV4_F32) y[e] = round_f16(__uint_as_float(row.u[e]));
+      else {
+        const uint16_t h = (uint16_t)(row.u[e / 2] >> (16 * (e & 1)));
+        y[e] = round_f16(DT == YSKN_KV4_BF16 ? bf2f(h) : h2f(h));
+      }
+    }
+    float lo = y[0], hi = y[0];
+    #pragma unroll
+    for (int e = 1; e < CPL; ++e) { lo = fminf(lo, y[e]); hi = fmaxf(hi, y[e]); }
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) { lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o)); hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o)); }
+    const float sc = __fdiv_rn(__fsub_rn(hi, lo), 15.f);
+    const float inv = hi > lo ? __fdiv_rn(15.f, __fsub_rn(hi, lo)) : 0.f;
+    const size_t slot = (size_t)head * max_ctx + pos;
+    uint8_t* vq = kv.vq + slot * (HD / 2) + (size_t)lane * (CPL / 2);
     uint32_t packed = 0;
     #pragma unroll
-    for (int e = 0; e < CPL; e += 2) {
-      const uint32_t u = *reinterpret_cast<const uint32_t*>(rows + (size_t)t * HD + e);
-      packed |= (uint32_t)quant4(h2f((uint16_t)u), lo[e], inv[e]) << (4 * e);
-      packed |= (uint32_t)quant4(h2f((uint16_t)(u >> 16)), lo[e + 1], inv[e + 1]) << (4 * e + 4);
-    }
-    uint8_t* dst = kq + (size_t)t * (HD / 2);
-    if (CPL == 8) *reinterpret_cast<uint32_t*>(dst) = packed;
-    else if (CPL == 4) *reinterpret_cast<uint16_t*>(dst) = (uint16_t)packed;
-    else *dst = (uint8_t)packed;
+    for (int e = 0; e < CPL; ++e) packed |= (uint32_t)quant4(y[e], lo, inv) << (4 * e);
+    if (CPL == 8) *reinterpret_cast<uint32_t*>(vq) = packed;
+    else if (CPL == 4) *reinterpret_cast<uint16_t*>(vq) = (uint16_t)packed;
+    else *vq = (uint8_t)packed;
+    if (lane == 0) { kv.vscale[slot] = f2h(sc); kv.vzero[slot] = f2h(lo); }
   }
 }
 
-// One warp per (row, kv-head): K row -> fp16 shadow; V row -> int4 + fp16 scale/zero.  FUSE (one-row passes): a row that
-// completes its 32-token group quantises the group in the same launch, as the reference's epilogue does at M = 1
-// (src/post_kernels.cu:55-63, switched on by src/engine.cpp:186-187): the 31 older rows were stored by earlier passes and
-// the newest one by this very lane, so no other launch and no barrier is needed.
-template <int HD, int DT, bool FUSE>
-__global__ void __launch_bounds__(128) kv4_append_rows_kernel(yskn_kv_append_args A) {
-  constexpr int CPL = HD / 32;                       // channels per lane (2, 4 or 8)
-  const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+// One launch for any number of rows: K rows -> fp16 shadow and, where the pass appends a group's 32nd token, the group's int4 keys
+// (src/attention_gqa.cu:145-146; in the append launch, as the reference's epilogue does at M = 1: src/post_kernels.cu:55-63); V rows -> int4 + fp16
+// scale/zero.  Warps know their work by number: first the keys, (group that the pass touches, kv-head, 64 channels), then the values, (group,
+// kv-head, one of `vw` shares of its rows).  Nothing passes between warps.
+// Bound by HBM for a prompt (4 KB in, 2.6 KB out per token of four 256-channel heads), by trips to memory for a few rows, and by what room it
+// leaves the attention kernel behind it: see append_hd.
+template <int HD, int DT, bool PAIRS>
+__global__ void __launch_bounds__(256, 4) kv4_append_kernel(yskn_kv_append_args A, int groups, int vw, int wide) {
+  const int lane = threadIdx.x & 31, nk = groups * A.kvh * (HD / 64);
+  int w = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
   pdl_enter();
-  if (w >= A.M * A.kvh) return;
-  const int r = w / A.kvh, head = w % A.kvh, pos = *A.d_pos + r;
-  if (pos < 0 || pos >= A.max_ctx) return;
-  const size_t in0 = ((size_t)r * A.kvh + head) * HD + (size_t)lane * CPL;
-
-  uint16_t kh[CPL]; float y[CPL];
-  #pragma unroll
-  for (int e = 0; e < CPL; ++e) {
-    kh[e] = f2h(act_load<DT>(A.k_in, in0 + e));
-    y[e] = round_f16(act_load<DT>(A.v_in, in0 + e));
-  }
-  uint16_t* ksh = A.kv.kshadow + ((size_t)head * A.max_ctx + pos) * HD + (size_t)lane * CPL;
-  #pragma unroll
-  for (int e = 0; e < CPL; e += 2) *reinterpret_cast<uint32_t*>(ksh + e) = (uint32_t)kh[e] | ((uint32_t)kh[e + 1] << 16);
-
-  float lo = y[0], hi = y[0];
-  #pragma unroll
-  for (int e = 1; e < CPL; ++e) { lo = fminf(lo, y[e]); hi = fmaxf(hi, y[e]); }
-  #pragma unroll
-  for (int o = 16; o; o >>= 1) { lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o)); hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o)); }
-  const float sc = __fdiv_rn(__fsub_rn(hi, lo), 15.f);
-  const float inv = hi > lo ? __fdiv_rn(15.f, __fsub_rn(hi, lo)) : 0.f;
-  const size_t slot = (size_t)head * A.max_ctx + pos;
-  uint8_t* vq = A.kv.vq + slot * (HD / 2) + (size_t)lane * (CPL / 2);
-  uint32_t packed = 0;
-  #pragma unroll
-  for (int e = 0; e < CPL; ++e) packed |= (uint32_t)quant4(y[e], lo, inv) << (4 * e);
-  if (CPL == 8) *reinterpret_cast<uint32_t*>(vq) = packed;
-  else if (CPL == 4) *reinterpret_cast<uint16_t*>(vq) = (uint16_t)packed;
-  else *vq = (uint8_t)packed;
-  if (lane == 0) { A.kv.vscale[slot] = f2h(sc); A.kv.vzero[slot] = f2h(lo); }
-  if (FUSE && (pos & 31) == 31) group_quant_warp<HD>(A.kv, A.max_ctx, pos >> 5, head, lane);
+  const int pos0 = *A.d_pos, last = pos0 + A.M - 1;
+  const bool keys = w < nk;
+  if (!keys) w -= nk;
+  const int parts = keys ? HD / 64 : vw, part = w % parts, gh = w / parts, gi = (pos0 >> 5) + gh / A.kvh, head = gh % A.kvh, gend = gi * 32 + 31;
+  if (gh >= groups * A.kvh || gi < 0 || gi * 32 > last || gi * 32 >= A.max_ctx) return;
+  const int first = max(pos0, gi * 32), end = min(last, gend) + 1;               // rows of this pass in the group
+  if (keys) keys_warp<HD, DT, PAIRS>(A.kv, A.max_ctx, A.k_in, A.kvh, pos0, first, end, gi, head, part * 64 + 2 * lane, gend >= pos0 && gend <= last);
+  else values_warp<HD, DT>(A.kv, A.max_ctx, A.v_in, A.kvh, pos0, first + part, end, vw, head, lane, wide != 0);
 }
 
-// One warp per (candidate group, kv-head).  A group is quantised only in the pass that appends its
-// 32nd token (src/attention_gqa.cu:145-146); until then its rows exist only in the fp16 shadow.
+// The group step alone, from shadow rows that are there: one warp per (candidate group, kv-head, 64 channels).
 template <int HD>
 __global__ void __launch_bounds__(128) kv4_group_quant_kernel(yskn_kv_quant_args A, int kvh) {
-  const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int ncand = (A.M + 31) / 32 + 1;
+  const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5), part = w % (HD / 64), gh = w / (HD / 64);
   pdl_enter();
-  if (w >= ncand * kvh) return;
   const int pos0 = *A.d_pos, last = pos0 + A.M - 1;
-  const int gi = pos0 / 32 + w / kvh, head = w % kvh, gend = gi * 32 + 31;
-  if (gend < pos0 || gend > last || gend >= A.max_ctx) return;
-  group_quant_warp<HD>(A.kv, A.max_ctx, gi, head, lane);
+  const int gi = pos0 / 32 + gh / kvh, head = gh % kvh, gend = gi * 32 + 31;
+  if (gh >= ((A.M + 31) / 32 + 1) * kvh || gi < 0 || gend < pos0 || gend > last || gend >= A.max_ctx) return;
+  keys_warp<HD, YSKN_KV4_F16, true>(A.kv, A.max_ctx, nullptr, kvh, pos0, gi * 32, gi * 32, gi, head, part * 64 + 2 * lane, true);
 }
 
 // out[t][i] = (cos, sin)(float(t) * freq_i), freq_i = theta^(-2i/rd).  The fp32 product that defines the
@@ -152,13 +204,23 @@ __global__ void kv4_rope_table_kernel(float2* out, int max_ctx, float theta, int
   out[idx] = make_float2((float)c, (float)s);
 }
 
-template <int HD, bool FUSE> int append_dt(const yskn_kv_append_args& a, cudaStream_t st) {
-  const dim3 blocks((unsigned)((a.M * a.kvh + 3) / 4));
-  const char* who = "kv4_append_rows_kernel";
+// Blocks.  The attention kernel is launched while this one runs (programmatic launch) and sets itself up beside it where an SM has room: up to eight
+// rows come in blocks of two warps, which fit beside the decode kernel's block on its SM (61,440 of 65,536 registers).  The tcgen05 kernel takes all
+// of an SM's registers and finds no room beside any block; blocks of 32 warps on as few SMs as possible were slower than that (64 rows: 9.0 us
+// against 4.0 in blocks of four warps).
+template <int HD> int append_hd(const yskn_kv_append_args& a, cudaStream_t st) {
+  const int groups = (a.M + 30) / 32 + 1;                        // groups that M rows can touch
+  const int vw = a.M < 8 ? a.M : 8;
+  const int threads = a.M <= 8 ? 64 : a.M <= 64 ? 128 : 256;
+  const long long warps = (long long)groups * a.kvh * (HD / 64 + vw);
+  const dim3 blocks((unsigned)((warps * 32 + threads - 1) / threads));
+  const char* who = "kv4_append_kernel";
+  const int wide = ((uintptr_t)a.v_in & (HD / 16 - 1)) == 0;     // a lane's HD / 32 values in one load
+  const bool pairs = ((uintptr_t)a.k_in & 3) == 0;               // two keys in one load
   switch (a.in_dtype) {
-    case YSKN_KV4_F16: return launch_pdl(who, kv4_append_rows_kernel<HD, YSKN_KV4_F16, FUSE>, blocks, 128, 0, st, a);
-    case YSKN_KV4_BF16: return launch_pdl(who, kv4_append_rows_kernel<HD, YSKN_KV4_BF16, FUSE>, blocks, 128, 0, st, a);
-    case YSKN_KV4_F32: return launch_pdl(who, kv4_append_rows_kernel<HD, YSKN_KV4_F32, FUSE>, blocks, 128, 0, st, a);
+    case YSKN_KV4_F16: return launch_pdl(who, pairs ? kv4_append_kernel<HD, YSKN_KV4_F16, true> : kv4_append_kernel<HD, YSKN_KV4_F16, false>, blocks, threads, 0, st, a, groups, vw, wide);
+    case YSKN_KV4_BF16: return launch_pdl(who, pairs ? kv4_append_kernel<HD, YSKN_KV4_BF16, true> : kv4_append_kernel<HD, YSKN_KV4_BF16, false>, blocks, threads, 0, st, a, groups, vw, wide);
+    case YSKN_KV4_F32: return launch_pdl(who, kv4_append_kernel<HD, YSKN_KV4_F32, false>, blocks, threads, 0, st, a, groups, vw, wide);
     default: KV4_REJECT("yskn_kv4_append: unknown in_dtype %d", a.in_dtype);
   }
 }
@@ -192,7 +254,7 @@ int launch_rope_table(float* d_out, int max_ctx, float theta, int rd, cudaStream
 
 int launch_group_quant(const yskn_kv_quant_args& a, int kvh, int hd, cudaStream_t st) {
   if (a.M <= 0 || kvh <= 0 || !a.d_pos || a.max_ctx % 32) KV4_REJECT("yskn_kv4_group_quant: bad arguments (M %d, kvh %d, max_ctx %d)", a.M, kvh, a.max_ctx);
-  const dim3 blocks((unsigned)((((a.M + 31) / 32 + 1) * kvh + 3) / 4));
+  const dim3 blocks((unsigned)((((a.M + 31) / 32 + 1) * kvh * (hd / 64) + 3) / 4));
   const char* who = "kv4_group_quant_kernel";
   if (hd == 256) return launch_pdl(who, kv4_group_quant_kernel<256>, blocks, 128, 0, st, a, kvh);
   if (hd == 128) return launch_pdl(who, kv4_group_quant_kernel<128>, blocks, 128, 0, st, a, kvh);
@@ -203,20 +265,10 @@ int launch_group_quant(const yskn_kv_quant_args& a, int kvh, int hd, cudaStream_
 int launch_append(const yskn_kv_append_args& a, cudaStream_t st) {
   if (!a.k_in || !a.v_in || !a.d_pos || a.M <= 0 || a.kvh <= 0 || a.max_ctx % 32)
     KV4_REJECT("yskn_kv4_append: bad arguments (M %d, kvh %d, max_ctx %d)", a.M, a.kvh, a.max_ctx);
-  int rc;
-  if (a.M == 1) {                                                // one launch: the row's warp also closes its group
-    if (a.hd == 256) return append_dt<256, true>(a, st);
-    if (a.hd == 128) return append_dt<128, true>(a, st);
-    if (a.hd == 64) return append_dt<64, true>(a, st);
-    KV4_REJECT("yskn_kv4_append: unsupported head_dim %d (64, 128, 256)", a.hd);
-  }
-  if (a.hd == 256) rc = append_dt<256, false>(a, st);
-  else if (a.hd == 128) rc = append_dt<128, false>(a, st);
-  else if (a.hd == 64) rc = append_dt<64, false>(a, st);
-  else KV4_REJECT("yskn_kv4_append: unsupported head_dim %d (64, 128, 256)", a.hd);
-  if (rc) return rc;
-  yskn_kv_quant_args q; q.kv = a.kv; q.d_pos = a.d_pos; q.M = a.M; q.max_ctx = a.max_ctx;
-  return launch_group_quant(q, a.kvh, a.hd, st);
+  if (a.hd == 256) return append_hd<256>(a, st);
+  if (a.hd == 128) return append_hd<128>(a, st);
+  if (a.hd == 64) return append_hd<64>(a, st);
+  KV4_REJECT("yskn_kv4_append: unsupported head_dim %d (64, 128, 256)", a.hd);
 }
 
 }  // namespace kv4

@@ -218,85 +218,76 @@ __global__ void __launch_bounds__(CQ * HD) kv4_combine_kernel(CombineP P) {
   }
 }
 
-// Many rows (verify passes, prompts in few splits): one warp per (row, head), lane l owns channels 4l .. (and HD/2 + 4l .. of 256), no shared memory and
-// no barrier.  The partials are read once from memory, so what counts is how many loads are in flight: eight splits of a row per warp (8 KB).
+// Many rows (verify passes, prompts in few splits): one warp per 128 channels of a (row, head), lane l owns channels 4l .., no shared memory and no
+// barrier.  The partials are read once from memory, so what counts is how many loads are in flight: all of up to 20 splits (a verify pass of one
+// pair of query tiles has 18).
 template <int HD, int DT>
-__global__ void __launch_bounds__(256) kv4_combine_rows_kernel(CombineP P, int rows) {
-  constexpr int NV = HD / 128, B = 8;
-  const int lane = threadIdx.x & 31, w = blockIdx.x * 8 + (threadIdx.x >> 5);
+__global__ void __launch_bounds__(128) kv4_combine_rows_kernel(CombineP P, int items) {
+  constexpr int NV = HD / 128, B = 20;
+  const int lane = threadIdx.x & 31, item = blockIdx.x * 4 + (threadIdx.x >> 5);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (w >= rows) return;
-  const int r = w / P.nh, head = w % P.nh;
-  const size_t slot0 = (size_t)r * P.S * P.nh + head;
-  const float* acc = P.pacc + slot0 * HD + 4 * lane;
-  const size_t step = (size_t)P.nh * HD;
-  float4 v[B][NV];
+  if (item >= items) return;
+  const int w = item / NV, r = w / P.nh, head = w % P.nh, c = 128 * (item % NV) + 4 * lane;
+  const size_t slot0 = (size_t)r * P.S * P.nh + head, step = (size_t)P.nh * HD;
+  const float* acc = P.pacc + slot0 * HD + c;
+  float4 v[B];
   auto load = [&](int s0) {
     #pragma unroll
-    for (int k = 0; k < B; ++k)
-      #pragma unroll
-      for (int h = 0; h < NV; ++h) if (s0 + k < P.S) v[k][h] = __ldcg(reinterpret_cast<const float4*>(acc + (s0 + k) * step + 128 * h));
+    for (int k = 0; k < B; ++k) if (s0 + k < P.S) v[k] = __ldcg(reinterpret_cast<const float4*>(acc + (s0 + k) * step));
   };
+  float m0 = -1e30f, l0 = 0.f;                           // of split `lane`
+  if (lane < P.S) { m0 = __ldcg(P.pm + slot0 + (size_t)lane * P.nh); l0 = __ldcg(P.pl + slot0 + (size_t)lane * P.nh); }
   load(0);
-  float mx = -1e30f;
-  for (int s = lane; s < P.S; s += 32) mx = fmaxf(mx, __ldcg(P.pm + slot0 + (size_t)s * P.nh));
+  float mx = m0;
+  for (int s = lane + 32; s < P.S; s += 32) mx = fmaxf(mx, __ldcg(P.pm + slot0 + (size_t)s * P.nh));
   #pragma unroll
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  float4 sum[NV];
-  #pragma unroll
-  for (int h = 0; h < NV; ++h) sum[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-  float l = 0.f;
+  float wgt = m0 > -1e29f ? expf(m0 - mx) : 0.f, l = wgt * l0;
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
   #pragma unroll 1
-  for (int c0 = 0; c0 < P.S; c0 += 32) {                 // weights of 32 splits, one per lane
-    float wgt = 0.f;
-    if (c0 + lane < P.S) {
-      const float m = __ldcg(P.pm + slot0 + (size_t)(c0 + lane) * P.nh);
-      if (m > -1e29f) wgt = expf(m - mx);
-      l += wgt * __ldcg(P.pl + slot0 + (size_t)(c0 + lane) * P.nh);
-    }
-    #pragma unroll 1
-    for (int s0 = c0; s0 < min(c0 + 32, P.S); s0 += B) {
-      if (s0 > 0) load(s0);
-      #pragma unroll
-      for (int k = 0; k < B; ++k) {
-        const float f = __shfl_sync(0xffffffffu, wgt, (s0 + k) & 31);
-        if (s0 + k < P.S) {
-          #pragma unroll
-          for (int h = 0; h < NV; ++h) {
-            sum[h].x = fmaf(f, v[k][h].x, sum[h].x); sum[h].y = fmaf(f, v[k][h].y, sum[h].y);
-            sum[h].z = fmaf(f, v[k][h].z, sum[h].z); sum[h].w = fmaf(f, v[k][h].w, sum[h].w);
-          }
+  for (int s0 = 0; ; ) {                                 // batches of B splits; the weights of 32 splits are spread over the lanes
+    #pragma unroll
+    for (int k = 0; k < B; ++k) {
+      const int s = s0 + k;
+      if (s > 0 && (s & 31) == 0) {                      // the next 32 weights
+        wgt = 0.f;
+        if (s + lane < P.S) {
+          const float m = __ldcg(P.pm + slot0 + (size_t)(s + lane) * P.nh);
+          if (m > -1e29f) wgt = expf(m - mx);
+          l += wgt * __ldcg(P.pl + slot0 + (size_t)(s + lane) * P.nh);
         }
       }
+      const float f = __shfl_sync(0xffffffffu, wgt, s & 31);
+      if (s < P.S) { sum.x = fmaf(f, v[k].x, sum.x); sum.y = fmaf(f, v[k].y, sum.y); sum.z = fmaf(f, v[k].z, sum.z); sum.w = fmaf(f, v[k].w, sum.w); }
     }
+    s0 += B;
+    if (s0 >= P.S) break;
+    load(s0);
   }
   #pragma unroll
   for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  const float o[4] = {sum.x, sum.y, sum.z, sum.w};
+  const size_t e0 = (size_t)w * HD + c;
+  uint16_t u[4];
   #pragma unroll
-  for (int h = 0; h < NV; ++h) {
-    const float o[4] = {sum[h].x, sum[h].y, sum[h].z, sum[h].w};
-    const size_t e0 = (size_t)w * HD + 128 * h + 4 * lane;
-    uint16_t u[4];
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float y = round_f16(o[k] / l);
-      if (P.bv) y = __fadd_rn(y, act_load<DT>(P.bv, (size_t)(head / P.g) * HD + 128 * h + 4 * lane + k));
-      if (P.gate) { const float gt = act_load<DT>(P.gate, e0 + k); y = __fmul_rn(y, __fdiv_rn(1.f, __fadd_rn(1.f, expf(-gt)))); }
-      u[k] = act_store16<DT>(y);
-    }
-    *reinterpret_cast<uint2*>(P.o16 + e0) = make_uint2((uint32_t)u[0] | ((uint32_t)u[1] << 16), (uint32_t)u[2] | ((uint32_t)u[3] << 16));
+  for (int k = 0; k < 4; ++k) {
+    float y = round_f16(o[k] / l);
+    if (P.bv) y = __fadd_rn(y, act_load<DT>(P.bv, (size_t)(head / P.g) * HD + c + k));
+    if (P.gate) { const float gt = act_load<DT>(P.gate, e0 + k); y = __fmul_rn(y, __fdiv_rn(1.f, __fadd_rn(1.f, expf(-gt)))); }
+    u[k] = act_store16<DT>(y);
   }
+  *reinterpret_cast<uint2*>(P.o16 + e0) = make_uint2((uint32_t)u[0] | ((uint32_t)u[1] << 16), (uint32_t)u[2] | ((uint32_t)u[3] << 16));
 }
 
 template <int HD, int DT, bool TI, bool TO, bool PEER>
 int launch_k(const CombineP& P, size_t smem, cudaStream_t st) {
   const long long blocks = (long long)P.nh * P.M;
-  // Above 296 rows x heads the warp-per-row form (measured with 64 rows in 9 splits, behind the attention kernel:
-  // 13.2 -> 5.2 us; the pass 123 -> 112 us with the append kernel in one launch)
+  // Above 296 rows x heads, where the blocks below no longer fit the GPU at once, the form for many rows (64 rows in 9 splits, behind the attention
+  // kernel: 13.2 -> 5.2 us)
   if constexpr (!TI && !TO && !PEER && HD >= 128)
-    if (blocks > 296 && blocks < (1ll << 30) && !((uintptr_t)P.pacc & 15) && !((uintptr_t)P.o16 & 7))
-      return launch_pdl("kv4_combine_rows_kernel", kv4_combine_rows_kernel<HD, DT>, dim3((unsigned)((blocks + 7) / 8)), 256, 0, st, P, (int)blocks);
+    if (blocks > 296 && blocks < (1ll << 28) && !((uintptr_t)P.pacc & 15) && !((uintptr_t)P.o16 & 7))
+      return launch_pdl("kv4_combine_rows_kernel", kv4_combine_rows_kernel<HD, DT>, dim3((unsigned)((blocks * (HD / 128) + 3) / 4)), 128, 0, st, P, (int)blocks * (HD / 128));
   const int CQ = (P.S < 8 || (TI && !TO && PEER)) ? 1 : (blocks <= 296 ? 4 : 2);   // 296 = two 1,024-thread blocks on each of 148 SMs; the merge of pushed triples folds nothing
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(P.nh, P.M); cfg.blockDim = dim3(CQ * HD); cfg.dynamicSmemBytes = smem; cfg.stream = st;

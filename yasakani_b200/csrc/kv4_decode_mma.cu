@@ -196,6 +196,9 @@ __device__ __forceinline__ float lds_h(uint32_t a) {
 }
 
 // ---------------------------------------------------------------- kernel
+// Tensor maps of one cache.  The scales and zeros come as tiles too: as plain bulk copies of 2 KB and 256 bytes they slowed the whole stream down
+// (262,144 tokens: XX us).
+struct Maps { CUtensorMap k, v, ks, kz, vs, vz; };
 struct DecodeP {
   yskn_attn_g_args A;
   Shard sh;
@@ -214,8 +217,7 @@ struct DecodeP {
 // 55.6 us with their append and merge, eight rows over 172 tokens 48.8 -> 38 us.
 template <int HD, int RD, int DT, bool Q>
 __global__ void __launch_bounds__(NTHREADS, 1)
-kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV,
-                      const __grid_constant__ CUtensorMap mapR, const DecodeP P) {
+kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__ CUtensorMap mapR, const DecodeP P) {
   using L = Lay<HD, RD, Q>;
   constexpr int NW = L::NW, NR = L::NR, NP = L::NP, NRd = NR > 0 ? NR : 1;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -301,8 +303,7 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
       const size_t row0 = (size_t)kvh * A.max_ctx;              // first row of this kv-head in the [Hkv*max_ctx] arrays
       const int slot = multi ? P.ms.slot[it.r] : 0;
       const yskn_kv_layer kvl = multi ? P.ms.layers[slot] : A.kv;
-      const CUtensorMap* const mk = multi ? static_cast<const CUtensorMap*>(P.ms.maps) + 2 * slot : &mapK;
-      const CUtensorMap* const mv = multi ? static_cast<const CUtensorMap*>(P.ms.maps) + 2 * slot + 1 : &mapV;
+      const Maps* const mp = multi ? static_cast<const Maps*>(P.ms.maps) + slot : &maps;
       for (int u = it.u0; u < it.u0 + it.nu; ++u) {
         const int s = k % NSTAGE;
         // an early unit: one of the first ring fills, int4 only, every token below the base position
@@ -320,20 +321,20 @@ kv4_decode_mma_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_con
         go = __shfl_sync(0xffffffffu, ok, 0) != 0;
         if (!go) break;
         const bool tail = has_tail && u == nu4;
-        const int ngr = tail ? 1 : min(L::UG, nq - u * L::UG);   // groups in this unit
         const int g0 = tail ? nq : u * L::UG;                    // its first group (local index)
         const uint32_t st = sbase + L::OFF_STAGES + s * L::STAGE, bar = bar_full + 8 * s;
-        if (lane == 0) mbar_expect_tx(bar, 2 * L::UG * L::KB + ngr * (2 * L::SCB * (tail ? 0 : 1) + 128) + L::UG * L::ROPEB);   // SHADOW == UG*KB
+        if (lane == 0) mbar_expect_tx(bar, 2 * L::UG * L::KB + 2 * L::UG * ((tail ? 0 : L::SCB) + 64) + L::UG * L::ROPEB);   // SHADOW == UG*KB
         __syncwarp();                                            // the barrier is armed before any copy is issued
-        const size_t tok0 = row0 + (size_t)g0 * 32, gb = ((size_t)kvh * (A.max_ctx / 32) + g0) * HD;
-        switch (lane) {                                          // one copy per lane: seven issue slots in parallel
-          case 0: if (tail) bulk_1d(st + L::OFF_K, kvl.kshadow + tok0 * HD, L::SHADOW, bar);
-                  else tma_2d(st + L::OFF_K, mk, 0, (int)tok0, bar); break;
-          case 1: tma_2d(st + L::OFF_V, mv, 0, (int)tok0, bar); break;   // always the swizzled tile; rows past the unit are unused
-          case 2: if (!tail) bulk_1d(st + L::OFF_KS, kvl.kscale + gb, ngr * L::SCB, bar); break;
-          case 3: if (!tail) bulk_1d(st + L::OFF_KZ, kvl.kzero + gb, ngr * L::SCB, bar); break;
-          case 4: bulk_1d(st + L::OFF_VS, kvl.vscale + tok0, ngr * 64, bar); break;
-          case 5: bulk_1d(st + L::OFF_VZ, kvl.vzero + tok0, ngr * 64, bar); break;
+        // One copy per lane: seven issue slots in parallel.  Whole units always: what lies behind the last group of a unit, or of the array, is unused.
+        const int tok0 = (int)row0 + g0 * 32, grp0 = kvh * (A.max_ctx / 32) + g0;
+        switch (lane) {
+          case 0: if (tail) bulk_1d(st + L::OFF_K, kvl.kshadow + (size_t)tok0 * HD, L::SHADOW, bar);
+                  else tma_2d(st + L::OFF_K, &mp->k, 0, tok0, bar); break;
+          case 1: tma_2d(st + L::OFF_V, &mp->v, 0, tok0, bar); break;
+          case 2: if (!tail) tma_2d(st + L::OFF_KS, &mp->ks, 0, grp0, bar); break;
+          case 3: if (!tail) tma_2d(st + L::OFF_KZ, &mp->kz, 0, grp0, bar); break;
+          case 4: tma_2d(st + L::OFF_VS, &mp->vs, g0 * 32, kvh, bar); break;
+          case 5: tma_2d(st + L::OFF_VZ, &mp->vz, g0 * 32, kvh, bar); break;
           case 6: if (RD > 0) tma_2d(st + L::OFF_ROPE, &mapR, 0, g0 + P.sh.start / 32, bar); break;   // rows 32*(g0..g0+3) of the table
           default: break;
         }
@@ -712,23 +713,40 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Tensor map over a packed array viewed as [rows][rowbytes] bytes, box = 128 rows (one unit), swizzle = row width.
-bool make_map(CUtensorMap* out, const void* base, uint64_t rows, int rowbytes) {
-  struct Key { const void* p; uint64_t rows; int rb; bool operator==(const Key& o) const { return p == o.p && rows == o.rows && rb == o.rb; } };
-  struct Hash { size_t operator()(const Key& k) const { return std::hash<const void*>()(k.p) ^ (k.rows * 1315423911u) ^ (size_t)k.rb; } };
-  static std::mutex mu; static std::unordered_map<Key, CUtensorMap, Hash> cache;
-  std::lock_guard<std::mutex> lk(mu);
-  const Key key{base, rows, rowbytes};
-  auto it = cache.find(key);
-  if (it != cache.end()) { *out = it->second; return true; }
+// 2-D tensor map [rows][cols] of 8- or 16-bit elements, box = box_rows x box_cols.
+bool make_map(CUtensorMap* out, const void* base, int elem, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle sw) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)rowbytes, rows}, strides[1] = {(cuuint64_t)rowbytes};
-  const cuuint32_t box[2] = {(cuuint32_t)rowbytes, 128}, estr[2] = {1, 1};
-  const CUtensorMapSwizzle sw = rowbytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-  if (fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return false;
-  if (cache.size() > 4096) cache.clear();
+  const cuuint64_t dims[2] = {cols, rows}, strides[1] = {cols * elem};
+  const cuuint32_t box[2] = {box_cols, box_rows}, estr[2] = {1, 1};
+  return fn(out, elem == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The maps of one cache: units of 128 tokens of the packed rows (swizzle = row width), four rows of the group arrays, 128 values of the token arrays.
+bool make_maps(Maps* out, const yskn_kv_layer& l, int kvh, int max_ctx, int hd) {
+  struct Key {
+    const void* p[6]; int kvh, max_ctx, hd;
+    bool operator==(const Key& o) const { return memcmp(p, o.p, sizeof(p)) == 0 && kvh == o.kvh && max_ctx == o.max_ctx && hd == o.hd; }
+  };
+  struct Hash {
+    size_t operator()(const Key& k) const {
+      size_t h = (size_t)k.max_ctx * 1315423911u ^ (size_t)(k.kvh * 512 + k.hd);
+      for (const void* p : k.p) h = (h ^ std::hash<const void*>()(p)) * 0x100000001B3ull;
+      return h;
+    }
+  };
+  static std::mutex mu; static std::unordered_map<Key, Maps, Hash> cache;
+  std::lock_guard<std::mutex> lk(mu);
+  const Key key{{l.kq, l.vq, l.kscale, l.kzero, l.vscale, l.vzero}, kvh, max_ctx, hd};
+  auto it = cache.find(key);
+  if (it != cache.end()) { *out = it->second; return true; }
+  const uint64_t rows = (uint64_t)kvh * max_ctx;
+  const CUtensorMapSwizzle sw = hd == 256 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, none = CU_TENSOR_MAP_SWIZZLE_NONE;
+  if (!make_map(&out->k, l.kq, 1, rows, hd / 2, 128, hd / 2, sw) || !make_map(&out->v, l.vq, 1, rows, hd / 2, 128, hd / 2, sw) ||
+      !make_map(&out->ks, l.kscale, 2, rows / 32, hd, 4, hd, none) || !make_map(&out->kz, l.kzero, 2, rows / 32, hd, 4, hd, none) ||
+      !make_map(&out->vs, l.vscale, 2, kvh, max_ctx, 1, 128, none) || !make_map(&out->vz, l.vzero, 2, kvh, max_ctx, 1, 128, none)) return false;
+  if (cache.size() > 1024) cache.clear();
   cache.emplace(key, *out);
   return true;
 }
@@ -754,7 +772,7 @@ bool make_rope_map(CUtensorMap* out, const float* rope, int rd, uint64_t groups)
 }
 
 template <int HD, int RD, int DT, bool Q>
-int launch_q(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, cudaStream_t st) {
+int launch_q(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const Maps& mp, const CUtensorMap& mr, cudaStream_t st) {
   using L = Lay<HD, RD, Q>;
   auto kern = kv4_decode_mma_kernel<HD, RD, DT, Q>;
   static std::atomic<unsigned long long> attr{0};               // once per device, like the reference's launchers once per process
@@ -768,24 +786,24 @@ int launch_q(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_k
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
-  KV4_CUDA(cudaLaunchKernelEx(&cfg, kern, mk, mv, mr, P));
+  KV4_CUDA(cudaLaunchKernelEx(&cfg, kern, mp, mr, P));
   return launch_status("kv4_decode_mma_kernel");
 }
 
 // One CTA fills an SM, so a grid of up to one block per SM starts at once and has nothing to take over; a larger one runs as a queue.
 template <int HD, int RD, int DT>
-int launch_t(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, cudaStream_t st) {
+int launch_t(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const Maps& mp, const CUtensorMap& mr, cudaStream_t st) {
   int dev = 0, sms = 0;
   KV4_CUDA(cudaGetDevice(&dev));
   KV4_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if ((long long)a.splits * a.kvh * a.M > sms) return launch_q<HD, RD, DT, true>(a, g, sh, early, ms, mk, mv, mr, st);
-  return launch_q<HD, RD, DT, false>(a, g, sh, early, ms, mk, mv, mr, st);
+  if ((long long)a.splits * a.kvh * a.M > sms) return launch_q<HD, RD, DT, true>(a, g, sh, early, ms, mp, mr, st);
+  return launch_q<HD, RD, DT, false>(a, g, sh, early, ms, mp, mr, st);
 }
 
 template <int HD, int RD>
-int launch_dt(const yskn_attn_g_args& a, int g, int dt, Shard sh, int early, const yskn_kv4_ms_rows& ms, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr, cudaStream_t st) {
-  if (dt == YSKN_KV4_BF16) return launch_t<HD, RD, YSKN_KV4_BF16>(a, g, sh, early, ms, mk, mv, mr, st);
-  return launch_t<HD, RD, YSKN_KV4_F16>(a, g, sh, early, ms, mk, mv, mr, st);
+int launch_dt(const yskn_attn_g_args& a, int g, int dt, Shard sh, int early, const yskn_kv4_ms_rows& ms, const Maps& mp, const CUtensorMap& mr, cudaStream_t st) {
+  if (dt == YSKN_KV4_BF16) return launch_t<HD, RD, YSKN_KV4_BF16>(a, g, sh, early, ms, mp, mr, st);
+  return launch_t<HD, RD, YSKN_KV4_F16>(a, g, sh, early, ms, mp, mr, st);
 }
 
 }  // namespace
@@ -800,17 +818,16 @@ int ms_prepare(const yskn_kv_layer* h_layers, int n_slots, int kvh, int hd, int 
   if (!h_layers || !d_layers || !d_maps || n_slots <= 0 || n_slots > 64) KV4_REJECT("yskn_kv4_ms_prepare: bad arguments (n_slots %d)", n_slots);
   if (kvh <= 0 || (hd != 128 && hd != 256) || max_ctx <= 0 || max_ctx % 64) KV4_REJECT("yskn_kv4_ms_prepare: bad shape (kvh %d, hd %d, max_ctx %d)", kvh, hd, max_ctx);
   if ((uintptr_t)d_maps & 127) KV4_REJECT("yskn_kv4_ms_prepare: the map table must be 128-byte aligned");
-  std::vector<CUtensorMap> maps(2 * (size_t)n_slots);
-  const uint64_t rows = (uint64_t)kvh * max_ctx;
+  std::vector<Maps> maps((size_t)n_slots);
   for (int s = 0; s < n_slots; ++s) {
     const yskn_kv_layer& l = h_layers[s];
     const uintptr_t al = (uintptr_t)l.kq | (uintptr_t)l.vq | (uintptr_t)l.kscale | (uintptr_t)l.kzero | (uintptr_t)l.kshadow | (uintptr_t)l.vscale | (uintptr_t)l.vzero;
     if (!l.kq || !l.vq || !l.kscale || !l.kzero || !l.kshadow || !l.vscale || !l.vzero || (al & 15))
       KV4_REJECT("yskn_kv4_ms_prepare: cache arrays of slot %d missing or not 16-byte aligned", s);
-    if (!make_map(&maps[2 * s], l.kq, rows, hd / 2) || !make_map(&maps[2 * s + 1], l.vq, rows, hd / 2))
+    if (!make_maps(&maps[s], l, kvh, max_ctx, hd))
       KV4_REJECT("yskn_kv4_ms_prepare: cuTensorMapEncodeTiled failed or is unavailable");
   }
-  KV4_CUDA(cudaMemcpyAsync(d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, st));
+  KV4_CUDA(cudaMemcpyAsync(d_maps, maps.data(), maps.size() * sizeof(Maps), cudaMemcpyHostToDevice, st));
   KV4_CUDA(cudaMemcpyAsync(d_layers, h_layers, (size_t)n_slots * sizeof(yskn_kv_layer), cudaMemcpyHostToDevice, st));
   KV4_CUDA(cudaStreamSynchronize(st));                            // the host vectors go out of scope
   return 0;
@@ -825,19 +842,19 @@ int launch_decode_mma(const yskn_attn_g_args& a, int g, int hd, int rd, int act_
                              : (uintptr_t)a.kv.kq | (uintptr_t)a.kv.vq | (uintptr_t)a.kv.kscale | (uintptr_t)a.kv.kzero | (uintptr_t)a.kv.kshadow |
                                (uintptr_t)a.kv.vscale | (uintptr_t)a.kv.vzero | (uintptr_t)a.rope;
   if (al & 15) KV4_REJECT("yskn_kv4_attention: cache arrays and rope table must be 16-byte aligned");
-  CUtensorMap mk, mv, mr;
-  const uint64_t rows = (uint64_t)a.kvh * a.max_ctx;
-  if (multi) { memset(&mk, 0, sizeof(mk)); memset(&mv, 0, sizeof(mv)); }      // the kernel takes the maps of the row's sequence from ms->maps
-  else if (!make_map(&mk, a.kv.kq, rows, hd / 2) || !make_map(&mv, a.kv.vq, rows, hd / 2))
+  Maps mp;
+  CUtensorMap mr;
+  if (multi) memset(&mp, 0, sizeof(mp));                          // the kernel takes the maps of the row's sequence from ms->maps
+  else if (!make_maps(&mp, a.kv, a.kvh, a.max_ctx, hd))
     KV4_REJECT("yskn_kv4_attention: cuTensorMapEncodeTiled failed or is unavailable");
   const yskn_kv4_ms_rows msv = multi ? *ms : yskn_kv4_ms_rows{nullptr, nullptr, nullptr, nullptr, 0};
   if (multi) early = 0;                                           // rows of one sequence in the same pass are appended by the predecessor
   // The rope table must cover positions [0, shard start + shard length); groups past that read as zero and are never used.
-  if (rd == 0) mr = mk;
+  if (rd == 0) mr = mp.k;
   else if (!make_rope_map(&mr, a.rope, rd, ((uint64_t)sh.start + (uint64_t)sh.len) / 32))
     KV4_REJECT("yskn_kv4_attention: cuTensorMapEncodeTiled failed for the rope table");
-  if (hd == 256) return rd ? launch_dt<256, 64>(a, g, act_dtype, sh, early, msv, mk, mv, mr, st) : launch_dt<256, 0>(a, g, act_dtype, sh, early, msv, mk, mv, mr, st);
-  return rd ? launch_dt<128, 128>(a, g, act_dtype, sh, early, msv, mk, mv, mr, st) : launch_dt<128, 0>(a, g, act_dtype, sh, early, msv, mk, mv, mr, st);
+  if (hd == 256) return rd ? launch_dt<256, 64>(a, g, act_dtype, sh, early, msv, mp, mr, st) : launch_dt<256, 0>(a, g, act_dtype, sh, early, msv, mp, mr, st);
+  return rd ? launch_dt<128, 128>(a, g, act_dtype, sh, early, msv, mp, mr, st) : launch_dt<128, 0>(a, g, act_dtype, sh, early, msv, mp, mr, st);
 }
 
 int decode_status_fetch(int* out) {
