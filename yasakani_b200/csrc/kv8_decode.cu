@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(KV8_WARPS * 32, 1) kv8_decode_kernel(const Kv8
 // 24,000 rows of one split.
 __device__ __forceinline__ float kv8_round(int dt, float v) { return dt == YSKN_KV4_BF16 ? bf2f(f2bf(v)) : h2f(f2h(v)); }
 template <int DT> __device__ __forceinline__ float kv8_gated(float y, float gt) {   // y * sigmoid(gate), each factor and the product rounded (src/q35_kernels.cu:1423-1424)
-  return kv8_round(DT, __fmul_rn(y, kv8_round(DT, __fdiv_rn(1.f, __fadd_rn(1.f, expf(-gt))))));
+  return kv8_round(DT, __fmul_rn(y, kv8_round(DT, __frcp_rn(__fadd_rn(1.f, expf(-gt))))));
 }
 
 // Many splits: one block per (head, row), four runs of splits x 256 channels, every thread's loads issued at once; one warp
@@ -311,8 +311,27 @@ __global__ void __launch_bounds__(256) kv8_combine_rows_kernel(const float* pm, 
       v[4 * k] += w * a.x; v[4 * k + 1] += w * a.y; v[4 * k + 2] += w * a.z; v[4 * k + 3] += w * a.w;
     }
   }
+  // v / L2, correctly rounded: with r = 1 / L2 rounded and q = v * r, fma(v - q * L2, r, q) is the rounded quotient while nothing leaves the normal
+  // range (Markstein, IBM J. Res. Dev. 34, 1990); three operations instead of a division per value.  Other rows divide.
+  const float r = __frcp_rn(L2);
+  float odd = 0.f;                                         // NaN when a value is not finite
   #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __fdiv_rn(v[i], L2);
+  for (int i = 0; i < 32; ++i) odd = fmaf(v[i], 0.f, odd);
+  if (L2 > 1e-18f && L2 < 1e18f && odd == 0.f) {
+    #pragma unroll
+    for (int i = 0; i < 32; ++i) { const float q = __fmul_rn(v[i], r); v[i] = fmaf(fmaf(-q, L2, v[i]), r, q); }
+  } else {
+    #pragma unroll 1
+    for (int k = 0; k < 32; k += 4) {                      // rolled: rows without keys, sums beyond the range
+      float t[4];
+      #pragma unroll
+      for (int i = 0; i < 32; i += 4) if (i == k) { t[0] = v[i]; t[1] = v[i + 1]; t[2] = v[i + 2]; t[3] = v[i + 3]; }
+      #pragma unroll
+      for (int e = 0; e < 4; ++e) t[e] = __fdiv_rn(t[e], L2);
+      #pragma unroll
+      for (int i = 0; i < 32; i += 4) if (i == k) { v[i] = t[0]; v[i + 1] = t[1]; v[i + 2] = t[2]; v[i + 3] = t[3]; }
+    }
+  }
   if (inverse_rotate) { hadamard256(v, ll); apply_signs(v, ll); }
   if (!live) return;
   const size_t e0 = (size_t)row * KV8_HD + 4 * ll;
