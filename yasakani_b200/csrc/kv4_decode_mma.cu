@@ -23,15 +23,21 @@
 // into A-fragment registers:
 //   * a 32-bit word holds 8 nibbles; one AND reads nibbles (x, x+4) in place as two fp16 subnormals, n * 2^-24 at bits 0..3 of a
 //     half, n * 2^-20 at bits 4..7: exactly one A register, because the contraction order over channels is free.  The tensor core
-//     multiplies subnormals exactly and sums in fp32, so the factor is taken out of the sum (one accumulator per factor).  K's
-//     per-channel scale is folded into Q once per group (q' = q*scale); the zero points become a per-head bias, sum q*zero, formed
-//     by two more MMA rows.
+//     forms products with subnormals exactly, so the factor is taken out of the fp32 sum (one accumulator per factor); it aligns them
+//     for the sum by the exponent 2^-14 of a subnormal, though, not by their leading bit, see V.  K's per-channel scale is folded into Q
+//     once per group (q' = q*scale); the zero points become a per-head bias, sum q*zero, formed by two more MMA rows.
 //   * for V the contraction runs over tokens: a transposed 8x8 shared-memory load (ldmatrix.trans) hands a lane the same
 //     four channels of two consecutive tokens in one register, which is the pairing an A register wants.  V's per-token
 //     scale is folded into P and its zero point into a per-head scalar.  No offset may ride along in these sums: the tensor
 //     core's fp32 accumulators truncate, and one that carried 1024 * sum(p) lost about 2e-3 of the output at 262,144 tokens.
-//     Before the subnormals, offsets (1024 + n, 64 + n) were added by the logic op and taken out again by subtractions and by MMA rows
-//     of ones: 262,144 tokens 85.6 -> 82.2 us, eight sequences 124.2 -> 116.9 us (both tiles of a group in step, see below, included).
+//     A warp's sum of O runs over up to 1,000 tokens, so the truncation at the alignment above counts here, and the nibbles are read
+//     at bits 3..6 (n * 2^-21) and 7..10 (n * 2^-17; bit 10 is the exponent's last, under which the format is still linear), for
+//     one shift more per word.  Error of the rows against double precision at 262,144 / 65,536 / 32,768 tokens, mean of six caches,
+//     even channels and odd ones: 1.59e-3 1.58e-3 / 1.15e-3 1.14e-3 / 1.18e-3 1.18e-3.  At bits 0..3 and 4..7: 2.29e-3 1.59e-3 /
+//     1.34e-3 1.15e-3 / 1.29e-3 1.18e-3.  With offsets (1024 + n taken out by a subtraction, 64 + n by MMA rows of ones): 1.54e-3 6.70e-3 /
+//     1.14e-3 1.26e-3 / 1.16e-3 1.19e-3.  For K, whose sums run over a head's channels only, the position changes nothing (0.1 %).
+//     Time with offsets, and now: 262,144 tokens 85.7 -> 81.2 us, eight sequences 124.2 -> 115.8 us (both tiles of a group in
+//     step, see below, included).
 //   * RoPE: Q is rotated back by the group's first position (one table row per group), the remaining angle
 //     (0..31 tokens) is applied to the rotary channels of K with the table's first 32 rows.  cos/sin of
 //     (t0 + dt) are thereby formed by angle addition from the caller's table entries for t0 and dt.  The table's own
@@ -163,10 +169,11 @@ __device__ __forceinline__ uint32_t hneg2(uint32_t a) { uint32_t d; asm("neg.f16
 // A 32-bit word of a packed row holds nibbles 0..7.  One AND pairs nibbles (X, X+4) as the two halves of a register
 // WITHOUT moving them (one shift, w >> 8, serves X = 2, 3), and the halves are fp16 subnormals: a nibble at bits 0..3 reads as n * 2^-24, at
 // bits 4..7 as n * 2^-20.  The tensor core multiplies subnormals exactly, so the factor leaves behind the fp32 sum, and nothing is added to the
-// operands.  Rotary words need the value itself: under exponent 2^10 (0x6400) or 2^6 (0x5400) the halves read as 1024 + n or 64 + n, and the
+// operands.  V's words are first shifted by 3 (w << 3 for X = 0, 1 and w >> 5 for X = 2, 3): n * 2^-21 and n * 2^-17.  Rotary words need the value itself: under exponent 2^10 (0x6400) or 2^6 (0x5400) the halves read as 1024 + n or 64 + n, and the
 // constant leaves by an exact subtraction.
 constexpr uint32_t NIB_E = 0x000F000Fu, NIB_O = 0x00F000F0u;
 constexpr float NIB_E_INV = 16777216.f, NIB_O_INV = 1048576.f;     // 2^24, 2^20
+constexpr float VNIB_E_INV = 2097152.f, VNIB_O_INV = 131072.f;     // 2^21, 2^17
 constexpr uint32_t NEG_E = 0xE400E400u, NEG_O = 0xD400D400u;       // -(1024, 1024), -(64, 64)
 // (a & m) | c as ONE LOP3.  LOP3 takes a single immediate, so with two literal constants the compiler emits AND then OR
 // (measured: 562 LOP3 per group instead of ~280); the masks and offsets are therefore kept in registers that the
@@ -569,16 +576,17 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
       }
       // ---- O^T += V^T P^T.  A transposed 8x8 load hands lane (g, j) the 16-bit element g of token rows 2j and 2j+1 of a
       //      16-byte chunk: four channels (4g .. 4g+3 of the chunk's 32) of two consecutive tokens, which is the pairing along
-      //      the contraction that an A register wants.  MMA row g = the channel at bits 0..3 (2^-24), row g+8 = the one at bits 4..7 (2^-20).
+      //      the contraction that an A register wants.  MMA row g = the channel at bits 3..6 of the shifted word (2^-21), row g+8 = the one at bits 7..10 (2^-17).
       #pragma unroll
       for (int t = 0; t < 2; ++t)
         #pragma unroll
         for (int q = 0; q < HD / 64; ++q)
           #pragma unroll
           for (int p = 0; p < 2; ++p) {
-            const uint32_t lo = vx[t][q][2 * p], hi = vx[t][q][2 * p + 1], lo8 = lo >> 8, hi8 = hi >> 8;
-            mma16816(acc[(2 * q + p) * 2], lo & NIB_E, lo & NIB_O, hi & NIB_E, hi & NIB_O, pb[2 * t], pb[2 * t + 1]);
-            mma16816(acc[(2 * q + p) * 2 + 1], lo8 & NIB_E, lo8 & NIB_O, hi8 & NIB_E, hi8 & NIB_O, pb[2 * t], pb[2 * t + 1]);
+            constexpr uint32_t E = NIB_E << 3, O = NIB_O << 3;
+            const uint32_t lo = vx[t][q][2 * p], hi = vx[t][q][2 * p + 1], lo0 = lo << 3, hi0 = hi << 3, lo2 = lo >> 5, hi2 = hi >> 5;
+            mma16816(acc[(2 * q + p) * 2], lo0 & E, lo0 & O, hi0 & E, hi0 & O, pb[2 * t], pb[2 * t + 1]);
+            mma16816(acc[(2 * q + p) * 2 + 1], lo2 & E, lo2 & O, hi2 & E, hi2 & O, pb[2 * t], pb[2 * t + 1]);
           }
     };
 
@@ -662,8 +670,8 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
         #pragma unroll
         for (int t = 0; t < L::NH; ++t) {                        // m-tile: (even | odd channel) x (head 2j | 2j+1)
           const int mt = half * L::NH + t;
-          mbuf[(warp * L::NH + t) * 32 + lane] = make_float4(fmaf(acc[mt][0], NIB_E_INV, zacc[0]) * sc0, fmaf(acc[mt][1], NIB_E_INV, zacc[1]) * sc1,
-                                                             fmaf(acc[mt][2], NIB_O_INV, zacc[0]) * sc0, fmaf(acc[mt][3], NIB_O_INV, zacc[1]) * sc1);
+          mbuf[(warp * L::NH + t) * 32 + lane] = make_float4(fmaf(acc[mt][0], VNIB_E_INV, zacc[0]) * sc0, fmaf(acc[mt][1], VNIB_E_INV, zacc[1]) * sc1,
+                                                             fmaf(acc[mt][2], VNIB_O_INV, zacc[0]) * sc0, fmaf(acc[mt][3], VNIB_O_INV, zacc[1]) * sc1);
         }
         if (Q && more && half == 0) {                            // nobody still reads the Q fragments of this item
           #pragma unroll
