@@ -605,7 +605,10 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
       const uint32_t st = sbase + L::OFF_STAGES + s * L::STAGE;
       if (!mbar_wait(bar_full + 8 * s, (k / NSTAGE) & 1)) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; break; }
       const uint32_t bar_free = bar_empty + 8 * s;
-      if (none) { if (lane == 0) mbar_arrive(bar_free); }
+      if (none) {
+        __syncwarp();                                            // no lane still polls the barrier of a stage that may now be refilled
+        if (lane == 0) mbar_arrive(bar_free);
+      }
       else if (tail) group(std::true_type{}, st, bar_free, 0, len - nq * 32);
       else group(std::false_type{}, st, bar_free, sub, 32);
     }
