@@ -187,7 +187,7 @@ int yskn_kv4_attention_ex(const yskn_attn_g_args* a, const yskn_kv4_attn_ext* x,
   return attention_dispatch(a, g, hd, rd, act_dtype, Shard{0, a->max_ctx}, (cudaStream_t)cuda_stream, x);
 }
 
-size_t yskn_kv4_ms_maps_bytes(int n_slots) { return n_slots > 0 ? (size_t)n_slots * 6 * 128 : 0; }
+size_t yskn_kv4_ms_maps_bytes(int n_slots) { return n_slots > 0 ? (size_t)n_slots * 2 * 128 : 0; }
 
 int yskn_kv4_ms_prepare(const yskn_kv_layer* h_layers, int n_slots, int kvh, int hd, int max_ctx, yskn_kv_layer* d_layers, void* d_maps,
                         void* cuda_stream) {

@@ -13,8 +13,8 @@
 // Work split.  grid (splits, Hkv, M), one CTA per SM when splits*Hkv*M = 148.  A CTA owns a run of 128-token units
 // (four 32-token groups) of one kv-head.  One producer warp streams each unit into an mbarrier ring with seven
 // copies: K 128 x HD/2 bytes and V 128 x HD/2 bytes by tiled TMA (128-byte swizzle), four K scale rows, four K zero
-// rows, 128 V scales, 128 V zeros (bulk copies) and the four rope rows of the groups' first positions (one strided
-// TMA tile).  Few, large copies matter: the number of copies in flight per SM is limited, not only their bytes.
+// rows, 128 V scales, 128 V zeros (tiles; bulk copies in a multi-request pass) and the four rope rows of the groups' first
+// positions (one strided TMA tile).  Few, large copies matter: the number of copies in flight per SM is limited, not only their bytes.
 // Seven consumer warps take the groups round-robin and keep their own (m, l, O) state.  A group is two 16-token
 // MMA tiles:
 //   S^T[16 tok x 8 heads]  = K[16 tok x HD] . Q^T[HD x 8 heads]          (m16n8k16, HD/16 steps)
@@ -203,9 +203,11 @@ __device__ __forceinline__ float lds_h(uint32_t a) {
 }
 
 // ---------------------------------------------------------------- kernel
-// Tensor maps of one cache.  The scales and zeros come as tiles too: as plain bulk copies of 2 KB and 256 bytes the same step took 82.2 instead of
-// 81.1 us at 262,144 tokens.
+// Tensor maps of one cache.  The scales and zeros come as tiles too: as bulk copies of 2 KB and 256 bytes the same step took 82.2 instead of
+// 81.1 us at 262,144 tokens.  In a multi-request pass they are bulk copies all the same, because its table in device memory holds the maps of K and V
+// only (yskn_kv4_ms_rows): eight sequences 116.3 us, with a table of six maps 115.8.
 struct Maps { CUtensorMap k, v, ks, kz, vs, vz; };
+static_assert(sizeof(Maps) == 6 * 128, "yskn_kv4_ms_maps_bytes and the header give 128 bytes a map");
 struct DecodeP {
   yskn_attn_g_args A;
   Shard sh;
@@ -222,7 +224,7 @@ struct DecodeP {
 // bit of it, does not depend on Q.  Before, each item paid its launch, set-up, first-copy latency and merge by itself, and the longest
 // rows of a batch came last: eight sequences of 2,048 .. 131,072 tokens 171 -> 124 us with their merge, five rows over 20,011 tokens 67.6 ->
 // 55.6 us with their append and merge, eight rows over 172 tokens 48.8 -> 38 us.
-template <int HD, int RD, int DT, bool Q>
+template <int HD, int RD, int DT, bool Q, bool multi>
 __global__ void __launch_bounds__(NTHREADS, 1)
 kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__ CUtensorMap mapR, const DecodeP P) {
   using L = Lay<HD, RD, Q>;
@@ -244,7 +246,6 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
 
-  const bool multi = P.ms.pos != nullptr;                       // rows of several sequences: per-row position and cache
   // ---- which groups an item (split, kv-head, row) covers (local token indices of this shard)
   struct Item { int split, kvh, r, base_local, len, nq, nu4, u0, nu; bool has_tail; };
   auto item_at = [&](int x, int y, int z) {
@@ -310,7 +311,7 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
       const size_t row0 = (size_t)kvh * A.max_ctx;              // first row of this kv-head in the [Hkv*max_ctx] arrays
       const int slot = multi ? P.ms.slot[it.r] : 0;
       const yskn_kv_layer kvl = multi ? P.ms.layers[slot] : A.kv;
-      const Maps* const mp = multi ? static_cast<const Maps*>(P.ms.maps) + slot : &maps;
+      const CUtensorMap* const mk = multi ? static_cast<const CUtensorMap*>(P.ms.maps) + 2 * slot : &maps.k;   // K, V; of one cache all six
       for (int u = it.u0; u < it.u0 + it.nu; ++u) {
         const int s = k % NSTAGE;
         // an early unit: one of the first ring fills, int4 only, every token below the base position
@@ -330,18 +331,21 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
         const bool tail = has_tail && u == nu4;
         const int g0 = tail ? nq : u * L::UG;                    // its first group (local index)
         const uint32_t st = sbase + L::OFF_STAGES + s * L::STAGE, bar = bar_full + 8 * s;
-        if (lane == 0) mbar_expect_tx(bar, 2 * L::UG * L::KB + 2 * L::UG * ((tail ? 0 : L::SCB) + 64) + L::UG * L::ROPEB);   // SHADOW == UG*KB
+        // Tiles are whole units always: what lies behind the last group of a unit, or of the array, is unused.  Bulk copies (the table of a
+        // multi-request pass holds the maps of K and V only) end with the unit's last group, which may be the array's.
+        const int ngr = !multi ? L::UG : tail ? 1 : min(L::UG, nq - u * L::UG);
+        if (lane == 0) mbar_expect_tx(bar, 2 * L::UG * L::KB + 2 * ngr * ((tail ? 0 : L::SCB) + 64) + L::UG * L::ROPEB);   // SHADOW == UG*KB
         __syncwarp();                                            // the barrier is armed before any copy is issued
-        // One copy per lane: seven issue slots in parallel.  Whole units always: what lies behind the last group of a unit, or of the array, is unused.
         const int tok0 = (int)row0 + g0 * 32, grp0 = kvh * (A.max_ctx / 32) + g0;
+        // One copy per lane: seven issue slots in parallel
         switch (lane) {
           case 0: if (tail) bulk_1d(st + L::OFF_K, kvl.kshadow + (size_t)tok0 * HD, L::SHADOW, bar);
-                  else tma_2d(st + L::OFF_K, &mp->k, 0, tok0, bar); break;
-          case 1: tma_2d(st + L::OFF_V, &mp->v, 0, tok0, bar); break;
-          case 2: if (!tail) tma_2d(st + L::OFF_KS, &mp->ks, 0, grp0, bar); break;
-          case 3: if (!tail) tma_2d(st + L::OFF_KZ, &mp->kz, 0, grp0, bar); break;
-          case 4: tma_2d(st + L::OFF_VS, &mp->vs, g0 * 32, kvh, bar); break;
-          case 5: tma_2d(st + L::OFF_VZ, &mp->vz, g0 * 32, kvh, bar); break;
+                  else tma_2d(st + L::OFF_K, mk, 0, tok0, bar); break;
+          case 1: tma_2d(st + L::OFF_V, mk + 1, 0, tok0, bar); break;
+          case 2: if (!tail) { if (multi) bulk_1d(st + L::OFF_KS, kvl.kscale + (size_t)grp0 * HD, ngr * L::SCB, bar); else tma_2d(st + L::OFF_KS, mk + 2, 0, grp0, bar); } break;
+          case 3: if (!tail) { if (multi) bulk_1d(st + L::OFF_KZ, kvl.kzero + (size_t)grp0 * HD, ngr * L::SCB, bar); else tma_2d(st + L::OFF_KZ, mk + 3, 0, grp0, bar); } break;
+          case 4: if (multi) bulk_1d(st + L::OFF_VS, kvl.vscale + tok0, ngr * 64, bar); else tma_2d(st + L::OFF_VS, mk + 4, g0 * 32, kvh, bar); break;
+          case 5: if (multi) bulk_1d(st + L::OFF_VZ, kvl.vzero + tok0, ngr * 64, bar); else tma_2d(st + L::OFF_VZ, mk + 5, g0 * 32, kvh, bar); break;
           case 6: if (RD > 0) tma_2d(st + L::OFF_ROPE, &mapR, 0, g0 + P.sh.start / 32, bar); break;   // rows 32*(g0..g0+3) of the table
           default: break;
         }
@@ -734,6 +738,11 @@ bool make_map(CUtensorMap* out, const void* base, int elem, uint64_t rows, uint6
             CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Packed rows in units of 128 tokens, swizzle = row width.
+bool make_unit_map(CUtensorMap* out, const void* base, int kvh, int max_ctx, int hd) {
+  return make_map(out, base, 1, (uint64_t)kvh * max_ctx, hd / 2, 128, hd / 2, hd == 256 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
 // The maps of one cache: units of 128 tokens of the packed rows (swizzle = row width), four rows of the group arrays, 128 values of the token arrays.
 bool make_maps(Maps* out, const yskn_kv_layer& l, int kvh, int max_ctx, int hd) {
   struct Key {
@@ -753,8 +762,8 @@ bool make_maps(Maps* out, const yskn_kv_layer& l, int kvh, int max_ctx, int hd) 
   auto it = cache.find(key);
   if (it != cache.end()) { *out = it->second; return true; }
   const uint64_t rows = (uint64_t)kvh * max_ctx;
-  const CUtensorMapSwizzle sw = hd == 256 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, none = CU_TENSOR_MAP_SWIZZLE_NONE;
-  if (!make_map(&out->k, l.kq, 1, rows, hd / 2, 128, hd / 2, sw) || !make_map(&out->v, l.vq, 1, rows, hd / 2, 128, hd / 2, sw) ||
+  const CUtensorMapSwizzle none = CU_TENSOR_MAP_SWIZZLE_NONE;
+  if (!make_unit_map(&out->k, l.kq, kvh, max_ctx, hd) || !make_unit_map(&out->v, l.vq, kvh, max_ctx, hd) ||
       !make_map(&out->ks, l.kscale, 2, rows / 32, hd, 4, hd, none) || !make_map(&out->kz, l.kzero, 2, rows / 32, hd, 4, hd, none) ||
       !make_map(&out->vs, l.vscale, 2, kvh, max_ctx, 1, 128, none) || !make_map(&out->vz, l.vzero, 2, kvh, max_ctx, 1, 128, none)) return false;
   if (cache.size() > 1024) cache.clear();
@@ -782,10 +791,10 @@ bool make_rope_map(CUtensorMap* out, const float* rope, int rd, uint64_t groups)
   return true;
 }
 
-template <int HD, int RD, int DT, bool Q>
-int launch_q(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const Maps& mp, const CUtensorMap& mr, cudaStream_t st) {
+template <int HD, int RD, int DT, bool Q, bool multi>
+int launch_m(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const Maps& mp, const CUtensorMap& mr, cudaStream_t st) {
   using L = Lay<HD, RD, Q>;
-  auto kern = kv4_decode_mma_kernel<HD, RD, DT, Q>;
+  auto kern = kv4_decode_mma_kernel<HD, RD, DT, Q, multi>;
   static std::atomic<unsigned long long> attr{0};               // once per device, like the reference's launchers once per process
   if (first_use_on_device(attr)) {
     KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
@@ -799,6 +808,12 @@ int launch_q(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_k
   cfg.attrs = at; cfg.numAttrs = 1;
   KV4_CUDA(cudaLaunchKernelEx(&cfg, kern, mp, mr, P));
   return launch_status("kv4_decode_mma_kernel");
+}
+
+template <int HD, int RD, int DT, bool Q>
+int launch_q(const yskn_attn_g_args& a, int g, Shard sh, int early, const yskn_kv4_ms_rows& ms, const Maps& mp, const CUtensorMap& mr, cudaStream_t st) {
+  if (ms.pos) return launch_m<HD, RD, DT, Q, true>(a, g, sh, early, ms, mp, mr, st);
+  return launch_m<HD, RD, DT, Q, false>(a, g, sh, early, ms, mp, mr, st);
 }
 
 // One CTA fills an SM, so a grid of up to one block per SM starts at once and has nothing to take over; a larger one runs as a queue.
@@ -829,16 +844,16 @@ int ms_prepare(const yskn_kv_layer* h_layers, int n_slots, int kvh, int hd, int 
   if (!h_layers || !d_layers || !d_maps || n_slots <= 0 || n_slots > 64) KV4_REJECT("yskn_kv4_ms_prepare: bad arguments (n_slots %d)", n_slots);
   if (kvh <= 0 || (hd != 128 && hd != 256) || max_ctx <= 0 || max_ctx % 64) KV4_REJECT("yskn_kv4_ms_prepare: bad shape (kvh %d, hd %d, max_ctx %d)", kvh, hd, max_ctx);
   if ((uintptr_t)d_maps & 127) KV4_REJECT("yskn_kv4_ms_prepare: the map table must be 128-byte aligned");
-  std::vector<Maps> maps((size_t)n_slots);
+  std::vector<CUtensorMap> maps(2 * (size_t)n_slots);
   for (int s = 0; s < n_slots; ++s) {
     const yskn_kv_layer& l = h_layers[s];
     const uintptr_t al = (uintptr_t)l.kq | (uintptr_t)l.vq | (uintptr_t)l.kscale | (uintptr_t)l.kzero | (uintptr_t)l.kshadow | (uintptr_t)l.vscale | (uintptr_t)l.vzero;
     if (!l.kq || !l.vq || !l.kscale || !l.kzero || !l.kshadow || !l.vscale || !l.vzero || (al & 15))
       KV4_REJECT("yskn_kv4_ms_prepare: cache arrays of slot %d missing or not 16-byte aligned", s);
-    if (!make_maps(&maps[s], l, kvh, max_ctx, hd))
+    if (!make_unit_map(&maps[2 * s], l.kq, kvh, max_ctx, hd) || !make_unit_map(&maps[2 * s + 1], l.vq, kvh, max_ctx, hd))
       KV4_REJECT("yskn_kv4_ms_prepare: cuTensorMapEncodeTiled failed or is unavailable");
   }
-  KV4_CUDA(cudaMemcpyAsync(d_maps, maps.data(), maps.size() * sizeof(Maps), cudaMemcpyHostToDevice, st));
+  KV4_CUDA(cudaMemcpyAsync(d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, st));
   KV4_CUDA(cudaMemcpyAsync(d_layers, h_layers, (size_t)n_slots * sizeof(yskn_kv_layer), cudaMemcpyHostToDevice, st));
   KV4_CUDA(cudaStreamSynchronize(st));                            // the host vectors go out of scope
   return 0;
