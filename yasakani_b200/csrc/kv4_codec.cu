@@ -169,13 +169,13 @@ __global__ void __launch_bounds__(256, 4) kv4_append_kernel(yskn_kv_append_args 
   const int lane = threadIdx.x & 31, nk = groups * A.kvh * (HD / 64);
   int w = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
   pdl_enter();
-  const int pos0 = *A.d_pos;
-  if (pos0 >= A.max_ctx) return;                     // no row fits, and no index below leaves 32 bits
-  const int last = min(pos0 + A.M, A.max_ctx) - 1;
+  const int pos0 = *A.d_pos, last = (int)((unsigned)pos0 + (unsigned)A.M - 1u);
   const bool keys = w < nk;
   if (!keys) w -= nk;
   const int parts = keys ? HD / 64 : vw, part = w % parts, gh = w / parts, gi = (pos0 >> 5) + gh / A.kvh, head = gh % A.kvh, gend = gi * 32 + 31;
-  if (gh >= groups * A.kvh || gi < 0 || gi * 32 > last) return;
+  // A group outside the cache is told by its number, which no position makes wrap; positions whose last row would wrap have no other groups.  (A
+  // comparison of the position ahead of all this cost every decode step 0.2 us.)
+  if (gh >= groups * A.kvh || (unsigned)gi >= (unsigned)A.max_ctx / 32u || gi * 32 > last) return;
   const int first = max(pos0, gi * 32), end = min(last, gend) + 1;               // rows of this pass in the group
   if (keys) keys_warp<HD, DT, PAIRS>(A.kv, A.max_ctx, A.k_in, A.kvh, pos0, first, end, gi, head, part * 64 + 2 * lane, gend >= pos0 && gend <= last);
   else values_warp<HD, DT>(A.kv, A.max_ctx, A.v_in, A.kvh, pos0, first + part, end, vw, head, lane, wide != 0);
@@ -186,10 +186,8 @@ template <int HD>
 __global__ void __launch_bounds__(128) kv4_group_quant_kernel(yskn_kv_quant_args A, int kvh) {
   const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5), part = w % (HD / 64), gh = w / (HD / 64);
   pdl_enter();
-  const int pos0 = *A.d_pos;
-  if (pos0 >= A.max_ctx) return;
-  const int last = pos0 + A.M - 1, gi = pos0 / 32 + gh / kvh, head = gh % kvh, gend = gi * 32 + 31;
-  if (gh >= ((A.M + 31) / 32 + 1) * kvh || gi < 0 || gend < pos0 || gend > last || gend >= A.max_ctx) return;
+  const int pos0 = *A.d_pos, last = (int)((unsigned)pos0 + (unsigned)A.M - 1u), gi = pos0 / 32 + gh / kvh, head = gh % kvh, gend = gi * 32 + 31;
+  if (gh >= ((A.M + 31) / 32 + 1) * kvh || (unsigned)gi >= (unsigned)A.max_ctx / 32u || gend < pos0 || gend > last) return;
   keys_warp<HD, YSKN_KV4_F16, true>(A.kv, A.max_ctx, nullptr, kvh, pos0, gi * 32, gi * 32, gi, head, part * 64 + 2 * lane, true);
 }
 
