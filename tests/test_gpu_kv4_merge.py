@@ -29,3 +29,9 @@ def test_merge_matches_double_precision(M, nh, g, hd, S, dtype, shift):
     # type: half an ulp, 2^-11 or 2^-8 of the value; fp32 arithmetic between the two is far below either
     bound = bare.abs() * 2.0 ** -10 + want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.01 + 1e-6
     assert ((o16.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("M", [19, 37, 38])                       # 304, 592 and 608 rows x heads: with more than 20 splits a warp each from 593 on
+@pytest.mark.parametrize("S", [20, 21, 37])
+def test_merge_on_both_sides_of_the_line_for_128_channels(M, S):
+    test_merge_matches_double_precision(M, 16, 8, 128, S, torch.float16, 0)
