@@ -205,14 +205,15 @@ __global__ void kv4_rope_table_kernel(float2* out, int max_ctx, float theta, int
   out[idx] = make_float2((float)c, (float)s);
 }
 
-// Blocks.  The attention kernel is launched while this one runs (programmatic launch) and sets itself up beside it where an SM has room: up to eight
-// rows come in blocks of two warps, which fit beside the decode kernel's block on its SM (61,440 of 65,536 registers).  The tcgen05 kernel takes all
-// of an SM's registers and finds no room beside any block; blocks of 32 warps on as few SMs as possible were slower than that (64 rows: 9.0 us
-// against 4.0 in blocks of four warps).
+// Blocks.  The attention kernel is launched while this one runs (programmatic launch) and sets itself up beside it where an SM has room.  Of the decode
+// kernel's forms, one CTA of 256 threads an SM, only the single-wave one of head_dim 256 leaves room (232 registers a thread, 61,440 of 65,536 by
+// blocks; the queue and the rotary forms of 128 channels take 254 or 255), and there blocks of 64, 128 and 256 threads came out the same for up to
+// eight rows (one row 19.8, 11.3 and 81.5 us, five rows 50.4).  The tcgen05 kernel takes all of an SM's registers; blocks of 32 warps on as few SMs
+// as possible were slower than its wait for room (64 rows: 9.0 us against 4.0 in blocks of four warps).
 template <int HD> int append_hd(const yskn_kv_append_args& a, cudaStream_t st) {
   const int groups = (a.M + 30) / 32 + 1;                        // groups that M rows can touch
   const int vw = a.M < 8 ? a.M : 8;
-  const int threads = a.M <= 8 ? 64 : a.M <= 64 ? 128 : 256;
+  const int threads = a.M <= 64 ? 128 : 256;
   const long long warps = (long long)groups * a.kvh * (HD / 64 + vw);
   const dim3 blocks((unsigned)((warps * 32 + threads - 1) / threads));
   const char* who = "kv4_append_kernel";
