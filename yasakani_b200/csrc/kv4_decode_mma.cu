@@ -435,7 +435,7 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
 
     // One 32-token group.  TAIL: the open group (fp16 shadow rows, `nvalid` visible tokens); else an int4 group.
     // `st` = stage base, `sub` = which of the unit's four groups (0 for the open group).
-    auto group = [&](auto tail_c, const uint32_t st, const uint32_t bar_free, const int sub, const int nvalid) {
+    auto group = [&](auto tail_c, const uint32_t st, const int sub, const int nvalid) {
       constexpr bool TAIL = decltype(tail_c)::value;
       const uint32_t s_k = st + L::OFF_K + sub * L::KB, s_v = st + L::OFF_V + sub * L::KB, s_ks = st + L::OFF_KS + sub * L::SCB,
                      s_kz = st + L::OFF_KZ + sub * L::SCB, s_vs = st + L::OFF_VS + sub * 64, s_rope = st + L::OFF_ROPE + sub * L::ROPEB;
@@ -546,9 +546,6 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
         const bool v = !TAIL || 8 * y + g < nvalid;
         vs[y] = v ? lds_h(s_vs + 2 * g + 16 * y) : 0.f; vz[y] = v ? lds_h(s_vs + L::UG * 64 + 2 * g + 16 * y) : 0.f;
       }
-      // All of the group has been read: its part of the stage goes back here, with the softmax and P.V still ahead.
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_free);                      // one of the four arrivals that free the stage
       // ---- softmax over the group (log2 domain); heads 2j, 2j+1
       float s[4][2];
       #pragma unroll
@@ -608,13 +605,12 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
       if (!Q && none) continue;
       const uint32_t st = sbase + L::OFF_STAGES + s * L::STAGE;
       if (!mbar_wait(bar_full + 8 * s, (k / NSTAGE) & 1)) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; break; }
-      const uint32_t bar_free = bar_empty + 8 * s;
-      if (none) {
-        __syncwarp();                                            // no lane still polls the barrier of a stage that may now be refilled
-        if (lane == 0) mbar_arrive(bar_free);
+      if (!none) {
+        if (tail) group(std::true_type{}, st, 0, len - nq * 32);
+        else group(std::false_type{}, st, sub, 32);
       }
-      else if (tail) group(std::true_type{}, st, bar_free, 0, len - nq * 32);
-      else group(std::false_type{}, st, bar_free, sub, 32);
+      __syncwarp();                                              // no lane still reads the stage or polls its barrier
+      if (lane == 0) mbar_arrive(bar_empty + 8 * s);             // one of the four arrivals that free the stage
     }
 
     // Q: the item after this one, and its queries on their way while this one is merged
