@@ -104,7 +104,6 @@ template <int HD, int RD, bool Q> struct Lay {
   static constexpr int TOTAL = Q ? OFF_MERGE + MERGE : OFF_ML + NCW * 4 * 16;
   static_assert(Q || MERGE <= NSTAGE * STAGE, "merge buffer must fit in the ring");
   static_assert(SHADOW == UG * KB, "the open group's fp16 rows take the place of the unit's packed K");
-  static_assert(NCW <= 2 * UG, "a warp passes over at most one unit between two slots");
   static_assert(NR % 2 == 0 && NR <= NW, "rotary width must be a multiple of 64 and at most head_dim");
   static_assert(TOTAL <= 227 * 1024, "shared memory budget of one CTA");
 };
@@ -605,11 +604,7 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
       const bool tail = has_tail && u == nu4, none = tail ? sub != 0 : u * L::UG + sub >= nq;   // the unit holds fewer than four groups
       if (!Q && none) continue;
       const uint32_t st = sbase + L::OFF_STAGES + s * L::STAGE;
-      // A wait tells a stage's phases apart by parity only, so a warp waits for every unit of its item, also for the one before where that has no
-      // slot of its own: its stage's next unit would else be taken for there, should the unit itself come in after the next ones.
-      bool here = mbar_wait(bar_full + 8 * s, (k / NSTAGE) & 1);
-      if (sub < NCW - L::UG && u > u0) here = mbar_wait(bar_full + 8 * ((k - 1) % NSTAGE), ((k - 1) / NSTAGE) & 1) && here;
-      if (!here) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; break; }
+      if (!mbar_wait(bar_full + 8 * s, (k / NSTAGE) & 1)) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; break; }
       if (!none) {
         if (tail) group(std::true_type{}, st, 0, len - nq * 32);
         else group(std::false_type{}, st, sub, 32);
