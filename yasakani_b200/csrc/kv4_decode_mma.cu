@@ -94,7 +94,8 @@ template <int HD, int RD, bool Q> struct Lay {
   static constexpr int OFF_RELT = OFF_QFRAG + QFRAG;
   static constexpr int OFF_BARS = OFF_RELT + RELT;         // full[NSTAGE], empty[NSTAGE]
   static constexpr int OFF_MISC = OFF_BARS + 2 * NSTAGE * 8;   // abort flag
-  static constexpr int OFF_RESP = (OFF_MISC + 4 + 15) / 16 * 16, OFF_CLC = OFF_RESP + 32;   // queue: two cancel responses, their full / empty barriers
+  static constexpr int OFF_TAG = OFF_MISC + 4;             // [NSTAGE] the unit last issued into each stage
+  static constexpr int OFF_RESP = (OFF_TAG + 4 * NSTAGE + 15) / 16 * 16, OFF_CLC = OFF_RESP + 32;   // queue: two cancel responses, their full / empty barriers
   static constexpr int OFF_ORDER = OFF_CLC + 32, OFF_POS = OFF_ORDER + 64;                   // queue: rows by length; their positions
   static constexpr int OFF_ML = (OFF_POS + 256 + 15) / 16 * 16;                              // (m, l) of heads 2j, 2j+1 per (warp, j)
   static constexpr int NH = HD / 32;                       // m-tiles of one half
@@ -268,11 +269,13 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
   const uint32_t bar_full = sbase + L::OFF_BARS, bar_empty = bar_full + NSTAGE * 8;
   const uint32_t bar_clc = sbase + L::OFF_CLC, resp = sbase + L::OFF_RESP;       // Q: full[2], empty[2]; two responses
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + L::OFF_MISC);
+  volatile int* s_tag = reinterpret_cast<volatile int*>(smem + L::OFF_TAG);
   if (sbase & 1023u) { if (threadIdx.x == 0) atomicExch(&g_decode_status, 3); return; }   // the swizzled tiles need a 1 KB base
   if (threadIdx.x == 0) {
     // a stage is free again once the consumers of its four groups have arrived (without Q units with fewer groups are never reused)
     for (int s = 0; s < NSTAGE; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, L::UG); }
     if (Q) for (int s = 0; s < 2; ++s) { mbar_init(bar_clc + 8 * s, 1); mbar_init(bar_clc + 16 + 8 * s, NCW); }
+    for (int s = 0; s < NSTAGE; ++s) s_tag[s] = -1;
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -334,6 +337,7 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
         // Tiles are whole units always: what lies behind the last group of a unit, or of the array, is unused.  Bulk copies (the table of a
         // multi-request pass holds the maps of K and V only) end with the unit's last group, which may be the array's.
         const int ngr = !multi ? L::UG : tail ? 1 : min(L::UG, nq - u * L::UG);
+        if (lane == 0) s_tag[s] = k;
         if (lane == 0) mbar_expect_tx(bar, 2 * L::UG * L::KB + 2 * ngr * ((tail ? 0 : L::SCB) + 64) + L::UG * L::ROPEB);   // SHADOW == UG*KB
         __syncwarp();                                            // the barrier is armed before any copy is issued
         const int tok0 = (int)row0 + g0 * 32, grp0 = kvh * (A.max_ctx / 32) + g0;
@@ -604,7 +608,12 @@ kv4_decode_mma_kernel(const __grid_constant__ Maps maps, const __grid_constant__
       const bool tail = has_tail && u == nu4, none = tail ? sub != 0 : u * L::UG + sub >= nq;   // the unit holds fewer than four groups
       if (!Q && none) continue;
       const uint32_t st = sbase + L::OFF_STAGES + s * L::STAGE;
-      if (!mbar_wait(bar_full + 8 * s, (k / NSTAGE) & 1)) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; break; }
+      // A wait tells a stage's phases apart by parity only, and a warp has no slot in some units: while such a unit is still on its way, the wait for
+      // the next one in its stage would return on the phase before both.  So the unit is seen issued first, which is behind the end of that phase.
+      const uint32_t full = bar_full + 8 * s, parity = (k / NSTAGE) & 1;
+      uint32_t polls = 0;
+      while (s_tag[s] != k && ++polls < WAIT_LIMIT) mbar_try_wait(full, parity);
+      if (polls >= WAIT_LIMIT || !mbar_wait(full, parity)) { atomicExch(&g_decode_status, 1); *s_abort = 1; ok = false; break; }
       if (!none) {
         if (tail) group(std::true_type{}, st, 0, len - nq * 32);
         else group(std::false_type{}, st, sub, 32);
