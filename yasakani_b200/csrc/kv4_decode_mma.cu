@@ -36,7 +36,7 @@
 //     even channels and odd ones: 1.59e-3 1.58e-3 / 1.15e-3 1.14e-3 / 1.18e-3 1.18e-3.  At bits 0..3 and 4..7: 2.29e-3 1.59e-3 /
 //     1.34e-3 1.15e-3 / 1.29e-3 1.18e-3.  With offsets (1024 + n taken out by a subtraction, 64 + n by MMA rows of ones): 1.54e-3 6.70e-3 /
 //     1.14e-3 1.26e-3 / 1.16e-3 1.19e-3.  For K, whose sums run over a head's channels only, the position changes nothing (0.1 %).
-//     Time with offsets, and now: 262,144 tokens 85.7 -> 81.2 us, eight sequences 124.2 -> 115.8 us (both tiles of a group in
+//     Time with offsets, and now: 262,144 tokens 85.7 -> 82.0 us, eight sequences 124.2 -> 115.7 us (both tiles of a group in
 //     step, see below, included).
 //   * RoPE: Q is rotated back by the group's first position (one table row per group), the remaining angle
 //     (0..31 tokens) is applied to the rotary channels of K with the table's first 32 rows.  cos/sin of
@@ -66,7 +66,7 @@ namespace {
 #ifndef KV4_DECODE_NCW
 #define KV4_DECODE_NCW 7                     // consumer warps per CTA
 #endif
-// 8 warps = 2 per SM sub-partition, one CTA per SM, up to 255 registers a thread.  Measured at 262,144 tokens:
+// 8 warps = 2 per SM sub-partition, one CTA per SM, up to 255 registers a thread.  Measured at 262,144 tokens, with the offsets' arithmetic:
 // 4 / 6 / 8 / 12 / 16 warps (255 / 255 / 255 / 168 / 128 registers) = 127 / 111 / 83.5 / 90.2 / 107 us per step
 constexpr int NCW = KV4_DECODE_NCW;
 constexpr int NTHREADS = (NCW + 1) * 32;

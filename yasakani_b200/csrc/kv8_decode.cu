@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(256) kv8_combine_rows_kernel(const float* pm, 
   // v / L2, correctly rounded.  With r = 1 / L2 rounded and q = v * r, q - (q * L2 - v) * r in two fused steps is the rounded quotient while the values
   // and the residual stay normal (Markstein, IBM J. Res. Dev. 34, 1990; his theorem asks for a q within one unit in the last place, and q may
   // be off by 1.5: the 40.7 million pairs of 24-bit values whose quotient lies near enough to a tie for that to matter were all tried).  Three
-  // operations instead of a division per value: 24,000 rows of one split 24.2 -> 22 us.  The bounds keep |q| and the residual's last bit
+  // operations instead of a division per value: 24,000 rows of one split, behind memory, 26.8 -> 24.7 us.  The bounds keep |q| and the residual's last bit
   // normal; the residual has the sign that leaves a zero its own.  Other rows divide.
   const float r = __frcp_rn(L2);
   float big = 0.f;                                         // largest |v|, past NaN, which stays NaN on either way
