@@ -41,3 +41,9 @@ def test_merge_matches_double_precision(M, nh, S, dtype):
     ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
     err = np.abs(o16.double().cpu().numpy() - want)
     assert (err <= 2.5 * ulp * np.abs(want) + 1e-6).all(), err.max()
+
+
+@pytest.mark.parametrize("M,nh,S", [(37, 4, 3), (149, 1, 1), (50, 3, 8), (25, 6, 9), (19, 8, 32), (19, 8, 33), (10, 24, 64)])
+def test_row_form_edges(M, nh, S):
+    """Both sides of the line between the forms, whole and broken batches of eight splits, one and two weights a lane."""
+    test_merge_matches_double_precision(M, nh, S, torch.bfloat16)

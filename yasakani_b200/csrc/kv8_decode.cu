@@ -285,85 +285,149 @@ __global__ void __launch_bounds__(KV8_CQ * 256) kv8_combine_kernel(const float* 
   o16[e] = act_store16<DT>(y);
 }
 
-// One to four splits (prefill): eight lanes per row as in the row codec, four rows per warp, no shared memory and no barrier.
-template <int DT>
-__global__ void __launch_bounds__(256) kv8_combine_rows_kernel(const float* pm, const float* pl, const float* pacc, int S, int nh, long long rows,
+// Many rows: one warp per row, lane l owns channels 4l .. 4l + 3 and 128 + 4l .., no shared memory and no barrier; up to eight splits of loads are in
+// flight at once.  Bound by instruction issue for a prompt (56 operations a value, most of them the sigmoid, the butterflies and the quotient), by two trips to
+// memory for the rows of a verify pass.  The form it replaces took eight lanes a row (four rows a warp, 32 values a lane: a quarter of the warps, for
+// one to four splits only).  Replays over partials in L2, before -> now: 384 rows of 18 splits 7.5 -> 4.1 us, 2,400 of 6 splits 36.5 -> 4.5, 4,032 of 4 splits
+// 13.6 -> 5.7, 24,000 of one split 21.3 -> 14.2.
+template <int DT, bool ONE>
+__global__ void __launch_bounds__(128) kv8_combine_rows_kernel(const float* pm, const float* pl, const float* pacc, int S, int nh, long long rows,
                                                                const void* gate, uint16_t* o16, int inverse_rotate) {
-  const int lane = threadIdx.x & 31, ll = lane & 7;
-  const long long row = (long long)blockIdx.x * 32 + (threadIdx.x >> 5) * 4 + (lane >> 3);       // row = token * nh + head
-  const bool live = row < rows;
+  constexpr int B = ONE ? 1 : 8;
+  const int lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);          // row = token * nh + head
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const long long tok = live ? row / nh : 0;
-  const int head = live ? (int)(row - tok * nh) : 0;
-  auto slot = [&](int s) -> size_t { return ((size_t)tok * S + s) * nh + head; };
-  float M2 = -1e30f, L2 = 0.f, v[32];
-  #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = 0.f;
-  for (int s = 0; s < S; ++s) M2 = fmaxf(M2, __ldcg(pm + slot(s)));
-  for (int s = 0; s < S; ++s) {
-    const float m = __ldcg(pm + slot(s)), w = m > -1e29f ? expf(m - M2) : 0.f;
-    L2 += w * __ldcg(pl + slot(s));
-    const float4* src = reinterpret_cast<const float4*>(pacc + slot(s) * KV8_HD) + ll;
+  if (row >= rows) return;
+  const long long tok = row / nh;
+  const int head = (int)(row - tok * nh);
+  const size_t slot0 = (size_t)tok * S * nh + head, step = (size_t)nh * KV8_HD;
+  const float* acc = pacc + slot0 * KV8_HD + 4 * lane;
+  const size_t e0 = (size_t)row * KV8_HD + 4 * lane;
+  float4 a[B][2];
+  auto load = [&](int s0) {
     #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float4 a = __ldcg(src + 8 * k);
-      v[4 * k] += w * a.x; v[4 * k + 1] += w * a.y; v[4 * k + 2] += w * a.z; v[4 * k + 3] += w * a.w;
+    for (int k = 0; k < B; ++k)
+      if (s0 + k < S) {
+        a[k][0] = __ldcg(reinterpret_cast<const float4*>(acc + (s0 + k) * step));
+        a[k][1] = __ldcg(reinterpret_cast<const float4*>(acc + (s0 + k) * step + 128));
+      }
+  };
+  float m0 = -1e30f, m1 = -1e30f, l0 = 0.f, l1 = 0.f, w0, w1 = 0.f, L2;      // of splits `lane` and `lane + 32` (at most 64 splits)
+  if (ONE) { m0 = __ldcg(pm + slot0); l0 = __ldcg(pl + slot0); }
+  else if (lane < S) { m0 = __ldcg(pm + slot0 + (size_t)lane * nh); l0 = __ldcg(pl + slot0 + (size_t)lane * nh); }
+  if (!ONE && lane + 32 < S) { m1 = __ldcg(pm + slot0 + (size_t)(lane + 32) * nh); l1 = __ldcg(pl + slot0 + (size_t)(lane + 32) * nh); }
+  load(0);
+  uint2 g[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)};
+  if (gate) {
+    g[0] = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(gate) + e0);
+    g[1] = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(gate) + e0 + 128);
+  }
+  if (ONE) { w0 = m0 > -1e29f ? 1.f : 0.f; L2 = w0 * l0; }
+  else {
+    float mx = fmaxf(m0, m1);
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    w0 = m0 > -1e29f ? expf(m0 - mx) : 0.f; w1 = m1 > -1e29f ? expf(m1 - mx) : 0.f;
+    L2 = w0 * l0 + w1 * l1;
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) L2 += __shfl_xor_sync(0xffffffffu, L2, o);
+  }
+  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // v[e] = channel 4 lane + e, v[4 + e] = channel 128 + 4 lane + e
+  #pragma unroll 1
+  for (int s0 = 0; ; ) {
+    #pragma unroll
+    for (int k = 0; k < B; ++k) {
+      const int s = s0 + k;
+      const float w = ONE ? w0 : __shfl_sync(0xffffffffu, s < 32 ? w0 : w1, s & 31);
+      if (s < S) {
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          v[4 * h] += w * a[k][h].x; v[4 * h + 1] += w * a[k][h].y; v[4 * h + 2] += w * a[k][h].z; v[4 * h + 3] += w * a[k][h].w;
+        }
+      }
     }
+    s0 += B;
+    if (ONE || s0 >= S) break;
+    load(s0);
   }
   // v / L2, correctly rounded.  With r = 1 / L2 rounded and q = v * r, q - (q * L2 - v) * r in two fused steps is the rounded quotient while the values
   // and the residual stay normal (Markstein, IBM J. Res. Dev. 34, 1990; his theorem asks for a q within one unit in the last place, and q may
   // be off by 1.5: the 40.7 million pairs of 24-bit values whose quotient lies near enough to a tie for that to matter were all tried).  Three
-  // operations instead of a division per value: 24,000 rows of one split, behind memory, 26.8 -> 24.7 us.  The bounds keep |q| and the residual's last bit
-  // normal; the residual has the sign that leaves a zero its own.  Other rows divide.
+  // operations instead of a division per value.  The bounds keep |q| and the residual's last bit normal; the residual has the sign that leaves a
+  // zero its own.  Lanes with other values divide.
   const float r = __frcp_rn(L2);
   float big = 0.f;                                         // largest |v|, past NaN, which stays NaN on either way
   uint32_t small = 0xFFFFFFFFu;                            // smallest |v| that is not 0: its bits twice, less 1
   #pragma unroll
-  for (int i = 0; i < 32; ++i) { big = fmaxf(big, fabsf(v[i])); small = min(small, 2u * __float_as_uint(v[i]) - 1u); }
+  for (int i = 0; i < 8; ++i) { big = fmaxf(big, fabsf(v[i])); small = min(small, 2u * __float_as_uint(v[i]) - 1u); }
   constexpr uint32_t SMALL = 2u * ((127u - 60u) << 23) - 1u;
   if (L2 >= 0x1p-20f && L2 <= 0x1p60f && big <= 0x1p100f && small >= SMALL) {
     #pragma unroll
-    for (int i = 0; i < 32; ++i) { const float q = __fmul_rn(v[i], r); v[i] = fmaf(-fmaf(q, L2, -v[i]), r, q); }
+    for (int i = 0; i < 8; ++i) { const float q = __fmul_rn(v[i], r); v[i] = fmaf(-fmaf(q, L2, -v[i]), r, q); }
   } else {
     #pragma unroll 1
-    for (int k = 0; k < 32; k += 4) {                      // rolled: rows without keys, sums beyond the range
-      float t[4];
+    for (int i = 0; i < 8; ++i) {                          // rolled (rows without keys, sums beyond the range): the values go round by one each time
+      const float t = __fdiv_rn(v[0], L2);
       #pragma unroll
-      for (int i = 0; i < 32; i += 4) if (i == k) { t[0] = v[i]; t[1] = v[i + 1]; t[2] = v[i + 2]; t[3] = v[i + 3]; }
-      #pragma unroll
-      for (int e = 0; e < 4; ++e) t[e] = __fdiv_rn(t[e], L2);
-      #pragma unroll
-      for (int i = 0; i < 32; i += 4) if (i == k) { v[i] = t[0]; v[i + 1] = t[1]; v[i + 2] = t[2]; v[i + 3] = t[3]; }
+      for (int k = 0; k < 7; ++k) v[k] = v[k + 1];
+      v[7] = t;
     }
   }
-  if (inverse_rotate) { hadamard256(v, ll); apply_signs(v, ll); }
-  if (!live) return;
-  const size_t e0 = (size_t)row * KV8_HD + 4 * ll;
-  #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    uint2 g = make_uint2(0u, 0u);
-    if (gate) g = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(gate) + e0 + 32 * k);
-    const uint16_t gb[4] = {(uint16_t)g.x, (uint16_t)(g.x >> 16), (uint16_t)g.y, (uint16_t)(g.y >> 16)};
-    uint32_t w[4];
+  if (inverse_rotate) {                                    // stages h = 1 ... 128 in order: lower index a + b, upper lower - upper
     #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float y = kv8_round(DT, v[4 * k + i]);
-      if (gate) y = kv8_gated<DT>(y, DT == YSKN_KV4_F16 ? h2f(gb[i]) : bf2f(gb[i]));
-      w[i] = act_store16<DT>(y);
+    for (int rb = 1; rb < 4; rb *= 2)                      // h = 1, 2
+      #pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (!(i & rb)) { const float lo = v[i], up = v[i + rb]; v[i] = __fadd_rn(lo, up); v[i + rb] = __fsub_rn(lo, up); }
+    #pragma unroll
+    for (int m = 1; m < 32; m *= 2) {                      // h = 4 ... 64: the lanes
+      const float flip = (lane & m) ? -1.f : 1.f;          // the product is exact: one rounding, as of the sum
+      #pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = fmaf(v[i], flip, __shfl_xor_sync(0xffffffffu, v[i], m));
     }
-    *reinterpret_cast<uint2*>(o16 + e0 + 32 * k) = make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+    const int w = lane >> 3, b = 4 * (lane & 7);
+    const uint32_t sg[2] = {c_signs.w[w] >> b, c_signs.w[w + 4] >> b};
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {                          // h = 128, then 1/16 and the signs
+      const float lo = v[i], up = v[i + 4];
+      v[i] = __fmul_rn(__fadd_rn(lo, up), __uint_as_float(0x3d800000u | (((sg[0] >> i) & 1u) << 31)));
+      v[i + 4] = __fmul_rn(__fsub_rn(lo, up), __uint_as_float(0x3d800000u | (((sg[1] >> i) & 1u) << 31)));
+    }
+  }
+  auto pack = [](float lo, float hi) {                     // two values rounded to the output type
+    uint32_t d;
+    if (DT == YSKN_KV4_BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+  };
+  auto low = [](uint32_t d) { return DT == YSKN_KV4_BF16 ? __uint_as_float(d << 16) : h2f((uint16_t)d); };
+  auto high = [](uint32_t d) { return DT == YSKN_KV4_BF16 ? __uint_as_float(d & 0xffff0000u) : h2f((uint16_t)(d >> 16)); };
+  auto sigm = [](float gt) { return __frcp_rn(__fadd_rn(1.f, expf(-gt))); };
+  #pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t u[2] = {pack(v[4 * h], v[4 * h + 1]), pack(v[4 * h + 2], v[4 * h + 3])};
+    if (gate) {                                            // y * sigmoid(gate): each factor and the product rounded (src/q35_kernels.cu:1423-1424)
+      const uint32_t gg[2] = {g[h].x, g[h].y};
+      #pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t sg = pack(sigm(low(gg[i])), sigm(high(gg[i])));
+        u[i] = pack(__fmul_rn(low(u[i]), low(sg)), __fmul_rn(high(u[i]), high(sg)));
+      }
+    }
+    *reinterpret_cast<uint2*>(o16 + e0 + 128 * h) = make_uint2(u[0], u[1]);
   }
 }
 
 template <int DT>
 int launch_kv8_combine_dt(const float* pm, const float* pl, const float* pacc, int S, int M, int nh, const void* gate, uint16_t* o16, int inverse_rotate, cudaStream_t st) {
-  // The row form reads 16-byte pieces and wants enough rows to fill the GPU: with up to four splits and at least 2,048 rows (half a
-  // block of 32 rows per SM) it wins; a few long sums want the block form's parallel loads.
+  // The form of a warp per row wants enough rows: up to one block of 1,024 threads per SM the block form's parallel loads win (96 rows of 37 splits 3.1
+  // against 4.9 us), beyond it its blocks queue up (192 rows: 37 splits 5.5 against 5.0, 18 splits 5.1 against 3.9).  It reads 16-byte pieces.
   const long long rows = (long long)M * nh;
   const bool aligned = !((((uintptr_t)pacc) & 15) | (((uintptr_t)o16 | (uintptr_t)gate) & 7));
-  if (S <= 4 && rows >= 2048 && aligned)
-    return launch_pdl("kv8_combine_rows_kernel", kv8_combine_rows_kernel<DT>, dim3((unsigned)((rows + 31) / 32)), 256, 0, st, pm, pl, pacc, S, nh, rows, gate, o16, inverse_rotate);
+  if (rows > 148 && aligned)
+    return launch_pdl("kv8_combine_rows_kernel", S == 1 ? kv8_combine_rows_kernel<DT, true> : kv8_combine_rows_kernel<DT, false>, dim3((unsigned)((rows + 3) / 4)), 128, 0, st,
+                      pm, pl, pacc, S, nh, rows, gate, o16, inverse_rotate);
   return launch_pdl("kv8_combine_kernel", kv8_combine_kernel<DT>, dim3(nh, M), KV8_CQ * 256, 0, st, pm, pl, pacc, S, nh, gate, o16, inverse_rotate);
 }
 
