@@ -362,25 +362,26 @@ __device__ __forceinline__ void tc_prefetch_l2(const void* p) { asm volatile("pr
 __device__ __forceinline__ void tc_sts128(uint32_t a, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-// Queries of one CTA (128 operand rows = (token, head) pairs) as fp16 rows in the swizzled Q blocks; rows without a query are zero.
+// Queries of one CTA (operand rows = (token, head) pairs) as fp16 rows in the swizzled Q blocks.  Rows of the tile beyond its tokens keep what the shared memory
+// held: what they yield is used nowhere.
 // PAIRS: chunks in the order of tc_row_to_pairs.  Thread t of nt; eight 16-byte loads are in flight per thread before the first one is converted.
 template <int HD, bool PAIRS>
 __device__ __forceinline__ void tc_stage_q(uint32_t sq, int q_block, const uint16_t* q16, bool bf16, int tok0, int G, int TOK, int M, int nh, int head0,
                                            int t, int nt) {
   constexpr int NW = HD / 8, B = 8;
   #pragma unroll 1
-  for (int base = t; base < 128 * NW; base += B * nt) {
+  for (int base = t; base < TOK * G * NW; base += B * nt) {
     uint4 u[B];
     #pragma unroll
     for (int b = 0; b < B; ++b) {
       const int it = base + b * nt, row = it / NW, w = it % NW, tk = tok0 + row / G;
       u[b] = make_uint4(0u, 0u, 0u, 0u);
-      if (it < 128 * NW && row < TOK * G && tk < M) u[b] = tc_ldg128(q16 + ((size_t)tk * nh + head0 + row % G) * HD + 8 * w);
+      if (it < TOK * G * NW && tk < M) u[b] = tc_ldg128(q16 + ((size_t)tk * nh + head0 + row % G) * HD + 8 * w);
     }
     #pragma unroll
     for (int b = 0; b < B; ++b) {
       const int it = base + b * nt, row = it / NW, w = it % NW;
-      if (it >= 128 * NW) break;
+      if (it >= TOK * G * NW) break;
       uint32_t o4[4] = {u[b].x, u[b].y, u[b].z, u[b].w};
       if (bf16) {
         #pragma unroll
@@ -464,7 +465,7 @@ template <int HD> struct TcLay {
 };
 
 struct TcP {
-  const int* d_pos; int M, splits, G, nh, max_ctx, ks_rows; float qscale;
+  const int* d_pos; int M, splits, G, tpc, nh, max_ctx, ks_rows; float qscale;
   float* pm; float* pl; float* pacc;
   uint16_t* o16; const uint16_t* bv;                       // splits == 1 and o16 set: store the finished rows, no partials
   yskn_kv_layer kv; const float* rope; int rd;             // the fused form reads the packed cache itself
@@ -498,6 +499,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sb = s_u32(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nquad = (P.tpc * P.G + 31) / 32;                         // quadrants of 32 rows that hold queries: softmax warps of the others have no part
   const uint32_t rank = cluster_ctarank();                           // 0 = leader: issues the MMAs, owns the "full"/"ready" barriers
   // barriers (8 bytes each), same offsets in both CTAs:
   //   leader's copy only: kfull[NK] vfull[NV] pready[2] phalf[2] qfull     each CTA's copy: kempty[NK] vempty[NV] sready[2] pvdone[2]
@@ -514,13 +516,13 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     for (int i = 0; i < L::NK; ++i) { bar_init(b_kfull + 8 * i, FUSED ? 2 * TC_KW : 1); bar_init(b_kempty + 8 * i, 1); }
     for (int i = 0; i < L::NV; ++i) { bar_init(b_vfull + 8 * i, FUSED ? 2 * TC_VW : 1); bar_init(b_vempty + 8 * i, 1); }
     for (int i = 0; i < 2; ++i) { bar_init(b_sready + 8 * i, 1); bar_init(b_pvdone + 8 * i, 1); }
-    // P of a tile: all softmax warps of both CTAs in the converting forms; the four of the tile's warpgroup otherwise, half of the keys at a time
-    for (int i = 0; i < 2; ++i) { bar_init(b_pready + 8 * i, FUSED ? 2 * TC_SW : TC_SW); bar_init(b_phalf + 8 * i, TC_SW); }
+    // P of a tile: all softmax warps with queries of both CTAs in the converting forms; those of the tile's warpgroup otherwise, half of the keys at a time
+    for (int i = 0; i < 2; ++i) { bar_init(b_pready + 8 * i, (FUSED ? 4 : 2) * nquad); bar_init(b_phalf + 8 * i, 2 * nquad); }
     bar_init(b_q, STAGED_Q ? 2 * TC_SW : 1);                         // queries that are converted or reordered are staged by the softmax warps
     *s_abort = 0;
-    for (int i = 0; i < 128; ++i) reinterpret_cast<volatile uint32_t*>(smem + L::OFF_XCH + 2 * 2 * 128 * 4)[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (threadIdx.x < 128) reinterpret_cast<volatile uint32_t*>(smem + L::OFF_XCH + 2 * 2 * 128 * 4)[threadIdx.x] = 0;   // tags of the exchange
   if (warp == TC_SW + 1) {                                           // the same warp of both CTAs allocates for the pair
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sb + L::OFF_BAR + 184), "n"(L::TM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -540,7 +542,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   // ---- geometry: uniform over the pair except tok0
-  const int G = P.G, TOK = 128 / G, kvh = blockIdx.z, S = P.splits, split = blockIdx.y;
+  const int G = P.G, TOK = P.tpc, kvh = blockIdx.z, S = P.splits, split = blockIdx.y;
   const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;               // heaviest query tiles first; gridDim.x is even
   const int tok0 = qt * TOK;                                         // this CTA's first token
   const int tokA = (qt & ~1) * TOK;                                  // the pair's first token (always < M)
@@ -562,7 +564,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     // Every copy reports to the leader's "full" barrier; the leader posts the byte count of both CTAs' parts.
     if (lane == 0 && n > 0) {
       if (!STAGED_Q) {
-        if (rank == 0) bar_expect_tx(b_q, 2 * L::KBLK * G * TOK * 128);
+        if (rank == 0) bar_expect_tx(b_q, 2 * L::KBLK * G * (128 / G) * 128);   // whole boxes: tokens beyond this CTA's come along unused
         for (int kb = 0; kb < L::KBLK; ++kb) tma_load_4d_pair(sb + L::OFF_Q + kb * L::Q_BLOCK, &mapQ, 64 * kb, 0, kvh, tok0, lead_q);
       }
       int kit = 0; bool ok = true;
@@ -684,42 +686,37 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     if (n > 0 && is_k) {
       // ------------------------------------------------------------------- K role
       if constexpr (I8) {
-        constexpr int NKI = ((TC_BN / 2) * 16 + NKT - 1) / NKT;      // 64 keys x 16 chunks over the K threads
-        // The items of all tiles form one stream (NKI per tile); two are in flight ahead of the one being converted.  Rolled
-        // loops: the kernel's code has to stay inside the instruction cache.
-        auto k8_load = [&](int q, I8In& I) {                         // q-th item of this thread's stream
-          const int it = ct + NKT * (q % NKI), t = (j0 + q / NKI) * TC_BN + (TC_BN / 2) * (int)rank + (it >> 4);
-          if (q < n * NKI && it < (TC_BN / 2) * 16 && t < P.max_ctx) {
-            I.w = tc_ldg128(P.k8 + (row0 + t) * HD + 16 * (it & 15));
-            I.s = tc_ldg32(P.ks8 + row0 + t);
-          }
+        constexpr int NKI = (TC_BN / 2) * 16 / NKT;                  // 64 keys x 16 chunks over the K threads
+        static_assert(NKI * NKT == (TC_BN / 2) * 16, "every K thread has the same number of items");
+        // A thread keeps its items of a whole tile in registers; each is requested again, for the next tile, as soon as it has been converted.
+        auto k8_load = [&](int i, int u, I8In& I) {
+          const int it = ct + NKT * u, t = min((j0 + min(i, n - 1)) * TC_BN + (TC_BN / 2) * (int)rank + (it >> 4), P.max_ctx - 1);
+          I.w = tc_ldg128(P.k8 + (row0 + t) * HD + 16 * (it & 15));
+          I.s = tc_ldg32(P.ks8 + row0 + t);
         };
         auto k8_prefetch = [&](int tk) {                             // L2 prefetch of a half tile: 64 rows of 256 bytes, two lines each
           if (tk >= P.max_ctx) return;
           tc_prefetch_l2(P.k8 + (row0 + tk + (ct >> 1)) * HD + 128 * (ct & 1));
           if (ct < 2) tc_prefetch_l2(P.ks8 + row0 + tk + 32 * ct);
         };
-        I8In cur, n1, n2;
-        k8_load(0, cur); k8_load(1, n1);
+        I8In cur[NKI];
+        #pragma unroll
+        for (int u = 0; u < NKI; ++u) k8_load(0, u, cur[u]);
         if (n > 1) k8_prefetch((j0 + 1) * TC_BN + (TC_BN / 2) * (int)rank);
-        int q = 0;
         for (int i = 0; i < n && ok; ++i) {
           const int tk0 = (j0 + i) * TC_BN + (TC_BN / 2) * (int)rank, st = i % L::NK;
           const uint32_t sk = sb + L::OFF_K + st * L::K_HALF;
           if (i + 2 < n) k8_prefetch(tk0 + 2 * TC_BN);
           stage_wait(b_kempty + 8 * st, i, L::NK);
           if (!ok) break;
-          #pragma unroll 1
-          for (int u = 0; u < NKI; ++u, ++q) {
-            k8_load(q + 2, n2);
+          #pragma unroll
+          for (int u = 0; u < NKI; ++u) {
             const int it = ct + NKT * u, k = it >> 4, c = it & 15;
-            if (it < (TC_BN / 2) * 16) {
-              uint4 lo, hi;
-              i8_convert(cur, tk0 + k < P.max_ctx, lo, hi);
-              tc_sts128(sk + (c >> 2) * L::K_BLOCK + k * 128 + ((((2 * c) & 7) ^ (k & 7)) << 4), lo);
-              tc_sts128(sk + (c >> 2) * L::K_BLOCK + k * 128 + ((((2 * c + 1) & 7) ^ (k & 7)) << 4), hi);
-            }
-            cur = n1; n1 = n2;
+            uint4 lo, hi;
+            i8_convert(cur[u], tk0 + k < P.max_ctx, lo, hi);
+            tc_sts128(sk + (c >> 2) * L::K_BLOCK + k * 128 + ((((2 * c) & 7) ^ (k & 7)) << 4), lo);
+            tc_sts128(sk + (c >> 2) * L::K_BLOCK + k * 128 + ((((2 * c + 1) & 7) ^ (k & 7)) << 4), hi);
+            k8_load(i + 1, u, cur[u]);
           }
           publish(lead_kfull + 8 * st);
         }
@@ -730,48 +727,52 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       const uint32_t* kq32 = reinterpret_cast<const uint32_t*>(P.kv.kq);
       auto k_addr = [&](uint32_t sk, int w, int k) { return sk + (w >> 3) * L::K_BLOCK + k * 128 + (((w & 7) ^ (k & 7)) << 4); };
       const TcNib nk = tc_nib_consts();
-      // Work of a tile in warp items.  Plain: 32 (word column, octet of keys) pairs, x = col + npl * octet, so that consecutive lanes take
-      // consecutive columns; warp w takes items w, w + 4.  Rotary (up to four word pairs per key): nrp pairs x 32 / nrp keys of one group, nrp items
-      // per group; for a 64-channel rotary part six plain and eight rotary items share out as 2 + 1, 2 + 1, 1 + 3, 1 + 3.
-      const int wq = ct >> 5, np1 = npl > 0 ? npl : 1, nplain = npl * 8;
-      struct PlainIn { uint32_t w[8]; uint4 s, z; };
-      int pg[2], ps[2], pd[2];                                       // a lane's two items: word offset, scale offset, stage offset
+      // Each of the four warps has 16 of the half tile's keys, which lie in one 32-token group.  Plain item: a word column of four of them (npl columns x 4
+      // quads of keys over 32 lanes; a column's scales serve four words).  Rotary item: a word pair (p, p + nrp) of one key; for a 64-channel rotary part
+      // two per lane beside three plain ones.  A thread keeps the words, scales and rope entries of its items of a whole tile in registers, and requests
+      // each again for the next tile as soon as it has been used: requests made one item ahead were waited for in every phase (a tile took the K warps 5.5 k
+      // cycles for 350 instructions each).
+      constexpr int NPU = NWD / 8;                                   // plain items of a lane when nothing is rotated
+      const int wq = ct >> 5, np1 = npl > 0 ? npl : 1, wkey = 16 * wq;
+      struct PlainIn { uint32_t w[4]; uint4 s, z; };
+      uint32_t pk[NPU], ps[NPU], pd[NPU];                            // byte offsets of a lane's items: first word, scales, stage
       #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int x = 32 * (wq + TC_KW * u) + lane, col = nrw + x % np1, key = 8 * (x / np1);
-        pg[u] = x < nplain ? key * (HD / 8) + col : -1; ps[u] = (key >> 5) * HD + 8 * col;
-        pd[u] = (col >> 3) * L::K_BLOCK + key * 128 + ((col & 7) << 4);
+      for (int u = 0; u < NPU; ++u) {
+        const int x = min(lane + 32 * u, 4 * np1 - 1);               // lanes beyond the last item repeat it
+        const int col = npl > 0 ? nrw + x % np1 : 0, key = wkey + 4 * (x / np1);    // key is a multiple of 4: its four rows swizzle by (key & 4) + e
+        pk[u] = key * (HD / 2) + 4 * col; ps[u] = (key >> 5) * HD * 2 + 16 * col;
+        pd[u] = (col >> 3) * L::K_BLOCK + key * 128 + (((col & 7) ^ (key & 4)) << 4);
       }
-      const int pn = 32 * wq >= nplain ? 0 : (32 * (wq + TC_KW) < nplain ? 2 : 1);       // items of this warp
-      static_assert(NWD * 8 <= 32 * TC_KW * 2, "two plain items per warp cover a half tile");
       auto tile_key = [&](int i) { return (j0 + i) * TC_BN + (TC_BN / 2) * (int)rank; };   // first key of this CTA's half of K tile i
-      auto plain_load = [&](int i, int u, PlainIn& I) {
-        const int tk = tile_key(i), off = u ? pg[1] : pg[0];
-        if (i < n && off >= 0 && tk < P.max_ctx) {
-          const uint32_t* src = kq32 + (row0 + tk) * (HD / 8) + off;
-          #pragma unroll
-          for (int e = 0; e < 8; ++e) I.w[e] = tc_ldg32(src + e * (HD / 8));
-          const size_t gb = (grp0 + tk / 32) * HD + (u ? ps[1] : ps[0]);
-          I.s = tc_ldg128(P.kv.kscale + gb); I.z = tc_ldg128(P.kv.kzero + gb);
-        }
+      // Loads are never skipped: past the last tile, or for a half tile outside the cache, they take keys that are there and nobody uses.  (A load under a
+      // branch merges two values at the loop's end, and the copy waits for the load.)
+      auto load_key = [&](int i) { return min(tile_key(min(i, n - 1)), P.max_ctx - TC_BN / 2); };
+      struct KAt { const uint8_t* kq; const uint8_t* ks; const uint8_t* kz; const uint8_t* rope; };   // a half tile in the cache's arrays
+      auto k_at = [&](int i) {
+        const size_t t = row0 + load_key(i);
+        const size_t gb = (t / 32) * (HD * 2);
+        return KAt{reinterpret_cast<const uint8_t*>(P.kv.kq) + t * (HD / 2), reinterpret_cast<const uint8_t*>(P.kv.kscale) + gb,
+                   reinterpret_cast<const uint8_t*>(P.kv.kzero) + gb, reinterpret_cast<const uint8_t*>(P.rope) + (size_t)load_key(i) * half * 8};
+      };
+      auto plain_load = [&](const KAt& at, int u, PlainIn& I) {
+        const uint8_t* src = at.kq + pk[u];
+        #pragma unroll
+        for (int e = 0; e < 4; ++e) I.w[e] = tc_ldg32(src + e * (HD / 2));
+        I.s = tc_ldg128(at.ks + ps[u]); I.z = tc_ldg128(at.kz + ps[u]);
       };
       auto plain_store = [&](int u, uint32_t sk, const PlainIn& I) {
-        if ((u ? pg[1] : pg[0]) < 0) return;
-        const uint32_t base = sk + (u ? pd[1] : pd[0]);                // keys are a multiple of 8 further on: key e swizzles by e
+        const uint32_t base = sk + pd[u];
         uint32_t sc[4], zz[4];
         tc_row_to_pairs(I.s, sc); tc_row_to_pairs(I.z, zz);
+        uint4 out[4];                                                // four words converted, then four stores: independent chains interleave
         #pragma unroll
-        for (int h = 0; h < 8; h += 4) {                               // four words converted, then four stores: independent chains interleave
-          uint4 out[4];
-          #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            uint32_t nb[4];
-            tc_nibs(I.w[h + e], nb, nk);
-            out[e] = make_uint4(tc_hfma2(nb[0], sc[0], zz[0]), tc_hfma2(nb[1], sc[1], zz[1]), tc_hfma2(nb[2], sc[2], zz[2]), tc_hfma2(nb[3], sc[3], zz[3]));
-          }
-          #pragma unroll
-          for (int e = 0; e < 4; ++e) tc_sts128((base ^ (uint32_t)((h + e) << 4)) + (h + e) * 128, out[e]);
+        for (int e = 0; e < 4; ++e) {
+          uint32_t nb[4];
+          tc_nibs(I.w[e], nb, nk);
+          out[e] = make_uint4(tc_hfma2(nb[0], sc[0], zz[0]), tc_hfma2(nb[1], sc[1], zz[1]), tc_hfma2(nb[2], sc[2], zz[2]), tc_hfma2(nb[3], sc[3], zz[3]));
         }
+        #pragma unroll
+        for (int e = 0; e < 4; ++e) tc_sts128((base ^ (uint32_t)(e << 4)) + e * 128, out[e]);
       };
       struct RotIn { uint32_t wa, wb; uint4 sa, za, sb, zb; uint4 r[4]; };   // shadow items keep their two fp16 rows in sa, za
       // one rotary item = key k, word pair (p, p + nrp): 8 + 8 channels (c, c + rd/2) and their 8 (cos, sin) pairs
@@ -821,32 +822,28 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       auto zero_k = [&](uint32_t sk) {                               // a half tile past max_ctx: nothing to read
         for (int it = ct; it < (TC_BN / 2) * NWD; it += NKT) tc_sts128(k_addr(sk, it % NWD, it / NWD), make_uint4(0u, 0u, 0u, 0u));
       };
-      // Rotary items in the compact mapping (rotary width of at most 64 channels): a warp stays in one 32-key group, so the group's scale / zero
-      // chunks are loaded once per tile.  Wider rotary parts take the items one after the other (rot_load / rot_store).
+      // Rotary items in the compact mapping (rotary width of at most 64 channels): a lane keeps its word pair.  Wider rotary parts take the items one after
+      // the other (rot_load / rot_store).
+      constexpr int NRU = 2;                                         // 16 keys x nrp pairs over 32 lanes, nrp <= 4
       const bool compact = nrp >= 1 && nrp <= 4;
-      const int rlight = nrp == 4 ? 1 : nrp >> 1;                    // rotary items of warps 0 and 1 (group = warp & 1); 2 and 3 take the rest
-      const int r0 = wq < 2 ? 0 : rlight, rn = !compact ? 0 : (wq < 2 ? rlight : nrp - rlight);
-      const int cp = lane & (nrp - 1), cg = wq & 1, cstep = compact ? 32 >> lp : 0, cc = compact ? cstep * r0 + (lane >> lp) : 0;
+      const int cp = lane & (nrp - 1), cstep = compact ? 32 >> lp : 0, cc = compact ? lane >> lp : 16;
       struct RotS { uint4 sa, za, sb, zb; };                         // the group's scale / zero chunks of the two words
       struct RotI { uint32_t wa, wb; uint4 r[4]; };                  // one key: the two words and the 8 (cos, sin) pairs
-      auto rots_load = [&](int tk0, RotS& R) {
-        const size_t gb = (grp0 + tk0 / 32 + cg) * HD;
-        R.sa = tc_ldg128(P.kv.kscale + gb + 8 * cp); R.za = tc_ldg128(P.kv.kzero + gb + 8 * cp);
-        R.sb = tc_ldg128(P.kv.kscale + gb + 8 * (cp + nrp)); R.zb = tc_ldg128(P.kv.kzero + gb + 8 * (cp + nrp));
+      const uint32_t rs0 = (wq >> 1) * HD * 2 + 16 * cp, rk0 = (wkey + (cc & 15)) * (HD / 2) + 4 * cp, rr0 = ((wkey + (cc & 15)) * half + 8 * cp) * 8;
+      auto rots_load = [&](const KAt& at, RotS& R) {
+        R.sa = tc_ldg128(at.ks + rs0); R.za = tc_ldg128(at.kz + rs0);
+        R.sb = tc_ldg128(at.ks + rs0 + 16 * nrp); R.zb = tc_ldg128(at.kz + rs0 + 16 * nrp);
       };
-      auto roti_load = [&](int i, int u, RotI& R) {                  // item u of this warp in tile i
-        const int tk = tile_key(i);
-        if (i < n && u < rn && tk < P.max_ctx) {
-          const int t = tk + 32 * cg + cc + cstep * u;
-          const uint32_t* rowp = kq32 + (row0 + t) * (HD / 8);
-          R.wa = tc_ldg32(rowp + cp); R.wb = tc_ldg32(rowp + cp + nrp);
-          const float* rp = P.rope + ((size_t)t * half + 8 * cp) * 2;
-          #pragma unroll
-          for (int e = 0; e < 4; ++e) R.r[e] = tc_ldg128(rp + 4 * e);
-        }
+      auto roti_load = [&](const KAt& at, int u, RotI& R) {          // item u of this lane: key cc + cstep u of the warp's sixteen
+        const uint8_t* rowp = at.kq + rk0 + u * cstep * (HD / 2);
+        R.wa = tc_ldg32(rowp); R.wb = tc_ldg32(rowp + 4 * nrp);
+        const uint8_t* rp = at.rope + rr0 + u * cstep * half * 8;
+        #pragma unroll
+        for (int e = 0; e < 4; ++e) R.r[e] = tc_ldg128(rp + 16 * e);
       };
       auto roti_store = [&](int u, uint32_t sk, const RotS& Sc, const RotI& R) {
-        const int p = cp, q = cp + nrp, k = 32 * cg + cc + cstep * u;
+        if (cc + cstep * u >= 16) return;
+        const int p = cp, q = cp + nrp, k = wkey + cc + cstep * u;
         uint32_t sa[4], za[4], sb4[4], zb[4], na[4], nb[4], a[4], b[4], lo[4], hi[4];
         tc_row_to_pairs(Sc.sa, sa); tc_row_to_pairs(Sc.za, za); tc_row_to_pairs(Sc.sb, sb4); tc_row_to_pairs(Sc.zb, zb);
         tc_nibs(R.wa, na, nk); tc_nibs(R.wb, nb, nk);
@@ -865,10 +862,19 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         tc_sts128(k_addr(sk, p, k), make_uint4(lo[0], lo[1], lo[2], lo[3]));
         tc_sts128(k_addr(sk, q, k), make_uint4(hi[0], hi[1], hi[2], hi[3]));
       };
-      PlainIn pc, pnx;                                               // plain stream: current item, next item
-      RotI rc, rcn;                                                  // rotary stream (compact mapping)
-      plain_load(0, 0, pc);
-      roti_load(0, 0, rc);
+      PlainIn pc[NPU];
+      RotI rc[NRU];
+      RotS rs;
+      {
+        const KAt at = k_at(0);
+        #pragma unroll
+        for (int u = 0; u < NPU; ++u) plain_load(at, u, pc[u]);
+        if (compact) {
+          rots_load(at, rs);
+          #pragma unroll
+          for (int u = 0; u < NRU; ++u) if (cstep * u < 16) roti_load(at, u, rc[u]);
+        }
+      }
       int kit = 0;
       // L2 prefetch of a half tile two tiles ahead (64 packed rows, the scale and zero rows of its two groups; one line per
       // thread), so that the register loads a phase ahead find their lines in L2
@@ -886,35 +892,25 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         const int tk0 = tile_key(i);
         const bool kin = tk0 < P.max_ctx;                            // max_ctx is a multiple of 64: the half tile is inside or outside as a whole
         if (i + 2 < n) k_prefetch(tk0 + 2 * TC_BN);
-        // ---- item 1: the int4 keys.  The converters never idle, so a request must be made a whole phase before its data
-        //      is used: each plain item is requested while the one before it is converted (the first of a tile during the
-        //      previous tile's last plain item, i.e. a whole rotary phase ahead), each rotary item likewise (the first of a
-        //      tile a whole plain phase ahead), the tile's rotary scales before its plain phase.  Rolled loops, one expansion
-        //      of each conversion: the kernel's code has to stay inside the instruction cache.
+        // ---- item 1: the int4 keys
         {
           const int st = kit % L::NK;
           const uint32_t sk = sb + L::OFF_K + st * L::K_HALF;
-          RotS RS;
-          if (kin && compact) rots_load(tk0, RS);
           stage_wait(b_kempty + 8 * st, kit, L::NK);
           if (!ok) break;
           if (!kin) zero_k(sk);                                      // only the last tile of the last split can lie outside: nothing is loaded after it
           else {
-            #pragma unroll 1
-            for (int u = 0; u < pn; ++u) {
-              const bool more = u + 1 < pn;
-              plain_load(more ? i : i + 1, more ? 1 : 0, pnx);
-              plain_store(u, sk, pc);
-              pc = pnx;
+            const KAt at = k_at(i + 1);
+            #pragma unroll
+            for (int u = 0; u < NPU; ++u) {
+              if (32 * u < 4 * npl) { plain_store(u, sk, pc[u]); plain_load(at, u, pc[u]); }
             }
             if (compact) {
-              #pragma unroll 1
-              for (int u = 0; u < rn; ++u) {
-                const bool more = u + 1 < rn;
-                roti_load(more ? i : i + 1, more ? u + 1 : 0, rcn);
-                roti_store(u, sk, RS, rc);
-                rc = rcn;
+              #pragma unroll
+              for (int u = 0; u < NRU; ++u) {
+                if (cstep * u < 16) { roti_store(u, sk, rs, rc[u]); roti_load(at, u, rc[u]); }
               }
+              rots_load(at, rs);
             } else {
               RotIn R1;
               #pragma unroll 1
@@ -932,17 +928,24 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           if (!ok) break;
           if (!kin) zero_k(sk);
           else {
-            // plain channels: a copy, kept as a small loop (edge tiles are few; the kernel's code must stay inside the
-            // instruction cache)
+            // plain channels: a copy, four loads in flight (one after the other they were 6 us of the last split)
             #pragma unroll 1
-            for (int it = ct; it < (TC_BN / 2) * NWD; it += NKT) {
-              const int k = it / NWD, w = it % NWD;
-              if (w < nrw) continue;
-              uint4 x = make_uint4(0u, 0u, 0u, 0u);
-              if (tk0 + k < end) x = tc_ldg128(P.kv.kshadow + (row0 + tk0 + k) * HD + 8 * w);
-              uint32_t o4[4];
-              tc_row_to_pairs(x, o4);
-              tc_sts128(k_addr(sk, w, k), make_uint4(o4[0], o4[1], o4[2], o4[3]));
+            for (int base = ct; base < (TC_BN / 2) * NWD; base += 4 * NKT) {
+              uint4 x[4];
+              #pragma unroll
+              for (int b = 0; b < 4; ++b) {
+                const int it = base + b * NKT, k = it / NWD, w = it % NWD;
+                x[b] = make_uint4(0u, 0u, 0u, 0u);
+                if (it < (TC_BN / 2) * NWD && w >= nrw && tk0 + k < end) x[b] = tc_ldg128(P.kv.kshadow + (row0 + tk0 + k) * HD + 8 * w);
+              }
+              #pragma unroll
+              for (int b = 0; b < 4; ++b) {
+                const int it = base + b * NKT, k = it / NWD, w = it % NWD;
+                if (it >= (TC_BN / 2) * NWD || w < nrw) continue;
+                uint32_t o4[4];
+                tc_row_to_pairs(x[b], o4);
+                tc_sts128(k_addr(sk, w, k), make_uint4(o4[0], o4[1], o4[2], o4[3]));
+              }
             }
             RotIn R1;
             #pragma unroll 1
@@ -958,38 +961,35 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       if constexpr (I8) {
         constexpr int NVI8 = (TC_BN * 8 + NVT - 1) / NVT;            // 128 keys x 8 chunks (this CTA's 128 channels) over the V threads
         const int vt = ct - NKT;
-        auto v8_load = [&](int q, I8In& I) {                         // q-th item of this thread's stream (NVI8 per tile)
-          const int it = vt + NVT * (q % NVI8), t = (j0 + q / NVI8) * TC_BN + (it >> 3);
-          if (q < n * NVI8 && it < TC_BN * 8 && t < end) {
-            I.w = tc_ldg128(P.v8 + (row0 + t) * HD + 128 * (int)rank + 16 * (it & 7));
-            I.s = tc_ldg32(P.vs8 + row0 + t);
-          }
+        auto v8_load = [&](int i, int u, I8In& I) {                  // item u of this thread in tile i
+          const int it = vt + NVT * u, t = min((j0 + min(i, n - 1)) * TC_BN + (it >> 3), end - 1);
+          I.w = tc_ldg128(P.v8 + (row0 + t) * HD + 128 * (int)rank + 16 * (it & 7));
+          I.s = tc_ldg32(P.vs8 + row0 + t);
         };
         auto v8_prefetch = [&](int j) {                              // L2 prefetch of a tile's 128 half rows (one line each) and scales
           for (int x = vt; x < TC_BN; x += NVT) if (j * TC_BN + x < end) tc_prefetch_l2(P.v8 + (row0 + j * TC_BN + x) * HD + 128 * (int)rank);
           if (vt < 4 && j * TC_BN + 32 * vt < end) tc_prefetch_l2(P.vs8 + row0 + j * TC_BN + 32 * vt);
         };
-        I8In cur, n1, n2;
-        v8_load(0, cur); v8_load(1, n1);
+        I8In cur[NVI8];
+        #pragma unroll
+        for (int u = 0; u < NVI8; ++u) v8_load(0, u, cur[u]);
         if (n > 1) v8_prefetch(j0 + 1);
-        int q = 0;
         for (int i = 0; i < n && ok; ++i) {
           const int j = j0 + i, st = i % L::NV;
           const uint32_t sv = sb + L::OFF_V + st * L::V_HALF;
           if (i + 2 < n) v8_prefetch(j + 2);
           stage_wait(b_vempty + 8 * st, i, L::NV);
           if (!ok) break;
-          #pragma unroll 1
-          for (int u = 0; u < NVI8; ++u, ++q) {
-            v8_load(q + 2, n2);
+          #pragma unroll
+          for (int u = 0; u < NVI8; ++u) {
             const int it = vt + NVT * u, k = it >> 3, c = it & 7;
             if (it < TC_BN * 8) {
               uint4 lo, hi;
-              i8_convert(cur, j * TC_BN + k < end, lo, hi);          // tokens that do not exist yet read as zero
+              i8_convert(cur[u], j * TC_BN + k < end, lo, hi);       // tokens that do not exist yet read as zero
               tc_sts128(sv + (c >> 2) * L::V_BLOCK + k * 128 + ((((2 * c) & 7) ^ (k & 7)) << 4), lo);
               tc_sts128(sv + (c >> 2) * L::V_BLOCK + k * 128 + ((((2 * c + 1) & 7) ^ (k & 7)) << 4), hi);
             }
-            cur = n1; n1 = n2;
+            v8_load(i + 1, u, cur[u]);
           }
           publish(lead_vfull + 8 * st);
         }
@@ -1000,25 +1000,27 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       const int vt = ct - NKT, part = vt % PARTS, vk0 = vt / PARTS;  // item u of this thread in a tile: key vk0 + VSTEP u, its part of the half row
       const TcNib nk = tc_nib_consts();
       struct VIn { uint4 w; uint32_t s, z; };
-      // The items of all tiles form one stream (tile by tile, NVI items each); two items are in flight ahead of the one being
-      // converted.  A rolled loop: the lines are in L2 already (prefetched two tiles ahead), and small code matters more
-      // here than the last cycles of latency.
-      const uint8_t* vsrc = P.kv.vq + row0 * (HD / 2) + (HD / 4) * (int)rank + 16 * part;
-      int li = 0, lu = 0;                                            // tile and item of the next load
-      auto v_item_load = [&](VIn& I) {
-        const int k = vk0 + VSTEP * lu, t = (j0 + li) * TC_BN + k;
-        if (li < n && k < TC_BN && t < end) {
-          I.w = tc_ldg128(vsrc + (size_t)t * (HD / 2));
-          I.s = tc_ldg16(P.kv.vscale + row0 + t); I.z = tc_ldg16(P.kv.vzero + row0 + t);
-        }
-        if (++lu == NVI) { lu = 0; ++li; }
+      // As for K: the items of a whole tile in registers, each requested again for the next tile once it has been converted.
+      struct VAt { const uint8_t* q; const uint16_t* s; const uint16_t* z; int last; };     // a tile in the cache's arrays, its last token
+      auto v_at = [&](int i) {
+        const int t = (j0 + min(i, n - 1)) * TC_BN;
+        return VAt{P.kv.vq + (row0 + t) * (HD / 2) + (HD / 4) * (int)rank + 16 * part, P.kv.vscale + row0 + t, P.kv.vzero + row0 + t, end - 1 - t};
+      };
+      auto v_item_load = [&](const VAt& at, int u, VIn& I) {
+        const uint32_t k = (uint32_t)min(vk0 + VSTEP * u, at.last);
+        I.w = tc_ldg128(at.q + k * (HD / 2));
+        I.s = tc_ldg16(at.s + k); I.z = tc_ldg16(at.z + k);
       };
       auto v_prefetch = [&](int j) {                                 // L2 prefetch of a tile's half rows and per-token scales
         for (int x = vt; x < TC_BN; x += NVT) if (j * TC_BN + x < end) tc_prefetch_l2(P.kv.vq + (row0 + j * TC_BN + x) * (HD / 2) + (HD / 4) * (int)rank);
         if (vt < 4 && j * TC_BN + 64 * (vt & 1) < end) tc_prefetch_l2((vt & 2 ? P.kv.vzero : P.kv.vscale) + row0 + j * TC_BN + 64 * (vt & 1));
       };
-      VIn cur, n1, n2;
-      v_item_load(cur); v_item_load(n1);
+      VIn vin[NVI];
+      {
+        const VAt at = v_at(0);
+        #pragma unroll
+        for (int u = 0; u < NVI; ++u) v_item_load(at, u, vin[u]);
+      }
       if (n > 1) v_prefetch(j0 + 1);
       const uint32_t vdst = (part >> 1) * L::V_BLOCK + (4 * (part & 1) << 4);     // chunk 4*part + e of the half row = chunk (4 (part & 1)) ^ e of its block
       for (int i = 0; i < n && ok; ++i) {
@@ -1027,15 +1029,16 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         if (i + 2 < n) v_prefetch(j + 2);
         stage_wait(b_vempty + 8 * st, i, L::NV);
         if (!ok) break;
-        #pragma unroll 1
+        const VAt at = v_at(i + 1);
+        #pragma unroll
         for (int u = 0; u < NVI; ++u) {
-          v_item_load(n2);
+          VIn& cur = vin[u];
           const int k = vk0 + VSTEP * u;
           if (k < TC_BN) {
             // no branches inside an item: a token that does not exist yet gets scale = zero = 0 (nibbles are finite whatever
             // the word holds), and the four words are converted before the four stores, so their chains interleave
             const bool live = j * TC_BN + k < end;
-            const uint32_t s2 = live ? cur.s | (cur.s << 16) : 0u, z2 = live ? cur.z | (cur.z << 16) : 0u;
+            const uint32_t s2 = live ? __byte_perm(cur.s, 0u, 0x1010) : 0u, z2 = live ? __byte_perm(cur.z, 0u, 0x1010) : 0u;
             const uint32_t ww[4] = {cur.w.x, cur.w.y, cur.w.z, cur.w.w};
             uint4 out[4];
             #pragma unroll
@@ -1048,7 +1051,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
             #pragma unroll
             for (int e = 0; e < 4; ++e) tc_sts128(base ^ (uint32_t)(e << 4), out[e]);
           }
-          cur = n1; n1 = n2;
+          v_item_load(at, u, cur);
         }
         publish(lead_vfull + 8 * st);
       }
@@ -1073,6 +1076,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         if (lane == 0) bar_arrive_cluster(lead_q);
       }
     }
+    if (quad >= nquad) return;
     // The row's two threads swap one float per tile through shared memory: value first, then a sequence number the
     // partner polls (bounded, like every wait here; a named barrier could not give up).
     volatile float* xval = reinterpret_cast<volatile float*>(smem + L::OFF_XCH);
@@ -1280,41 +1284,67 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     if (ok && n > 0 && !bar_wait(b_pvdone + 8 * ((n - 1) & 1), ((n - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; }
     tc_fence_after();
     if constexpr (FUSED) { if (ok) l += swap_with_partner(l, n + 1); }   // the row's sum = the two halves' sums
-    if (ok && !*s_abort) {
+    if (__all_sync(0xffffffffu, ok && !*s_abort)) {
       const size_t pidx = ((size_t)tok * S + split) * P.nh + kvh * G + head;
       const bool direct = P.o16 != nullptr && S == 1;                // one split: this CTA holds the whole row, finish it here
       auto ocol = [](int c) { return FORM == 1 ? tc_col(c) : c; };   // the int4 form's V chunks keep their channels in pair order
       if (valid && !direct && hf == 0) { P.pm[pidx] = (n > 0 && m > -1e29f) ? m * TC_LN2 : -1e30f; P.pl[pidx] = n > 0 ? l : 0.f; }
-      #pragma unroll 1
-      for (int c = hf; c < HD / 32; c += 2) {
-        float o[32];
+      auto o_chunk = [&](int c, float (&o)[32]) {                    // 32 columns of this row's O
         if (n > 0) tmem_ld32(trow + L::TM_O + 32 * c, o);
         else {
           #pragma unroll
           for (int k = 0; k < 32; ++k) o[k] = 0.f;
         }
-        if (valid && direct) {                                       // y = round_f16(o / l) (+ V bias), as the merge kernel
-          const size_t oi = ((size_t)tok * P.nh + kvh * G + head) * HD + 32 * c;
-          uint32_t w[16];
-          #pragma unroll
-          for (int k = 0; k < 32; k += 2) {
-            float y0 = round_f16(o[ocol(k)] / l), y1 = round_f16(o[ocol(k + 1)] / l);
-            if (act_bf16) {
-              if (P.bv) { y0 = __fadd_rn(y0, bf2f(P.bv[kvh * HD + 32 * c + k])); y1 = __fadd_rn(y1, bf2f(P.bv[kvh * HD + 32 * c + k + 1])); }
-              w[k / 2] = (uint32_t)f2bf(y0) | ((uint32_t)f2bf(y1) << 16);
-              continue;
-            }
-            if (P.bv) { y0 = __fadd_rn(y0, h2f(P.bv[kvh * HD + 32 * c + k])); y1 = __fadd_rn(y1, h2f(P.bv[kvh * HD + 32 * c + k + 1])); }
-            w[k / 2] = (uint32_t)f2h(y0) | ((uint32_t)f2h(y1) << 16);
+      };
+      auto finish = [&](int c, const float (&o)[32]) {               // y = round_f16(o / l) (+ V bias), as the merge kernel
+        uint4* dst = reinterpret_cast<uint4*>(P.o16 + ((size_t)tok * P.nh + kvh * G + head) * HD + 32 * c);
+        uint32_t w[16];
+        #pragma unroll
+        for (int k = 0; k < 32; k += 2) {
+          float y0 = round_f16(o[ocol(k)] / l), y1 = round_f16(o[ocol(k + 1)] / l);
+          if (act_bf16) {
+            if (P.bv) { y0 = __fadd_rn(y0, bf2f(P.bv[kvh * HD + 32 * c + k])); y1 = __fadd_rn(y1, bf2f(P.bv[kvh * HD + 32 * c + k + 1])); }
+            w[k / 2] = (uint32_t)f2bf(y0) | ((uint32_t)f2bf(y1) << 16);
+            continue;
           }
-          uint4* dst = reinterpret_cast<uint4*>(P.o16 + oi);
-          #pragma unroll
-          for (int k = 0; k < 4; ++k) dst[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
-        } else if (valid) {
-          float4* dst = reinterpret_cast<float4*>(P.pacc + pidx * HD + 32 * c);
-          #pragma unroll
-          for (int k = 0; k < 8; ++k) dst[k] = make_float4(o[ocol(4 * k)], o[ocol(4 * k + 1)], o[ocol(4 * k + 2)], o[ocol(4 * k + 3)]);
+          if (P.bv) { y0 = __fadd_rn(y0, h2f(P.bv[kvh * HD + 32 * c + k])); y1 = __fadd_rn(y1, h2f(P.bv[kvh * HD + 32 * c + k + 1])); }
+          w[k / 2] = (uint32_t)f2h(y0) | ((uint32_t)f2h(y1) << 16);
         }
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) dst[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+      };
+      if (!FUSED && direct) {                                        // a loop of its own: as a branch of the one below it cost 1,000 rows 58 -> 60 us
+        #pragma unroll 1
+        for (int c = hf; c < HD / 32; c += 2) {
+          float o[32];
+          o_chunk(c, o);
+          if (valid) finish(c, o);
+        }
+        return;
+      }
+      // Partials: a row's two threads take a half of its channels each, and the halves go through shared memory (every operand there has been consumed), so
+      // that a warp stores whole lines: 16 bytes a lane at a row's distance took the store unit 32 cycles an instruction, 4.6 us for a tile of 96 rows.
+      constexpr int PITCH = HD * 4 + 16, LPR = HD / 8;               // bytes of a row (eight lanes' 16-byte pieces fall on different banks); lanes that cover half a row
+      static_assert(128 * PITCH <= L::OFF_BAR, "the rows fit where the operands were");
+      #pragma unroll 1
+      for (int c = hf * (HD / 64); c < (hf + 1) * (HD / 64); ++c) {
+        float o[32];
+        o_chunk(c, o);
+        if (FUSED && direct) { if (valid) finish(c, o); continue; }
+        #pragma unroll
+        for (int k = 0; k < 8; ++k)
+          tc_sts128(sb + rho * PITCH + 128 * c + 16 * k, make_uint4(__float_as_uint(o[ocol(4 * k)]), __float_as_uint(o[ocol(4 * k + 1)]),
+                                                                    __float_as_uint(o[ocol(4 * k + 2)]), __float_as_uint(o[ocol(4 * k + 3)])));
+      }
+      if (FUSED && direct) return;
+      __syncwarp();
+      #pragma unroll 4
+      for (int r0 = 0; r0 < 32; r0 += 32 / LPR) {
+        const int r = r0 + lane / LPR, off = hf * 2 * HD + 16 * (lane % LPR);
+        const long long to = __shfl_sync(0xffffffffu, valid ? (long long)pidx : -1ll, r);
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(sb + (quad * 32 + r) * PITCH + off));
+        if (to >= 0) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(P.pacc) + (size_t)to * (4 * HD) + off) = v;
       }
     }
   };
@@ -1416,6 +1446,14 @@ int tc_launch_pdl(K kern, dim3 grid, int threads, int smem_bytes, cudaStream_t s
   return 0;
 }
 
+// Query tiles of a pass (an even number: CTA pairs), its tokens shared out evenly: a CTA's softmax work is what its rows are (16 rows of six heads:
+// 48 and 48, three quarters of the warps idle, where 96 and none left one CTA with all of it).
+int tc_tiles(int M, int g, int* tokens_per_cta) {
+  const int tok = 128 / g, pairs = (M + 2 * tok - 1) / (2 * tok);
+  *tokens_per_cta = (M + 2 * pairs - 1) / (2 * pairs);
+  return 2 * pairs;
+}
+
 struct TcWs { uint16_t* kd; uint16_t* vd; uint16_t* ks; int ks_rows; size_t bytes; };
 TcWs carve(void* ws, int kvh, int hd, int max_ctx, int M) {
   TcWs w; const size_t plane = (size_t)kvh * max_ctx * hd * 2;
@@ -1446,8 +1484,8 @@ int launch_tc_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, const TcWs&
   auto kern = bf16 ? kv4_tc_attn_kernel<HD, 3> : kv4_tc_attn_kernel<HD, 0>;
   static std::atomic<unsigned long long> attr[2] = {{0}, {0}};
   if (first_use_on_device(attr[bf16 != 0])) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  const int tok = 128 / g, qtiles = ((a.M + tok - 1) / tok + 1) & ~1;        // CTA pairs: an even number of query tiles
-  TcP P{a.d_pos, a.M, a.splits, g, a.nh, a.max_ctx, w.ks_rows, a.qscale, a.pm, a.pl, a.pacc, o16, bv, a.kv, a.rope, rd,
+  int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, w.ks_rows, a.qscale, a.pm, a.pl, a.pacc, o16, bv, a.kv, a.rope, rd,
         static_cast<const uint16_t*>(a.q16), bf16, nullptr, nullptr, nullptr, nullptr};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), TC_THREADS, L::TOTAL, st, mq, mkd, mvd, mks, P)) return rc;
   return launch_status("kv4_tc_attn_kernel");
@@ -1462,8 +1500,8 @@ int launch_tc_fused_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, uint1
   auto kern = kv4_tc_attn_kernel<HD, 1>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  const int tok = 128 / g, qtiles = ((a.M + tok - 1) / tok + 1) & ~1;
-  TcP P{a.d_pos, a.M, a.splits, g, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, o16, bv, a.kv, a.rope, rd, static_cast<const uint16_t*>(a.q16), bf16,
+  int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, o16, bv, a.kv, a.rope, rd, static_cast<const uint16_t*>(a.q16), bf16,
         nullptr, nullptr, nullptr, nullptr};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), tc_threads(true), L::TOTAL, st, mq, mq, mq, mq, P)) return rc;
   return launch_status("kv4_tc_attn_kernel (fused)");
@@ -1529,8 +1567,8 @@ int launch_kv8_attention_tc(const yskn_kv8_attn_args& a, int act_dtype, cudaStre
   auto kern = kv4_tc_attn_kernel<256, 2>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  const int tok = 128 / g, qtiles = ((a.M + tok - 1) / tok + 1) & ~1;
-  TcP P{a.d_pos, a.M, a.splits, g, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, nullptr, nullptr, yskn_kv_layer{}, nullptr, 0,
+  int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, nullptr, nullptr, yskn_kv_layer{}, nullptr, 0,
         a.q16, bf16, a.k8, a.v8, a.ks, a.vs};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), tc_threads(true), L::TOTAL, st, mq, mq, mq, mq, P)) return rc;
   return launch_status("kv4_tc_attn_kernel (INT8 rows)");
@@ -1557,8 +1595,8 @@ int launch_kv8_attention_tc_ws(const yskn_kv8_attn_args& a, int act_dtype, void*
   auto kern = kv4_tc_attn_kernel<256, 4>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  const int g = a.nh / a.kvh, tok = 128 / g, qtiles = ((a.M + tok - 1) / tok + 1) & ~1;
-  TcP P{a.d_pos, a.M, a.splits, g, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, nullptr, nullptr, yskn_kv_layer{}, nullptr, 0,
+  const int g = a.nh / a.kvh; int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, nullptr, nullptr, yskn_kv_layer{}, nullptr, 0,
         a.q16, act_dtype == YSKN_KV4_BF16, nullptr, nullptr, nullptr, nullptr};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), TC_THREADS, L::TOTAL, st, mq, mkd, mvd, mq, P)) return rc;
   return launch_status("kv4_tc_attn_kernel (INT8 rows, workspace)");
