@@ -22,3 +22,37 @@ def test_token_shares_match_exact_oracle(oracle, shape, ctx, M, splits, fused):
     from yasakani_b200 import kv4
     got, want = _run_tc(kv4, oracle, shape, ctx, M, splits, seed=77, fused=fused)
     assert_close(got, want, f"{shape} ctx {ctx} M {M} splits {splits} fused {fused}")
+
+
+@pytest.mark.parametrize("workspace", [True, False], ids=["workspace", "converting"])
+@pytest.mark.parametrize("bf16", [False, True], ids=["fp16", "bf16"])
+def test_finished_rows_are_the_rounded_quotients(workspace, bf16):
+    """Rows of one split against the same pass in partials and the merge kernel, which divides: equal bits, whatever the values are (ordinary, tiny and
+    zero values of both signs, infinities in a cached row), with a bias."""
+    import torch
+    from yasakani_b200 import kv4
+    M, hq, hkv, hd, max_ctx = 70, 8, 2, 128, 128
+    dt = torch.bfloat16 if bf16 else torch.float16
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    k, v, q = rnd(M, hkv, hd).to(dt), rnd(M, hkv, hd).to(dt), rnd(M, hq, hd).to(dt)
+    v[:20] *= 1e-6
+    v[20:24] = 0.0
+    v[24:26] = -0.0
+    layer = kv4.KvLayer(hkv, hd, max_ctx)
+    pos = torch.zeros(1, dtype=torch.int32, device="cuda")
+    kv4.launch_kv_append(layer, k, v, pos, M)
+    layer.vzero[0, 60:] = float("inf")                            # rows from 60 on sum infinities in the first kv-head
+    rope = torch.empty((max_ctx, hd // 2, 2), dtype=torch.float32, device="cuda")
+    kv4.launch_rope_table_g(rope, max_ctx, 1e4, hd)
+    bv = rnd(hkv, hd).to(dt)
+    pm, pl, pacc = kv4.attn_scratch(M, 1, hq, hd)
+    ws = kv4.tc_workspace(layer, M) if workspace else None
+    a, b = (torch.empty((M, hq, hd), dtype=dt, device="cuda") for _ in range(2))
+    kv4.launch_attention_prefill_tc(q, layer, M, pos, 1, pm, pl, pacc, rope, hq, kv4.default_qscale(hd), hd, a, ws, bv=bv)
+    kv4.launch_attention_tc(q, layer, M, pos, 1, pm, pl, pacc, rope, hq, kv4.default_qscale(hd), hd, ws)
+    kv4.launch_attn_combine_gqa(pm, pl, pacc, 1, M, b, hq, hq // hkv, bv=bv)
+    torch.cuda.synchronize()
+    assert kv4.device_status() == 0
+    same = (a.view(torch.int16) == b.view(torch.int16)) | (torch.isnan(a) & torch.isnan(b))
+    assert bool(same.all()), int((~same).sum())

@@ -358,25 +358,29 @@ __device__ __forceinline__ uint32_t tc_ldg16(const void* p) { unsigned short v; 
 __device__ __forceinline__ uint4 tc_ldg128(const void* p) {
   uint4 v; asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p)); return v;
 }
+__device__ __forceinline__ void tc_prefetch_bulk(const void* p, uint32_t bytes) {    // 16-byte aligned, a multiple of 16 bytes
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void tc_prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void tc_sts128(uint32_t a, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 // Queries of one CTA (operand rows = (token, head) pairs) as fp16 rows in the swizzled Q blocks.  Rows of the tile beyond its tokens keep what the shared memory
 // held: what they yield is used nowhere.
-// PAIRS: chunks in the order of tc_row_to_pairs.  Thread t of nt; eight 16-byte loads are in flight per thread before the first one is converted.
-template <int HD, bool PAIRS>
+// PAIRS: chunks in the order of tc_row_to_pairs.  Thread t of nt; B 16-byte loads are in flight per thread before the first one is converted.
+template <int HD, bool PAIRS, int B>
 __device__ __forceinline__ void tc_stage_q(uint32_t sq, int q_block, const uint16_t* q16, bool bf16, int tok0, int G, int TOK, int M, int nh, int head0,
                                            int t, int nt) {
-  constexpr int NW = HD / 8, B = 8;
+  constexpr int NW = HD / 8;
+  const uint32_t recip = 65536u / (uint32_t)G + 1u;                  // row / G for row < 128
   #pragma unroll 1
   for (int base = t; base < TOK * G * NW; base += B * nt) {
     uint4 u[B];
     #pragma unroll
     for (int b = 0; b < B; ++b) {
-      const int it = base + b * nt, row = it / NW, w = it % NW, tk = tok0 + row / G;
+      const int it = base + b * nt, row = it / NW, w = it % NW, tl = (int)((uint32_t)row * recip >> 16), tk = tok0 + tl;
       u[b] = make_uint4(0u, 0u, 0u, 0u);
-      if (it < TOK * G * NW && tk < M) u[b] = tc_ldg128(q16 + ((size_t)tk * nh + head0 + row % G) * HD + 8 * w);
+      if (it < TOK * G * NW && tk < M) u[b] = tc_ldg128(q16 + ((size_t)tk * nh + head0 + row - tl * G) * HD + 8 * w);
     }
     #pragma unroll
     for (int b = 0; b < B; ++b) {
@@ -390,6 +394,58 @@ __device__ __forceinline__ void tc_stage_q(uint32_t sq, int q_block, const uint1
       if (PAIRS) tc_row_to_pairs(make_uint4(o4[0], o4[1], o4[2], o4[3]), o4);
       tc_sts128(sq + (w >> 3) * q_block + row * 128 + (((w & 7) ^ (row & 7)) << 4), make_uint4(o4[0], o4[1], o4[2], o4[3]));
     }
+  }
+}
+// Finished rows of a pass of one split: y = round_f16(o / l) (+ V bias) as the merge kernel, every other 32 columns of O from hf on.  A function of its own,
+// so that its code does not move the loops of the kernel about (a fused pass of 64 rows, which never comes here, took 92 to 99 us with it in line).
+template <int HD, bool PAIRS>
+__device__ __noinline__ void tc_finish_row(uint32_t tcol, int hf, bool any, bool valid, float l, bool bf16, const uint16_t* bv, uint16_t* out) {
+  const float rl = __frcp_rn(l);
+  #pragma unroll 1
+  for (int c = hf; c < HD / 32; c += 2) {
+    float o[32];
+    if (any) tmem_ld32(tcol + 32 * c, o);
+    else {
+      #pragma unroll
+      for (int k = 0; k < 32; ++k) o[k] = 0.f;
+    }
+    if (!valid) continue;
+    // o / l, correctly rounded, by the rounded reciprocal and one residual (the proof is that of kv8_combine_rows_kernel); a division instead is a branch a
+    // value, 128 one after the other: 7 us of an item that took 23.  Where the residual is no longer normal (|o| < 2^-60) the quotient is below 2^-40 and
+    // rounds to a zero of its sign either way; infinities and sums beyond the range divide.
+    float big = 0.f;
+    #pragma unroll
+    for (int k = 0; k < 32; ++k) big = fmaxf(big, fabsf(o[k]));
+    if (l >= 0x1p-20f && l <= 0x1p60f && big <= 0x1p100f) {
+      #pragma unroll
+      for (int k = 0; k < 32; ++k) { const float q = __fmul_rn(o[k], rl); o[k] = fmaf(-fmaf(q, l, -o[k]), rl, q); }
+    } else {
+      #pragma unroll 1
+      for (int k = 0; k < 32; ++k) {                                 // rolled: the values go round by one each time
+        const float t = __fdiv_rn(o[0], l);
+        #pragma unroll
+        for (int e = 0; e < 31; ++e) o[e] = o[e + 1];
+        o[31] = t;
+      }
+    }
+    uint32_t w[16];
+    #pragma unroll
+    for (int k = 0; k < 32; k += 2) w[k / 2] = PAIRS ? tc_pack(o[tc_col(k)], o[tc_col(k + 1)]) : tc_pack(o[k], o[k + 1]);
+    if (bf16 || bv) {
+      #pragma unroll
+      for (int k = 0; k < 32; k += 2) {
+        float y0 = h2f((uint16_t)w[k / 2]), y1 = h2f((uint16_t)(w[k / 2] >> 16));
+        if (bv) {
+          const uint16_t b0 = bv[32 * c + k], b1 = bv[32 * c + k + 1];
+          y0 = __fadd_rn(y0, bf16 ? bf2f(b0) : h2f(b0)); y1 = __fadd_rn(y1, bf16 ? bf2f(b1) : h2f(b1));
+        }
+        if (bf16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[k / 2]) : "f"(y1), "f"(y0));
+        else w[k / 2] = tc_pack(y0, y1);
+      }
+    }
+    uint4* dst = reinterpret_cast<uint4*>(out + 32 * c);
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) dst[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
   }
 }
 // ------------------------------------------------------------------------------------------------ INT8 rows -> fp16 workspace
@@ -841,11 +897,17 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         #pragma unroll
         for (int e = 0; e < 4; ++e) R.r[e] = tc_ldg128(rp + 16 * e);
       };
+      auto rots_pairs = [&](RotS& R) {                               // into the order of the nibble reads, once a tile
+        uint32_t t[4];
+        tc_row_to_pairs(R.sa, t); R.sa = make_uint4(t[0], t[1], t[2], t[3]); tc_row_to_pairs(R.za, t); R.za = make_uint4(t[0], t[1], t[2], t[3]);
+        tc_row_to_pairs(R.sb, t); R.sb = make_uint4(t[0], t[1], t[2], t[3]); tc_row_to_pairs(R.zb, t); R.zb = make_uint4(t[0], t[1], t[2], t[3]);
+      };
       auto roti_store = [&](int u, uint32_t sk, const RotS& Sc, const RotI& R) {
         if (cc + cstep * u >= 16) return;
         const int p = cp, q = cp + nrp, k = wkey + cc + cstep * u;
-        uint32_t sa[4], za[4], sb4[4], zb[4], na[4], nb[4], a[4], b[4], lo[4], hi[4];
-        tc_row_to_pairs(Sc.sa, sa); tc_row_to_pairs(Sc.za, za); tc_row_to_pairs(Sc.sb, sb4); tc_row_to_pairs(Sc.zb, zb);
+        const uint32_t sa[4] = {Sc.sa.x, Sc.sa.y, Sc.sa.z, Sc.sa.w}, za[4] = {Sc.za.x, Sc.za.y, Sc.za.z, Sc.za.w};
+        const uint32_t sb4[4] = {Sc.sb.x, Sc.sb.y, Sc.sb.z, Sc.sb.w}, zb[4] = {Sc.zb.x, Sc.zb.y, Sc.zb.z, Sc.zb.w};
+        uint32_t na[4], nb[4], a[4], b[4], lo[4], hi[4];
         tc_nibs(R.wa, na, nk); tc_nibs(R.wb, nb, nk);
         #pragma unroll
         for (int x = 0; x < 4; ++x) { a[x] = tc_hfma2(na[x], sa[x], za[x]); b[x] = tc_hfma2(nb[x], sb4[x], zb[x]); }
@@ -876,15 +938,13 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         }
       }
       int kit = 0;
-      // L2 prefetch of a half tile two tiles ahead (64 packed rows, the scale and zero rows of its two groups; one line per
-      // thread), so that the register loads a phase ahead find their lines in L2
+      // L2 prefetch of a half tile two tiles ahead (64 packed rows, the scale and zero rows of its two groups: three contiguous pieces), so that the register
+      // loads a tile ahead find their lines in L2
       auto k_prefetch = [&](int tk) {
-        if (tk >= P.max_ctx) return;
-        if (ct < TC_BN / 2) tc_prefetch_l2(P.kv.kq + (row0 + tk + ct) * (HD / 2));
-        else if (ct < TC_BN / 2 + 4 * (HD / 64)) {
-          const int x = ct - TC_BN / 2, arr = x & 1, grp = (x >> 1) & 1, line = x >> 2;      // line < HD/64 (128-byte lines of an HD x fp16 row)
-          tc_prefetch_l2((arr ? P.kv.kzero : P.kv.kscale) + (grp0 + tk / 32 + grp) * HD + 64 * line);
-        }
+        if (tk >= P.max_ctx || ct != 0) return;
+        tc_prefetch_bulk(P.kv.kq + (row0 + tk) * (HD / 2), (TC_BN / 2) * (HD / 2));
+        tc_prefetch_bulk(P.kv.kscale + (grp0 + tk / 32) * HD, 2 * HD * 2);
+        tc_prefetch_bulk(P.kv.kzero + (grp0 + tk / 32) * HD, 2 * HD * 2);
       };
       if (n > 1) k_prefetch(j0 * TC_BN + TC_BN + (TC_BN / 2) * (int)rank);
       for (int i = 0; i < n && ok; ++i) {
@@ -906,6 +966,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
               if (32 * u < 4 * npl) { plain_store(u, sk, pc[u]); plain_load(at, u, pc[u]); }
             }
             if (compact) {
+              rots_pairs(rs);
               #pragma unroll
               for (int u = 0; u < NRU; ++u) {
                 if (cstep * u < 16) { roti_store(u, sk, rs, rc[u]); roti_load(at, u, rc[u]); }
@@ -1011,9 +1072,11 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         I.w = tc_ldg128(at.q + k * (HD / 2));
         I.s = tc_ldg16(at.s + k); I.z = tc_ldg16(at.z + k);
       };
-      auto v_prefetch = [&](int j) {                                 // L2 prefetch of a tile's half rows and per-token scales
-        for (int x = vt; x < TC_BN; x += NVT) if (j * TC_BN + x < end) tc_prefetch_l2(P.kv.vq + (row0 + j * TC_BN + x) * (HD / 2) + (HD / 4) * (int)rank);
-        if (vt < 4 && j * TC_BN + 64 * (vt & 1) < end) tc_prefetch_l2((vt & 2 ? P.kv.vzero : P.kv.vscale) + row0 + j * TC_BN + 64 * (vt & 1));
+      auto v_prefetch = [&](int j) {                                 // L2 prefetch of 64 of a tile's rows (the other CTA takes the other 64) and their scales
+        const int t = j * TC_BN + (TC_BN / 2) * (int)rank;
+        if (t >= P.max_ctx || vt != 0) return;
+        tc_prefetch_bulk(P.kv.vq + (row0 + t) * (HD / 2), (TC_BN / 2) * (HD / 2));
+        tc_prefetch_l2(P.kv.vscale + row0 + t); tc_prefetch_l2(P.kv.vzero + row0 + t);     // these two arrays may lie at any even address
       };
       VIn vin[NVI];
       {
@@ -1070,7 +1133,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     if constexpr (STAGED_Q) {
       if (n > 0) {
         // bf16 activations, or the chunk order of the int4 form: these eight warps write this CTA's query rows (there is no Q copy)
-        tc_stage_q<HD, FORM == 1>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, act_bf16, tok0, G, TOK, P.M, P.nh, kvh * G, threadIdx.x, 32 * TC_SW);
+        tc_stage_q<HD, FORM == 1, FUSED ? 8 : 16>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, act_bf16, tok0, G, TOK, P.M, P.nh, kvh * G, threadIdx.x, 32 * TC_SW);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) bar_arrive_cluster(lead_q);
@@ -1211,69 +1274,71 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       const bool edge = i >= npipe;
       const int buf = edge ? 0 : (i & 1);
       const uint32_t scol = trow + (buf ? L::TM_S1 : L::TM_S0) + 64 * hf;   // this thread's 64 S columns; P goes over the first 32
-      float x[64];                                                   // raw scores of this thread's 64 keys
       if (!bar_wait(b_sready + 8 * buf, srd[buf] & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
-      tc_fence_after();
-      tmem_ld64(scol, x);
       ++srd[buf];
       if (edge) {
         if (!bar_wait(b_sready + 8, srd[1] & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
-        tc_fence_after();
         ++srd[1];
-        // each 32-key quarter is one group: before the row's own -> int4 keys; own group -> shadow keys up to the row; later -> nothing
-        #pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
+      }
+      tc_fence_after();
+      // Two walks over the 64 keys in pieces of 32, first the maximum, then the exponentials, in one rolled loop: the loops of all roles have to stay inside the
+      // instruction cache together, and the scores are read from tensor memory a second time for it.
+      // Online softmax in the log2 domain on p = 2^(x*cs - m); lazy rescale (the running max may lag by up to 2^8).
+      float tmax = -INFINITY, nm = 0.f, ls0 = 0.f, ls1 = 0.f;
+      #pragma unroll 1
+      for (int step = 0; step < 4 && ok; ++step) {
+        const int h2 = step & 1;
+        if (step == 2) {
+          tmax = fmaxf(tmax, swap_with_partner(tmax, i + 1)) * cs;    // the row's two threads swap their maxima
+          const bool bump = valid && tmax > m + 8.f;
+          const float mn = bump ? tmax : m, alpha = bump ? tc_ex2(m - mn) : 1.f;
+          m = mn; l *= alpha; nm = -m;
+          // ---- O may be rescaled once P.V of tile i-1 is done (P.V of this tile waits for the signal below)
+          if (i > 0 && __any_sync(0xffffffffu, bump)) {              // rows that did not bump multiply by exactly 1
+            if (!bar_wait(b_pvdone + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
+            tc_fence_after();
+            #pragma unroll 1
+            for (int c = hf; c < HD / 32; c += 2) {                  // the row's two threads take alternate 32-column chunks of O
+              float o[32];
+              tmem_ld32(trow + L::TM_O + 32 * c, o);
+              #pragma unroll
+              for (int k = 0; k < 32; ++k) o[k] *= alpha;
+              tmem_st32(trow + L::TM_O + 32 * c, o);
+            }
+          }
+        }
+        float x[32];                                                 // raw scores
+        tmem_ld32(scol + 32 * h2, x);
+        if (edge) {
+          // each 32-key quarter is one group: before the row's own -> int4 keys; own group -> shadow keys up to the row; later -> nothing
           float a[32];
           tmem_ld32(trow + L::TM_S1 + 64 * hf + 32 * h2, a);
           const int gk = 4 * j + 2 * hf + h2, tb = j * TC_BN + 64 * hf + 32 * h2;
           #pragma unroll
-          for (int k = 0; k < 32; ++k) x[32 * h2 + k] = gk < cr ? x[32 * h2 + k] : (gk == cr && tb + k <= pr) ? a[k] : -INFINITY;
+          for (int k = 0; k < 32; ++k) x[k] = gk < cr ? x[k] : (gk == cr && tb + k <= pr) ? a[k] : -INFINITY;
         }
-      }
-      if (I8 && i >= nbulk) {                                        // INT8 rows: the tiles that hold the new rows are masked causally
-        const int tb = j * TC_BN + 64 * hf;
-        #pragma unroll
-        for (int k = 0; k < 64; ++k) x[k] = tb + k <= pr ? x[k] : -INFINITY;
-      }
-      // ---- online softmax in the log2 domain on p = 2^(x*cs - m); lazy rescale (the running max may lag by up to 2^8)
-      float tmax = fmaxf(x[0], x[1]);
-      #pragma unroll
-      for (int k = 2; k < 64; k += 2) tmax = fmaxf(tmax, fmaxf(x[k], x[k + 1]));
-      tmax = fmaxf(tmax, swap_with_partner(tmax, i + 1)) * cs;        // the row's two threads swap their maxima
-      const bool bump = valid && tmax > m + 8.f;
-      const float mn = bump ? tmax : m, alpha = bump ? tc_ex2(m - mn) : 1.f;
-      m = mn; l *= alpha;
-      uint32_t pk[32];
-      {
-        const float nm = -m;
-        float ls0 = 0.f, ls1 = 0.f;
-        #pragma unroll
-        for (int k = 0; k < 64; k += 4) {
-          const float p0 = tc_ex2(fmaf(x[k], cs, nm)), p1 = tc_ex2(fmaf(x[k + 1], cs, nm));        // exp2(-inf) = 0 for masked keys
-          const float p2 = tc_ex2(fmaf(x[k + 2], cs, nm)), p3 = tc_ex2(fmaf(x[k + 3], cs, nm));
-          ls0 += p0 + p1; ls1 += p2 + p3; pk[k / 2] = tc_pack(p0, p1); pk[k / 2 + 1] = tc_pack(p2, p3);
-        }
-        l += ls0 + ls1;
-      }
-      if (__any_sync(0xffffffffu, !valid) && !valid) {               // rows of the tile that hold no query: P = 0, state untouched
-        #pragma unroll
-        for (int k = 0; k < 32; ++k) pk[k] = 0u;
-        l = 0.f;
-      }
-      // ---- O may be rescaled once P.V of tile i-1 is done (P.V of this tile waits for the signal below)
-      if (i > 0 && __any_sync(0xffffffffu, bump)) {                  // rows that did not bump multiply by exactly 1
-        if (!bar_wait(b_pvdone + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
-        tc_fence_after();
-        #pragma unroll 1
-        for (int c = hf; c < HD / 32; c += 2) {                      // the row's two threads take alternate 32-column chunks of O
-          float o[32];
-          tmem_ld32(trow + L::TM_O + 32 * c, o);
+        if (I8 && i >= nbulk) {                                      // INT8 rows: the tiles that hold the new rows are masked causally
+          const int tb = j * TC_BN + 64 * hf + 32 * h2;
           #pragma unroll
-          for (int k = 0; k < 32; ++k) o[k] *= alpha;
-          tmem_st32(trow + L::TM_O + 32 * c, o);
+          for (int k = 0; k < 32; ++k) x[k] = tb + k <= pr ? x[k] : -INFINITY;
+        }
+        if (step < 2) {
+          #pragma unroll
+          for (int k = 0; k < 32; k += 2) tmax = fmaxf(tmax, fmaxf(x[k], x[k + 1]));
+        } else {
+          uint32_t pk[16];
+          #pragma unroll
+          for (int k = 0; k < 32; k += 4) {
+            const float p0 = tc_ex2(fmaf(x[k], cs, nm)), p1 = tc_ex2(fmaf(x[k + 1], cs, nm));      // exp2(-inf) = 0 for masked keys
+            const float p2 = tc_ex2(fmaf(x[k + 2], cs, nm)), p3 = tc_ex2(fmaf(x[k + 3], cs, nm));
+            ls0 += p0 + p1; ls1 += p2 + p3;
+            pk[k / 2] = valid ? tc_pack(p0, p1) : 0u; pk[k / 2 + 1] = valid ? tc_pack(p2, p3) : 0u;   // rows of the tile that hold no query: P = 0
+          }
+          tmem_st16u(scol + 16 * h2, pk);                            // P as the A operand of P.V, over S columns this thread has read
         }
       }
-      tmem_st32u(scol, pk);                                          // P as the A operand of P.V, over S columns this thread has read
+      if (!ok) break;
+      l = valid ? l + (ls0 + ls1) : 0.f;
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -1289,37 +1354,9 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       const bool direct = P.o16 != nullptr && S == 1;                // one split: this CTA holds the whole row, finish it here
       auto ocol = [](int c) { return FORM == 1 ? tc_col(c) : c; };   // the int4 form's V chunks keep their channels in pair order
       if (valid && !direct && hf == 0) { P.pm[pidx] = (n > 0 && m > -1e29f) ? m * TC_LN2 : -1e30f; P.pl[pidx] = n > 0 ? l : 0.f; }
-      auto o_chunk = [&](int c, float (&o)[32]) {                    // 32 columns of this row's O
-        if (n > 0) tmem_ld32(trow + L::TM_O + 32 * c, o);
-        else {
-          #pragma unroll
-          for (int k = 0; k < 32; ++k) o[k] = 0.f;
-        }
-      };
-      auto finish = [&](int c, const float (&o)[32]) {               // y = round_f16(o / l) (+ V bias), as the merge kernel
-        uint4* dst = reinterpret_cast<uint4*>(P.o16 + ((size_t)tok * P.nh + kvh * G + head) * HD + 32 * c);
-        uint32_t w[16];
-        #pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-          float y0 = round_f16(o[ocol(k)] / l), y1 = round_f16(o[ocol(k + 1)] / l);
-          if (act_bf16) {
-            if (P.bv) { y0 = __fadd_rn(y0, bf2f(P.bv[kvh * HD + 32 * c + k])); y1 = __fadd_rn(y1, bf2f(P.bv[kvh * HD + 32 * c + k + 1])); }
-            w[k / 2] = (uint32_t)f2bf(y0) | ((uint32_t)f2bf(y1) << 16);
-            continue;
-          }
-          if (P.bv) { y0 = __fadd_rn(y0, h2f(P.bv[kvh * HD + 32 * c + k])); y1 = __fadd_rn(y1, h2f(P.bv[kvh * HD + 32 * c + k + 1])); }
-          w[k / 2] = (uint32_t)f2h(y0) | ((uint32_t)f2h(y1) << 16);
-        }
-        #pragma unroll
-        for (int k = 0; k < 4; ++k) dst[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
-      };
-      if (!FUSED && direct) {                                        // a loop of its own: as a branch of the one below it cost 1,000 rows 58 -> 60 us
-        #pragma unroll 1
-        for (int c = hf; c < HD / 32; c += 2) {
-          float o[32];
-          o_chunk(c, o);
-          if (valid) finish(c, o);
-        }
+      if (direct) {                                                  // one split: this CTA holds the whole row
+        tc_finish_row<HD, FORM == 1>(trow + L::TM_O, hf, n > 0, valid, l, act_bf16, P.bv ? P.bv + kvh * HD : nullptr,
+                                     P.o16 + ((size_t)tok * P.nh + kvh * G + head) * HD);
         return;
       }
       // Partials: a row's two threads take a half of its channels each, and the halves go through shared memory (every operand there has been consumed), so
@@ -1329,14 +1366,16 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       #pragma unroll 1
       for (int c = hf * (HD / 64); c < (hf + 1) * (HD / 64); ++c) {
         float o[32];
-        o_chunk(c, o);
-        if (FUSED && direct) { if (valid) finish(c, o); continue; }
+        if (n > 0) tmem_ld32(trow + L::TM_O + 32 * c, o);
+        else {
+          #pragma unroll
+          for (int k = 0; k < 32; ++k) o[k] = 0.f;
+        }
         #pragma unroll
         for (int k = 0; k < 8; ++k)
           tc_sts128(sb + rho * PITCH + 128 * c + 16 * k, make_uint4(__float_as_uint(o[ocol(4 * k)]), __float_as_uint(o[ocol(4 * k + 1)]),
                                                                     __float_as_uint(o[ocol(4 * k + 2)]), __float_as_uint(o[ocol(4 * k + 3)])));
       }
-      if (FUSED && direct) return;
       __syncwarp();
       #pragma unroll 4
       for (int r0 = 0; r0 < 32; r0 += 32 / LPR) {
