@@ -101,3 +101,20 @@ def test_attention_over_packed_rows_equals_attention_over_the_unpacked_rows(orac
     got = o16.float().cpu().numpy()
     err = np.abs(got - want)
     assert (err <= 2e-3 + 1e-2 * np.abs(want)).all(), f"max err {err.max():.3e}"
+
+
+@pytest.mark.parametrize("nm", [1, 2, 5, 16])
+def test_both_encoder_forms_over_every_step_width(oracle, nm):
+    """Few rows take blocks of up to ten warps, many rows blocks of up to five: the same rows through both (one, all and several rounds of the
+    multipliers; the last row count of the one and the first of the other) against the oracle, bit for bit."""
+    from yasakani_b200 import kvx
+    blob = make_blob(nm=nm)
+    x, _, _ = _rows(40, 11)
+    grp, pos = np.arange(40, dtype=np.int32), np.full(40, 50, np.int32)     # records 0 .. 39 hold every step width and a flat one
+    want = oracle.tb_encode(blob, x, grp, pos)
+    prof = kvx.TrellisProfile(blob)
+    for n in (40, 592, 593):
+        rep = np.arange(n) % 40
+        y, pay, side = kvx.tb_encode(prof, *(torch.from_numpy(np.ascontiguousarray(a[rep])).cuda() for a in (x, grp, pos)))
+        assert np.array_equal(y.cpu().numpy().view(np.uint32), want["y"].view(np.uint32)[rep]), n
+        assert np.array_equal(pay.cpu().numpy().view(np.uint32).reshape(n, 40), want["pay"][rep]) and np.array_equal(side.cpu().numpy().view(np.uint32), want["side"][rep]), n

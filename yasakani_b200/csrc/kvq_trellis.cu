@@ -11,6 +11,7 @@
 // order), and every product that feeds a rounding decision is an explicit _rn operation, so no FMA contraction moves a bit.
 #include "kv4_common.cuh"
 #include <cstring>
+#include <type_traits>
 
 namespace kv4 {
 namespace {
@@ -36,15 +37,19 @@ __device__ __forceinline__ TbGroup tb_group(const uint8_t* b, int g) {
 // nothing is read through it (0: the header, which every blob has).
 __device__ __forceinline__ unsigned tb_table(const uint8_t* b, const TbGroup& P) { return P.ok && P.mode == 0 ? tb_u32(b + P.off_t + 4u * (unsigned)P.tix) : 0u; }
 
-// ---- encoder: one block of four warps per row, one warp per chain of 64 values.
+// ---- encoder: one block per row, one warp per multiplier and pair of chains, sixteen lanes per chain of 64 values.
 //
 // A step of the search takes new(d) = min over the 2^KK predecessors {j * UU + u}, u = d >> KK, of old(p), plus (x - code[d])^2: every
 // state is a candidate of one group u only, so 256 candidates and 256 costs a step.  What bounds it is instruction issue
-// (integer), so the whole step stays in registers: a lane holds eight states, four values of j for two values of u,
-//   p = jhi << (SH+2) | jlo << SH | umid << 1 | ulo,     registers e = (jlo, ulo), lane = (jhi, umid)     (SH = 8 - KK, UU = 2^SH)
-// the minimum over jlo is in the lane (one fused add-minimum per state), the first exchange over jhi halves the lane's two
-// values of u (each lane of the pair keeps one), the other exchanges are plain; the new states of a lane need 4 (KK = 3, 4) or
-// 1 (KK = 5) of the UU minima, one shuffle each: 6 / 7 / 4 shuffles and about 35 instructions a step, no shared memory on the path and no barrier.
+// (integer), so the whole step stays in registers: a lane holds sixteen states p = j << SH | u (SH = 8 - KK, UU = 2^SH), one multiply-add for each cost and
+// one fused add-minimum for each candidate, and both chains of a warp go through the same instructions, the few that hand minima on among them:
+//   KK   lane (4 bits)          registers                 minima handed on            exchanged
+//   3    u4 u3 u1 u0            j (8), u2                 8 shuffles                  none (a lane has every j of its two u)
+//   4    top bit of j, u3 .. u1 the other bits of j, u0   8 shuffles                  1 (each lane of a pair keeps one u)
+//   5    top bit of j, u        the other bits of j (16)  4 shuffles                  1
+// (The new states of a lane need the minima of the groups p >> KK.  For KK = 3 the bit of u in the registers is u2: the lane's states of both values need the
+// same eight, and which of its two values a lane hands on follows from j alone.)  About 48 instructions a step of two chains; the form it replaces
+// had a lane hold eight states of one chain: 55 a step of one, of which 39 were exchanges, masks and stores.
 // x^2 is left out of the costs: it adds the same number to every state of a step.  A cost travels as a key, cost << 5 | j, whose j is part
 // of the state's own constant: the minimum over keys is the minimum cost with the first j on ties (the reference's rule,
 // src/kvq_gpu.cuh:101-102) and carries its back pointer, one byte per group and step.
@@ -52,134 +57,150 @@ __device__ __forceinline__ unsigned tb_table(const uint8_t* b, const TbGroup& P)
 // two states; any state is reached from any other in three steps, so the costs of a step spread over at most 3 D.  They are
 // brought back to one of them every four steps: |cost| <= 3 D + 4 F < 2^26 for C <= 1400, and a key fits 32 bits.  Profiles with larger codes
 // take 64-bit keys (the same code, no bringing back).
-// 4,096 rows, 5 multipliers, on a B200: 1,335 us (one warp per (row, multiplier, chain), costs in shared memory, every lane walking its
-// group's predecessors; a second kernel for choice and packing) -> 448 (minima kept instead of back pointers, candidates recomputed on
-// the way back: 76 instructions a step) -> 321 (55 a step; issue slots 77 % busy, integer ALU 65 %, the
-// multiply pipe 53 %).
+// 4,096 rows, 5 multipliers, on a B200: 1,335 us (one warp per (row, multiplier, chain), costs in shared memory, every lane walking its group's predecessors; a
+// second kernel for choice and packing) -> 448 (minima kept instead of back pointers, candidates recomputed on the way back) -> 321 (eight states a
+// lane, a warp per chain that walks the multipliers) -> 243.  Issue slots 63 % busy, integer ALU 45 %, multiply pipe 49 %, shuffles and shared memory 45 %; 25 warps
+// an SM at 72 registers instead of 20 at 96 are slower (262), 15 at 128 too (273).
+// Blocks of ten warps (every multiplier and pair of chains at once) for a few rows, which are bound by the chains of 64 dependent steps; of five, twice as
+// many an SM, for more rows than two rounds of the former: with unpacking 100 rows 28.0 / 33.9 us, 600 53.5 / 55.6, 1,000 84.8 / 80.9, 4,096 270 / 250 (ten / five).
 constexpr int TB_NM = 16;                                // multipliers at most (the blob's limit)
+constexpr int TB_WIDE = 10, TB_NARROW = 5, TB_WIDE_ROWS = 2 * 2 * 148;     // warps of a block at most, two forms; rows that the wide one takes
 struct TbRowSmem {
-  uint8_t bp[4][64 * 32];                                // back pointers of each chain: [t][u], the low five bits
-  short code[256]; float red[8]; int cmax[4]; uint8_t fld[256];
-  struct Mult { uint8_t st[256]; float err[8]; } mult[1];  // one per multiplier: its states and its error sums
-  static size_t bytes(int nm) { return sizeof(TbRowSmem) + (nm - 1) * sizeof(Mult); }
+  short code[256]; float res[256]; float red[8]; int cmax[16]; uint8_t fld[256];
+  TbGroup grp; float coef[2];                              // what the search does not need waits here, not in registers
+  struct Warp { int xs[128]; uint8_t bp[2][64 * 32]; };    // scaled values; back pointers of each chain: [t][u], the low five bits
+  struct Mult { uint8_t st[256]; float err[8]; };          // one per multiplier: its states and its error sums
+  static int warps(int nm, int most) { return 2 * nm < 4 ? 4 : 2 * nm < most ? 2 * nm : most; }      // four at least: they hold the row
+  static size_t bytes(int nm, int most) { return sizeof(TbRowSmem) + warps(nm, most) * sizeof(Warp) + nm * sizeof(Mult); }
 };
+static_assert(sizeof(TbRowSmem) % 16 == 0 && sizeof(TbRowSmem::Warp) % 16 == 0, "xs is read sixteen bytes at a time");
 struct TbP { const uint8_t* blob; int nm; const float* x; const int* grp; const int* pos; int rows; float* y; uint8_t* pay; int pay_stride; uint32_t* side; int whole; };
 
 __device__ __forceinline__ int tb_addmin(int a, int b, int c) { return __viaddmin_s32(a, b, c); }
 __device__ __forceinline__ long long tb_addmin(long long a, long long b, long long c) { return min(a + b, c); }
 
-// States of the best path of this warp's chain for the scaled values xa (steps 0-31, a lane each) and xb (steps 32-63): returned
-// as (state of step lane, state of step lane + 32).  K = int or long long, the type of the keys.
-template <int KK, class K> __device__ __forceinline__ int2 tb_search(uint8_t* bp, const short* code, int xa, int xb, int lane) {
-  constexpr int SH = 8 - KK, UU = 1 << SH, NQ = KK == 5 ? 1 : 4;
+// States of the best path of this half warp's chain of scaled values xs (bp, xs and states are the chain's own).  K = int or long long, the type of the keys.
+template <int KK, class K> __device__ __forceinline__ void tb_search(uint8_t* bp, const short* code, const int* xs, uint8_t* states, int lane) {
+  constexpr int SH = 8 - KK, UU = 1 << SH, NQ = KK == 5 ? 4 : 8;
   constexpr bool NARROW = sizeof(K) == 4;
-  const int umid = lane & ((1 << (SH - 1)) - 1), jhi = lane >> (SH - 1);
-  K m2c[8], c2[8];
-  int src[NQ];
+  const int l = lane & 15, half = lane & 16;
+  auto state = [&](int e) {
+    return KK == 3 ? ((e >> 1) << 5) | ((l >> 2) << 3) | ((e & 1) << 2) | (l & 3) : KK == 4 ? ((l >> 3) << 7) | ((e >> 1) << 4) | ((l & 7) << 1) | (e & 1)
+                                                                                           : ((l >> 3) << 7) | (e << 3) | (l & 7);
+  };
+  int m2c[16], c2[16];                                   // 32-bit keys: a cost is x * m2c + c2; 64-bit ones read the code again (c (c - 2x) fits 32 bits)
+  if (NARROW)
+    #pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const int p = state(e), c = code[p];
+      m2c[e] = -2 * c * 32; c2[e] = c * c * 32 + (p >> SH);
+    }
+  int src[NQ];                                           // the lane that holds the minimum of group (new state >> KK)
   #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int p = (jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1), c = code[p];
-    m2c[e] = (K)(-2 * c) * 32; c2[e] = (K)c * c * 32 + (p >> SH);
-  }
-  #pragma unroll
-  for (int q = 0; q < NQ; ++q) {                         // the lane that holds the minimum of group (new state >> KK)
-    const int g = ((jhi << (SH + 2)) | (q << SH) | (umid << 1)) >> KK;
-    src[q] = ((g & 1) << (SH - 1)) | (g >> 1);
-  }
-  const bool upper = (lane >> (SH - 1)) & 1;             // of a pair of lanes the upper one keeps the odd u
-  const int my_u = (umid << 1) | (upper ? 1 : 0);
+  for (int q = 0; q < NQ; ++q)
+    src[q] = half | (KK == 3 ? ((q >> 1) << 2) | (l >> 2) : KK == 4 ? ((q & 1) << 3) | ((l >> 3) << 2) | (q >> 1) : ((l >> 3) << 2) | q);
+  const bool upper = l >> 3;                             // KK = 4: of a pair of lanes the upper one keeps the odd u
+  const int my_u = KK == 3 ? ((l >> 2) << 3) | (l & 3) : KK == 4 ? ((l & 7) << 1) | (upper ? 1 : 0) : l & 7;
   // Only state 0 exists at first.  Every state is reachable after three steps, so the others have to stay behind by more than 6 F
   // (5e7 for C = 1400) until then, and within the width of a key.
-  K keep = my_u == 0 ? (K)(-(1 << 25)) * 32 : (K)(NARROW ? (1 << 24) + (1 << 23) : 0x40000000) * 32;
-  uint8_t* mine = bp + (lane < UU ? my_u : 0);           // lanes below UU hold every u once (the jhi bits above the first are zero)
-  auto costs = [&](int x, K (&t)[8], K (&m)[NQ]) {
-    keep &= ~(K)31;
+  constexpr K FAR = (K)(NARROW ? (1 << 24) + (1 << 23) : 0x40000000) * 32;
+  K ka = my_u == 0 ? (K)(-(1 << 25)) * 32 : FAR, kb = FAR;          // minima of the lane's groups (kb: KK = 3, the one with u2 = 1)
+  uint8_t* mine = bp + my_u;
+  auto costs = [&](int x, K (&t)[16], K (&m)[NQ]) {
+    ka &= ~(K)31;
+    if (KK == 3) kb &= ~(K)31;
     #pragma unroll
-    for (int q = 0; q < NQ; ++q) m[q] = __shfl_sync(0xffffffffu, keep, src[q]);
+    for (int q = 0; q < NQ; ++q) m[q] = __shfl_sync(0xffffffffu, KK == 3 && (q & 1) ? kb : ka, src[q]);
     #pragma unroll
-    for (int e = 0; e < 8; ++e) t[e] = x * m2c[e] + c2[e];
+    for (int e = 0; e < 16; ++e)
+      if (NARROW) t[e] = x * m2c[e] + c2[e];
+      else { const int p = state(e), c = code[p]; t[e] = (K)(c * (c - 2 * x)) * 32 + (p >> SH); }
   };
+  auto mi = [](int e) { return KK == 5 ? e >> 2 : e >> 1; };
   auto step = [&](int x, int t) {                        // the minima of step t + 1 from those of step t
-    K ct[8], m[NQ];
+    K ct[16], m[NQ];
     costs(x, ct, m);
-    K a = ct[0] + m[0], b = ct[1] + m[0];
+    K a = ct[0] + m[0], b = ct[1] + m[mi(1)];
     #pragma unroll
-    for (int q = 1; q < 4; ++q) {
-      a = tb_addmin(ct[2 * q], m[NQ == 1 ? 0 : q], a);
-      b = tb_addmin(ct[2 * q + 1], m[NQ == 1 ? 0 : q], b);
+    for (int e = 2; e < 16; e += 2) {
+      a = tb_addmin(ct[e], m[mi(e)], a);
+      b = tb_addmin(ct[e + 1], m[mi(e + 1)], b);
     }
-    const K other = __shfl_xor_sync(0xffffffffu, upper ? a : b, 1 << (SH - 1));
-    keep = min(upper ? b : a, other);
-    #pragma unroll
-    for (int k = SH; k < 5; ++k) keep = min(keep, __shfl_xor_sync(0xffffffffu, keep, 1 << k));
-    if (lane < UU) mine[(t + 1) * UU] = (uint8_t)keep;
+    if (KK == 3) {
+      ka = a; kb = b;
+      mine[(t + 1) * UU] = (uint8_t)a; mine[(t + 1) * UU + 4] = (uint8_t)b;
+    } else {
+      if (KK == 4) ka = min(upper ? b : a, __shfl_xor_sync(0xffffffffu, upper ? a : b, 8));
+      else { ka = min(a, b); ka = min(ka, __shfl_xor_sync(0xffffffffu, ka, 8)); }
+      if (KK == 4 || l < UU) mine[(t + 1) * UU] = (uint8_t)ka;
+    }
   };
   #pragma unroll 1
   for (int t = 0; t < 60; t += 4) {
-    const int xs = t < 32 ? xa : xb;
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) step(__shfl_sync(0xffffffffu, xs, (t + i) & 31), t + i);
-    if (NARROW) keep -= __shfl_sync(0xffffffffu, keep, 0) & ~(K)31;
+    const int4 x = *reinterpret_cast<const int4*>(xs + t);
+    step(x.x, t); step(x.y, t + 1); step(x.z, t + 2); step(x.w, t + 3);
+    if (NARROW) { const K b0 = __shfl_sync(0xffffffffu, ka, half) & ~(K)31; ka -= b0; if (KK == 3) kb -= b0; }
   }
-  #pragma unroll
-  for (int t = 60; t < 63; ++t) step(__shfl_sync(0xffffffffu, xb, t - 32), t);
+  const int4 x = *reinterpret_cast<const int4*>(xs + 60);
+  step(x.x, 60); step(x.y, 61); step(x.z, 62);
   // best final state: smallest (cost, state)
-  K ct[8], m[NQ];
-  costs(__shfl_sync(0xffffffffu, xb, 31), ct, m);
+  K ct[16], m[NQ];
+  costs(x.w, ct, m);
   K best = 0; int bs = 0;
   #pragma unroll
-  for (int e = 0; e < 8; ++e) {                          // a lane's states grow with jlo, then ulo
-    const K c = (ct[e] + m[NQ == 1 ? 0 : e >> 1]) & ~(K)31;
-    if (e == 0 || c < best) { best = c; bs = (jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1); }
+  for (int e = 0; e < 16; ++e) {
+    const K c = (ct[e] + m[mi(e)]) & ~(K)31;
+    const int p = state(e);
+    if (e == 0 || c < best || (c == best && p < bs)) { best = c; bs = p; }
   }
   #pragma unroll
-  for (int o = 16; o; o >>= 1) {
+  for (int o = 8; o; o >>= 1) {
     const K c = __shfl_xor_sync(0xffffffffu, best, o); const int b2 = __shfl_xor_sync(0xffffffffu, bs, o);
     if (c < best || (c == best && b2 < bs)) { best = c; bs = b2; }
   }
   __syncwarp();                                          // the back pointers are complete
-  int2 out = make_int2(0, 0);
   int st = bs;
-  #pragma unroll 1
-  for (int half = 1; half >= 0; --half) {
-    int keep_st = 0;
-    #pragma unroll 8
-    for (int i = 31; i >= 0; --i) {
-      if (lane == i) keep_st = st;
-      const int u = st >> KK;
-      st = ((bp[(32 * half + i) * UU + u] & 31) << SH) | u;      // (the row of step 0 is read but never used)
-    }
-    if (half) out.y = keep_st; else out.x = keep_st;
+  #pragma unroll 8
+  for (int t = 63; t >= 0; --t) {
+    if (l == 0) states[t] = (uint8_t)st;
+    const int u = st >> KK;
+    st = ((bp[t * UU + u] & 31) << SH) + u;              // (the row of step 0 is read but never used)
   }
-  __syncwarp();                                          // they may be overwritten
-  return out;
+  __syncwarp();                                          // they may be overwritten, and the states are complete
 }
 
-__global__ void __launch_bounds__(128, 7) tb_encode_kernel(TbP A) {
+template <int W>
+__global__ void __launch_bounds__(W * 32, 20 / W) tb_encode_kernel(TbP A) {
   extern __shared__ __align__(16) unsigned char tbe_smem[];
   TbRowSmem& S = *reinterpret_cast<TbRowSmem*>(tbe_smem);
-  const int row = blockIdx.x, c = threadIdx.x >> 5, lane = threadIdx.x & 31, d0 = 64 * c + lane, d1 = d0 + 32;     // this thread's two values
+  const int nt = blockDim.x, nwarps = nt >> 5;
+  TbRowSmem::Warp* const warps = reinterpret_cast<TbRowSmem::Warp*>(tbe_smem + sizeof(TbRowSmem));
+  TbRowSmem::Mult* const mult = reinterpret_cast<TbRowSmem::Mult*>(warps + nwarps);
+  const int row = blockIdx.x, c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool own = c < 4;                                // the first four warps hold the row, two values a thread
+  const int d0 = 64 * (c & 3) + lane, d1 = d0 + 32;
   const uint8_t* b = A.blob;
-  const TbGroup P = tb_group(b, A.grp[row]);
+  TbGroup P = tb_group(b, A.grp[row]);
   const int words = A.pay_stride / 4;
   unsigned* pay = A.pay ? reinterpret_cast<unsigned*>(A.pay + (size_t)row * A.pay_stride) : nullptr;
   float ra = A.x[(size_t)row * 256 + d0], rb = A.x[(size_t)row * 256 + d1];
   if (!P.ok || A.pos[row] < P.guard) {                   // stored as it is
-    if (A.y) { A.y[(size_t)row * 256 + d0] = ra; A.y[(size_t)row * 256 + d1] = rb; }
+    if (A.y && own) { A.y[(size_t)row * 256 + d0] = ra; A.y[(size_t)row * 256 + d1] = rb; }
     if (A.whole) {
-      for (int w = threadIdx.x; w < words; w += 128) pay[w] = 0u;
+      for (int w = threadIdx.x; w < words; w += nt) pay[w] = 0u;
       if (threadIdx.x < 2) A.side[2 * row + threadIdx.x] = 0u;
     }
     return;
   }
   // the reference's row sum: a xor-butterfly over each run of 32 values, then the eight runs in order (src/kvq_fast.cuh:33-43)
-  auto runs = [&](float va, float vb, float* out) {
+  auto run_sum = [&](float v) {
     #pragma unroll
-    for (int o = 16; o; o >>= 1) { va += __shfl_xor_sync(0xffffffffu, va, o); vb += __shfl_xor_sync(0xffffffffu, vb, o); }
-    if (lane == 0) { out[2 * c] = va; out[2 * c + 1] = vb; }
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
   };
   auto rowsum = [&](float va, float vb) -> float {
-    runs(va, vb, S.red);
+    va = run_sum(va); vb = run_sum(vb);
+    if (own && lane == 0) { S.red[2 * c] = va; S.red[2 * c + 1] = vb; }
     __syncthreads();
     float t = 0.f;
     #pragma unroll
@@ -187,27 +208,29 @@ __global__ void __launch_bounds__(128, 7) tb_encode_kernel(TbP A) {
     __syncthreads();
     return t;
   };
-  const uint8_t* mup = b + P.go + 8;
-  const uint8_t* Up = mup + (P.has_mu ? 512 : 0);
   auto f16at = [&](const uint8_t* p, int d) { return __half2float(__ushort_as_half((unsigned short)tb_u16(p + 2 * d))); };
-  float mua = 0.f, mub = 0.f, u0a = 0.f, u0b = 0.f, u1a = 0.f, u1b = 0.f, c0 = 0.f, c1 = 0.f;
-  if (P.has_mu) { mua = f16at(mup, d0); mub = f16at(mup, d1); ra = __fsub_rn(ra, mua); rb = __fsub_rn(rb, mub); }
-  if (P.m > 0) {
-    u0a = f16at(Up, d0); u0b = f16at(Up, d1);
-    c0 = tb_f16r(rowsum(__fmul_rn(ra, u0a), __fmul_rn(rb, u0b)));
-    ra = __fsub_rn(ra, __fmul_rn(c0, u0a)); rb = __fsub_rn(rb, __fmul_rn(c0, u0b));
-  }
-  if (P.m > 1) {
-    u1a = f16at(Up + 512, d0); u1b = f16at(Up + 512, d1);
-    c1 = tb_f16r(rowsum(__fmul_rn(ra, u1a), __fmul_rn(rb, u1b)));
-    ra = __fsub_rn(ra, __fmul_rn(c1, u1a)); rb = __fsub_rn(rb, __fmul_rn(c1, u1b));
+  float c0 = 0.f, c1 = 0.f;
+  {
+    const uint8_t* mup = b + P.go + 8;
+    const uint8_t* Up = mup + (P.has_mu ? 512 : 0);
+    if (P.has_mu) { ra = __fsub_rn(ra, f16at(mup, d0)); rb = __fsub_rn(rb, f16at(mup, d1)); }
+    if (P.m > 0) {
+      const float ua = f16at(Up, d0), ub = f16at(Up, d1);
+      c0 = tb_f16r(rowsum(__fmul_rn(ra, ua), __fmul_rn(rb, ub)));
+      ra = __fsub_rn(ra, __fmul_rn(c0, ua)); rb = __fsub_rn(rb, __fmul_rn(c0, ub));
+    }
+    if (P.m > 1) {
+      const float ua = f16at(Up + 512, d0), ub = f16at(Up + 512, d1);
+      c1 = tb_f16r(rowsum(__fmul_rn(ra, ua), __fmul_rn(rb, ub)));
+      ra = __fsub_rn(ra, __fmul_rn(c1, ua)); rb = __fsub_rn(rb, __fmul_rn(c1, ub));
+    }
   }
   float xqa, xqb, psc; int fa, fb, kb;
   if (P.mode == 1) {                                     // flat 4-bit codes (src/kvq_fast.cuh:193-198)
     float am = fmaxf(fabsf(ra), fabsf(rb));
     #pragma unroll
     for (int o = 16; o; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-    if (lane == 0) S.red[c] = am;
+    if (own && lane == 0) S.red[c] = am;
     __syncthreads();
     am = fmaxf(fmaxf(S.red[0], S.red[1]), fmaxf(S.red[2], S.red[3]));
     float s7 = __fdiv_rn(am, 7.f); if (s7 == 0.f) s7 = 1.f;
@@ -217,50 +240,68 @@ __global__ void __launch_bounds__(128, 7) tb_encode_kernel(TbP A) {
     const unsigned to = tb_table(b, P);
     const float gain = tb_f32(b + to + 4);
     int cm = 0;
-    for (int i = threadIdx.x; i < 256; i += 128) { const int v = (short)tb_u16(b + to + 12 + 2 * i); S.code[i] = (short)v; cm = max(cm, abs(v)); }
+    for (int i = threadIdx.x; i < 256; i += nt) { const int v = (short)tb_u16(b + to + 12 + 2 * i); S.code[i] = (short)v; cm = max(cm, abs(v)); }
     cm = __reduce_max_sync(0xffffffffu, cm);
     if (lane == 0) S.cmax[c] = cm;
-    float rms = __fsqrt_rn(__fdiv_rn(rowsum(__fmul_rn(ra, ra), __fmul_rn(rb, rb)), 256.f));     // its barriers also publish the codes
+    if (own) { S.res[d0] = ra; S.res[d1] = rb; }
+    if (threadIdx.x == 0) { S.grp = P; S.coef[0] = c0; S.coef[1] = c1; }
+    float rms = __fsqrt_rn(__fdiv_rn(rowsum(__fmul_rn(ra, ra), __fmul_rn(rb, rb)), 256.f));     // its barriers also publish the codes and the row
     if (rms == 0.f) rms = 1.f;
-    const bool narrow = max(max(S.cmax[0], S.cmax[1]), max(S.cmax[2], S.cmax[3])) <= 1400;
+    for (int w = 0; w < nwarps; ++w) cm = max(cm, S.cmax[w]);
+    const bool narrow = cm <= 1400;
     auto scale = [&](int mi) { const float s = tb_f16r(__fmul_rn(rms, tb_f32(b + P.off_m + 4u * (unsigned)mi))); return s == 0.f ? 1.f : s; };
     auto value = [&](int st, float s) { return __fmul_rn(__fmul_rn(__fmul_rn((float)(int)S.code[st], 0.00390625f), gain), s); };
     #pragma unroll 1
-    for (int mi = 0; mi < A.nm; ++mi) {
+    for (int unit = c; unit < 2 * A.nm; unit += nwarps) {                    // a multiplier and two of the four chains
+      const int mi = unit >> 1, e0 = 128 * (unit & 1);
       const float s = scale(mi);
-      const int xa = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(ra, s), 256.f)), -2048.f), 2048.f);
-      const int xb = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(rb, s), 256.f)), -2048.f), 2048.f);
-      int2 st = make_int2(0, 0);
-      if (P.kk == 3) st = narrow ? tb_search<3, int>(S.bp[c], S.code, xa, xb, lane) : tb_search<3, long long>(S.bp[c], S.code, xa, xb, lane);
-      else if (P.kk == 4) st = narrow ? tb_search<4, int>(S.bp[c], S.code, xa, xb, lane) : tb_search<4, long long>(S.bp[c], S.code, xa, xb, lane);
-      else if (P.kk == 5) st = narrow ? tb_search<5, int>(S.bp[c], S.code, xa, xb, lane) : tb_search<5, long long>(S.bp[c], S.code, xa, xb, lane);
-      const float da = __fsub_rn(ra, value(st.x, s)), db = __fsub_rn(rb, value(st.y, s));
-      runs(__fmul_rn(da, da), __fmul_rn(db, db), S.mult[mi].err);
-      S.mult[mi].st[d0] = (uint8_t)st.x; S.mult[mi].st[d1] = (uint8_t)st.y;
+      TbRowSmem::Warp& B = warps[c];
+      #pragma unroll
+      for (int r = 0; r < 4; ++r)
+        B.xs[32 * r + lane] = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(S.res[e0 + 32 * r + lane], s), 256.f)), -2048.f), 2048.f);
+      __syncwarp();
+      const int h = lane >> 4;
+      uint8_t* const st = mult[mi].st + e0;
+      auto search = [&](auto kk) {
+        constexpr int KK = decltype(kk)::value;
+        if (narrow) tb_search<KK, int>(B.bp[h], S.code, B.xs + 64 * h, st + 64 * h, lane); else tb_search<KK, long long>(B.bp[h], S.code, B.xs + 64 * h, st + 64 * h, lane);
+      };
+      if (P.kk == 3) search(std::integral_constant<int, 3>{});
+      else if (P.kk == 4) search(std::integral_constant<int, 4>{});
+      else if (P.kk == 5) search(std::integral_constant<int, 5>{});
+      else { for (int r = 0; r < 4; ++r) st[32 * r + lane] = 0; __syncwarp(); }
+      #pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float d = __fsub_rn(S.res[e0 + 32 * r + lane], value(st[32 * r + lane], s)), e = run_sum(__fmul_rn(d, d));
+        if (lane == 0) mult[mi].err[4 * (unit & 1) + r] = e;
+      }
     }
     __syncthreads();
     float best_e = 0.f; int best = 0;
     for (int mi = 0; mi < A.nm; ++mi) {                  // the smallest squared error, the first on ties
       float e = 0.f;
       #pragma unroll
-      for (int w = 0; w < 8; ++w) e = __fadd_rn(e, S.mult[mi].err[w]);
+      for (int w = 0; w < 8; ++w) e = __fadd_rn(e, mult[mi].err[w]);
       if (mi == 0 || e < best_e) { best_e = e; best = mi; }
     }
+    P = S.grp; c0 = S.coef[0]; c1 = S.coef[1];
     const float s = scale(best);
-    const int sa = S.mult[best].st[d0], sb = S.mult[best].st[d1];
+    const int sa = mult[best].st[d0], sb = mult[best].st[d1];
     xqa = value(sa, s); xqb = value(sb, s);
     fa = sa & ((1 << P.kk) - 1); fb = sb & ((1 << P.kk) - 1); psc = s; kb = P.kk;
   }
-  if (A.y) {
-    if (P.m > 0) { xqa = __fadd_rn(xqa, __fmul_rn(c0, u0a)); xqb = __fadd_rn(xqb, __fmul_rn(c0, u0b)); }
-    if (P.m > 1) { xqa = __fadd_rn(xqa, __fmul_rn(c1, u1a)); xqb = __fadd_rn(xqb, __fmul_rn(c1, u1b)); }
-    if (P.has_mu) { xqa = __fadd_rn(xqa, mua); xqb = __fadd_rn(xqb, mub); }
+  if (A.y && own) {
+    const uint8_t* mup = b + P.go + 8;
+    const uint8_t* Up = mup + (P.has_mu ? 512 : 0);
+    if (P.m > 0) { xqa = __fadd_rn(xqa, __fmul_rn(c0, f16at(Up, d0))); xqb = __fadd_rn(xqb, __fmul_rn(c0, f16at(Up, d1))); }
+    if (P.m > 1) { xqa = __fadd_rn(xqa, __fmul_rn(c1, f16at(Up + 512, d0))); xqb = __fadd_rn(xqb, __fmul_rn(c1, f16at(Up + 512, d1))); }
+    if (P.has_mu) { xqa = __fadd_rn(xqa, f16at(mup, d0)); xqb = __fadd_rn(xqb, f16at(mup, d1)); }
     A.y[(size_t)row * 256 + d0] = xqa; A.y[(size_t)row * 256 + d1] = xqb;
   }
   if (pay) {
-    S.fld[d0] = (uint8_t)fa; S.fld[d1] = (uint8_t)fb;
+    if (own) { S.fld[d0] = (uint8_t)fa; S.fld[d1] = (uint8_t)fb; }
     __syncthreads();
-    for (int w = threadIdx.x; w < (A.whole ? words : 8 * kb); w += 128) {     // MSB-first bit stream, 32 bits per word (src/kvq_fast.cuh:228-232)
+    for (int w = threadIdx.x; w < (A.whole ? words : 8 * kb); w += nt) {      // MSB-first bit stream, 32 bits per word (src/kvq_fast.cuh:228-232)
       unsigned v = 0u;
       if (w < 8 * kb) {
         const int e0 = 32 * w / kb;                      // the field that holds the word's first bit
@@ -799,8 +840,14 @@ int launch_tb_encode(const uint8_t* blob, int nm, const float* x, const int* grp
   if (rows <= 0 || nm < 1 || nm > TB_NM) KV4_REJECT("yskn_tb_encode: bad shape (rows %d, multipliers %d)", rows, nm);
   if (pay && (pay_stride < 160 || pay_stride % 4 || ((uintptr_t)pay & 3))) KV4_REJECT("yskn_tb_encode: payload rows need a stride of at least 160 bytes, a multiple of 4");
   static std::atomic<unsigned long long> attr{0};
-  if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(tb_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TbRowSmem::bytes(TB_NM)));
-  tb_encode_kernel<<<rows, 128, TbRowSmem::bytes(nm), st>>>(TbP{blob, nm, x, grp, pos, rows, y, pay, pay_stride, side, whole});
+  if (first_use_on_device(attr)) {
+    KV4_CUDA(cudaFuncSetAttribute(tb_encode_kernel<TB_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TbRowSmem::bytes(TB_NM, TB_WIDE)));
+    KV4_CUDA(cudaFuncSetAttribute(tb_encode_kernel<TB_NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TbRowSmem::bytes(TB_NM, TB_NARROW)));
+  }
+  const TbP P{blob, nm, x, grp, pos, rows, y, pay, pay_stride, side, whole};
+  const int most = rows <= TB_WIDE_ROWS ? TB_WIDE : TB_NARROW;
+  auto kern = most == TB_WIDE ? tb_encode_kernel<TB_WIDE> : tb_encode_kernel<TB_NARROW>;
+  kern<<<rows, 32 * TbRowSmem::warps(nm, most), TbRowSmem::bytes(nm, most), st>>>(P);
   return launch_status("tb_encode_kernel");
 }
 
