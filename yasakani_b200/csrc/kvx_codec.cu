@@ -53,32 +53,36 @@ __global__ void __launch_bounds__(256) kvx_rotate_kernel(const float* x, float* 
   if (live) store_row<YSKN_KV4_F32>(y, (size_t)row, ll, v);
 }
 
-// INT8 row from the rotated values: scale = max|v| / 127, q = rne(v / scale) clamped to +-127 (src/kvx_codec.cuh:50-70).
+// INT8 codes of a row from its rotated values: scale = max|v| / 127, q = rne(v / scale) clamped to +-127 (src/kvx_codec.cuh:50-70).
+struct Int8Scale {
+  float scale, inv;
+  __device__ __forceinline__ explicit Int8Scale(float amax) { scale = __fdiv_rn(amax, 127.f); inv = scale > 0.f ? __fdiv_rn(1.f, scale) : 0.f; }
+  // q = rne(fl(v / scale)).  v * (1 / scale) is within 3.8e-5 of the correctly rounded quotient (|q| <= 127), so rounding it gives
+  // the same integer unless it lies that close to a half-integer; only those elements (about one in 10^4) take the exact division.
+  __device__ __forceinline__ int code(float v) const {
+    const float t = __fmul_rn(v, inv);
+    int q = __float2int_rn(t);
+    // distance of t from the integer it rounds to; near 0.5 (or NaN: 1/scale overflowed) -> the reference's own arithmetic.
+    // |v| <= max|v| makes |v / scale| <= 127 (1 + 2^-23), so the reference's clamp to +-127 can only act on that path.
+    if (!(fabsf(__fsub_rn(t, (float)q)) <= 0.5f - 6.2e-5f)) q = max(-127, min(127, scale > 0.f ? __float2int_rn(__fdiv_rn(v, scale)) : 0));
+    return q;
+  }
+};
 __device__ __forceinline__ void store_int8_row(const float (&v)[32], int ll, bool live, int8_t* q8, float* scales, size_t row) {
   float amax = 0.f;
   #pragma unroll
   for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[i]));
   #pragma unroll
   for (int m = 4; m; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-  const float sc = __fdiv_rn(amax, 127.f);
-  // q = rne(fl(v / sc)).  v * (1 / sc) is within 3.8e-5 of the correctly rounded quotient (|q| <= 127), so rounding it gives
-  // the same integer unless it lies that close to a half-integer; only those elements (about one in 10^4) take the exact division.
-  const float inv = sc > 0.f ? __fdiv_rn(1.f, sc) : 0.f;
+  const Int8Scale sc(amax);
   #pragma unroll
   for (int k = 0; k < 8; ++k) {
     uint32_t w = 0u;
     #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float xv = v[4 * k + e], t = __fmul_rn(xv, inv);
-      int q = __float2int_rn(t);
-      // distance of t from the integer it rounds to; near 0.5 (or NaN: 1/scale overflowed) -> the reference's own arithmetic.
-      // |v| <= max|v| makes |v / scale| <= 127 (1 + 2^-23), so the reference's clamp to +-127 can only act on that path.
-      if (!(fabsf(__fsub_rn(t, (float)q)) <= 0.5f - 6.2e-5f)) q = max(-127, min(127, sc > 0.f ? __float2int_rn(__fdiv_rn(xv, sc)) : 0));
-      w |= ((uint32_t)q & 0xFFu) << (8 * e);
-    }
+    for (int e = 0; e < 4; ++e) w |= ((uint32_t)sc.code(v[4 * k + e]) & 0xFFu) << (8 * e);
     if (live) *reinterpret_cast<uint32_t*>(q8 + row * 256 + 32 * k + 4 * ll) = w;
   }
-  if (live && ll == 0) scales[row] = sc;
+  if (live && ll == 0) scales[row] = sc.scale;
 }
 
 template <int DT>
@@ -119,74 +123,138 @@ __global__ void __launch_bounds__(256) kvx_decode_kernel(const int8_t* q8, const
 // 2, 1 = register pairs) followed by the in-order sum of the eight warp sums.  NRH = rotary width / 64.
 __device__ __forceinline__ float rbf(float f) { return bf2f(f2bf(f)); }
 
+// One warp per row; lane l owns channels 4l .. 4l + 3 (v[0..3]) and 128 + 4l .. (v[4..7]), so a run of 32 channels is eight lanes.  Bound by instruction issue
+// and, for a few tokens, by the length of a warp's straight-line code.  (With eight lanes a row, four rows a warp, a warp had 1,000 instructions and
+// the GPU a quarter of the warps: steps of one token over 500 / 32,768 INT8 rows 13.9 / 25.5 us, now 11.4 / 22.8; 100 rows behind 3,000 tokens 40.0, now 32.7.)
 template <int NRH>
-__global__ void __launch_bounds__(256, 4) kvx_attn_post_kernel(yskn_kvx_attn_post_args A) {
-  const int lane = threadIdx.x & 31, ll = lane & 7;
+__global__ void __launch_bounds__(256) kvx_attn_post_kernel(yskn_kvx_attn_post_args A) {
+  const int lane = threadIdx.x & 31;
   asm volatile("griddepcontrol.wait;" ::: "memory");           // programmatic dependent launch, both directions
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int per_tok = A.nh + 2 * A.kvh;
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3);
-  const bool live = item < (long long)A.M * per_tok;
-  const int tok = live ? (int)(item / per_tok) : 0, u = live ? (int)(item % per_tok) : 0;
+  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (item >= (long long)A.M * per_tok) return;
+  const int tok = (int)(item / per_tok), u = (int)(item - (long long)tok * per_tok);
   const int kind = u < A.nh ? 0 : (u < A.nh + A.kvh ? 1 : 2);    // query / key / value head
   const int head = kind == 0 ? u : (kind == 1 ? u - A.nh : u - A.nh - A.kvh);
-  const int pos = *A.d_pos + tok;
-  const uint16_t* src = kind == 0 ? A.q_rows + ((size_t)tok * A.nh + head) * 512
-                                  : (kind == 1 ? A.k_rows : A.v_rows) + ((size_t)tok * A.kvh + head) * 256;
-  float v[32];
-  load_row<YSKN_KV4_BF16>(src, 0, ll, live, v);
-  if (live && kind == 0) {                                       // the gate half of the head's projection, as it is
-    uint2 gate[8];                                               // all loads ahead of the first store
-    #pragma unroll
-    for (int k = 0; k < 8; ++k) gate[k] = *reinterpret_cast<const uint2*>(src + 256 + 32 * k + 4 * ll);
-    #pragma unroll
-    for (int k = 0; k < 8; ++k) *reinterpret_cast<uint2*>(A.gate16 + ((size_t)tok * A.nh + head) * 256 + 32 * k + 4 * ll) = gate[k];
+  const uint16_t* src = (kind == 0 ? A.q_rows + ((size_t)tok * A.nh + head) * 512
+                                   : (kind == 1 ? A.k_rows : A.v_rows) + ((size_t)tok * A.kvh + head) * 256) + 4 * lane;
+  const uint2 in[2] = {*reinterpret_cast<const uint2*>(src), *reinterpret_cast<const uint2*>(src + 128)};
+  const size_t orow = ((size_t)tok * A.nh + head) * 256 + 4 * lane;
+  if (kind == 0) {                                               // the gate half of the head's projection, as it is
+    const uint2 g0 = *reinterpret_cast<const uint2*>(src + 256), g1 = *reinterpret_cast<const uint2*>(src + 384);
+    *reinterpret_cast<uint2*>(A.gate16 + orow) = g0; *reinterpret_cast<uint2*>(A.gate16 + orow + 128) = g1;
   }
-  // ---- RMS norm (all lanes of a warp run the shuffles unless its four rows are all value heads, which keep their rows)
-  float tot = 0.f;
-  const bool any_norm = !__all_sync(0xffffffffu, kind == 2);
+  const int pos = *A.d_pos + tok;
+  float v[8];
   #pragma unroll
-  for (int k = 0; k < 8 && any_norm; ++k) {
-    float t[4];
-    #pragma unroll
-    for (int e = 0; e < 4; ++e) t[e] = __fmul_rn(v[4 * k + e], v[4 * k + e]);
-    #pragma unroll
-    for (int m = 4; m; m >>= 1) {
-      #pragma unroll
-      for (int e = 0; e < 4; ++e) t[e] = __fadd_rn(t[e], __shfl_xor_sync(0xffffffffu, t[e], m));
-    }
-    tot = __fadd_rn(tot, __fadd_rn(__fadd_rn(t[0], t[2]), __fadd_rn(t[1], t[3])));
+  for (int h = 0; h < 2; ++h) {
+    v[4 * h] = __uint_as_float(in[h].x << 16); v[4 * h + 1] = __uint_as_float(in[h].x & 0xffff0000u);
+    v[4 * h + 2] = __uint_as_float(in[h].y << 16); v[4 * h + 3] = __uint_as_float(in[h].y & 0xffff0000u);
   }
   if (kind != 2) {
+    // ---- RMS norm
+    const uint16_t* wn = (kind == 0 ? A.qn_w : A.kn_w) + 4 * lane;
+    const uint2 wv[2] = {ld_table(reinterpret_cast<const uint2*>(wn)), ld_table(reinterpret_cast<const uint2*>(wn + 128))};
+    float run[2];                                                // sums of squares of runs lane / 8 and 4 + lane / 8
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float t[4];
+      #pragma unroll
+      for (int e = 0; e < 4; ++e) t[e] = __fmul_rn(v[4 * h + e], v[4 * h + e]);
+      #pragma unroll
+      for (int m = 4; m; m >>= 1)
+        #pragma unroll
+        for (int e = 0; e < 4; ++e) t[e] = __fadd_rn(t[e], __shfl_xor_sync(0xffffffffu, t[e], m));
+      run[h] = __fadd_rn(__fadd_rn(t[0], t[2]), __fadd_rn(t[1], t[3]));
+    }
+    float tot = 0.f;
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, run[k >> 2], 8 * (k & 3)));
     const float x = __fadd_rn(__fdiv_rn(tot, 256.f), A.eps);
     const float r = A.pm ? __fdiv_rn(1.f, __fsqrt_rn(x)) : rsqrtf(x);
-    const uint16_t* wn = kind == 0 ? A.qn_w : A.kn_w;
     #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint2 w = ld_table(reinterpret_cast<const uint2*>(wn + 32 * k + 4 * ll));
-      const uint16_t wb[4] = {(uint16_t)w.x, (uint16_t)(w.x >> 16), (uint16_t)w.y, (uint16_t)(w.y >> 16)};
-      #pragma unroll
-      for (int e = 0; e < 4; ++e) v[4 * k + e] = rbf(__fmul_rn(__fmul_rn(v[4 * k + e], r), __fadd_rn(1.f, bf2f(wb[e]))));
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t w2 = i & 2 ? wv[i >> 2].y : wv[i >> 2].x;
+      const float w = __uint_as_float(i & 1 ? w2 & 0xffff0000u : w2 << 16);
+      v[i] = rbf(__fmul_rn(__fmul_rn(v[i], r), __fadd_rn(1.f, w)));
     }
-    // ---- rotate-half over the first 64*NRH channels: pair (d, d + 32*NRH) sits in one lane (registers k and k + NRH)
-    #pragma unroll
-    for (int k = 0; k < NRH; ++k) {
-      const float4* rr = reinterpret_cast<const float4*>(A.rope + ((size_t)pos * (32 * NRH) + 32 * k + 4 * ll) * 2);
-      const float4 c01 = live ? ld_table(rr) : make_float4(0.f, 0.f, 0.f, 0.f), c23 = live ? ld_table(rr + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float cs[4] = {c01.x, c01.z, c23.x, c23.z}, sn[4] = {c01.y, c01.w, c23.y, c23.w};
+    // ---- rotate-half over the first 64 * NRH channels, pairs (d, d + 32 * NRH): the partner is NRH runs away
+    if constexpr (NRH > 0) {
+      float p[8];                                                // partners of v
       #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float lo = v[4 * k + e], hi = v[4 * (k + NRH) + e];
-        v[4 * k + e] = rbf(__fadd_rn(rbf(__fmul_rn(lo, cs[e])), rbf(__fmul_rn(-hi, sn[e]))));
-        v[4 * (k + NRH) + e] = rbf(__fadd_rn(rbf(__fmul_rn(hi, cs[e])), rbf(__fmul_rn(lo, sn[e]))));
+        if (NRH == 1 || NRH == 2) p[e] = __shfl_xor_sync(0xffffffffu, v[e], 8 * NRH);
+        else if (NRH == 4) { p[e] = v[4 + e]; p[4 + e] = v[e]; }
+        else {                                                   // runs 0, 1, 2 with 3, 4, 5: run 3 is the first half's last, 4 and 5 are the second half's first
+          const float a = __shfl_sync(0xffffffffu, v[e], lane < 8 ? lane + 24 : lane - 24), b = __shfl_sync(0xffffffffu, v[4 + e], lane - 8);
+          p[e] = lane < 8 || lane >= 24 ? a : b;
+          p[4 + e] = __shfl_sync(0xffffffffu, v[e], lane + 8);
+        }
+      }
+      #pragma unroll
+      for (int h = 0; h < (NRH > 2 ? 2 : 1); ++h) {
+        const int d = 128 * h + 4 * lane;
+        if (d >= 64 * NRH) continue;
+        const bool up = d >= 32 * NRH;                           // the upper channel of its pair
+        const float4* rr = reinterpret_cast<const float4*>(A.rope + ((size_t)pos * (32 * NRH) + d - (up ? 32 * NRH : 0)) * 2);
+        const float4 c01 = ld_table(rr), c23 = ld_table(rr + 1);
+        const float cs[4] = {c01.x, c01.z, c23.x, c23.z}, sn[4] = {c01.y, c01.w, c23.y, c23.w};
+        #pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float q = p[4 * h + e];
+          v[4 * h + e] = rbf(__fadd_rn(rbf(__fmul_rn(v[4 * h + e], cs[e])), rbf(__fmul_rn(up ? q : -q, sn[e]))));
+        }
       }
     }
   }
-  apply_signs(v, ll);
-  hadamard256(v, ll);
-  if (live && kind == 0) store_row<YSKN_KV4_BF16>(A.q16, (size_t)tok * A.nh + head, ll, v);
-  const bool cache = live && kind != 0 && pos >= 0 && pos < A.max_ctx;     // a position outside the cache stores nothing
-  store_int8_row(v, ll, cache, kind == 2 ? A.v8 : A.k8, kind == 2 ? A.vs : A.ks, (size_t)head * A.max_ctx + (cache ? pos : 0));
+  // ---- signs and butterflies, stages h = 1 ... 128 in order: lower index a + b, upper lower - upper
+  const uint32_t sg[2] = {c_signs.w[lane >> 3] >> (4 * (lane & 7)), c_signs.w[4 + (lane >> 3)] >> (4 * (lane & 7))};
+  #pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ (((sg[i >> 2] >> (i & 3)) & 1u) << 31));
+  #pragma unroll
+  for (int rb = 1; rb < 4; rb *= 2)
+    #pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (!(i & rb)) { const float lo = v[i], hi = v[i + rb]; v[i] = __fadd_rn(lo, hi); v[i + rb] = __fsub_rn(lo, hi); }
+  #pragma unroll
+  for (int m = 1; m < 32; m *= 2) {
+    const float flip = (lane & m) ? -1.f : 1.f;                  // the product is exact: one rounding, as of the sum
+    #pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = fmaf(v[i], flip, __shfl_xor_sync(0xffffffffu, v[i], m));
+  }
+  #pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float lo = v[i], hi = v[4 + i];
+    v[i] = __fmul_rn(__fadd_rn(lo, hi), 0.0625f); v[4 + i] = __fmul_rn(__fsub_rn(lo, hi), 0.0625f);
+  }
+  if (kind == 0) {
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint2 o;
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o.x) : "f"(v[4 * h + 1]), "f"(v[4 * h]));
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o.y) : "f"(v[4 * h + 3]), "f"(v[4 * h + 2]));
+      *reinterpret_cast<uint2*>(A.q16 + orow + 128 * h) = o;
+    }
+    return;
+  }
+  if (pos < 0 || pos >= A.max_ctx) return;                       // a position outside the cache stores nothing
+  float amax = 0.f;
+  #pragma unroll
+  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  #pragma unroll
+  for (int m = 16; m; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
+  const Int8Scale sc(amax);
+  const size_t row = (size_t)head * A.max_ctx + pos;
+  int8_t* dst = (kind == 2 ? A.v8 : A.k8) + row * 256 + 4 * lane;
+  #pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t w = 0u;
+    #pragma unroll
+    for (int e = 0; e < 4; ++e) w |= ((uint32_t)sc.code(v[4 * h + e]) & 0xFFu) << (8 * e);
+    *reinterpret_cast<uint32_t*>(dst + 128 * h) = w;
+  }
+  if (lane == 0) (kind == 2 ? A.vs : A.ks)[row] = sc.scale;
 }
 
 int grid_for(long long rows, unsigned* grid, const char* who) {
@@ -241,11 +309,11 @@ int launch_kvx_attn_post(const yskn_kvx_attn_post_args& a, cudaStream_t st) {
        (uintptr_t)a.k8 | (uintptr_t)a.v8) & 7)
     KV4_REJECT("yskn_kvx_attn_post: row arrays must be 8-byte aligned");
   if ((uintptr_t)a.rope & 15) KV4_REJECT("yskn_kvx_attn_post: the rope table must be 16-byte aligned");
-  // A few tokens are bound by the latency of one warp's straight-line code: one-warp blocks put every four rows on an SM of their own
-  // (one token of the 27B shape is 32 rows, a single block of 256 threads).  From a block per SM on, blocks of 32 rows.
+  // One-warp blocks spread a few tokens over the SMs; from eight rows an SM on, blocks of eight.
   const long long rows = (long long)a.M * (a.nh + 2 * a.kvh);
-  const int threads = rows < 148 * ROWS_PER_BLOCK ? 32 : 256;
-  unsigned grid; if (grid_for(rows * (256 / threads), &grid, "yskn_kvx_attn_post")) return -1;
+  const int threads = rows < 148 * 8 ? 32 : 256;
+  if (rows > (1ll << 33)) KV4_REJECT("yskn_kvx_attn_post: bad row count %lld", rows);
+  const unsigned grid = (unsigned)((rows + threads / 32 - 1) / (threads / 32));
   switch (a.rd / 64) {
     case 0: return launch_pdl("kvx_attn_post_kernel", kvx_attn_post_kernel<0>, dim3(grid), threads, 0, st, a);
     case 1: return launch_pdl("kvx_attn_post_kernel", kvx_attn_post_kernel<1>, dim3(grid), threads, 0, st, a);
