@@ -1,4 +1,4 @@
-"""The KV4 merge against double precision on both sides of the line between its two forms (rows x heads above 296 take a warp each): one split,
+"""The KV4 merge against double precision on both sides of the line between its two forms (many rows x heads take a warp each): one split,
 the edges of a batch of loads and of a warp's lanes of weights, empty splits, bias and gate, a partial buffer that is aligned for no wide load."""
 import pytest
 import torch
@@ -35,3 +35,9 @@ def test_merge_matches_double_precision(M, nh, g, hd, S, dtype, shift):
 @pytest.mark.parametrize("S", [20, 21, 37])
 def test_merge_on_both_sides_of_the_line_for_128_channels(M, S):
     test_merge_matches_double_precision(M, 16, 8, 128, S, torch.float16, 0)
+
+
+@pytest.mark.parametrize("M", [6, 7])                             # 144 and 168 rows x heads: with up to 20 splits a warp each from 149 on
+@pytest.mark.parametrize("S", [1, 20, 21, 37])
+def test_merge_on_both_sides_of_the_line_for_256_channels(M, S):
+    test_merge_matches_double_precision(M, 24, 6, 256, S, torch.bfloat16, 0)

@@ -283,15 +283,16 @@ __global__ void __launch_bounds__(128) kv4_combine_rows_kernel(CombineP P, int i
 template <int HD, int DT, bool TI, bool TO, bool PEER>
 int launch_k(const CombineP& P, size_t smem, cudaStream_t st) {
   const long long blocks = (long long)P.nh * P.M;
-  // The form for many rows (64 rows in 9 splits, behind the attention kernel: 13.2 -> 5.2 us) from where the blocks below no longer fit the GPU at
-  // once: two of 512 threads on each of 148 SMs for head_dim 256, four of 256 threads for 128.  us per merge of rows x heads, blocks / warps:
-  //   head_dim 256   18 splits   312: 4.2 / 2.8   1,536: 12.8 / 5.1      37 splits   288: 5.5 / 4.7   312: 5.9 / 4.9   1,536: 23.7 / 12.3
-  //   head_dim 128   18 splits   304: 2.6 / 2.2     576:  2.7 / 2.8   1,536: 6.2 / 3.2
-  //                  21 splits   304: 3.1 / 3.2     576:  3.2 / 4.1     768: 4.7 / 4.3     37 splits   576: 3.9 / 4.7   768: 5.6 / 4.9
-  // With up to 20 splits, which a warp requests at once, it wins from 296 for 128 channels too (and, not made use of, below: 192 rows x heads
-  // of 256 channels in 18 splits 4.9 / 2.6).
+  // The form of a warp per 128 channels and row (64 rows in 9 splits, behind the attention kernel: 13.2 -> 5.2 us) from where the blocks below no longer fit
+  // the GPU at once: two of 512 threads on each of 148 SMs for head_dim 256, four of 256 threads for 128.  us per merge of rows x heads, blocks / warps, replays:
+  //   head_dim 256   18-19 splits   48: 2.9 / 2.1    192: 5.1 / 2.5   288: 5.3 / 2.9   1,536: 12.8 / 5.1      37 splits   48: 3.0 / 3.3   192: 5.5 / 4.0   312: 5.9 / 4.9
+  //   head_dim 128   18 splits     304: 2.6 / 2.2    576: 2.7 / 2.8   1,536: 6.2 / 3.2
+  //                  21 splits     304: 3.1 / 3.2    576: 3.2 / 4.1     768: 4.7 / 4.3     37 splits   576: 3.9 / 4.7   768: 5.6 / 4.9
+  // Behind an attention kernel the lines are later than that, since the blocks are resident before it ends: whole steps of 48 / 96 / 192 / 288 rows x heads
+  // of 256 channels in 19 splits take 11.8 / 14.2 / 32.7 / 42.0 us with blocks and 12.6 / 15.1 / 31.5 / 40.7 with warps, of 192 in 37 splits 53.6 and 55.0.
+  // So up to 20 splits, which a warp requests at once, go to it from 149 rows x heads of 256 channels on.
   if constexpr (!TI && !TO && !PEER && HD >= 128)
-    if (blocks > (HD == 128 && P.S > 20 ? 592 : 296) && blocks < (1ll << 28) && !((uintptr_t)P.pacc & 15) && !((uintptr_t)P.o16 & 7))
+    if (blocks > (HD == 128 && P.S > 20 ? 592 : HD == 256 && P.S <= 20 ? 148 : 296) && blocks < (1ll << 28) && !((uintptr_t)P.pacc & 15) && !((uintptr_t)P.o16 & 7))
       return launch_pdl("kv4_combine_rows_kernel", kv4_combine_rows_kernel<HD, DT>, dim3((unsigned)((blocks * (HD / 128) + 3) / 4)), 128, 0, st, P, (int)blocks * (HD / 128));
   const int CQ = (P.S < 8 || (TI && !TO && PEER)) ? 1 : (blocks <= 296 ? 4 : 2);   // 296 = two 1,024-thread blocks on each of 148 SMs; the merge of pushed triples folds nothing
   cudaLaunchConfig_t cfg{};
