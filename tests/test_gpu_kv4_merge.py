@@ -41,3 +41,9 @@ def test_merge_on_both_sides_of_the_line_for_128_channels(M, S):
 @pytest.mark.parametrize("S", [1, 20, 21, 37])
 def test_merge_on_both_sides_of_the_line_for_256_channels(M, S):
     test_merge_matches_double_precision(M, 24, 6, 256, S, torch.bfloat16, 0)
+
+
+@pytest.mark.parametrize("M,nh", [(1, 16), (9, 16), (10, 16)])    # 16, 144 and 160 rows x heads: eight runs of splits up to 148
+@pytest.mark.parametrize("S", [40, 41, 74, 81, 160])
+def test_merge_of_many_splits_in_eight_runs(M, nh, S):
+    test_merge_matches_double_precision(M, nh, 8, 128, S, torch.float16, 0)

@@ -50,7 +50,8 @@ constexpr int CB = 10;                                   // loads in flight per 
 // mappings); with TRIPLE_IN, every thread polls (bounded) the slots it needs -- (m, l) of each rank and its own channel of
 // each rank's O -- until they carry this step's tag, and the last block of the grid opens the next step.
 // CQ = split runs per block: 4 when there are many splits to fetch and few blocks (decode: latency), 2 when the grid of
-// 1,024-thread blocks would not fit the GPU at once, 1 for short sums (both only where the form for many rows does not apply).
+// 1,024-thread blocks would not fit the GPU at once, 1 for short sums (both only where the form for many rows does not apply), 8 for more than 40 splits
+// of 128 channels in few blocks.
 template <int HD, int DT, bool TRIPLE_IN, bool TRIPLE_OUT, bool PEER, int CQ>
 __global__ void __launch_bounds__(CQ * HD) kv4_combine_kernel(CombineP P) {
   // TRIPLE_IN && TRIPLE_OUT && PEER = the fused exchange: fold the splits, push the triple, wait for the other ranks' triples, merge.
@@ -176,6 +177,8 @@ __global__ void __launch_bounds__(CQ * HD) kv4_combine_kernel(CombineP P) {
   s_part[q * HD + d] = o;
   __syncthreads();
   if (q != 0) return;
+  if (CQ == 8) o = ((s_part[d] + s_part[HD + d]) + (s_part[2 * HD + d] + s_part[3 * HD + d])) +
+                   ((s_part[4 * HD + d] + s_part[5 * HD + d]) + (s_part[6 * HD + d] + s_part[7 * HD + d]));
   if (CQ == 4) o = (s_part[d] + s_part[HD + d]) + (s_part[2 * HD + d] + s_part[3 * HD + d]);
   if (CQ == 2) o = s_part[d] + s_part[HD + d];
   float L2 = s_L2;
@@ -300,6 +303,14 @@ int launch_k(const CombineP& P, size_t smem, cudaStream_t st) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
+  if constexpr (!TI && !PEER && HD == 128)
+    // More than 40 splits are two round trips for four runs: eight, with 1,024 threads a block, while a block has an SM of its own (four rows of
+    // 16 heads in 74 splits over 2,000 tokens 18.8 -> 17.8 us with append and attention, one row over 100,000 24.2 -> 23.5)
+    if (P.S > 4 * CB && blocks <= 148 && smem + 4 * HD * sizeof(float) <= 48 * 1024) {
+      cfg.blockDim = dim3(8 * HD); cfg.dynamicSmemBytes = smem + 4 * HD * sizeof(float);
+      KV4_CUDA(cudaLaunchKernelEx(&cfg, kv4_combine_kernel<HD, DT, TI, TO, PEER, 8>, P));
+      return 0;
+    }
   if (CQ == 4) KV4_CUDA(cudaLaunchKernelEx(&cfg, kv4_combine_kernel<HD, DT, TI, TO, PEER, 4>, P));
   else if (CQ == 2) KV4_CUDA(cudaLaunchKernelEx(&cfg, kv4_combine_kernel<HD, DT, TI, TO, PEER, 2>, P));
   else KV4_CUDA(cudaLaunchKernelEx(&cfg, kv4_combine_kernel<HD, DT, TI, TO, PEER, 1>, P));
