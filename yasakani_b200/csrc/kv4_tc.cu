@@ -1133,7 +1133,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     if constexpr (STAGED_Q) {
       if (n > 0) {
         // bf16 activations, or the chunk order of the int4 form: these eight warps write this CTA's query rows (there is no Q copy)
-        tc_stage_q<HD, FORM == 1, FUSED ? 8 : 16>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, act_bf16, tok0, G, TOK, P.M, P.nh, kvh * G, threadIdx.x, 32 * TC_SW);
+        tc_stage_q<HD, FORM == 1, FUSED ? 4 : 16>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, act_bf16, tok0, G, TOK, P.M, P.nh, kvh * G, threadIdx.x, 32 * TC_SW);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) bar_arrive_cluster(lead_q);
