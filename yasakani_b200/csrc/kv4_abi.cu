@@ -375,12 +375,12 @@ int yskn_kv8_attention_tc(const yskn_kv8_attn_args* a, int act_dtype, void* cuda
   if (!a) KV4_REJECT("yskn_kv8_attention_tc: null argument struct");
   return launch_kv8_attention_tc(*a, act_dtype, (cudaStream_t)cuda_stream);
 }
-// Converting inside the kernel costs every pair of 128-row tiles its own pass over the keys (4.0 us per 128 keys, against 1.5 from
+// Converting inside the kernel costs every pair of 128-row tiles its own pass over the keys (2.3 us per 128 keys, against 1.3 from
 // fp16 rows); writing the rows first costs a launch and one pass over them.  The host does not know how many keys are visible, so
 // the line lies where the written rows win for any number of them, or lose less than that launch.  Attention alone, converting / written
-// rows, in us, behind 0 and 8,000 tokens: 127 rows 14.9 / 16.4 and 58 / 43; 300 rows 17.0 / 18.7 and 109 / 65; 384 rows 19.2 / 19.1 (in a cache
-// much larger than its contents 20.4) and 212 / 101; 500 rows 21.8 / 20.2 and 208 / 101; 1,000 rows 47.7 / 39 and 414 / 198, whatever the
-// capacity.  1,000 rows behind 3,001 tokens, with row epilogue and merge: 264 -> 149 us.
+// rows, in us, behind 0, 3,000 and 8,000 tokens: 127 rows 11.7 / 12.1, 25 / 23 and 45 / 41; 300 rows 14.7 / 15.0, 40 / 32 and 82 / 62; 384 rows 17.0 / 15.8 (a cache
+// much larger than its contents adds 1.3 to the written rows), 69 / 46 and 160 / 98; 500 rows 19.0 / 17.9, 72 / 48 and 162 / 100; 1,000 rows 39.6 / 33.3, 134 / 91 and
+// 328 / 197.
 // The workspace grows with the capacity, not with the visible keys.  It is taken up to 256 MiB (0.15 % of the GPU's memory); beyond it a
 // pass that needed no memory before would hold as much as several layers' caches, so larger caches keep the converting form.
 size_t yskn_kv8_workspace_bytes(const yskn_kv8_attn_args* a) {
