@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(256) kv8_tc_prep_kernel(const int8_t* k8, cons
 constexpr int TC_SW = 8;                                   // softmax warps: warp w owns rows 32*(w%4).., key columns 64*(w/4)..
 constexpr int TC_KW = 4, TC_VW = 3, TC_CW = TC_KW + TC_VW;  // converter warps of the fused forms: K half tiles, V half tiles
 // + producer warp, + MMA issuer warp; the fused form adds the converter warps and fills up to four warpgroups (16 warps x 128
-// registers at launch), so that setmaxnreg can move registers from the softmax warps (120 each) and the V converters (112) to the K converters (160)
+// registers at launch), so that setmaxnreg can move registers from the softmax warps to the converters
 // The workspace forms launch three warpgroups of 168 registers a thread (504 per scheduler lane): 208 for the two of softmax warps, whose threads hold
 // a whole row of a tile, 88 for producer and MMA issuer (two of its four warps have no role).
 constexpr int tc_threads(bool fused) { return fused ? 512 : 384; }
@@ -1387,14 +1387,18 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       }
     }
   };
-  // ---- roles.  In the converting forms each warpgroup first sets its register budget (120 / 120 / 112 / 160 per thread: 512
-  //      per scheduler lane) and the role code sits under that branch, so that each role is compiled for its own budget.
+  // ---- roles.  In the converting forms each warpgroup first sets its register budget (softmax twice, V, K: 512 per scheduler lane) and the role code sits
+  //      under that branch, so that each role is compiled for its own budget.  More registers are more of a role's arithmetic under way at once; steps of 64 / 16 int4 rows
+  //      and of 16 INT8 rows over 32,768 tokens, and of 350 behind 6,000, in us: 120 / 112 / 160 88.7 / 52.4 / 54.9 / 85.4; 104 / 136 / 168 87.9 / 52.4 / 53.5 / 84.4;
+  //      96 / 160 / 160 89.3 / 52.8 / 52.7 / 84.3; 96 / 176 / 144 96.5 / 56.6 / 52.2 / 83.0.
   if constexpr (FUSED) {
-    if (warp < TC_SW) { asm volatile("setmaxnreg.dec.sync.aligned.u32 120;"); role_softmax(); }
+    constexpr int RS = I8 ? 96 : 104, RV = I8 ? 176 : 136, RK = I8 ? 144 : 168;
+    static_assert(2 * RS + RV + RK == 512, "what the launch has: 16 warps of 128 registers");
+    if (warp < TC_SW) { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RS)); role_softmax(); }
     else if (warp < TC_SW + 4) {
-      asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RV));
       if (warp == TC_SW) role_mma(); else role_conv(false);
-    } else { asm volatile("setmaxnreg.inc.sync.aligned.u32 160;"); role_conv(true); }
+    } else { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RK)); role_conv(true); }
   } else {
     if (warp < TC_SW) { asm volatile("setmaxnreg.inc.sync.aligned.u32 208;"); role_softmax(); }
     else {
