@@ -14,7 +14,7 @@
 //     fp32 arithmetic, one rounding to fp16.  HBM-bound byte mover: one warp per (token, kv-head).
 //  2. kv4_tc_attn_kernel: a pair of CTAs (cluster of two, tcgen05 cta_group::2) = 256 query rows ((token, head) pairs
 //     of one kv-head, 128 per CTA) x one split of the keys, in tiles of 128 keys.  Per CTA:
-//       warp 8      TMA producer: its Q rows once (form 0), then its half of every K tile (64 keys) and V tile (HD/2 channels)
+//       warp 8      TMA producer: its Q rows once, then its half of every K tile (64 keys) and V tile (HD/2 channels)
 //                   into two mbarrier rings, one tiled copy each; the copies report to the leader CTA's barriers
 //       warp 9      (leader CTA only) one thread issues every tcgen05.mma of the pair: S = Q.K^T (M256 N128 K16 steps, Q and
 //                   K from shared memory, K-major, 128-byte swizzle) into one of two TMEM buffers, and O += P.V (M256
@@ -28,8 +28,8 @@
 //
 //  The attention kernel has five forms (template FORM): 0 = operand tiles by TMA from the workspace, as above; 3 = the same
 //  with bf16 queries and output rows; 4 = the same over a workspace of Family-B INT8 rows; 1 = no workspace and no prep launch,
-//  converter warps build the tiles from the packed KV4 cache inside the kernel; 2 = the same over Family-B INT8 rows.  Only form 0
-//  copies its queries by TMA, in the others the softmax warps stage them.  The converting forms (1, 2) run 16 warps: 0-7 softmax, 8 MMA
+//  converter warps build the tiles from the packed KV4 cache inside the kernel; 2 = the same over Family-B INT8 rows.  The workspace
+//  forms copy their queries by TMA (bf16 ones are converted where they land), in the others the softmax warps stage them.  The converting forms (1, 2) run 16 warps: 0-7 softmax, 8 MMA
 //  issue, 9-11 V tiles, 12-15 K tiles.
 //
 // Rows are independent of one another inside every step (an MMA output row depends on its own A row only, the lazy
@@ -178,7 +178,6 @@ __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) { asm vol
 __device__ __forceinline__ void bar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void bar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -194,6 +193,7 @@ __device__ __forceinline__ bool elect_one() {                         // true in
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 // Address of the leader CTA's copy (rank 0 of the pair) of a shared-memory location, in the cluster window.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t rank) { uint32_t r; asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank)); return r; }
 __device__ __forceinline__ uint32_t leader_addr(uint32_t local) { uint32_t r; asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(local)); return r; }
 // What the arrival publishes lives in tensor memory and is ordered by the tcgen05 fences around it, so the default
 // (CTA-scope) release is enough; a cluster-scope release costs several hundred cycles per call.
@@ -279,12 +279,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) 
                  "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])), "r"(__float_as_uint(v[23])), "r"(__float_as_uint(v[24])),
                  "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])), "r"(__float_as_uint(v[27])), "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])),
                  "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31])) : "memory");
-}
-__device__ __forceinline__ void tmem_st32u(uint32_t taddr, const uint32_t (&v)[32]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
-                 "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-                 "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
 }
 __device__ __forceinline__ void tmem_st16u(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -525,7 +519,7 @@ struct TcP {
   float* pm; float* pl; float* pacc;
   uint16_t* o16; const uint16_t* bv;                       // splits == 1 and o16 set: store the finished rows, no partials
   yskn_kv_layer kv; const float* rope; int rd;             // the fused form reads the packed cache itself
-  const uint16_t* q16; int bf16;                           // all forms but 0: the softmax warps stage Q (as fp16)
+  const uint16_t* q16; int bf16;                           // all forms but 0: the softmax warps stage Q (as fp16), or convert it
   const int8_t* k8; const int8_t* v8; const float* ks8; const float* vs8;     // FORM 2: INT8 rows and their scales
 };
 
@@ -558,10 +552,10 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   const int nquad = (P.tpc * P.G + 31) / 32;                         // quadrants of 32 rows that hold queries: softmax warps of the others have no part
   const uint32_t rank = cluster_ctarank();                           // 0 = leader: issues the MMAs, owns the "full"/"ready" barriers
   // barriers (8 bytes each), same offsets in both CTAs:
-  //   leader's copy only: kfull[NK] vfull[NV] pready[2] phalf[2] qfull     each CTA's copy: kempty[NK] vempty[NV] sready[2] pvdone[2]
+  //   leader's copy only: kfull[NK] vfull[NV] pready[2] phalf[2] qfull     each CTA's copy: kempty[NK] vempty[NV] sready[2] pvdone[2] qraw
   const uint32_t B0 = sb + L::OFF_BAR;
   const uint32_t b_kfull = B0, b_kempty = B0 + 32, b_vfull = B0 + 64, b_vempty = B0 + 96, b_sready = B0 + 128, b_pready = B0 + 144,
-                 b_pvdone = B0 + 160, b_q = B0 + 176, b_phalf = B0 + 192;
+                 b_pvdone = B0 + 160, b_q = B0 + 176, b_phalf = B0 + 192, b_qraw = B0 + 208;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + L::OFF_BAR + 184);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + L::OFF_BAR + 188);
   const uint32_t lead_kfull = leader_addr(b_kfull), lead_vfull = leader_addr(b_vfull), lead_pready = leader_addr(b_pready), lead_q = leader_addr(b_q),
@@ -574,7 +568,8 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     for (int i = 0; i < 2; ++i) { bar_init(b_sready + 8 * i, 1); bar_init(b_pvdone + 8 * i, 1); }
     // P of a tile: all softmax warps with queries of both CTAs in the converting forms; those of the tile's warpgroup otherwise, half of the keys at a time
     for (int i = 0; i < 2; ++i) { bar_init(b_pready + 8 * i, (FUSED ? 4 : 2) * nquad); bar_init(b_phalf + 8 * i, 2 * nquad); }
-    bar_init(b_q, STAGED_Q ? 2 * TC_SW : 1);                         // queries that are converted or reordered are staged by the softmax warps
+    if constexpr (STAGED_Q && !FUSED) bar_init(b_qraw, 1);
+    bar_init(b_q, STAGED_Q ? 2 * TC_SW : 1);                         // queries that are converted or reordered come from the softmax warps
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -622,6 +617,9 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       if (!STAGED_Q) {
         if (rank == 0) bar_expect_tx(b_q, 2 * L::KBLK * G * (128 / G) * 128);   // whole boxes: tokens beyond this CTA's come along unused
         for (int kb = 0; kb < L::KBLK; ++kb) tma_load_4d_pair(sb + L::OFF_Q + kb * L::Q_BLOCK, &mapQ, 64 * kb, 0, kvh, tok0, lead_q);
+      } else {                                                       // as they are, for this CTA's softmax warps to convert where they land
+        bar_expect_tx(b_qraw, L::KBLK * G * (128 / G) * 128);
+        for (int kb = 0; kb < L::KBLK; ++kb) tma_load_4d_pair(sb + L::OFF_Q + kb * L::Q_BLOCK, &mapQ, 64 * kb, 0, kvh, tok0, cluster_addr(b_qraw, rank));
       }
       int kit = 0; bool ok = true;
       for (int i = 0; i < n && ok; ++i) {
@@ -948,7 +946,6 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       };
       if (n > 1) k_prefetch(j0 * TC_BN + TC_BN + (TC_BN / 2) * (int)rank);
       for (int i = 0; i < n && ok; ++i) {
-        const int j = j0 + i;
         const int tk0 = tile_key(i);
         const bool kin = tk0 < P.max_ctx;                            // max_ctx is a multiple of 64: the half tile is inside or outside as a whole
         if (i + 2 < n) k_prefetch(tk0 + 2 * TC_BN);
@@ -1132,8 +1129,25 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     const float cs = P.qscale * TC_LOG2E;
     if constexpr (STAGED_Q) {
       if (n > 0) {
-        // bf16 activations, or the chunk order of the int4 form: these eight warps write this CTA's query rows (there is no Q copy)
-        tc_stage_q<HD, FORM == 1, FUSED ? 4 : 16>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, act_bf16, tok0, G, TOK, P.M, P.nh, kvh * G, threadIdx.x, 32 * TC_SW);
+        // The converting forms write their query rows themselves (fp16, in the chunk order of the int4 form); in the workspace forms they have come by TMA and
+        // bf16 ones are converted where they lie (read, converted and stored from global memory 64 KB took 3.3 us: 1,000 bf16 rows 55.7 -> 53.4 us,
+        // 1,000 INT8 rows behind 3,001 tokens 128.5 -> 127.1)
+        if constexpr (FUSED) tc_stage_q<HD, FORM == 1, 4>(sb + L::OFF_Q, L::Q_BLOCK, P.q16, act_bf16, tok0, G, TOK, P.M, P.nh, kvh * G, threadIdx.x, 32 * TC_SW);
+        else {
+          if (!bar_wait(b_qraw, 0)) { atomicExch(&g_tc_status, 4); *s_abort = 1; }
+          if (act_bf16) {
+            #pragma unroll 4
+            for (int it = threadIdx.x; it < TOK * G * (HD / 8); it += 32 * TC_SW) {
+              const int row = it / (HD / 8), w = it % (HD / 8);
+              const uint32_t a = sb + L::OFF_Q + (w >> 3) * L::Q_BLOCK + row * 128 + (((w & 7) ^ (row & 7)) << 4);
+              uint32_t o[4];
+              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]) : "r"(a) : "memory");
+              #pragma unroll
+              for (int e = 0; e < 4; ++e) o[e] = tc_pack(__uint_as_float(o[e] << 16), __uint_as_float(o[e] & 0xffff0000u));
+              tc_sts128(a, make_uint4(o[0], o[1], o[2], o[3]));
+            }
+          }
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) bar_arrive_cluster(lead_q);
@@ -1520,8 +1534,7 @@ int launch_tc_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, const TcWs&
   if (int rc = launch_pdl("kv4_tc_prep_kernel", kv4_tc_prep_kernel<HD>, dim3((unsigned)((span + 3) / 4), (unsigned)a.kvh), 128, 0, st, pp)) return rc;
   CUtensorMap mq, mkd, mvd, mks;
   const uint64_t rows = (uint64_t)a.kvh * a.max_ctx;
-  if (bf16) memset(&mq, 0, sizeof(mq));                               // the softmax warps stage Q
-  if ((!bf16 && !tc_map_q(&mq, a.q16, a.M, a.kvh, g, HD)) || !tc_map_rows(&mkd, w.kd, rows, HD, TC_BN / 2, L::KBLK) ||
+  if (!tc_map_q(&mq, a.q16, a.M, a.kvh, g, HD) || !tc_map_rows(&mkd, w.kd, rows, HD, TC_BN / 2, L::KBLK) ||
       !tc_map_rows(&mvd, w.vd, rows, HD, TC_BN, L::KBLK / 2) || !tc_map_rows(&mks, w.ks, (uint64_t)a.kvh * w.ks_rows, HD, TC_BN / 2, L::KBLK))
     KV4_REJECT("yskn_kv4_attention_tc: cuTensorMapEncodeTiled failed or is unavailable");
   auto kern = bf16 ? kv4_tc_attn_kernel<HD, 3> : kv4_tc_attn_kernel<HD, 0>;
@@ -1631,14 +1644,14 @@ int launch_kv8_attention_tc_ws(const yskn_kv8_attn_args& a, int act_dtype, void*
   if (int rc = launch_pdl("kv8_tc_prep_kernel", kv8_tc_prep_kernel, dim3((unsigned)runs, (unsigned)a.kvh, 2), 256, 0, st,
                           a.k8, a.v8, a.ks, a.vs, a.d_pos, a.M, a.max_ctx, kd, vd)) return rc;
   CUtensorMap mq, mkd, mvd;
-  memset(&mq, 0, sizeof(mq));                                         // unused: the softmax warps stage Q
+  const int g = a.nh / a.kvh;
   const uint64_t rows = (uint64_t)a.kvh * a.max_ctx;
-  if (!tc_map_rows(&mkd, kd, rows, 256, TC_BN / 2, L::KBLK) || !tc_map_rows(&mvd, vd, rows, 256, TC_BN, L::KBLK / 2))
+  if (!tc_map_q(&mq, a.q16, a.M, a.kvh, g, 256) || !tc_map_rows(&mkd, kd, rows, 256, TC_BN / 2, L::KBLK) || !tc_map_rows(&mvd, vd, rows, 256, TC_BN, L::KBLK / 2))
     KV4_REJECT("yskn_kv8_attention_ws: cuTensorMapEncodeTiled failed or is unavailable");
   auto kern = kv4_tc_attn_kernel<256, 4>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  const int g = a.nh / a.kvh; int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
   TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, nullptr, nullptr, yskn_kv_layer{}, nullptr, 0,
         a.q16, act_dtype == YSKN_KV4_BF16, nullptr, nullptr, nullptr, nullptr};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), TC_THREADS, L::TOTAL, st, mq, mkd, mvd, mq, P)) return rc;
