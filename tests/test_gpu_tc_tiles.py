@@ -56,3 +56,31 @@ def test_finished_rows_are_the_rounded_quotients(workspace, bf16):
     assert kv4.device_status() == 0
     same = (a.view(torch.int16) == b.view(torch.int16)) | (torch.isnan(a) & torch.isnan(b))
     assert bool(same.all()), int((~same).sum())
+
+
+# Rows 0 .. 49 of a pass from position 246: a wider pass ends behind another key tile, and its pairs of CTAs hold other tokens where they share a pass out evenly.
+@pytest.mark.parametrize("workspace,bf16", [(True, False), (True, True), (False, False)], ids=["fp16", "bf16", "converting"])
+@pytest.mark.parametrize("ctx,S", [(246, 1), (246, 3), (2030, 5)])
+def test_rows_are_the_same_bits_in_passes_of_other_widths(ctx, S, workspace, bf16):
+    import torch
+    from yasakani_b200 import kv4
+    hq, hkv, hd, rd, widths, max_ctx = 24, 4, 256, 64, (50, 64, 85, 130), (ctx + 130 + 63) // 64 * 64
+    dt = torch.bfloat16 if bf16 else torch.float16
+    g = torch.Generator(device="cuda").manual_seed(ctx + S)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16).to(dt)
+    k, v, q = rnd(ctx + 130, hkv, hd), rnd(ctx + 130, hkv, hd), rnd(130, hq, hd)
+    layer = kv4.KvLayer(hkv, hd, max_ctx)
+    kv4.launch_kv_append(layer, k, v, torch.zeros(1, dtype=torch.int32, device="cuda"), ctx + 130)
+    rope = torch.empty((max_ctx, rd // 2, 2), dtype=torch.float32, device="cuda")
+    kv4.launch_rope_table_g(rope, max_ctx, 1e4, rd)
+    pos, first = torch.tensor([ctx], dtype=torch.int32, device="cuda"), None
+    for M in widths:
+        out = kv4.attn_scratch(M, S, hq, hd)
+        kv4.launch_attention_tc(q[:M].contiguous(), layer, M, pos, S, *out, rope, hq, kv4.default_qscale(hd), rd, kv4.tc_workspace(layer, M) if workspace else None)
+        torch.cuda.synchronize()
+        assert kv4.device_status() == 0
+        # the last split ends with the pass, so rows of a narrower pass see its last tiles masked
+        bits = [t[:widths[0]].view(torch.int32) for t in out]
+        first = first or bits
+        for name, a, b in zip(("m", "l", "o"), first, bits):
+            assert torch.equal(a, b), f"{name} of {int((a != b).flatten(1).any(1).sum())} of {widths[0]} rows in a pass of {M}"

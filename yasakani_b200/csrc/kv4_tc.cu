@@ -33,8 +33,9 @@
 //  issue, 9-11 V tiles, 12-15 K tiles.
 //
 // Rows are independent of one another inside every step (an MMA output row depends on its own A row only, the lazy
-// rescale multiplies other rows by exactly 1), tiles start at multiples of 128 keys and split boundaries depend on
-// *d_pos and `splits` only, so within a form a row's result does not depend on how many rows the pass holds.  Forms differ in the order in
+// rescale multiplies other rows by exactly 1), tiles start at multiples of 128 keys, split boundaries depend on
+// *d_pos and `splits` only, and where a tile's place in the pair decides which warpgroup adds its weights (forms 0 and 3: bulk or edge tile) pairs start at
+// multiples of the tokens that 256 rows hold, so within a form a row's result does not depend on how many rows the pass holds.  Forms differ in the order in
 // which a row's weights are added (pl, and with it the last bit of the row): over INT8 rows a pass takes form 4 from 384 rows on, where its caller
 // lends a workspace, and form 2 otherwise.
 //
@@ -1503,11 +1504,12 @@ int tc_launch_pdl(K kern, dim3 grid, int threads, int smem_bytes, cudaStream_t s
   return 0;
 }
 
-// Query tiles of a pass (an even number: CTA pairs), its tokens shared out evenly: a CTA's softmax work is what its rows are (16 rows of six heads:
-// 48 and 48, three quarters of the warps idle, where 96 and none left one CTA with all of it).
-int tc_tiles(int M, int g, int* tokens_per_cta) {
+// Query tiles of a pass: an even number (CTA pairs) of as many tokens as 128 rows hold.  `even`: the pass's tokens shared out evenly instead, since a CTA's
+// softmax work is what its rows are (16 rows of six heads: 48 and 48, three quarters of the warps idle, where 96 and none left one CTA with all of it).
+// Not for the forms over the int4 workspace: their warpgroups take bulk and edge tiles differently, and the line between those is the pair's first token.
+int tc_tiles(int M, int g, bool even, int* tokens_per_cta) {
   const int tok = 128 / g, pairs = (M + 2 * tok - 1) / (2 * tok);
-  *tokens_per_cta = (M + 2 * pairs - 1) / (2 * pairs);
+  *tokens_per_cta = even ? (M + 2 * pairs - 1) / (2 * pairs) : tok;
   return 2 * pairs;
 }
 
@@ -1540,7 +1542,7 @@ int launch_tc_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, const TcWs&
   auto kern = bf16 ? kv4_tc_attn_kernel<HD, 3> : kv4_tc_attn_kernel<HD, 0>;
   static std::atomic<unsigned long long> attr[2] = {{0}, {0}};
   if (first_use_on_device(attr[bf16 != 0])) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  int tpc; const int qtiles = tc_tiles(a.M, g, false, &tpc);
   TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, w.ks_rows, a.qscale, a.pm, a.pl, a.pacc, o16, bv, a.kv, a.rope, rd,
         static_cast<const uint16_t*>(a.q16), bf16, nullptr, nullptr, nullptr, nullptr};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), TC_THREADS, L::TOTAL, st, mq, mkd, mvd, mks, P)) return rc;
@@ -1556,7 +1558,7 @@ int launch_tc_fused_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, uint1
   auto kern = kv4_tc_attn_kernel<HD, 1>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  int tpc; const int qtiles = tc_tiles(a.M, g, true, &tpc);
   TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, o16, bv, a.kv, a.rope, rd, static_cast<const uint16_t*>(a.q16), bf16,
         nullptr, nullptr, nullptr, nullptr};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), tc_threads(true), L::TOTAL, st, mq, mq, mq, mq, P)) return rc;
@@ -1623,7 +1625,7 @@ int launch_kv8_attention_tc(const yskn_kv8_attn_args& a, int act_dtype, cudaStre
   auto kern = kv4_tc_attn_kernel<256, 2>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  int tpc; const int qtiles = tc_tiles(a.M, g, true, &tpc);
   TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, nullptr, nullptr, yskn_kv_layer{}, nullptr, 0,
         a.q16, bf16, a.k8, a.v8, a.ks, a.vs};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), tc_threads(true), L::TOTAL, st, mq, mq, mq, mq, P)) return rc;
@@ -1651,7 +1653,7 @@ int launch_kv8_attention_tc_ws(const yskn_kv8_attn_args& a, int act_dtype, void*
   auto kern = kv4_tc_attn_kernel<256, 4>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  int tpc; const int qtiles = tc_tiles(a.M, g, &tpc);
+  int tpc; const int qtiles = tc_tiles(a.M, g, true, &tpc);
   TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, nullptr, nullptr, yskn_kv_layer{}, nullptr, 0,
         a.q16, act_dtype == YSKN_KV4_BF16, nullptr, nullptr, nullptr, nullptr};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), TC_THREADS, L::TOTAL, st, mq, mkd, mvd, mq, P)) return rc;
