@@ -47,3 +47,31 @@ def test_merge_on_both_sides_of_the_line_for_256_channels(M, S):
 @pytest.mark.parametrize("S", [40, 41, 74, 81, 160])
 def test_merge_of_many_splits_in_eight_runs(M, nh, S):
     test_merge_matches_double_precision(M, nh, 8, 128, S, torch.float16, 0)
+
+
+@pytest.mark.parametrize("M,nh", [(1, 16), (9, 16)])
+@pytest.mark.parametrize("S", [37, 41, 74, 160])
+def test_a_shards_triple_is_the_same_by_either_exchange(M, nh, S):
+    """The triple that is gathered and the one that is pushed hold the same bits, at the sizes where the merge of a whole sequence takes eight runs of
+    splits, and are the fold in double precision to the rounding of S additions."""
+    from yasakani_b200 import kv4
+    hd, gen = 128, torch.Generator(device="cuda").manual_seed(S)
+    pm = torch.randn((M, S, nh), generator=gen, device="cuda") * 3
+    pm[:, S // 2] = -1e30                                          # an empty split
+    pl = torch.rand((M, S, nh), generator=gen, device="cuda") * 50 + 1
+    pacc = torch.randn((M, S, nh, hd), generator=gen, device="cuda") * pl[..., None]
+    triple = torch.empty((M, nh, hd + 2), device="cuda")
+    kv4.launch_local_triple(pm, pl, pacc, S, M, nh, hd, triple)
+    buf = torch.zeros((kv4.exchange_bytes(1, M, nh, hd) + 3) // 4, device="cuda")
+    x, o16 = kv4.peer_exchange([buf.data_ptr()], 0), torch.empty((M, nh, hd), dtype=torch.float16, device="cuda")
+    kv4.launch_push_triple(pm, pl, pacc, S, M, nh, hd, x)
+    kv4.launch_merge_pushed(x, M, nh, 8, hd, o16)
+    torch.cuda.synchronize()
+    assert kv4.device_status() == 0
+    pushed = buf[:2 * triple.numel()].view(M, nh, hd + 2, 2)[..., 0]      # the first step's half: a value and the number of its step
+    assert torch.equal(pushed.view(torch.int32), triple.view(torch.int32)), int((pushed != triple).sum())
+    w = torch.exp(pm.double() - pm.double().amax(1, keepdim=True)) * (pm > -1e29)
+    o, l, mag = (w[..., None] * pacc.double()).sum(1), (w * pl.double()).sum(1), (w[..., None] * pacc.double().abs()).sum(1)
+    # a weight is within 8 units (its argument, below 32, is rounded by the subtraction; expf within two), and every sum adds at most S terms
+    assert ((triple[..., 2:].double() - o).abs() <= (S + 40) * 2.0 ** -24 * mag).all() and ((triple[..., 1].double() - l).abs() <= (S + 40) * 2.0 ** -24 * l).all()
+    assert torch.equal(triple[..., 0], pm.amax(1))

@@ -303,9 +303,10 @@ int launch_k(const CombineP& P, size_t smem, cudaStream_t st) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
-  if constexpr (!TI && !PEER && HD == 128)
+  if constexpr (!TI && !TO && !PEER && HD == 128)
     // More than 40 splits are two round trips for four runs: eight, with 1,024 threads a block, while a block has an SM of its own (four rows of
-    // 16 heads in 74 splits over 2,000 tokens 18.8 -> 17.8 us with append and attention, one row over 100,000 24.2 -> 23.5)
+    // 16 heads in 74 splits over 2,000 tokens 18.8 -> 17.8 us with append and attention, one row over 100,000 24.2 -> 23.5).  A shard's triple is folded in four
+    // by either exchange, so that the one that is gathered and the one that is pushed are the same bits.
     if (P.S > 4 * CB && blocks <= 148 && smem + 4 * HD * sizeof(float) <= 48 * 1024) {
       cfg.blockDim = dim3(8 * HD); cfg.dynamicSmemBytes = smem + 4 * HD * sizeof(float);
       KV4_CUDA(cudaLaunchKernelEx(&cfg, kv4_combine_kernel<HD, DT, TI, TO, PEER, 8>, P));
