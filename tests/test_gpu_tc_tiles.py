@@ -84,3 +84,47 @@ def test_rows_are_the_same_bits_in_passes_of_other_widths(ctx, S, workspace, bf1
         first = first or bits
         for name, a, b in zip(("m", "l", "o"), first, bits):
             assert torch.equal(a, b), f"{name} of {int((a != b).flatten(1).any(1).sum())} of {widths[0]} rows in a pass of {M}"
+
+
+@pytest.mark.parametrize("pos", [-200, -16, -9, -3, 190])
+@pytest.mark.parametrize("int8", [False, True], ids=["int4", "int8"])
+def test_positions_outside_the_cache_are_read_nowhere(int8, pos):
+    """A converting pass that begins below position 0, or ends behind the cache: rows without keys leave empty partials, the others equal those of the same
+    positions in a pass that lies inside."""
+    import torch
+    from yasakani_b200 import kv4, kvx
+    M, S, nh, kvh, hd, max_ctx = 16, 2, 24, 4, 256, 192
+    g = torch.Generator(device="cuda").manual_seed(9)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    q, k, v = rnd(M, nh, hd), rnd(max_ctx, kvh, hd), rnd(max_ctx, kvh, hd)
+    zero = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def attend(rows, at, out):
+        qq, p = q[rows].contiguous(), torch.tensor([at], dtype=torch.int32, device="cuda")
+        m = qq.shape[0]
+        if int8:
+            kvx.launch_kv8_attention_tc(qq, *arrays, m, p, S, *out, nh)
+        else:
+            kv4.launch_attention_tc(qq, layer, m, p, S, *out, rope, nh, kv4.default_qscale(hd), 64, None)
+    if int8:
+        (k8, ks), (v8, vs) = (kvx.encode(x.transpose(0, 1).reshape(-1, hd).float()) for x in (k, v))
+        arrays = k8.view(kvh, max_ctx, hd), v8.view(kvh, max_ctx, hd), ks.view(kvh, max_ctx), vs.view(kvh, max_ctx)
+    else:
+        layer = kv4.KvLayer(kvh, hd, max_ctx)
+        kv4.launch_kv_append(layer, k, v, zero, max_ctx)
+        rope = torch.empty((max_ctx, 32, 2), dtype=torch.float32, device="cuda")
+        kv4.launch_rope_table_g(rope, max_ctx, 1e4, 64)
+    out = kv4.attn_scratch(M, S, nh, hd)
+    attend(slice(None), pos, out)
+    torch.cuda.synchronize()
+    assert kv4.device_status() == 0
+    empty = [r for r in range(M) if pos + r < 0]
+    if empty:
+        assert (out[0][empty] == -1e30).all() and (out[1][empty] == 0).all() and (out[2][empty] == 0).all()
+    inside = [r for r in range(M) if 0 <= pos + r < max_ctx]
+    if inside:
+        want = kv4.attn_scratch(len(inside), S, nh, hd)
+        attend(slice(inside[0], inside[-1] + 1), max(pos, 0), want)
+        torch.cuda.synchronize()
+        for a, b in zip(out, want):
+            assert torch.isfinite(b).all() and torch.equal(a[inside].view(torch.int32), b.view(torch.int32))

@@ -599,8 +599,8 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   const int tok0 = qt * TOK;                                         // this CTA's first token
   const int tokA = (qt & ~1) * TOK;                                  // the pair's first token (always < M)
   const int pos0 = *P.d_pos;
-  const int pmax = pos0 + min(tokA + 2 * TOK, P.M) - 1;              // last key any row of the pair sees
-  const int nt_all = pmax / TC_BN + 1;
+  const int pmax = min(pos0 + min(tokA + 2 * TOK, P.M), P.max_ctx) - 1;   // last key any row of the pair sees; negative: none does
+  const int nt_all = (pmax + TC_BN) / TC_BN;                         // so no tile lies outside the cache, whatever the position is
   const int per = (pos0 / TC_BN + 1 + S - 1) / S;                    // split width in tiles: a function of *d_pos and S only
   const int j0 = min(split * per, nt_all), j1 = split == S - 1 ? nt_all : min((split + 1) * per, nt_all);
   const int n = j1 - j0;
@@ -721,7 +721,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     constexpr int NKT = TC_KW * 32, NVT = TC_VW * 32, NWD = HD / 8, NWV = HD / 16;   // threads per role; packed words per K row; per V row in this CTA's channel half
     // warps 9-11 (warpgroup 2) convert V, warps 12-15 (warpgroup 3) convert K: ct = 0 .. NKT-1 for K, NKT .. NKT+NVT-1 for V
     const int ct = is_k ? (int)threadIdx.x - (TC_SW + 4) * 32 : (int)threadIdx.x - CONV0 * 32 + TC_KW * 32;
-    const int end = pos0 + P.M;                                      // tokens [0, end) exist
+    const int end = min(pos0 + P.M, P.max_ctx);                      // tokens [0, end) exist; every tile of the pair begins below it
     const size_t row0 = (size_t)kvh * P.max_ctx, grp0 = (size_t)kvh * (P.max_ctx / 32);
     bool ok = true;
     auto publish = [&](uint32_t lead_bar) {                          // this warp's part of the stage is written
@@ -735,7 +735,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     };
 
     // INT8 rows: item = (key, 16-byte chunk = 16 channels) -> two 16-byte chunks of fp16; cur holds this tile's items, each
-    // next-tile item is requested right before the same item of this tile is converted
+    // next-tile item is requested right after the same item of this tile has been converted
     struct I8In { uint4 w; uint32_t s; };
     auto i8_convert = [&](const I8In& I, bool live, uint4& lo, uint4& hi) { tc_i8_chunk(I.w, __uint_as_float(I.s), live, lo, hi); };
     if (n > 0 && is_k) {
