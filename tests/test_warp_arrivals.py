@@ -12,3 +12,17 @@ def test_every_arrival_for_a_warp_stands_behind_a_syncwarp():
     assert len(arrivals) >= 2
     for at in arrivals:
         assert code[:at].rstrip().endswith("__syncwarp();"), code[max(0, at - 120):at + 60]
+
+
+def test_lanes_that_went_apart_are_joined_ahead_of_the_next_warp_wide_instruction():
+    """tcgen05.ld and .st are instructions of the whole warp: where its lanes have polled or divided for themselves, an instruction that joins them, and
+    that no condition guards, stands in between."""
+    code = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(os.path.join(build.CSRC, "kv4_tc.cu")).read(), flags=re.S)
+    finish = code[code.index("tc_finish_row("):]
+    loop = finish[finish.index("for (int c = hf;"):]
+    assert "__syncwarp();" in loop[:loop.index("tmem_ld32")]
+    swap = code[code.index("swap_with_partner(tmax"):]
+    swap = swap[:swap.index("tmem_")]
+    assert re.search(r"if \(I8\) __syncwarp\(\);", swap) and re.search(r"if \(I8 \? [^:]* : __any_sync\(0xffffffffu, bump\) && ", swap)
+    swap = code[code.index("if (mown != m)"):]
+    assert re.search(r"if \(__any_sync\(0xffffffffu, bump\) && ", swap[:swap.index("tmem_")])

@@ -392,13 +392,15 @@ __device__ __forceinline__ void tc_stage_q(uint32_t sq, int q_block, const uint1
   }
 }
 // Finished rows of a pass of one split: y = round_f16(o / l) (+ V bias) as the merge kernel, every other 32 columns of O from hf on.  A function of its own,
-// so that its code does not move the loops of the kernel about (a fused pass of 64 rows, which never comes here, took 92 to 99 us with it in line).
+// so that its code does not move the loops of the kernel about (a fused pass of 64 rows, which never comes here, took 92 to 99 us with it in line).  It is
+// called with what setmaxnreg has left the softmax warps, 104 registers in form 1 and 208 in forms 0 and 3, and needs 49.
 template <int HD, bool PAIRS>
 __device__ __noinline__ void tc_finish_row(uint32_t tcol, int hf, bool any, bool valid, float l, bool bf16, const uint16_t* bv, uint16_t* out) {
   const float rl = __frcp_rn(l);
   #pragma unroll 1
   for (int c = hf; c < HD / 32; c += 2) {
     float o[32];
+    __syncwarp();                                                    // lanes without a row, and those that divided, have come round
     if (any) tmem_ld32(tcol + 32 * c, o);
     else {
       #pragma unroll
@@ -1236,7 +1238,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         xseq[hf * 128 + rho] = (uint16_t)(i + 1);
         if (mown != m) { l *= tc_ex2(mown - m); mown = m; }
         // ---- O may be rescaled once P.V of tile i-1 is done (P.V of this tile waits for the signals below)
-        if (i > 0 && __any_sync(0xffffffffu, bump)) {                // rows that did not bump multiply by exactly 1
+        if (__any_sync(0xffffffffu, bump) && i > 0) {                // rows that did not bump multiply by exactly 1; every tile asks: the warp is together again
           if (!bar_wait(b_pvdone + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
           tc_fence_after();
           #pragma unroll 1
@@ -1308,8 +1310,11 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           const bool bump = valid && tmax > m + 8.f;
           const float mn = bump ? tmax : m, alpha = bump ? tc_ex2(m - mn) : 1.f;
           m = mn; l *= alpha; nm = -m;
-          // ---- O may be rescaled once P.V of tile i-1 is done (P.V of this tile waits for the signal below)
-          if (i > 0 && __any_sync(0xffffffffu, bump)) {              // rows that did not bump multiply by exactly 1
+          // ---- O may be rescaled once P.V of tile i-1 is done (P.V of this tile waits for the signal below).  Each lane has polled for itself in the
+          //      exchange and the tcgen05.ld behind want the warp together, so every tile asks, the first too; over INT8 rows it joins first (with the
+          //      other way about, 64 int4 rows over 32,768 tokens took 0.9 % more and 383 INT8 rows behind 8,000 2 %).
+          if (I8) __syncwarp();
+          if (I8 ? i > 0 && __any_sync(0xffffffffu, bump) : __any_sync(0xffffffffu, bump) && i > 0) {   // rows that did not bump multiply by exactly 1
             if (!bar_wait(b_pvdone + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
             tc_fence_after();
             #pragma unroll 1
@@ -1369,7 +1374,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       const bool direct = P.o16 != nullptr && S == 1;                // one split: this CTA holds the whole row, finish it here
       auto ocol = [](int c) { return FORM == 1 ? tc_col(c) : c; };   // the int4 form's V chunks keep their channels in pair order
       if (valid && !direct && hf == 0) { P.pm[pidx] = (n > 0 && m > -1e29f) ? m * TC_LN2 : -1e30f; P.pl[pidx] = n > 0 ? l : 0.f; }
-      if (direct) {                                                  // one split: this CTA holds the whole row
+      if (!I8 && direct) {
         tc_finish_row<HD, FORM == 1>(trow + L::TM_O, hf, n > 0, valid, l, act_bf16, P.bv ? P.bv + kvh * HD : nullptr,
                                      P.o16 + ((size_t)tok * P.nh + kvh * G + head) * HD);
         return;
