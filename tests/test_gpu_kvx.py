@@ -152,6 +152,13 @@ def test_attn_post_equals_the_oracle_bit_for_bit(oracle, M, nh, kvh, rd, pos0):
     _same(_gpu_post(kvx, d, 1e-6, pos0, rd, max_ctx, fill=7), _oracle_post(oracle, d, 1e-6, pos0, rd, max_ctx, fill=7), f"M {M} nh {nh} kvh {kvh} rd {rd}")
 
 
+# 1,152 and 1,216 rows: blocks of one warp and, from 1,184 rows on, of eight; 2,793: a last block of one row
+@pytest.mark.parametrize("rd", [64, 192])
+@pytest.mark.parametrize("M,nh,kvh", [(36, 24, 4), (38, 24, 4), (399, 5, 1)])
+def test_attn_post_in_both_block_sizes(oracle, M, nh, kvh, rd):
+    test_attn_post_equals_the_oracle_bit_for_bit(oracle, M, nh, kvh, rd, 21)
+
+
 def test_attn_post_default_math_mode_is_within_one_bf16_step(oracle):
     """pm = 0 takes rsqrtf like the reference's default (an approximation: no CPU restatement); against the portable-math
     oracle the query rows may differ by one bf16 step and the INT8 payload by one count."""
