@@ -47,3 +47,9 @@ def test_merge_matches_double_precision(M, nh, S, dtype):
 def test_row_form_edges(M, nh, S):
     """Both sides of the line between the forms, whole and broken batches of eight splits, one and two weights a lane."""
     test_merge_matches_double_precision(M, nh, S, torch.bfloat16)
+
+
+@pytest.mark.parametrize("M,nh", [(37, 8), (27, 11)])             # 296 and 297 rows: with more than 32 splits a warp each from 297 on
+@pytest.mark.parametrize("S", [32, 33, 37, 64])
+def test_both_sides_of_the_line_for_many_splits(M, nh, S):
+    test_merge_matches_double_precision(M, nh, S, torch.float16)

@@ -432,10 +432,13 @@ __global__ void __launch_bounds__(128) kv8_combine_rows_kernel(const float* pm, 
 template <int DT>
 int launch_kv8_combine_dt(const float* pm, const float* pl, const float* pacc, int S, int M, int nh, const void* gate, uint16_t* o16, int inverse_rotate, cudaStream_t st) {
   // The form of a warp per row wants enough rows: up to one block of 1,024 threads per SM the block form's parallel loads win (96 rows of 37 splits 3.1
-  // against 4.9 us), beyond it its blocks queue up (192 rows: 37 splits 5.5 against 5.0, 18 splits 5.1 against 3.9).  It reads 16-byte pieces.
+  // against 4.9 us in replays, 192 rows of 18 splits 5.1 against 3.9).  With more than 32 splits, two weights a lane, the line is two blocks an SM: behind the
+  // attention kernel the blocks are resident before it ends, and whole steps of 192 rows in 24 / 37 splits over 8,000 tokens take 48.7 / 55.9 us with blocks and
+  // 48.3 / 59.9 with warps (168 rows in 37: 50.4 / 53.9; 288 rows in 33 over 3,000 tokens 30.3 / 28.9, in 37 30.3 / 33.9; 576 rows in 37 37.6 / 36.7).  Warps read
+  // 16-byte pieces.
   const long long rows = (long long)M * nh;
   const bool aligned = !((((uintptr_t)pacc) & 15) | (((uintptr_t)o16 | (uintptr_t)gate) & 7));
-  if (rows > 148 && aligned)
+  if (rows > (S > 32 ? 296 : 148) && aligned)
     return launch_pdl("kv8_combine_rows_kernel", S == 1 ? kv8_combine_rows_kernel<DT, true> : kv8_combine_rows_kernel<DT, false>, dim3((unsigned)((rows + 3) / 4)), 128, 0, st,
                       pm, pl, pacc, S, nh, rows, gate, o16, inverse_rotate);
   return launch_pdl("kv8_combine_kernel", kv8_combine_kernel<DT>, dim3(nh, M), KV8_CQ * 256, 0, st, pm, pl, pacc, S, nh, gate, o16, inverse_rotate);
