@@ -52,6 +52,27 @@ def test_encoder_key_widths(oracle, top):
     assert np.array_equal(side.cpu().numpy().view(np.uint32), want["side"])
 
 
+@pytest.mark.parametrize("nm", [1, 2, 5])
+# Costs of the oracle are 32-bit numbers below its infinity of 2^30 while three steps from the only state that exists at first cost less:
+# 3 (10,000 + 2,048)^2 = 4.4e8.  (The largest code that a table holds, 32,767, does not: 3.6e9.)
+@pytest.mark.parametrize("top", [1400, 2200, 10000])
+def test_key_widths_in_every_block_size(oracle, top, nm):
+    """One multiplier, few rows and many rows take blocks of their own, and the 64-bit search a warp per chain in two of them: the same rows through all."""
+    from yasakani_b200 import kvx
+    blob = _with_largest_code(make_blob(nm=nm), top)
+    rng = np.random.default_rng(top + nm)
+    x = (rng.standard_normal((40, 256)) * np.exp(rng.standard_normal((40, 1)))).astype(np.float32)
+    x[7, ::3] *= 40.0
+    grp, pos = np.arange(40, dtype=np.int32), np.full(40, 9, np.int32)
+    want = oracle.tb_encode(blob, x, grp, pos)
+    prof = kvx.TrellisProfile(blob)
+    for n in (40, 593):
+        rep = np.arange(n) % 40
+        y, pay, side = kvx.tb_encode(prof, *(torch.from_numpy(np.ascontiguousarray(a[rep])).cuda() for a in (x, grp, pos)))
+        assert np.array_equal(y.cpu().numpy().view(np.uint32), want["y"].view(np.uint32)[rep]), n
+        assert np.array_equal(pay.cpu().numpy().view(np.uint32).reshape(n, 40), want["pay"][rep]) and np.array_equal(side.cpu().numpy().view(np.uint32), want["side"][rep]), n
+
+
 @pytest.mark.parametrize("with_payload", [True, False])
 def test_encoder_leaves_the_callers_other_words_alone(oracle, with_payload):
     """The C entry writes a packed row's payload words and its side words, nothing else: rows of records that hold other data behind the

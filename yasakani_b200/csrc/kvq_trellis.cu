@@ -48,23 +48,27 @@ __device__ __forceinline__ unsigned tb_table(const uint8_t* b, const TbGroup& P)
 //   4    top bit of j, u3 .. u1 the other bits of j, u0   8 shuffles                  1 (each lane of a pair keeps one u)
 //   5    top bit of j, u        the other bits of j (16)  4 shuffles                  1
 // (The new states of a lane need the minima of the groups p >> KK.  For KK = 3 the bit of u in the registers is u2: the lane's states of both values need the
-// same eight, and which of its two values a lane hands on follows from j alone.)  About 48 instructions a step of two chains; the form it replaces
-// had a lane hold eight states of one chain: 55 a step of one, of which 39 were exchanges, masks and stores.
+// same eight, and which of its two values a lane hands on follows from j alone.)  About 48 instructions a step of two chains; the form before it,
+// a warp per chain with eight states a lane, takes 55 a step of one, of which 39 are exchanges, masks and stores (tb_search_chain).
 // x^2 is left out of the costs: it adds the same number to every state of a step.  A cost travels as a key, cost << 5 | j, whose j is part
 // of the state's own constant: the minimum over keys is the minimum cost with the first j on ties (the reference's rule,
 // src/kvq_gpu.cuh:101-102) and carries its back pointer, one byte per group and step.
 // Width of the keys: |f| = |c^2 - 2xc| <= F = C^2 + 4096 C with C = max |code| and |x| <= 2048, and f differs by at most D = 8192 C between
 // two states; any state is reached from any other in three steps, so the costs of a step spread over at most 3 D.  They are
 // brought back to one of them every four steps: |cost| <= 3 D + 4 F < 2^26 for C <= 1400, and a key fits 32 bits.  Profiles with larger codes
-// take 64-bit keys (the same code, no bringing back).
+// take 64-bit keys (no bringing back).
 // 4,096 rows, 5 multipliers, on a B200: 1,335 us (one warp per (row, multiplier, chain), costs in shared memory, every lane walking its group's predecessors; a
 // second kernel for choice and packing) -> 448 (minima kept instead of back pointers, candidates recomputed on the way back) -> 321 (eight states a
 // lane, a warp per chain that walks the multipliers) -> 243.  Issue slots 63 % busy, integer ALU 45 %, multiply pipe 49 %, shuffles and shared memory 45 %; 25 warps
 // an SM at 72 registers instead of 20 at 96 are slower (262), 15 at 128 too (273).
+// Where a warp per chain stays: with one multiplier, whose two pairs of chains would leave two of the block's four warps idle (28 warps an SM; 4,096 rows 83 us
+// by pairs, 75 by chains; 64-bit keys 318 and 178), and with 64-bit keys and many rows, where sixteen states a lane do not fit the registers and the codes are read again
+// every step (4,096 rows of 2 / 5 / 16 multipliers 362 / 972 / 3,237 us by pairs, 327 / 838 / 2,625 by chains; 8 rows, bound by the dependent steps, 23.5 / 40 / 122
+// and 31.7 / 46 / 136).
 // Blocks of ten warps (every multiplier and pair of chains at once) for a few rows, which are bound by the chains of 64 dependent steps; of five, twice as
 // many an SM, for more rows than two rounds of the former: with unpacking 100 rows 28.0 / 33.9 us, 600 53.5 / 55.6, 1,000 84.8 / 80.9, 4,096 270 / 250 (ten / five).
 constexpr int TB_NM = 16;                                // multipliers at most (the blob's limit)
-constexpr int TB_WIDE = 10, TB_NARROW = 5, TB_WIDE_ROWS = 2 * 2 * 148;     // warps of a block at most, two forms; rows that the wide one takes
+constexpr int TB_WIDE = 10, TB_NARROW = 5, TB_ONE = 4, TB_WIDE_ROWS = 2 * 2 * 148;     // warps of a block at most, three forms; rows that the wide one takes
 struct TbRowSmem {
   short code[256]; float res[256]; float red[8]; int cmax[16]; uint8_t fld[256];
   TbGroup grp; float coef[2];                              // what the search does not need waits here, not in registers
@@ -78,6 +82,29 @@ struct TbP { const uint8_t* blob; int nm; const float* x; const int* grp; const 
 
 __device__ __forceinline__ int tb_addmin(int a, int b, int c) { return __viaddmin_s32(a, b, c); }
 __device__ __forceinline__ long long tb_addmin(long long a, long long b, long long c) { return min(a + b, c); }
+
+// Only state 0 exists at first.  Every state is reachable after three steps, so the others have to stay behind by more than 6 F
+// (5e7 for C = 1400) until then, and within the width of a key.
+template <class K> constexpr K TB_START = (K)(-(1 << 25)) * 32;
+template <class K> constexpr K TB_FAR = (K)(sizeof(K) == 4 ? (1 << 24) + (1 << 23) : 0x40000000) * 32;
+
+// The best final state of a chain, smallest (cost, state) over 2 O lanes, and the way back from it; `first` is 0 in the lane that stores.
+template <int KK, int O, class K> __device__ __forceinline__ void tb_walk(const uint8_t* bp, K best, int st, uint8_t* states, int first) {
+  constexpr int SH = 8 - KK, UU = 1 << SH;
+  #pragma unroll
+  for (int o = O; o; o >>= 1) {
+    const K c = __shfl_xor_sync(0xffffffffu, best, o); const int b2 = __shfl_xor_sync(0xffffffffu, st, o);
+    if (c < best || (c == best && b2 < st)) { best = c; st = b2; }
+  }
+  __syncwarp();                                          // the back pointers are complete
+  #pragma unroll 8
+  for (int t = 63; t >= 0; --t) {
+    if (first == 0) states[t] = (uint8_t)st;
+    const int u = st >> KK;
+    st = ((bp[t * UU + u] & 31) << SH) + u;              // (the row of step 0 is read but never used)
+  }
+  __syncwarp();                                          // they may be overwritten, and the states are complete
+}
 
 // States of the best path of this half warp's chain of scaled values xs (bp, xs and states are the chain's own).  K = int or long long, the type of the keys.
 template <int KK, class K> __device__ __forceinline__ void tb_search(uint8_t* bp, const short* code, const int* xs, uint8_t* states, int lane) {
@@ -101,10 +128,7 @@ template <int KK, class K> __device__ __forceinline__ void tb_search(uint8_t* bp
     src[q] = half | (KK == 3 ? ((q >> 1) << 2) | (l >> 2) : KK == 4 ? ((q & 1) << 3) | ((l >> 3) << 2) | (q >> 1) : ((l >> 3) << 2) | q);
   const bool upper = l >> 3;                             // KK = 4: of a pair of lanes the upper one keeps the odd u
   const int my_u = KK == 3 ? ((l >> 2) << 3) | (l & 3) : KK == 4 ? ((l & 7) << 1) | (upper ? 1 : 0) : l & 7;
-  // Only state 0 exists at first.  Every state is reachable after three steps, so the others have to stay behind by more than 6 F
-  // (5e7 for C = 1400) until then, and within the width of a key.
-  constexpr K FAR = (K)(NARROW ? (1 << 24) + (1 << 23) : 0x40000000) * 32;
-  K ka = my_u == 0 ? (K)(-(1 << 25)) * 32 : FAR, kb = FAR;          // minima of the lane's groups (kb: KK = 3, the one with u2 = 1)
+  K ka = my_u == 0 ? TB_START<K> : TB_FAR<K>, kb = TB_FAR<K>;          // minima of the lane's groups (kb: KK = 3, the one with u2 = 1)
   uint8_t* mine = bp + my_u;
   auto costs = [&](int x, K (&t)[16], K (&m)[NQ]) {
     ka &= ~(K)31;
@@ -153,24 +177,77 @@ template <int KK, class K> __device__ __forceinline__ void tb_search(uint8_t* bp
     const int p = state(e);
     if (e == 0 || c < best || (c == best && p < bs)) { best = c; bs = p; }
   }
+  tb_walk<KK, 8>(bp, best, bs, states, l);
+}
+
+// The same with the whole warp on one chain, eight states a lane,
+//   p = jhi << (SH+2) | jlo << SH | umid << 1 | ulo,     registers e = (jlo, ulo), lane = (jhi, umid):
+// the minimum over jlo is in the lane, the first exchange over jhi halves the lane's two values of u (each lane of the pair keeps one), the others are plain;
+// the new states need 4 (KK = 3, 4) or 1 (KK = 5) of the UU minima.
+template <int KK, class K> __device__ __forceinline__ void tb_search_chain(uint8_t* bp, const short* code, const int* xs, uint8_t* states, int lane) {
+  constexpr int SH = 8 - KK, UU = 1 << SH, NQ = KK == 5 ? 1 : 4;
+  constexpr bool NARROW = sizeof(K) == 4;
+  const int umid = lane & ((1 << (SH - 1)) - 1), jhi = lane >> (SH - 1);
+  auto state = [&](int e) { return (jhi << (SH + 2)) | ((e >> 1) << SH) | (umid << 1) | (e & 1); };    // a lane's states grow with e
+  int m2c[8];                                            // a cost is one multiply-add, a wide one for 64-bit keys
+  K c2[8];
+  int src[NQ];
   #pragma unroll
-  for (int o = 8; o; o >>= 1) {
-    const K c = __shfl_xor_sync(0xffffffffu, best, o); const int b2 = __shfl_xor_sync(0xffffffffu, bs, o);
-    if (c < best || (c == best && b2 < bs)) { best = c; bs = b2; }
+  for (int e = 0; e < 8; ++e) {
+    const int p = state(e), c = code[p];
+    m2c[e] = -2 * c * 32; c2[e] = (K)c * c * 32 + (p >> SH);
   }
-  __syncwarp();                                          // the back pointers are complete
-  int st = bs;
-  #pragma unroll 8
-  for (int t = 63; t >= 0; --t) {
-    if (l == 0) states[t] = (uint8_t)st;
-    const int u = st >> KK;
-    st = ((bp[t * UU + u] & 31) << SH) + u;              // (the row of step 0 is read but never used)
+  #pragma unroll
+  for (int q = 0; q < NQ; ++q) {                         // the lane that holds the minimum of group (new state >> KK)
+    const int g = ((jhi << (SH + 2)) | (q << SH) | (umid << 1)) >> KK;
+    src[q] = ((g & 1) << (SH - 1)) | (g >> 1);
   }
-  __syncwarp();                                          // they may be overwritten, and the states are complete
+  const bool upper = (lane >> (SH - 1)) & 1;             // of a pair of lanes the upper one keeps the odd u
+  const int my_u = (umid << 1) | (upper ? 1 : 0);
+  K keep = my_u == 0 ? TB_START<K> : TB_FAR<K>;
+  uint8_t* mine = bp + (lane < UU ? my_u : 0);           // lanes below UU hold every u once (the jhi bits above the first are zero)
+  auto costs = [&](int x, K (&t)[8], K (&m)[NQ]) {
+    keep &= ~(K)31;
+    #pragma unroll
+    for (int q = 0; q < NQ; ++q) m[q] = __shfl_sync(0xffffffffu, keep, src[q]);
+    #pragma unroll
+    for (int e = 0; e < 8; ++e) t[e] = (K)x * m2c[e] + c2[e];
+  };
+  auto step = [&](int x, int t) {                        // the minima of step t + 1 from those of step t
+    K ct[8], m[NQ];
+    costs(x, ct, m);
+    K a = ct[0] + m[0], b = ct[1] + m[0];
+    #pragma unroll
+    for (int q = 1; q < 4; ++q) {
+      a = tb_addmin(ct[2 * q], m[NQ == 1 ? 0 : q], a);
+      b = tb_addmin(ct[2 * q + 1], m[NQ == 1 ? 0 : q], b);
+    }
+    keep = min(upper ? b : a, __shfl_xor_sync(0xffffffffu, upper ? a : b, 1 << (SH - 1)));
+    #pragma unroll
+    for (int k = SH; k < 5; ++k) keep = min(keep, __shfl_xor_sync(0xffffffffu, keep, 1 << k));
+    if (lane < UU) mine[(t + 1) * UU] = (uint8_t)keep;
+  };
+  #pragma unroll 1
+  for (int t = 0; t < 60; t += 4) {
+    const int4 x = *reinterpret_cast<const int4*>(xs + t);
+    step(x.x, t); step(x.y, t + 1); step(x.z, t + 2); step(x.w, t + 3);
+    if (NARROW) keep -= __shfl_sync(0xffffffffu, keep, 0) & ~(K)31;
+  }
+  const int4 x = *reinterpret_cast<const int4*>(xs + 60);
+  step(x.x, 60); step(x.y, 61); step(x.z, 62);
+  K ct[8], m[NQ];
+  costs(x.w, ct, m);
+  K best = 0; int bs = 0;
+  #pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const K c = (ct[e] + m[NQ == 1 ? 0 : e >> 1]) & ~(K)31;
+    if (e == 0 || c < best) { best = c; bs = state(e); }
+  }
+  tb_walk<KK, 16>(bp, best, bs, states, lane);
 }
 
 template <int W>
-__global__ void __launch_bounds__(W * 32, 20 / W) tb_encode_kernel(TbP A) {
+__global__ void __launch_bounds__(W * 32, W == TB_ONE ? 7 : 20 / W) tb_encode_kernel(TbP A) {
   extern __shared__ __align__(16) unsigned char tbe_smem[];
   TbRowSmem& S = *reinterpret_cast<TbRowSmem*>(tbe_smem);
   const int nt = blockDim.x, nwarps = nt >> 5;
@@ -251,31 +328,45 @@ __global__ void __launch_bounds__(W * 32, 20 / W) tb_encode_kernel(TbP A) {
     const bool narrow = cm <= 1400;
     auto scale = [&](int mi) { const float s = tb_f16r(__fmul_rn(rms, tb_f32(b + P.off_m + 4u * (unsigned)mi))); return s == 0.f ? 1.f : s; };
     auto value = [&](int st, float s) { return __fmul_rn(__fmul_rn(__fmul_rn((float)(int)S.code[st], 0.00390625f), gain), s); };
-    #pragma unroll 1
-    for (int unit = c; unit < 2 * A.nm; unit += nwarps) {                    // a multiplier and two of the four chains
-      const int mi = unit >> 1, e0 = 128 * (unit & 1);
+    // a unit: a multiplier and the N = 128 or 64 values from e0 on that this warp searches
+    auto unit_of = [&](int mi, int e0, auto n, auto search) {
+      constexpr int R = decltype(n)::value / 32;
       const float s = scale(mi);
       TbRowSmem::Warp& B = warps[c];
       #pragma unroll
-      for (int r = 0; r < 4; ++r)
+      for (int r = 0; r < R; ++r)
         B.xs[32 * r + lane] = (int)fminf(fmaxf(rintf(__fmul_rn(__fdiv_rn(S.res[e0 + 32 * r + lane], s), 256.f)), -2048.f), 2048.f);
       __syncwarp();
-      const int h = lane >> 4;
       uint8_t* const st = mult[mi].st + e0;
-      auto search = [&](auto kk) {
-        constexpr int KK = decltype(kk)::value;
-        if (narrow) tb_search<KK, int>(B.bp[h], S.code, B.xs + 64 * h, st + 64 * h, lane); else tb_search<KK, long long>(B.bp[h], S.code, B.xs + 64 * h, st + 64 * h, lane);
-      };
-      if (P.kk == 3) search(std::integral_constant<int, 3>{});
-      else if (P.kk == 4) search(std::integral_constant<int, 4>{});
-      else if (P.kk == 5) search(std::integral_constant<int, 5>{});
-      else { for (int r = 0; r < 4; ++r) st[32 * r + lane] = 0; __syncwarp(); }
+      if (P.kk == 3) search(std::integral_constant<int, 3>{}, B, st);
+      else if (P.kk == 4) search(std::integral_constant<int, 4>{}, B, st);
+      else if (P.kk == 5) search(std::integral_constant<int, 5>{}, B, st);
+      else { for (int r = 0; r < R; ++r) st[32 * r + lane] = 0; __syncwarp(); }
       #pragma unroll
-      for (int r = 0; r < 4; ++r) {
+      for (int r = 0; r < R; ++r) {
         const float d = __fsub_rn(S.res[e0 + 32 * r + lane], value(st[32 * r + lane], s)), e = run_sum(__fmul_rn(d, d));
-        if (lane == 0) mult[mi].err[4 * (unit & 1) + r] = e;
+        if (lane == 0) mult[mi].err[e0 / 32 + r] = e;
       }
-    }
+    };
+    auto pairs = [&](auto key) {
+      #pragma unroll 1
+      for (int unit = c; unit < 2 * A.nm; unit += nwarps)
+        unit_of(unit >> 1, 128 * (unit & 1), std::integral_constant<int, 128>{}, [&](auto kk, TbRowSmem::Warp& B, uint8_t* st) {
+          const int h = lane >> 4;
+          tb_search<decltype(kk)::value, decltype(key)>(B.bp[h], S.code, B.xs + 64 * h, st + 64 * h, lane);
+        });
+    };
+    auto chains = [&](auto key) {
+      #pragma unroll 1
+      for (int unit = c; unit < 4 * A.nm; unit += nwarps)
+        unit_of(unit >> 2, 64 * (unit & 3), std::integral_constant<int, 64>{}, [&](auto kk, TbRowSmem::Warp& B, uint8_t* st) {
+          tb_search_chain<decltype(kk)::value, decltype(key)>(B.bp[0], S.code, B.xs, st, lane);
+        });
+    };
+    if constexpr (W == TB_ONE) { if (narrow) chains(int{}); else chains((long long)0); }
+    else if (narrow) pairs(int{});
+    else if constexpr (W == TB_WIDE) pairs((long long)0);
+    else chains((long long)0);
     __syncthreads();
     float best_e = 0.f; int best = 0;
     for (int mi = 0; mi < A.nm; ++mi) {                  // the smallest squared error, the first on ties
@@ -857,10 +948,11 @@ int launch_tb_encode(const uint8_t* blob, int nm, const float* x, const int* grp
   if (first_use_on_device(attr)) {
     KV4_CUDA(cudaFuncSetAttribute(tb_encode_kernel<TB_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TbRowSmem::bytes(TB_NM, TB_WIDE)));
     KV4_CUDA(cudaFuncSetAttribute(tb_encode_kernel<TB_NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TbRowSmem::bytes(TB_NM, TB_NARROW)));
+    KV4_CUDA(cudaFuncSetAttribute(tb_encode_kernel<TB_ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TbRowSmem::bytes(1, TB_ONE)));
   }
   const TbP P{blob, nm, x, grp, pos, rows, y, pay, pay_stride, side, whole};
-  const int most = rows <= TB_WIDE_ROWS ? TB_WIDE : TB_NARROW;
-  auto kern = most == TB_WIDE ? tb_encode_kernel<TB_WIDE> : tb_encode_kernel<TB_NARROW>;
+  const int most = nm == 1 ? TB_ONE : rows <= TB_WIDE_ROWS ? TB_WIDE : TB_NARROW;
+  auto kern = most == TB_ONE ? tb_encode_kernel<TB_ONE> : most == TB_WIDE ? tb_encode_kernel<TB_WIDE> : tb_encode_kernel<TB_NARROW>;
   kern<<<rows, 32 * TbRowSmem::warps(nm, most), TbRowSmem::bytes(nm, most), st>>>(P);
   return launch_status("tb_encode_kernel");
 }
