@@ -55,9 +55,10 @@ __global__ void __launch_bounds__(KV8_WARPS * 32, 1) kv8_decode_kernel(const Kv8
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   // Programmatic dependent launch: this grid may be scheduled while the row epilogue in front of it drains, and waits here before it
   // reads the position, the queries and the new rows; the merge behind it may be scheduled early in turn.
-  // Nothing is read ahead of that wait, but the block's first keys are asked into L2 while the epilogue runs, from wherever the position points now (a stale one
-  // asks for the wrong lines of the cache's own arrays, no more): one token over 32,768 rows 22.8 -> 21.6 us.  (Tried on the int4 decode kernel
-  // too: behind its append, 2 us, reading the position early costs more than it brings, 19.7 -> 20.8 us.)
+  // One thing is read ahead of that wait: the position, past L1, and for nothing but the address from which the block's first keys are asked into L2 while the
+  // epilogue runs.  It may be stale or be written at that moment; held within the cache it then asks for the wrong lines of the cache's own arrays, no more, and
+  // all that a result depends on, the position again first of all, is read behind the wait: one token over 32,768 rows 22.8 -> 21.6 us.  (Tried on the int4
+  // decode kernel too: behind its append, 2 us, reading the position early costs more than it brings, 19.7 -> 20.8 us.)
   if (threadIdx.x < 2 && r == 0) {
     const int keys = max(0, min(__ldcg(A.d_pos), A.max_ctx)), tl = keys / 16, n = (tl + (int)gridDim.x - 1) / (int)gridDim.x;   // past L1: read again behind the wait
     const int t0 = min(tl, split * n), nt = min(min(n, tl - t0), KV8_AHEAD);
@@ -384,26 +385,9 @@ __global__ void __launch_bounds__(128) kv8_combine_rows_kernel(const float* pm, 
       v[7] = t;
     }
   }
-  if (inverse_rotate) {                                    // stages h = 1 ... 128 in order: lower index a + b, upper lower - upper
-    #pragma unroll
-    for (int rb = 1; rb < 4; rb *= 2)                      // h = 1, 2
-      #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (!(i & rb)) { const float lo = v[i], up = v[i + rb]; v[i] = __fadd_rn(lo, up); v[i + rb] = __fsub_rn(lo, up); }
-    #pragma unroll
-    for (int m = 1; m < 32; m *= 2) {                      // h = 4 ... 64: the lanes
-      const float flip = (lane & m) ? -1.f : 1.f;          // the product is exact: one rounding, as of the sum
-      #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = fmaf(v[i], flip, __shfl_xor_sync(0xffffffffu, v[i], m));
-    }
-    const int w = lane >> 3, b = 4 * (lane & 7);
-    const uint32_t sg[2] = {c_signs.w[w] >> b, c_signs.w[w + 4] >> b};
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) {                          // h = 128, then 1/16 and the signs
-      const float lo = v[i], up = v[i + 4];
-      v[i] = __fmul_rn(__fadd_rn(lo, up), __uint_as_float(0x3d800000u | (((sg[0] >> i) & 1u) << 31)));
-      v[i + 4] = __fmul_rn(__fsub_rn(lo, up), __uint_as_float(0x3d800000u | (((sg[1] >> i) & 1u) << 31)));
-    }
+  if (inverse_rotate) {                                    // 1/16 and the signs in one factor
+    const LaneSigns sg = lane_signs(lane);
+    hadamard256_warp(v, lane, [&](int i) { return __uint_as_float(0x3d800000u | (((sg.w[i >> 2] >> (i & 3)) & 1u) << 31)); });
   }
   auto pack = [](float lo, float hi) {                     // two values rounded to the output type
     uint32_t d;

@@ -208,26 +208,11 @@ __global__ void __launch_bounds__(256) kvx_attn_post_kernel(yskn_kvx_attn_post_a
       }
     }
   }
-  // ---- signs and butterflies, stages h = 1 ... 128 in order: lower index a + b, upper lower - upper
-  const uint32_t sg[2] = {c_signs.w[lane >> 3] >> (4 * (lane & 7)), c_signs.w[4 + (lane >> 3)] >> (4 * (lane & 7))};
+  // ---- signs and butterflies
+  const LaneSigns sg = lane_signs(lane);
   #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ (((sg[i >> 2] >> (i & 3)) & 1u) << 31));
-  #pragma unroll
-  for (int rb = 1; rb < 4; rb *= 2)
-    #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (!(i & rb)) { const float lo = v[i], hi = v[i + rb]; v[i] = __fadd_rn(lo, hi); v[i + rb] = __fsub_rn(lo, hi); }
-  #pragma unroll
-  for (int m = 1; m < 32; m *= 2) {
-    const float flip = (lane & m) ? -1.f : 1.f;                  // the product is exact: one rounding, as of the sum
-    #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = fmaf(v[i], flip, __shfl_xor_sync(0xffffffffu, v[i], m));
-  }
-  #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float lo = v[i], hi = v[4 + i];
-    v[i] = __fmul_rn(__fadd_rn(lo, hi), 0.0625f); v[4 + i] = __fmul_rn(__fsub_rn(lo, hi), 0.0625f);
-  }
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ (((sg.w[i >> 2] >> (i & 3)) & 1u) << 31));
+  hadamard256_warp(v, lane, [](int) { return 0.0625f; });
   if (kind == 0) {
     #pragma unroll
     for (int h = 0; h < 2; ++h) {

@@ -1,4 +1,4 @@
-// The sign-Hadamard-256 rotation of Family B (kvx_rotate, src/kvx_codec.cuh:35-49) on rows held in registers, eight lanes per row.
+// The sign-Hadamard-256 rotation of Family B (kvx_rotate, src/kvx_codec.cuh:35-49) on rows held in registers: eight lanes per row, or a warp.
 #pragma once
 #include "kv4_common.cuh"
 
@@ -56,6 +56,31 @@ __device__ __forceinline__ void hadamard256(float (&v)[32], int ll) {
   }
   #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __fmul_rn(v[i], 0.0625f);
+}
+
+// The same with a warp per row: lane l holds v[e] = element 4l + e and v[4 + e] = element 128 + 4l + e (e 0..3).  Sign bits of those eight: bit e of w[0] and w[1].
+struct LaneSigns { uint32_t w[2]; };
+__device__ __forceinline__ LaneSigns lane_signs(int lane) {
+  return {{c_signs.w[lane >> 3] >> (4 * (lane & 7)), c_signs.w[4 + (lane >> 3)] >> (4 * (lane & 7))}};
+}
+// Stages h = 1, 2 in the registers, 4 ... 64 over the lanes, 128 in the registers, then each element times its factor(element's index in v).
+template <class F> __device__ __forceinline__ void hadamard256_warp(float (&v)[8], int lane, F factor) {
+  #pragma unroll
+  for (int rb = 1; rb < 4; rb *= 2)
+    #pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (!(i & rb)) { const float lo = v[i], up = v[i + rb]; v[i] = __fadd_rn(lo, up); v[i + rb] = __fsub_rn(lo, up); }
+  #pragma unroll
+  for (int m = 1; m < 32; m *= 2) {
+    const float flip = (lane & m) ? -1.f : 1.f;            // the product is exact: one rounding, as of the sum
+    #pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = fmaf(v[i], flip, __shfl_xor_sync(0xffffffffu, v[i], m));
+  }
+  #pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float lo = v[i], up = v[i + 4];
+    v[i] = __fmul_rn(__fadd_rn(lo, up), factor(i)); v[i + 4] = __fmul_rn(__fsub_rn(lo, up), factor(i + 4));
+  }
 }
 
 }  // namespace
