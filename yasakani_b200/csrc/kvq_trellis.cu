@@ -505,7 +505,6 @@ constexpr uint32_t TBA_SMEM = sizeof(TbAttnSm) + TBA_TAB + (TBA_MERGE > 2 * TBA_
 struct TbRule { int packed_ok, mode, kb, guard, m, has_mu; float gain; };     // per-group constants of the unpack rule
 
 __device__ __forceinline__ uint32_t tba_lds(uint32_t a) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
-__device__ __forceinline__ void tba_sts(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ uint32_t tba_pack(float lo, float hi) { uint32_t d; asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo)); return d; }
 __device__ __forceinline__ void tba_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
