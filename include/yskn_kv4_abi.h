@@ -403,7 +403,7 @@ YSKN_KV4_API int yskn_kv8_attention_tc(const yskn_kv8_attn_args* a, int act_dtyp
 /* yskn_kv8_attention_tc over a caller-owned workspace of 1,024 * kvh * max_ctx bytes (16-byte aligned; its contents need not survive the
  * call's work on the stream): the visible keys become fp16 rows once, in a launch of their own, instead of once per 256 query
  * rows.  Same operands bit for bit; pl is summed in another order, so a row's last bit depends on the form.  yskn_kv8_workspace_bytes: that size where
- * the pass is the faster for it whatever the position and the capacity, to within a microsecond (at least 384 rows, and at most 256 MiB), 0 where
+ * the pass is the faster for it whatever the position and the capacity (at least 384 rows, and at most 256 MiB), 0 where
  * yskn_kv8_attention is to be called as it is. */
 YSKN_KV4_API size_t yskn_kv8_workspace_bytes(const yskn_kv8_attn_args* a);
 YSKN_KV4_API int yskn_kv8_attention_ws(const yskn_kv8_attn_args* a, int act_dtype, void* d_workspace, size_t workspace_bytes, void* cuda_stream);

@@ -50,8 +50,8 @@ static int attention_dispatch(const yskn_attn_g_args* a, int g, int hd, int rd, 
   const bool mma_ok = decode_mma_supports(g, hd, rd, a->M);
   const int algo = current_algo();
   // Wide passes (more rows than the warp-level decode kernel takes) go to the tcgen05 kernel.  Up to TC_FUSED_MAX_ROWS rows it
-  // converts the packed cache inside the kernel (every CTA pair converts the tiles it reads; measured at 32,768 tokens: 61 / 65 / 111 us
-  // for 16 / 32 / 64 rows against 105 / 109 / 136 us with a full dequantisation in front); longer
+  // converts the packed cache inside the kernel (every CTA pair converts the tiles it reads; measured at 32,768 tokens, attention alone: 43 / 43 / 71 us
+  // for 16 / 32 / 64 rows against 94 / 93 / 110 us with a full dequantisation in front); longer
   // passes dequantise once into a workspace, if the caller has lent one (valid_tokens = 0: the whole workspace is brought
   // up to date on every call), and take the converting form otherwise.
   if (a->M > 8 && algo != ALGO_SCALAR && sh.start == 0 && sh.len == a->max_ctx && !(((uintptr_t)a->q16 | (uintptr_t)a->pacc) & 15)) {
@@ -377,10 +377,12 @@ int yskn_kv8_attention_tc(const yskn_kv8_attn_args* a, int act_dtype, void* cuda
 }
 // Converting inside the kernel costs every pair of 128-row tiles its own pass over the keys (2.3 us per 128 keys, against 1.3 from
 // fp16 rows); writing the rows first costs a launch and one pass over them.  The host does not know how many keys are visible, so
-// the line lies where the written rows win for any number of them, or lose less than that launch.  Attention alone, converting / written
-// rows, in us, behind 0, 3,000 and 8,000 tokens: 127 rows 11.7 / 12.1, 25 / 23 and 45 / 41; 300 rows 14.7 / 15.0, 40 / 32 and 82 / 62; 384 rows 17.0 / 15.8 (a cache
-// much larger than its contents adds 1.3 to the written rows), 69 / 46 and 160 / 98; 500 rows 19.0 / 17.9, 72 / 48 and 162 / 100; 1,000 rows 39.6 / 33.3, 134 / 91 and
-// 328 / 197.
+// the written rows are taken only where they win for any number of them in a cache of any size.  They do from 384 rows on, by 5 % at the least; the line is
+// on the safe side, since it was drawn when they lost below it and passes below it have never taken memory.  Attention alone, replays, converting /
+// written rows, in us, behind 0 tokens of a full cache, 0 of one of 65,536, 3,000 and 8,000:
+//   127 rows   10.9 / 10.8   10.9 / 11.9   23.7 / 20.7   41.9 / 38.9         384 rows   16.4 / 14.2   16.2 / 15.3   67.7 / 44.0   151 / 96
+//   256 rows   12.2 / 11.9   12.2 / 12.9   38.5 / 29.5   78.5 / 59.1         500 rows   18.1 / 15.8   18.1 / 16.6   69.2 / 45.8   151 / 98
+//   340 rows   15.6 / 15.3   15.6 / 15.4   42.3 / 31.7   78.5 / 63.4       1,000 rows   38.4 / 31.4   38.7 / 31.4  131.2 / 89.3   287 / 189
 // The workspace grows with the capacity, not with the visible keys.  It is taken up to 256 MiB (0.15 % of the GPU's memory); beyond it a
 // pass that needed no memory before would hold as much as several layers' caches, so larger caches keep the converting form.
 size_t yskn_kv8_workspace_bytes(const yskn_kv8_attn_args* a) {

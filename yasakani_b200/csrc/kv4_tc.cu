@@ -1409,8 +1409,10 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   };
   // ---- roles.  In the converting forms each warpgroup first sets its register budget (softmax twice, V, K: 512 per scheduler lane) and the role code sits
   //      under that branch, so that each role is compiled for its own budget.  More registers are more of a role's arithmetic under way at once; steps of 64 / 16 int4 rows
-  //      and of 16 INT8 rows over 32,768 tokens, and of 350 behind 6,000, in us: 120 / 112 / 160 88.7 / 52.4 / 54.9 / 85.4; 104 / 136 / 168 87.9 / 52.4 / 53.5 / 84.4;
-  //      96 / 160 / 160 89.3 / 52.8 / 52.7 / 84.3; 96 / 176 / 144 96.5 / 56.6 / 52.2 / 83.0.
+  //      and of 16 INT8 rows over 32,768 tokens, and of 350 behind 6,000, repeated over one cache, in us: 120 / 112 / 160 88.7 / 52.4 / 54.9 / 85.4; 104 / 136 / 168 87.9 /
+  //      52.4 / 53.5 / 84.4; 96 / 160 / 160 89.3 / 52.8 / 52.7 / 84.3; 96 / 176 / 144 96.5 / 56.6 / 52.2 / 83.0.  Any change of the code's layout moves these times by a
+  //      per cent or two, so what the table shows is that int4 rows lose 10 % when their K converters have 144 registers and INT8 rows gain 5 and 3 % when V's have more;
+  //      the first three splits are the same for int4 rows.
   if constexpr (FUSED) {
     constexpr int RS = I8 ? 96 : 104, RV = I8 ? 176 : 136, RK = I8 ? 144 : 168;
     static_assert(2 * RS + RV + RK == 512, "what the launch has: 16 warps of 128 registers");
