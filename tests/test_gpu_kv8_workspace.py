@@ -139,3 +139,20 @@ def test_scratch_is_no_tensor_and_no_part_of_another_streams_capture():
     graph.replay()
     torch.cuda.synchronize()
     assert (x == 2).all()
+
+
+@pytest.mark.parametrize("ctx,S", [(246, 1), (246, 3), (2030, 5)])
+@pytest.mark.parametrize("written", [True, False], ids=["written", "converting"])
+def test_rows_are_the_same_bits_in_passes_of_other_widths(written, ctx, S):
+    """Rows 0 .. 49 of passes that end behind other key tiles and share their rows out over other pairs of CTAs."""
+    from yasakani_b200 import kv4
+    q, k8, v8, ks, vs, pos = _case(ctx, 130, torch.bfloat16, seed=5)
+    ws = torch.full((1024 * KVH * k8.shape[1],), 0xFF, dtype=torch.uint8, device="cuda") if written else None
+    first = None
+    for M in (50, 64, 85, 130):
+        out = kv4.attn_scratch(M, S, NH, 256)
+        assert _entry((q[:M].contiguous(), k8, v8, ks, vs, pos), M, S, out, ws) == 0
+        torch.cuda.synchronize()
+        bits = [t[:50].view(torch.int32) for t in out]
+        first = first or bits
+        assert kv4.device_status() == 0 and all(torch.equal(a, b) for a, b in zip(first, bits)), M
