@@ -58,19 +58,16 @@ def test_finished_rows_are_the_rounded_quotients(workspace, bf16):
     assert bool(same.all()), int((~same).sum())
 
 
-# Rows 0 .. 49 of a pass from position 246: a wider pass ends behind another key tile, and its pairs of CTAs hold other tokens where they share a pass out evenly.
-@pytest.mark.parametrize("workspace,bf16", [(True, False), (True, True), (False, False)], ids=["fp16", "bf16", "converting"])
-@pytest.mark.parametrize("ctx,S", [(246, 1), (246, 3), (2030, 5)])
-def test_rows_are_the_same_bits_in_passes_of_other_widths(ctx, S, workspace, bf16):
+def _same_rows_in_passes_of(widths, ctx, S, workspace, dt, hq, hkv, hd, rd):
     import torch
     from yasakani_b200 import kv4
-    hq, hkv, hd, rd, widths, max_ctx = 24, 4, 256, 64, (50, 64, 85, 130), (ctx + 130 + 63) // 64 * 64
-    dt = torch.bfloat16 if bf16 else torch.float16
+    top = widths[-1]
+    max_ctx = (ctx + top + 63) // 64 * 64
     g = torch.Generator(device="cuda").manual_seed(ctx + S)
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16).to(dt)
-    k, v, q = rnd(ctx + 130, hkv, hd), rnd(ctx + 130, hkv, hd), rnd(130, hq, hd)
+    k, v, q = rnd(ctx + top, hkv, hd), rnd(ctx + top, hkv, hd), rnd(top, hq, hd)
     layer = kv4.KvLayer(hkv, hd, max_ctx)
-    kv4.launch_kv_append(layer, k, v, torch.zeros(1, dtype=torch.int32, device="cuda"), ctx + 130)
+    kv4.launch_kv_append(layer, k, v, torch.zeros(1, dtype=torch.int32, device="cuda"), ctx + top)
     rope = torch.empty((max_ctx, rd // 2, 2), dtype=torch.float32, device="cuda")
     kv4.launch_rope_table_g(rope, max_ctx, 1e4, rd)
     pos, first = torch.tensor([ctx], dtype=torch.int32, device="cuda"), None
@@ -84,6 +81,22 @@ def test_rows_are_the_same_bits_in_passes_of_other_widths(ctx, S, workspace, bf1
         first = first or bits
         for name, a, b in zip(("m", "l", "o"), first, bits):
             assert torch.equal(a, b), f"{name} of {int((a != b).flatten(1).any(1).sum())} of {widths[0]} rows in a pass of {M}"
+
+
+# Rows 0 .. 49 of a pass from position 246: a wider pass ends behind another key tile, and its pairs of CTAs hold other tokens where they share a pass out evenly.
+@pytest.mark.parametrize("workspace,bf16", [(True, False), (True, True), (False, False)], ids=["fp16", "bf16", "converting"])
+@pytest.mark.parametrize("ctx,S", [(246, 1), (246, 3), (2030, 5)])
+def test_rows_are_the_same_bits_in_passes_of_other_widths(ctx, S, workspace, bf16):
+    import torch
+    _same_rows_in_passes_of((50, 64, 85, 130), ctx, S, workspace, torch.bfloat16 if bf16 else torch.float16, 24, 4, 256, 64)
+
+
+@pytest.mark.parametrize("hq,hkv,hd,rd", [(16, 2, 128, 128), (8, 4, 128, 64), (16, 4, 128, 32), (8, 4, 256, 64)])      # eight, two, four heads a kv-head; 256 channels
+@pytest.mark.parametrize("ctx", [0, 100])
+def test_rows_are_the_same_bits_on_both_sides_of_the_even_shares(ctx, hq, hkv, hd, rd):
+    """Converting passes of up to 128 rows share their tokens out evenly, longer ones of 128 channels fill their pairs where a pair is part of a key tile."""
+    import torch
+    _same_rows_in_passes_of((40, 128, 129, 300), ctx, 2, False, torch.float16, hq, hkv, hd, rd)
 
 
 @pytest.mark.parametrize("pos", [-200, -16, -9, -3, 190])

@@ -1565,7 +1565,12 @@ int launch_tc_fused_hd(const yskn_attn_g_args& a, int g, int rd, int bf16, uint1
   auto kern = kv4_tc_attn_kernel<HD, 1>;
   static std::atomic<unsigned long long> attr{0};
   if (first_use_on_device(attr)) KV4_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  int tpc; const int qtiles = tc_tiles(a.M, g, true, &tpc);
+  // The tiles that a pair's own tokens lie in are converted twice.  Where the tokens of a pair are a whole part of a key tile (2, 4 or 8 heads a kv-head), even shares of
+  // more than a tile of tokens lie across one tile more.  Rows of eight heads of 128 channels, one split, us from position 0 and behind 2,500 tokens: 150 rows 20.6 and
+  // 61.2 with whole shares before the requests a tile ahead, 21.6 and 59.1 with them and even shares, 19.3 and 60.7 with whole ones; 300 rows 23.1 and 63.9, 23.9 and
+  // 63.3, 22.1 and 63.9.  With 256 channels even shares have not cost anything (150 rows 27.8 and 75.5, 25.9 and 60.2, whole ones 22.2 and 63.5).
+  const bool whole = HD == 128 && (g == 2 || g == 4 || g == 8) && a.M > TC_BN;
+  int tpc; const int qtiles = tc_tiles(a.M, g, !whole, &tpc);
   TcP P{a.d_pos, a.M, a.splits, g, tpc, a.nh, a.max_ctx, 0, a.qscale, a.pm, a.pl, a.pacc, o16, bv, a.kv, a.rope, rd, static_cast<const uint16_t*>(a.q16), bf16,
         nullptr, nullptr, nullptr, nullptr};
   if (int rc = tc_launch_pdl(kern, dim3(qtiles, a.splits, a.kvh), tc_threads(true), L::TOTAL, st, mq, mq, mq, mq, P)) return rc;
