@@ -393,7 +393,7 @@ __device__ __forceinline__ void tc_stage_q(uint32_t sq, int q_block, const uint1
 }
 // Finished rows of a pass of one split: y = round_f16(o / l) (+ V bias) as the merge kernel, every other 32 columns of O from hf on.  A function of its own,
 // so that its code does not move the loops of the kernel about (a fused pass of 64 rows, which never comes here, took 92 to 99 us with it in line).  It is
-// called with what setmaxnreg has left the softmax warps, 104 registers in form 1 and 208 in forms 0 and 3, and needs 49.
+// called with what setmaxnreg has left the softmax warps, 104 or 120 registers in form 1 and 208 in forms 0 and 3, and needs 49.
 template <int HD, bool PAIRS>
 __device__ __noinline__ void tc_finish_row(uint32_t tcol, int hf, bool any, bool valid, float l, bool bf16, const uint16_t* bv, uint16_t* out) {
   const float rl = __frcp_rn(l);
@@ -939,13 +939,22 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         }
       }
       int kit = 0;
-      // L2 prefetch of a half tile two tiles ahead (64 packed rows, the scale and zero rows of its two groups: three contiguous pieces), so that the register
-      // loads a tile ahead find their lines in L2
+      // L2 prefetch of a half tile two tiles ahead (64 packed rows, the scale and zero rows of its two groups), so that the register loads a tile ahead find their lines
+      // in L2.  256 channels: three contiguous pieces by one thread, which is less code.  128 channels: a line a thread; pieces cost passes that fill the GPU 5 to 10 %
+      // there (2,000 rows of six heads behind 8,000 tokens, 64 / 16 channels rotated, 370 / 370 us by lines and 410 / 413 by pieces).
       auto k_prefetch = [&](int tk) {
-        if (tk >= P.max_ctx || ct != 0) return;
-        tc_prefetch_bulk(P.kv.kq + (row0 + tk) * (HD / 2), (TC_BN / 2) * (HD / 2));
-        tc_prefetch_bulk(P.kv.kscale + (grp0 + tk / 32) * HD, 2 * HD * 2);
-        tc_prefetch_bulk(P.kv.kzero + (grp0 + tk / 32) * HD, 2 * HD * 2);
+        if (tk >= P.max_ctx) return;
+        if constexpr (HD == 128) {
+          if (ct < TC_BN / 2) tc_prefetch_l2(P.kv.kq + (row0 + tk + ct) * (HD / 2));
+          else if (ct < TC_BN / 2 + 4 * (HD / 64)) {
+            const int x = ct - TC_BN / 2, arr = x & 1, grp = (x >> 1) & 1, line = x >> 2;
+            tc_prefetch_l2((arr ? P.kv.kzero : P.kv.kscale) + (grp0 + tk / 32 + grp) * HD + 64 * line);
+          }
+        } else if (ct == 0) {
+          tc_prefetch_bulk(P.kv.kq + (row0 + tk) * (HD / 2), (TC_BN / 2) * (HD / 2));
+          tc_prefetch_bulk(P.kv.kscale + (grp0 + tk / 32) * HD, 2 * HD * 2);
+          tc_prefetch_bulk(P.kv.kzero + (grp0 + tk / 32) * HD, 2 * HD * 2);
+        }
       };
       if (n > 1) k_prefetch(j0 * TC_BN + TC_BN + (TC_BN / 2) * (int)rank);
       for (int i = 0; i < n && ok; ++i) {
@@ -1072,11 +1081,16 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         I.w = tc_ldg128(at.q + k * (HD / 2));
         I.s = tc_ldg16(at.s + k); I.z = tc_ldg16(at.z + k);
       };
-      auto v_prefetch = [&](int j) {                                 // L2 prefetch of 64 of a tile's rows (the other CTA takes the other 64) and their scales
-        const int t = j * TC_BN + (TC_BN / 2) * (int)rank;
-        if (t >= P.max_ctx || vt != 0) return;
-        tc_prefetch_bulk(P.kv.vq + (row0 + t) * (HD / 2), (TC_BN / 2) * (HD / 2));
-        tc_prefetch_l2(P.kv.vscale + row0 + t); tc_prefetch_l2(P.kv.vzero + row0 + t);     // these two arrays may lie at any even address
+      auto v_prefetch = [&](int j) {                                 // L2 prefetch of a tile's half rows, or of 64 of its rows (the other CTA takes the other 64)
+        if constexpr (HD == 128) {
+          for (int x = vt; x < TC_BN; x += NVT) if (j * TC_BN + x < end) tc_prefetch_l2(P.kv.vq + (row0 + j * TC_BN + x) * (HD / 2) + (HD / 4) * (int)rank);
+          if (vt < 4 && j * TC_BN + 64 * (vt & 1) < end) tc_prefetch_l2((vt & 2 ? P.kv.vzero : P.kv.vscale) + row0 + j * TC_BN + 64 * (vt & 1));
+        } else {
+          const int t = j * TC_BN + (TC_BN / 2) * (int)rank;
+          if (t >= P.max_ctx || vt != 0) return;
+          tc_prefetch_bulk(P.kv.vq + (row0 + t) * (HD / 2), (TC_BN / 2) * (HD / 2));
+          tc_prefetch_l2(P.kv.vscale + row0 + t); tc_prefetch_l2(P.kv.vzero + row0 + t);     // these two arrays may lie at any even address
+        }
       };
       VIn vin[NVI];
       {
@@ -1298,11 +1312,16 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         ++srd[1];
       }
       tc_fence_after();
-      // Two walks over the 64 keys in pieces of 32, first the maximum, then the exponentials, in one rolled loop: the loops of all roles have to stay inside the
-      // instruction cache together, and the scores are read from tensor memory a second time for it.
+      // Two walks over the 64 keys in pieces of 32, first the maximum, then the exponentials.  256 channels: one rolled loop, since the loops of all roles have to stay
+      // inside the instruction cache together, and the scores are read from tensor memory a second time for it.  128 channels: converter loops of half the length leave
+      // room for the walks in line, and half the channels leave the softmax as the pace, so scores stay in registers (120 a thread): 64 rows of six heads, 64 / 16 channels rotated, over
+      // 8,000 tokens 126 / 121 us rolled, 98 / 100 in line (121 / 110 before the requests a tile ahead); rotated as a whole 147 and 146.
       // Online softmax in the log2 domain on p = 2^(x*cs - m); lazy rescale (the running max may lag by up to 2^8).
       float tmax = -INFINITY, nm = 0.f, ls0 = 0.f, ls1 = 0.f;
-      #pragma unroll 1
+      constexpr bool KEEP = HD == 128;
+      float xs[KEEP ? 2 : 1][32];                                    // raw scores
+      constexpr int STEPS = KEEP ? 4 : 1;
+      #pragma unroll STEPS
       for (int step = 0; step < 4 && ok; ++step) {
         const int h2 = step & 1;
         if (step == 2) {
@@ -1327,9 +1346,9 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
             }
           }
         }
-        float x[32];                                                 // raw scores
-        tmem_ld32(scol + 32 * h2, x);
-        if (edge) {
+        float (&x)[32] = xs[KEEP ? h2 : 0];
+        if (!KEEP || step < 2) tmem_ld32(scol + 32 * h2, x);
+        if (edge && (!KEEP || step < 2)) {
           // each 32-key quarter is one group: before the row's own -> int4 keys; own group -> shadow keys up to the row; later -> nothing
           float a[32];
           tmem_ld32(trow + L::TM_S1 + 64 * hf + 32 * h2, a);
@@ -1412,13 +1431,13 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   //      and of 16 INT8 rows over 32,768 tokens, and of 350 behind 6,000, repeated over one cache, in us: 120 / 112 / 160 88.7 / 52.4 / 54.9 / 85.4; 104 / 136 / 168 87.9 /
   //      52.4 / 53.5 / 84.4; 96 / 160 / 160 89.3 / 52.8 / 52.7 / 84.3; 96 / 176 / 144 96.5 / 56.6 / 52.2 / 83.0.  Any change of the code's layout moves these times by a
   //      per cent or two, so what the table shows is that int4 rows lose 10 % when their K converters have 144 registers and INT8 rows gain 5 and 3 % when V's have more;
-  //      the first three splits are the same for int4 rows.
+  //      the first three splits are the same for int4 rows.  128 channels keep 120 / 112 / 160: softmax threads hold 64 scores there.
   if constexpr (FUSED) {
-    constexpr int RS = I8 ? 96 : 104, RV = I8 ? 176 : 136, RK = I8 ? 144 : 168;
+    constexpr int RS = I8 ? 96 : HD == 128 ? 120 : 104, RV = I8 ? 176 : HD == 128 ? 112 : 136, RK = I8 ? 144 : HD == 128 ? 160 : 168;
     static_assert(2 * RS + RV + RK == 512, "what the launch has: 16 warps of 128 registers");
     if (warp < TC_SW) { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RS)); role_softmax(); }
     else if (warp < TC_SW + 4) {
-      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RV));
+      if constexpr (RV < 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RV)); else asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RV));
       if (warp == TC_SW) role_mma(); else role_conv(false);
     } else { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RK)); role_conv(true); }
   } else {
