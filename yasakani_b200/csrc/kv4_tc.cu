@@ -1252,7 +1252,7 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         xseq[hf * 128 + rho] = (uint16_t)(i + 1);
         if (mown != m) { l *= tc_ex2(mown - m); mown = m; }
         // ---- O may be rescaled once P.V of tile i-1 is done (P.V of this tile waits for the signals below)
-        if (__any_sync(0xffffffffu, bump) && i > 0) {                // rows that did not bump multiply by exactly 1; every tile asks: the warp is together again
+        if (__any_sync(0xffffffffu, bump && i > 0)) {                // rows that did not bump multiply by exactly 1; every tile asks: the warp is together again
           if (!bar_wait(b_pvdone + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
           tc_fence_after();
           #pragma unroll 1
@@ -1330,10 +1330,8 @@ kv4_tc_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           const float mn = bump ? tmax : m, alpha = bump ? tc_ex2(m - mn) : 1.f;
           m = mn; l *= alpha; nm = -m;
           // ---- O may be rescaled once P.V of tile i-1 is done (P.V of this tile waits for the signal below).  Each lane has polled for itself in the
-          //      exchange and the tcgen05.ld behind want the warp together, so every tile asks, the first too; over INT8 rows it joins first (with the
-          //      other way about, 64 int4 rows over 32,768 tokens took 0.9 % more and 383 INT8 rows behind 8,000 2 %).
-          if (I8) __syncwarp();
-          if (I8 ? i > 0 && __any_sync(0xffffffffu, bump) : __any_sync(0xffffffffu, bump) && i > 0) {   // rows that did not bump multiply by exactly 1
+          //      exchange and the tcgen05.ld behind want the warp together, so every tile asks, the first too.
+          if (__any_sync(0xffffffffu, bump && i > 0)) {              // rows that did not bump multiply by exactly 1
             if (!bar_wait(b_pvdone + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1)) { atomicExch(&g_tc_status, 4); *s_abort = 1; ok = false; break; }
             tc_fence_after();
             #pragma unroll 1
