@@ -59,7 +59,7 @@ __device__ __forceinline__ unsigned tb_table(const uint8_t* b, const TbGroup& P)
 // take 64-bit keys (no bringing back).
 // 4,096 rows, 5 multipliers, on a B200: 1,335 us (one warp per (row, multiplier, chain), costs in shared memory, every lane walking its group's predecessors; a
 // second kernel for choice and packing) -> 448 (minima kept instead of back pointers, candidates recomputed on the way back) -> 321 (eight states a
-// lane, a warp per chain that walks the multipliers) -> 243.  Issue slots 63 % busy, integer ALU 45 %, multiply pipe 49 %, shuffles and shared memory 45 %; 25 warps
+// lane, a warp per chain that walks the multipliers) -> 238.  Issue slots 64 % busy, integer ALU 49 %, shuffles and shared memory 49 %; 25 warps
 // an SM at 72 registers instead of 20 at 96 are slower (262), 15 at 128 too (273).
 // Where a warp per chain stays: with one multiplier, whose two pairs of chains would leave two of the block's four warps idle (28 warps an SM; 4,096 rows 83 us
 // by pairs, 75 by chains; 64-bit keys 318 and 178), and with 64-bit keys and many rows, where sixteen states a lane do not fit the registers and the codes are read again
